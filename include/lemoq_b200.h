@@ -113,6 +113,20 @@ LEMOQ_API int lemoq_w8_rows_tokens(const void* planes, int T, const int8_t* code
                          int group_size, const int32_t* seg_offsets, int E, int gate_up, void* y, void* stream);
 
 /* ---------------------------------------------------------------------------
+ * The same sums on the 5th-generation tensor cores, straight from the fp16
+ * activations: y[t, n] = fp16(sum_g scale[e, n, g] * sum_{k in g} codes[e, n, k] * x[t, k])
+ * (+ resid[t, n], an fp16 add, when resid is not NULL), from a handful of tokens to
+ * whole prompts.  ref: as above (src/lemoq/quant/linear.py:365,
+ * src/lemoq/kernels/moe_static.py:329).  Arguments as above; K % 128 == 0 without an upper limit, N any
+ * positive number (even for gate_up).  exact == 0 allows the form for prompts, which
+ * rounds scale * code to fp16 before the product (the fp16 weights a dequantising
+ * matmul would have used).  err_flag (may be NULL): LEMOQ_FLAG_WAIT_TIMEOUT.
+ */
+LEMOQ_API int lemoq_w8_gemm(const void* x, int T, const int8_t* codes, const void* scale, int N, int K, int group_size,
+                         const int32_t* seg_offsets, int E, int gate_up, int exact, const void* resid, void* y, int* err_flag,
+                         void* stream);
+
+/* ---------------------------------------------------------------------------
  * Row bookkeeping of the expert-parallel exchange (batched decode over several
  * GPUs, benchmark configuration 5).  These have no counterpart in the reference
  * (it has no multi-GPU code).  The contract: expert e lives on rank e / (experts / world),
@@ -372,6 +386,22 @@ LEMOQ_API const char* lemoq_step_engine(lemoq_step* step);
  * kernel: at its start, where it begins each phase of each layer (the phases of different blocks overlap, so
  * these are one block's view), and at its end; NULL when the step runs as chained kernels. */
 LEMOQ_API const unsigned long long* lemoq_step_phase_stamps(lemoq_step* step);
+
+/* ---------------------------------------------------------------------------
+ * A prompt of T tokens through the whole model: the K and V rows go into slots
+ * positions[t] of the fp16 caches (layers[i].keys / .values), row t attends to slots
+ * [0, positions[t]], logits (T, vocab) fp16 of every row.  Of desc the model fields are
+ * read (sizes, eps, norm_topk_prob, embed, final_norm, lm_head_*, rope_*), not the step's
+ * scalars.  ref: the eager prefill of benchmarks/cudagraph.py:520, i.e. per layer
+ * src/lemoq/quant/linear.py:365 and src/lemoq/kernels/moe_static.py:329.
+ * head_dim 128, hidden and ffn multiples of 128, hidden and heads * 128 <= 4096, experts a
+ * multiple of 8 and <= 128, top_k <= 32, group_size a multiple of 128; other shapes are
+ * refused (LEMOQ_ERR_UNSUPPORTED; lemoq_prompt_workspace_bytes returns 0).  tokens, positions:
+ * (T) int64 on the device.  err_flag (may be NULL): LEMOQ_FLAG_*.
+ */
+LEMOQ_API size_t lemoq_prompt_workspace_bytes(const lemoq_step_desc* desc, int T);
+LEMOQ_API int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens,
+                     const int64_t* positions, int T, void* logits, void* workspace, size_t workspace_bytes, int* err_flag, void* stream);
 
 #define LEMOQ_FLAG_BAD_POSITION 1
 #define LEMOQ_FLAG_BAD_LENGTH 2

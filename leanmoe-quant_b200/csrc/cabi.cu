@@ -1,4 +1,5 @@
 // extern "C" entry points: argument validation + launch.  No allocation, no sync.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -14,6 +15,18 @@ int set_error(int code, const char* fmt, ...) {
     vsnprintf(g_err, sizeof(g_err), fmt, ap);
     va_end(ap);
     return code;
+}
+
+int sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 static LaunchCfg cfg_of(void* stream) {

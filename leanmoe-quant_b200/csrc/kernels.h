@@ -101,6 +101,22 @@ bool stream_moe_eligible(const MoeParams& p);
 int launch_stream_gate_up(const MoeParams& p, const LaunchCfg& lc);
 int launch_stream_down(const MoeParams& p, const LaunchCfg& lc);
 
+// ---- W8 rows x many tokens on the tensor cores (w8_gemm.cu) ----------------------------
+struct W8GemmParams {
+    const __half* x = nullptr;       // (T, K), sorted by expert when seg is given
+    const int8_t* codes = nullptr;   // (E, N, K)
+    const __half* scale = nullptr;   // (E, N, K / group_size)
+    const int32_t* seg = nullptr;    // (E + 1) token offsets on the device, or null: one segment [0, T)
+    const __half* resid = nullptr;   // optional (T, N): y = fp16(acc) + resid
+    __half* y = nullptr;             // (T, N); gate/up: (T, N / 2) = silu(row n) * row N / 2 + n
+    int T = 0, N = 0, K = 0, group_size = 128, E = 1;
+    bool gate_up = false;
+    bool exact = true;               // never round code x scale to fp16 (large token counts only: small ones are always exact)
+    int* err_flag = nullptr;
+};
+int launch_w8_gemm(const W8GemmParams& g, const LaunchCfg& lc);
+int sm_count();  // of the current device, looked up once per device
+
 // ---- attention --------------------------------------------------------------------
 struct AttnParams {
     // q source: either a finished (H, D) fp16 q (fused == 0), or the raw packed qkv

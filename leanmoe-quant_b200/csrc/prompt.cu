@@ -1,0 +1,132 @@
+// A whole prompt through the model: T tokens, all layers, logits of every row, the K/V rows left in the fp16 caches.
+//
+// Eleven kernels per layer, launched from here with programmatic dependent launch: the prompt of a short question is
+// bound by the 6.9 GB of weights all experts together have (1.1 ms), so a launch gap or a host call per expert is what it
+// must not pay; a long prompt is bound by the tensor cores (w8_gemm.cu, prompt_attn.cu).
+#include <algorithm>
+
+#include "prompt.h"
+
+namespace lemoq {
+namespace {
+
+size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+struct PromptBuffers {
+    __half *x, *x1, *h, *qkv, *q, *ctx, *pairs, *act;
+    float* top_w;
+    int32_t *top_i, *place, *pair_of, *seg;
+};
+
+size_t carve_prompt(const lemoq_step_desc& d, int T, char* base, PromptBuffers* b) {
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char* at = base + off;
+        off += up256(bytes);
+        return at;
+    };
+    const size_t t = T, A = static_cast<size_t>(d.heads) * d.head_dim, P = t * d.top_k;
+    PromptBuffers o;
+    o.x = reinterpret_cast<__half*>(take(2 * t * d.hidden));
+    o.x1 = reinterpret_cast<__half*>(take(2 * t * d.hidden));
+    o.h = reinterpret_cast<__half*>(take(2 * t * d.hidden));
+    o.qkv = reinterpret_cast<__half*>(take(2 * t * 3 * A));
+    o.q = reinterpret_cast<__half*>(take(2 * t * A));
+    o.ctx = reinterpret_cast<__half*>(take(2 * t * A));
+    o.pairs = reinterpret_cast<__half*>(take(2 * P * d.hidden));  // the experts' inputs, then their outputs
+    o.act = reinterpret_cast<__half*>(take(2 * P * d.ffn));
+    o.top_w = reinterpret_cast<float*>(take(4 * P));
+    o.top_i = reinterpret_cast<int32_t*>(take(4 * P));
+    o.place = reinterpret_cast<int32_t*>(take(4 * P));
+    o.pair_of = reinterpret_cast<int32_t*>(take(4 * P));
+    o.seg = reinterpret_cast<int32_t*>(take(4 * (static_cast<size_t>(d.experts) + 1)));
+    if (b) *b = o;
+    return off;
+}
+
+int validate_prompt(const lemoq_step_desc& d) {
+    LEMOQ_REQUIRE(d.layers > 0 && d.hidden > 0 && d.heads > 0 && d.experts > 0 && d.top_k > 0 && d.ffn > 0 && d.vocab > 0 && d.max_len > 0,
+                  LEMOQ_ERR_INVALID, "prompt: all sizes must be positive");
+    LEMOQ_REQUIRE(d.head_dim == 128, LEMOQ_ERR_UNSUPPORTED, "prompt: head_dim must be 128");
+    LEMOQ_REQUIRE(d.hidden % 128 == 0 && d.hidden <= 4096 && d.heads <= 32 && d.ffn % 128 == 0, LEMOQ_ERR_UNSUPPORTED,
+                  "prompt: hidden and ffn must be multiples of 128, hidden and heads * 128 at most 4096");
+    LEMOQ_REQUIRE(d.experts % 8 == 0 && d.experts <= 128 && d.top_k <= 32 && d.top_k <= d.experts, LEMOQ_ERR_UNSUPPORTED,
+                  "prompt: experts must be a multiple of 8, at most 128, top_k at most 32");
+    LEMOQ_REQUIRE(d.group_size > 0 && d.group_size % 128 == 0 && d.hidden % d.group_size == 0 && d.ffn % d.group_size == 0 &&
+                      d.heads * 128 % d.group_size == 0,
+                  LEMOQ_ERR_UNSUPPORTED, "prompt: group_size must be a multiple of 128 that divides every row");
+    return LEMOQ_OK;
+}
+
+}  // namespace
+}  // namespace lemoq
+
+using namespace lemoq;
+
+extern "C" size_t lemoq_prompt_workspace_bytes(const lemoq_step_desc* desc, int T) {
+    if (!desc || T <= 0 || validate_prompt(*desc) != LEMOQ_OK) return 0;
+    return carve_prompt(*desc, T, nullptr, nullptr);
+}
+
+extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens, const int64_t* positions, int T, void* logits,
+                                void* workspace, size_t workspace_bytes, int* err_flag, void* stream) {
+    LEMOQ_REQUIRE(desc && layers && tokens && positions && logits && workspace, LEMOQ_ERR_INVALID, "prompt: null pointer");
+    const lemoq_step_desc& d = *desc;
+    if (int rc = validate_prompt(d)) return rc;
+    LEMOQ_REQUIRE(T > 0 && static_cast<int64_t>(T) * d.top_k <= (1 << 24), LEMOQ_ERR_INVALID, "prompt: T=%d out of range", T);
+    LEMOQ_REQUIRE(d.embed && d.final_norm && d.lm_head_codes && d.lm_head_scale && d.rope_cos && d.rope_sin, LEMOQ_ERR_INVALID,
+                  "prompt: null pointer in descriptor");
+    LEMOQ_REQUIRE(aligned16(logits) && aligned16(workspace), LEMOQ_ERR_INVALID, "prompt: logits and workspace must be 16-byte aligned");
+    PromptBuffers b;
+    const size_t need = carve_prompt(d, T, static_cast<char*>(workspace), &b);
+    LEMOQ_REQUIRE(workspace_bytes >= need, LEMOQ_ERR_INVALID, "prompt: workspace of %zu bytes, needs %zu", workspace_bytes, need);
+
+    LaunchCfg lc;
+    lc.stream = static_cast<cudaStream_t>(stream);
+    LaunchCfg chained = lc;
+    chained.pdl = true;
+    auto half = [](const void* p) { return reinterpret_cast<const __half*>(p); };
+    const int A = d.heads * 128, P = T * d.top_k;
+
+    auto gemm = [&](const __half* x, int rows, const int8_t* codes, const void* scale, int N, int K, const __half* resid, __half* y) {
+        W8GemmParams g;
+        g.x = x; g.T = rows; g.codes = codes; g.scale = half(scale); g.N = N; g.K = K; g.group_size = d.group_size;
+        g.resid = resid; g.y = y; g.exact = false; g.err_flag = err_flag;
+        return launch_w8_gemm(g, chained);
+    };
+#define LEMOQ_TRY(call)            \
+    do {                           \
+        if (int rc_ = (call)) return rc_; \
+    } while (0)
+
+    LEMOQ_TRY(launch_embed_norm(tokens, half(d.embed), d.vocab, T, d.hidden, half(layers[0].ln1), d.eps, b.x, b.h, err_flag, lc));
+    for (int i = 0; i < d.layers; ++i) {
+        const lemoq_layer_desc& L = layers[i];
+        LEMOQ_TRY(gemm(b.h, T, L.qkv_codes, L.qkv_scale, 3 * A, d.hidden, nullptr, b.qkv));
+        QkvRows r;
+        r.qkv = b.qkv; r.q_norm = half(L.q_norm); r.k_norm = half(L.k_norm); r.rope_cos = half(d.rope_cos); r.rope_sin = half(d.rope_sin);
+        r.pos = positions; r.q = b.q; r.keys = reinterpret_cast<__half*>(L.keys); r.values = reinterpret_cast<__half*>(L.values);
+        r.eps = d.eps; r.T = T; r.heads = d.heads; r.S = d.max_len; r.err_flag = err_flag;
+        LEMOQ_TRY(launch_qkv_rows(r, chained));
+        PromptAttn a;
+        a.q = b.q; a.keys = half(L.keys); a.values = half(L.values); a.pos = positions; a.out = b.ctx;
+        a.T = T; a.heads = d.heads; a.S = d.max_len; a.scale = 1.0f / sqrtf(128.0f); a.err_flag = err_flag;
+        LEMOQ_TRY(launch_prompt_attn(a, chained));
+        LEMOQ_TRY(gemm(b.ctx, T, L.o_codes, L.o_scale, d.hidden, A, b.x, b.x1));
+        LEMOQ_TRY(launch_combine_norm(nullptr, nullptr, nullptr, T, 0, b.x1, d.hidden, half(L.ln2), d.eps, nullptr, b.h, chained));
+        LEMOQ_TRY(launch_route_rows(b.h, half(L.router), T, d.hidden, d.experts, d.top_k, d.norm_topk_prob, nullptr, b.top_w, b.top_i, chained));
+        LEMOQ_TRY(launch_pair_plan(b.top_i, P, d.experts, b.place, b.pair_of, b.seg, chained));
+        LEMOQ_TRY(launch_gather_rows(b.h, b.pair_of, P, d.top_k, d.hidden, b.pairs, chained));
+        W8GemmParams g;
+        g.x = b.pairs; g.T = P; g.codes = L.gu_codes; g.scale = half(L.gu_scale); g.N = 2 * d.ffn; g.K = d.hidden; g.group_size = d.group_size;
+        g.seg = b.seg; g.E = d.experts; g.gate_up = true; g.y = b.act; g.exact = false; g.err_flag = err_flag;
+        LEMOQ_TRY(launch_w8_gemm(g, chained));
+        g.x = b.act; g.codes = L.dn_codes; g.scale = half(L.dn_scale); g.N = d.hidden; g.K = d.ffn; g.gate_up = false; g.y = b.pairs;
+        LEMOQ_TRY(launch_w8_gemm(g, chained));
+        LEMOQ_TRY(launch_combine_norm(b.pairs, b.place, b.top_w, T, d.top_k, b.x1, d.hidden,
+                                      half(i + 1 < d.layers ? layers[i + 1].ln1 : d.final_norm), d.eps, b.x, b.h, chained));
+    }
+    LEMOQ_TRY(gemm(b.h, T, d.lm_head_codes, d.lm_head_scale, d.vocab, d.hidden, nullptr, reinterpret_cast<__half*>(logits)));
+#undef LEMOQ_TRY
+    return LEMOQ_OK;
+}

@@ -1,0 +1,45 @@
+// Launch interface of the kernels for many tokens at once (prompt_ops.cu, prompt_attn.cu).
+#pragma once
+
+#include "kernels.h"
+
+namespace lemoq {
+
+int launch_embed_norm(const int64_t* tokens, const __half* embed, int64_t vocab, int T, int H, const __half* w, float eps, __half* x, __half* h, int* err,
+                      const LaunchCfg& lc);
+// y == nullptr: h = norm(x1) only
+int launch_combine_norm(const __half* y, const int32_t* place, const float* top_w, int T, int K, const __half* x1, int H, const __half* w, float eps, __half* x2,
+                        __half* h, const LaunchCfg& lc);
+
+struct QkvRows {
+    const __half* qkv = nullptr;     // (T, 3A)
+    const __half *q_norm = nullptr, *k_norm = nullptr;        // (A)
+    const __half *rope_cos = nullptr, *rope_sin = nullptr;    // (S, 128)
+    const int64_t* pos = nullptr;    // (T) cache slot of each row
+    __half* q = nullptr;             // (T, A)
+    __half *keys = nullptr, *values = nullptr;                // (heads, S, 128)
+    float eps = 0.f;
+    int T = 0, heads = 0, S = 0;
+    int* err_flag = nullptr;
+};
+int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc);
+
+// logits (T, E) fp16 = h . router^T, softmax + top-k of every row.  E a multiple of 16, <= 128; H a multiple of 64.
+int launch_route_rows(const __half* h, const __half* router, int T, int H, int E, int top_k, int norm, __half* logits, float* top_w, int32_t* top_i,
+                      const LaunchCfg& lc);
+// Stable sort of the P = T * K pairs by expert: place[p] = row of pair p in expert order, pair_of[row] = p, seg[e] = first row of e.
+int launch_pair_plan(const int32_t* top_i, int P, int E, int32_t* place, int32_t* pair_of, int32_t* seg, const LaunchCfg& lc);
+int launch_gather_rows(const __half* h, const int32_t* pair_of, int P, int K, int H, __half* x_sorted, const LaunchCfg& lc);
+
+struct PromptAttn {
+    const __half* q = nullptr;       // (T, heads * 128)
+    const __half *keys = nullptr, *values = nullptr;  // (heads, S, 128)
+    const int64_t* pos = nullptr;    // (T): row t sees slots [0, pos[t]]
+    __half* out = nullptr;           // (T, heads * 128)
+    int T = 0, heads = 0, S = 0;
+    float scale = 0.f;
+    int* err_flag = nullptr;
+};
+int launch_prompt_attn(const PromptAttn& p, const LaunchCfg& lc);
+
+}  // namespace lemoq

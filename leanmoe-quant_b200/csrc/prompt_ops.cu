@@ -1,0 +1,372 @@
+// Row operations between the tensor-core kernels when many tokens go through a layer at once.  All of them are bounded by
+// the rows they read and write (L2-resident up to some thousand tokens); each does everything that touches its rows in one
+// pass, so that a layer is eleven launches:
+//
+//   embed_norm     embedding row, input RMSNorm                                   one block per token
+//   qkv_rows       q/k RMSNorm over the projection width, RoPE, rows into the caches one block per token
+//   route_rows     router logits (fp16 mma), softmax, top-k                         one block per 16 tokens
+//   pair_plan      stable counting sort of the (token, slot) pairs by expert         one block per expert
+//   gather_rows    activations into expert order                                    one block per pair
+//   combine_norm   routing-weighted sum in slot order (fp32) + residual, next norm   one block per token
+#include "prompt.h"
+#include "stream.cuh"
+
+namespace lemoq {
+namespace {
+
+constexpr int kRowThreads = 256;
+constexpr int kRowVecs = 2;  // 8-value vectors a thread keeps: rows up to 4096
+
+// RMSNorm of a row held as fp32 in registers (vector v at 8 * (tid + 256 v)); HF rounding chain, fp16 out.
+__device__ __forceinline__ void norm_row_store(const float (&f)[kRowVecs][8], int H, const __half* __restrict__ w, float eps, __half* __restrict__ y, float* red) {
+    float ss = 0.f;
+#pragma unroll
+    for (int v = 0; v < kRowVecs; ++v)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss = fmaf(f[v][j], f[v][j], ss);  // vectors beyond the row are zero
+    ss = block_sum(ss, red);
+    const float rstd = 1.0f / sqrtf(ss / static_cast<float>(H) + eps);
+#pragma unroll
+    for (int v = 0; v < kRowVecs; ++v) {
+        const int i = 8 * (threadIdx.x + kRowThreads * v);
+        if (i < H) {
+            const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + i));
+            const __half* wh = reinterpret_cast<const __half*>(&wv);
+            __align__(16) __half o[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(f[v][j] * rstd), wh[j]);
+            *reinterpret_cast<uint4*>(y + i) = *reinterpret_cast<const uint4*>(o);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kRowThreads) embed_norm_kernel(const int64_t* __restrict__ tokens, const __half* __restrict__ embed, int64_t vocab, int H,
+                                                                 const __half* __restrict__ w, float eps, __half* __restrict__ x, __half* __restrict__ h, int* err) {
+    __shared__ float red[40];
+    pdl_wait();
+    pdl_trigger();
+    const int64_t t = blockIdx.x, tok = checked_token(tokens + t, vocab, err);
+    float f[kRowVecs][8];
+#pragma unroll
+    for (int v = 0; v < kRowVecs; ++v) {
+        const int i = 8 * (threadIdx.x + kRowThreads * v);
+        uint4 e = make_uint4(0, 0, 0, 0);
+        if (i < H) {
+            e = ld_stream16(embed + tok * H + i);
+            *reinterpret_cast<uint4*>(x + t * H + i) = e;
+        }
+        unpack8_h(e, f[v]);
+    }
+    norm_row_store(f, H, w, eps, h + t * H, red);
+}
+
+// out[t] = fp16(sum_k w[t, k] * y[place[t, k]]) + x1[t]; then the next RMSNorm of it.  Without y: only the norm of x1.
+__global__ void __launch_bounds__(kRowThreads) combine_norm_kernel(const __half* __restrict__ y, const int32_t* __restrict__ place, const float* __restrict__ top_w,
+                                                                   int K, const __half* __restrict__ x1, int H, const __half* __restrict__ w, float eps,
+                                                                   __half* __restrict__ x2, __half* __restrict__ h) {
+    __shared__ float red[40];
+    pdl_wait();
+    pdl_trigger();
+    const int64_t t = blockIdx.x;
+    float f[kRowVecs][8];
+#pragma unroll
+    for (int v = 0; v < kRowVecs; ++v) {
+        const int i = 8 * (threadIdx.x + kRowThreads * v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[v][j] = 0.f;
+        if (i < H) {
+            uint4 r = ld_cg16(x1 + t * H + i);
+            if (y) {
+                for (int k = 0; k < K; ++k) {
+                    const float wk = __half2float(__float2half_rn(__ldg(top_w + t * K + k)));
+                    float g[8];
+                    unpack8_h(ld_cg16(y + static_cast<int64_t>(__ldg(place + t * K + k)) * H + i), g);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) f[v][j] = __fadd_rn(f[v][j], __fmul_rn(g[j], wk));
+                }
+                __half* rh = reinterpret_cast<__half*>(&r);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) rh[j] = __hadd(__float2half_rn(f[v][j]), rh[j]);
+                *reinterpret_cast<uint4*>(x2 + t * H + i) = r;
+            }
+            unpack8_h(r, f[v]);
+        }
+    }
+    norm_row_store(f, H, w, eps, h + t * H, red);
+}
+
+// One block per token, A = heads * 128 <= 4096.  qkv (T, 3A) -> q (T, A) normalised and rotated; the k and v rows go into
+// slot pos[t] of the fp16 caches (heads, S, 128).
+__global__ void __launch_bounds__(kRowThreads) qkv_rows_kernel(const QkvRows p) {
+    __shared__ float red[40];
+    __shared__ __align__(16) __half row[2][kRowThreads * 8 * kRowVecs];
+    pdl_wait();
+    pdl_trigger();
+    const int64_t t = blockIdx.x;
+    const int A = p.heads * 128, tid = threadIdx.x;
+    int64_t pos = p.pos[t];
+    if (pos < 0 || pos >= p.S) {
+        if (p.err_flag && tid == 0) atomicOr(p.err_flag, LEMOQ_FLAG_BAD_POSITION);
+        pos = pos < 0 ? 0 : p.S - 1;
+    }
+    const __half* src = p.qkv + t * 3 * A;
+    float f[2][kRowVecs][8];
+    float ss[2] = {0.f, 0.f};
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int v = 0; v < kRowVecs; ++v) {
+            const int i = 8 * (tid + kRowThreads * v);
+            unpack8_h(i < A ? ld_cg16(src + m * A + i) : make_uint4(0, 0, 0, 0), f[m][v]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss[m] = fmaf(f[m][v][j], f[m][v][j], ss[m]);
+        }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const float rstd = 1.0f / sqrtf(block_sum(ss[m], red) / static_cast<float>(A) + p.eps);
+        const __half* w = m ? p.k_norm : p.q_norm;
+#pragma unroll
+        for (int v = 0; v < kRowVecs; ++v) {
+            const int i = 8 * (tid + kRowThreads * v);
+            if (i < A) {
+                const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + i));
+                const __half* wh = reinterpret_cast<const __half*>(&wv);
+                __align__(16) __half o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(f[m][v][j] * rstd), wh[j]);
+                *reinterpret_cast<uint4*>(&row[m][i]) = *reinterpret_cast<const uint4*>(o);
+            }
+        }
+    }
+    __syncthreads();
+    const __half* cos = p.rope_cos + pos * 128;
+    const __half* sin = p.rope_sin + pos * 128;
+#pragma unroll
+    for (int v = 0; v < kRowVecs; ++v) {
+        const int i = 8 * (tid + kRowThreads * v);
+        if (i < A) {
+            const int d = i & 127, other = d < 64 ? i + 64 : i - 64;
+            const float sign = d < 64 ? -1.f : 1.f;
+            float c[8], s[8];
+            unpack8_h(__ldg(reinterpret_cast<const uint4*>(cos + d)), c);
+            unpack8_h(__ldg(reinterpret_cast<const uint4*>(sin + d)), s);
+            const int64_t slot = (static_cast<int64_t>(i >> 7) * p.S + pos) * 128 + d;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                float a[8], b[8];
+                unpack8_h(*reinterpret_cast<const uint4*>(&row[m][i]), a);
+                unpack8_h(*reinterpret_cast<const uint4*>(&row[m][other]), b);
+                __align__(16) __half o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = __float2half_rn(__fadd_rn(__fmul_rn(a[j], c[j]), __fmul_rn(sign * b[j], s[j])));
+                __half* dst = m ? p.keys + slot : p.q + t * A + i;
+                *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
+            }
+            *reinterpret_cast<uint4*>(p.values + slot) = ld_cg16(src + 2 * A + i);
+        }
+    }
+}
+
+// ---- router ---------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+constexpr int kRouteWarps = 8;
+constexpr int kRouteTokens = 16;
+
+// 16 tokens x all experts per block.  The warps split H; their partial sums meet in shared memory and are added in warp
+// order.  With 0.27 GFLOP per thousand tokens the work is too small for a tcgen05 pipeline to fill: what counts is one round
+// of loads.  A and B use the same permutation of k inside 32 values, so that 128-bit loads feed the fragments.
+template <int TILES>  // expert tiles of 8
+__global__ void __launch_bounds__(kRouteWarps * 32) route_rows_kernel(const __half* __restrict__ h, const __half* __restrict__ router, int T, int H, int E, int top_k,
+                                                                      int norm, __half* __restrict__ logits, float* __restrict__ top_w, int32_t* __restrict__ top_i) {
+    extern __shared__ float part[];  // [warp][16 tokens][E]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int t0 = blockIdx.x * kRouteTokens, tiles = E >> 3;
+    pdl_wait();
+    pdl_trigger();
+    float c[TILES][4];
+#pragma unroll
+    for (int n = 0; n < TILES; ++n) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
+    const __half* lo = h + static_cast<int64_t>(min(t0 + g, T - 1)) * H + 8 * q;
+    const __half* hi = h + static_cast<int64_t>(min(t0 + g + 8, T - 1)) * H + 8 * q;
+    const __half* wr = router + static_cast<int64_t>(g) * H + 8 * q;
+    for (int k = 32 * warp; k < H; k += 32 * kRouteWarps) {
+        const uint4 a = ld_cg16(lo + k), b = ld_cg16(hi + k);
+#pragma unroll
+        for (int n = 0; n < TILES; ++n) {
+            if (n < tiles) {
+                const uint4 w = __ldg(reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(8 * n) * H + k));
+                mma_f16(c[n], a.x, b.x, a.y, b.y, w.x, w.y);
+                mma_f16(c[n], a.z, b.z, a.w, b.w, w.z, w.w);
+            }
+        }
+    }
+    float* mine = part + warp * kRouteTokens * E;
+#pragma unroll
+    for (int n = 0; n < TILES; ++n) {
+        if (n < tiles) {
+            *reinterpret_cast<float2*>(mine + g * E + 8 * n + 2 * q) = make_float2(c[n][0], c[n][1]);
+            *reinterpret_cast<float2*>(mine + (g + 8) * E + 8 * n + 2 * q) = make_float2(c[n][2], c[n][3]);
+        }
+    }
+    __syncthreads();
+    constexpr int PER = TILES / 4 < 1 ? 1 : TILES / 4;  // experts of a lane: lane + 32 i
+    for (int j = warp; j < kRouteTokens; j += kRouteWarps) {
+        const int t = t0 + j;
+        if (t >= T) break;
+        float p[PER];
+        float mx = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int e = lane + 32 * i;
+            p[i] = -INFINITY;
+            if (e < E) {
+                float v = 0.f;
+#pragma unroll
+                for (int w = 0; w < kRouteWarps; ++w) v += part[(w * kRouteTokens + j) * E + e];
+                const __half r = __float2half_rn(v);
+                if (logits) logits[static_cast<int64_t>(t) * E + e] = r;
+                p[i] = __half2float(r);
+            }
+            mx = fmaxf(mx, p[i]);
+        }
+        mx = warp_max(mx);
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            if (lane + 32 * i < E) {
+                p[i] = expf(p[i] - mx);
+                sum += p[i];
+            }
+        }
+        sum = warp_sum(sum);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) p[i] = lane + 32 * i < E ? p[i] / sum : -1.f;
+        float kept = 0.f, wsum = 0.f;
+        int kept_i = 0;
+        for (int k = 0; k < top_k; ++k) {
+            float best = -1.f;
+            int bi = 0x7fffffff;
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+                if (p[i] > best) {  // ascending e inside a lane: the first maximum wins
+                    best = p[i];
+                    bi = lane + 32 * i;
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (ob > best || (ob == best && oi < bi)) {
+                    best = ob;
+                    bi = oi;
+                }
+            }
+            if (bi >= E) bi = 0;  // only with NaN logits: any valid expert
+            wsum += best;
+            if (lane == k) {
+                kept = best;
+                kept_i = bi;
+            }
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+                if (bi == lane + 32 * i) p[i] = -1.f;
+        }
+        if (lane < top_k) {
+            top_w[static_cast<int64_t>(t) * top_k + lane] = norm ? kept / wsum : kept;
+            top_i[static_cast<int64_t>(t) * top_k + lane] = kept_i;
+        }
+    }
+}
+
+// ---- pairs into expert order ----------------------------------------------------------------------------------------------
+constexpr int kPlanThreads = 512;
+
+// One block per expert: counts the pairs of lower experts, then gives its own pairs their rows in pair order.
+__global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const int32_t* __restrict__ top_i, int P, int E, int32_t* __restrict__ place,
+                                                                 int32_t* __restrict__ pair_of, int32_t* __restrict__ seg) {
+    __shared__ int s_warp[kPlanThreads / 32 + 1];
+    const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_wait();
+    pdl_trigger();
+    int below = 0;
+    for (int p = threadIdx.x; p < P; p += kPlanThreads) below += top_i[p] < e;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+    if (lane == 0) s_warp[warp] = below;
+    __syncthreads();
+    int base = 0;
+#pragma unroll
+    for (int w = 0; w < kPlanThreads / 32; ++w) base += s_warp[w];
+    __syncthreads();
+    if (threadIdx.x == 0) seg[e] = base;
+    for (int p0 = 0; p0 < P; p0 += kPlanThreads) {
+        const int p = p0 + threadIdx.x;
+        const bool hit = p < P && top_i[p] == e;
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) s_warp[warp] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < kPlanThreads / 32; ++w) {
+            const int n = s_warp[w];
+            before += w < warp ? n : 0;
+            all += n;
+        }
+        if (hit) {
+            const int row = base + before + __popc(m & ((1u << lane) - 1u));
+            place[p] = row;
+            pair_of[row] = p;
+        }
+        base += all;
+        __syncthreads();
+    }
+    if (e == E - 1 && threadIdx.x == 0) seg[E] = base;
+}
+
+__global__ void __launch_bounds__(kRowThreads) gather_rows_kernel(const __half* __restrict__ h, const int32_t* __restrict__ pair_of, int K, int H,
+                                                                  __half* __restrict__ x_sorted) {
+    pdl_wait();
+    pdl_trigger();
+    const int64_t r = blockIdx.x, t = pair_of[r] / K;
+    for (int i = 8 * threadIdx.x; i < H; i += 8 * kRowThreads)
+        *reinterpret_cast<uint4*>(x_sorted + r * H + i) = ld_cg16(h + t * H + i);
+}
+
+}  // namespace
+
+int launch_embed_norm(const int64_t* tokens, const __half* embed, int64_t vocab, int T, int H, const __half* w, float eps, __half* x, __half* h, int* err,
+                      const LaunchCfg& lc) {
+    return launch_kernel(embed_norm_kernel, dim3(T), dim3(kRowThreads), 0, lc, tokens, embed, vocab, H, w, eps, x, h, err);
+}
+
+int launch_combine_norm(const __half* y, const int32_t* place, const float* top_w, int T, int K, const __half* x1, int H, const __half* w, float eps, __half* x2,
+                        __half* h, const LaunchCfg& lc) {
+    return launch_kernel(combine_norm_kernel, dim3(T), dim3(kRowThreads), 0, lc, y, place, top_w, K, x1, H, w, eps, x2, h);
+}
+
+int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc) { return launch_kernel(qkv_rows_kernel, dim3(p.T), dim3(kRowThreads), 0, lc, p); }
+
+int launch_route_rows(const __half* h, const __half* router, int T, int H, int E, int top_k, int norm, __half* logits, float* top_w, int32_t* top_i,
+                      const LaunchCfg& lc) {
+    const dim3 grid((T + kRouteTokens - 1) / kRouteTokens), block(kRouteWarps * 32);
+    const size_t smem = static_cast<size_t>(kRouteWarps) * kRouteTokens * E * sizeof(float);
+    if (E <= 64) return launch_kernel(route_rows_kernel<8>, grid, block, smem, lc, h, router, T, H, E, top_k, norm, logits, top_w, top_i);
+    const cudaError_t err = cudaFuncSetAttribute(route_rows_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
+    return launch_kernel(route_rows_kernel<16>, grid, block, smem, lc, h, router, T, H, E, top_k, norm, logits, top_w, top_i);
+}
+
+int launch_pair_plan(const int32_t* top_i, int P, int E, int32_t* place, int32_t* pair_of, int32_t* seg, const LaunchCfg& lc) {
+    return launch_kernel(pair_plan_kernel, dim3(E), dim3(kPlanThreads), 0, lc, top_i, P, E, place, pair_of, seg);
+}
+
+int launch_gather_rows(const __half* h, const int32_t* pair_of, int P, int K, int H, __half* x_sorted, const LaunchCfg& lc) {
+    return launch_kernel(gather_rows_kernel, dim3(P), dim3(kRowThreads), 0, lc, h, pair_of, K, H, x_sorted);
+}
+
+}  // namespace lemoq

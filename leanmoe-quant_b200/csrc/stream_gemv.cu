@@ -307,18 +307,6 @@ __global__ void __launch_bounds__(kMaxStreamWarps * 32, 1) stream_down_kernel(Mo
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-static int sm_count() {
-    static int cached = 0;
-    if (cached) return cached;
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
-        cached = v;
-    else
-        cached = 148;
-    return cached;
-}
-
 template <typename Kern>
 static int set_smem(Kern kern, size_t smem) {
     if (smem > 227 * 1024) return set_error(LEMOQ_ERR_UNSUPPORTED, "streaming kernel needs %zu bytes of shared memory", smem);

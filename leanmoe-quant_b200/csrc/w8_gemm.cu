@@ -1,0 +1,518 @@
+// W8 rows against many tokens on the tensor cores: prompts (thousands of tokens), batches of tens, and the routed experts
+// of both (tokens sorted by expert, a segment per expert).
+//
+//   y[t, n] = sum_g scale[n, g] * ( sum_{k in group g} codes[n, k] * x[t, k] )        (+ resid[t, n], or SwiGLU of two rows)
+//
+// The weight rows are the M side of tcgen05.mma (128 rows a tile, lane = row), the tokens the N side: an expert with nine
+// tokens costs an N of 16 and not a tile of 128.  Two forms:
+//   exact   up to 64 tokens a tile.  int8 codes are exact in fp16, so the products are those of the integer kernels: the codes
+//           are widened, not scaled.  The fp32 sum of one group of 128 codes leaves TMEM, is scaled in fp32 and added to
+//           the row's accumulators in registers.
+//   scaled  up to 128 tokens a tile, for prompts: the widened code is multiplied by its group scale and rounded to fp16 (what
+//           dequantising the weights to fp16 in memory does), the sum over all of K stays in TMEM.
+//
+// One persistent block per SM, a tile = two M tiles (256 weight rows; for gate/up 128 gate rows and their 128 up rows)
+// x up to NT tokens of one expert:
+//   warp 16      TMA: per group of 128 k the codes (2 x 128 rows x 128 bytes) and the tokens (two halves of 64 k), swizzled
+//   warps 8-15   a warpgroup per M tile, thread = weight row: widen the codes of a group into TMEM (two buffers)
+//   warp 17      issues the MMAs: A = widened codes from TMEM, B = tokens from shared memory, D in TMEM
+//   warps 0-7    a warpgroup per M tile, thread = weight row: collect the sums (per group / at the end), finish the rows
+// TMEM: D of tile w at column 128 w (exact: two buffers of 64), A of tile w, buffer b at 256 + 128 w + 64 b.
+//
+// What bounds it: with few tokens per expert the bytes of the codes (HBM); with 128 per tile shared memory (160 KB of TMA
+// writes, code reads and B reads per group against 1024 cycles of MMAs).  A in TMEM instead of shared memory, because widened
+// codes in shared memory would add a write and a read of twice the codes' size.  Widening and collecting are different warps
+// because either is a chain of waits, and the TMA and MMA loops are one thread each because a vote after every wait cost
+// that warp 160 cycles (exact, NT = 16: 3200 cycles per group with both by the same warps and `lane == 0` issue, 1700 with
+// separate warps and elect.sync).
+#include "tc.cuh"
+
+#include <algorithm>
+#include <mutex>
+
+namespace lemoq {
+
+int encode_rows_map(CUtensorMap* map, const void* base, int elem_bytes, int64_t rows, int64_t cols, int box_rows, int64_t row_stride) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Encode encode = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) == cudaSuccess &&
+            found == cudaDriverEntryPointSuccess)
+            encode = reinterpret_cast<Encode>(fn);
+    });
+    if (!encode) return set_error(LEMOQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available in this driver");
+    if (row_stride == 0) row_stride = cols;
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_stride) * elem_bytes};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / elem_bytes), static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t elem[2] = {1, 1};
+    const CUresult rc = encode(map, elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims,
+                               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) return set_error(LEMOQ_ERR_CUDA, "cuTensorMapEncodeTiled: error %d", static_cast<int>(rc));
+    return LEMOQ_OK;
+}
+
+namespace {
+
+constexpr int kThreads = 640;       // five warpgroups: two collect, two widen, the fifth has the TMA warp and the MMA warp
+// Registers: 640 threads are launched with 96 each (61,440); 256 x 144 + 256 x 56 + 128 x 72 = 60,416 afterwards.
+constexpr int kExactTokens = 64, kScaledTokens = 128;  // most tokens of a tile
+constexpr int kRegsCollect = 144, kRegsWiden = 56, kRegsIssue = 72;
+constexpr int kTileRows = 256;      // weight rows of a tile (two M tiles of 128)
+constexpr int kCodeBytes = 2 * 128 * 128;
+constexpr int kSegCap = kMaxExperts + 1;
+constexpr uint32_t kColA = 256;     // first TMEM column of the widened codes
+
+template <int NT>
+struct Shape {
+    static constexpr int kBox = NT >= 128 ? 32 : 16;                    // token rows of one TMA box
+    static constexpr int kHalf = NT * 128;                              // bytes of one 64-wide half of the tokens
+    static constexpr int kStage = kCodeBytes + 2 * kHalf;
+    static constexpr bool kScaled = NT > kExactTokens;
+    static constexpr int kDBufs = kScaled ? 1 : 2;                      // accumulator buffers per M tile
+    static constexpr int kStages = NT >= 128 ? 3 : (NT == 64 ? 4 : 5);
+    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + 1024;
+};
+
+struct GemmShape {
+    int T, N, K, group, E, gate_up;
+    const int32_t* seg;    // (E + 1) or null: one segment [0, T)
+    const __half* scale;   // (E, N, K / group)
+    const __half* resid;   // (T, N) or null
+    __half* y;             // (T, N), or (T, N / 2) in gate/up mode
+    int* err_flag;
+};
+
+struct Tile {
+    int row0, row1;    // first weight row of the two M tiles inside the expert
+    int e, t0, n;      // expert, first token, tokens
+};
+
+// Tiles before expert e: first[e].  A tile number -> expert by binary search, then (M tile pair, token tile): neighbours in
+// the order share their weight rows and meet in L2.  The tokens of an expert are split evenly.
+template <int NT>
+__device__ __forceinline__ Tile tile_at(int i, const int* first, const int* tok, const GemmShape& p, int mt) {
+    int lo = 0, hi = p.E;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= i) lo = mid; else hi = mid;
+    }
+    Tile t;
+    t.e = lo;
+    const int cnt = tok[lo + 1] - tok[lo], nt = (cnt + NT - 1) / NT, r = i - first[lo], m = r / nt, b = r - m * nt;
+    const int per = ((cnt + nt - 1) / nt + 15) & ~15;
+    t.t0 = tok[lo] + b * per;
+    t.n = max(0, min(per, tok[lo + 1] - t.t0));
+    t.row0 = p.gate_up ? m * 128 : m * kTileRows;
+    t.row1 = p.gate_up ? p.N / 2 + m * 128 : m * kTileRows + 128;
+    return t;
+}
+
+// 16 codes -> 8 words of two exact fp16 each: bytes with the sign flipped dropped into 0x64__ are 1024 + 128 + c.
+template <bool SCALED>
+__device__ __forceinline__ void widen16(const uint4& w, __half scale, uint32_t* out) {
+    const uint32_t u[4] = {w.x ^ 0x80808080u, w.y ^ 0x80808080u, w.z ^ 0x80808080u, w.w ^ 0x80808080u};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        __half2 a = codes_half2(u[i], 0x4140), b = codes_half2(u[i], 0x4342);
+        if (SCALED) {
+            a = __hmul2(a, __half2half2(scale));
+            b = __hmul2(b, __half2half2(scale));
+        }
+        out[2 * i] = *reinterpret_cast<const uint32_t*>(&a);
+        out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                                                              const GemmShape p) {
+    using S = Shape<NT>;
+    constexpr int kStages = S::kStages;
+    extern __shared__ uint8_t raw[];
+    __shared__ __align__(8) uint64_t s_bar[2 * kStages + 7];
+    __shared__ int s_first[kSegCap], s_tok[kSegCap];
+    __shared__ uint32_t s_tmem;
+    __shared__ volatile int s_abort;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t stage0 = (smem_u32(raw) + 1023u) & ~1023u;
+    const uint32_t bars = smem_u32(s_bar);
+    auto full = [&](int s) { return bars + 8u * s; };
+    auto done = [&](int s) { return bars + 8u * (kStages + s); };
+    auto a_full = [&](int b) { return bars + 8u * (2 * kStages + b); };
+    auto d_free = [&](int b) { return bars + 8u * (2 * kStages + 2 + b); };
+    const uint32_t ex = bars + 8u * (2 * kStages + 4), drained = ex + 8u, d_full = ex + 16u;
+    constexpr int kD = S::kDBufs;
+    constexpr bool kScaled = S::kScaled;
+
+    if (tid == 0) {
+        s_abort = 0;
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(full(s), 1);
+            mbar_init(done(s), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(a_full(b), 8);
+            mbar_init(d_free(b), 8);
+        }
+        mbar_init(ex, 8);
+        mbar_init(drained, 1);
+        mbar_init(d_full, 1);
+        mbar_fence_init();
+    }
+    if (warp == 17) tmem_alloc(smem_u32(&s_tmem), 512);
+    if (tid == 512) {
+        tma_prefetch_map(&map_w);
+        tma_prefetch_map(&map_x);
+    }
+    pdl_wait();  // the segments and the tokens come from earlier kernels
+    pdl_trigger();
+    const int mt = p.gate_up ? (p.N / 2 + 127) / 128 : (p.N + kTileRows - 1) / kTileRows;
+    if (warp == 0) {  // tokens and tiles before each expert
+        int carry = 0;
+        for (int e0 = 0; e0 < p.E; e0 += 32) {
+            const int e = e0 + lane;
+            int a = 0, b = 0;
+            if (e < p.E) {
+                a = p.seg ? min(max(p.seg[e], 0), p.T) : 0;
+                b = p.seg ? min(max(p.seg[e + 1], a), p.T) : p.T;
+                s_tok[e] = a;
+                if (e == p.E - 1) s_tok[p.E] = b;
+            }
+            const int mine = (b - a + NT - 1) / NT * mt;
+            int v = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += up;
+            }
+            if (e < p.E) s_first[e] = carry + v - mine;
+            carry += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) s_first[p.E] = carry;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    const int tiles = s_first[p.E], groups = p.K >> 7;
+    volatile int* abort = &s_abort;
+
+    if (warp >= 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+    if (warp == 16) {
+        // ---- TMA: one thread ---------------------------------------------------------------------------------------
+        if (elect_one()) {
+            int s = 0, issued = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
+                const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
+                const int boxes = (t.n + S::kBox - 1) / S::kBox, base = t.e * p.N;
+                const uint32_t bytes = kCodeBytes + 2u * boxes * S::kBox * 128u;
+                for (int g = 0; g < groups; ++g) {
+                    if (!(ok = thread_wait(done(s), ph, abort))) break;
+                    const uint32_t at = stage0 + static_cast<uint32_t>(s) * S::kStage, bar = full(s);
+                    mbar_expect_tx(bar, bytes);
+                    tma_load_2d(at, &map_w, g * 128, base + t.row0, bar);
+                    tma_load_2d(at + kCodeBytes / 2, &map_w, g * 128, base + t.row1, bar);
+                    for (int b = 0; b < boxes; ++b) {
+                        tma_load_2d(at + kCodeBytes + b * S::kBox * 128, &map_x, g * 128, t.t0 + b * S::kBox, bar);
+                        tma_load_2d(at + kCodeBytes + S::kHalf + b * S::kBox * 128, &map_x, g * 128 + 64, t.t0 + b * S::kBox, bar);
+                    }
+                    ++issued;
+                    if (++s == kStages) { s = 0; ph ^= 1; }
+                }
+            }
+            if (!ok) {  // gave up: the copies in flight still land in this block's shared memory
+                for (int j = max(0, issued - kStages); j < issued; ++j) mbar_wait(full(j % kStages), (j / kStages) & 1);
+            }
+        }
+    } else if (warp == 17) {
+        // ---- MMA: one thread ---------------------------------------------------------------------------------------
+        if (elect_one()) {
+            int s = 0, it = 0, dn = 0;  // dn counts the accumulations: one per group (exact) or per tile (scaled)
+            bool ok = true;
+            for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
+                const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
+                const uint32_t idesc = idesc_f16(128, max(16, (t.n + 15) & ~15), false);
+                for (int g = 0; g < groups; ++g, ++it) {
+                    const int b = it & 1, db = kD == 2 ? dn & 1 : 0;
+                    const bool begins = !kScaled || g == 0, ends = !kScaled || g + 1 == groups;
+                    // a widening warp has seen the stage's copies land before it arrives: no wait on full(s) here
+                    if (!(ok = thread_wait(a_full(b), (it >> 1) & 1, abort))) break;
+                    if (begins && !(ok = thread_wait(d_free(db), ((kD == 2 ? dn >> 1 : dn) & 1) ^ 1, abort))) break;
+                    tc_fence_after();
+                    const uint64_t x0 = smem_desc_sw128(stage0 + static_cast<uint32_t>(s) * S::kStage + kCodeBytes, 1024);
+                    const uint32_t a = tmem + kColA + 64u * b, d = tmem + 64u * db;
+#pragma unroll
+                    for (int w = 0; w < 2; ++w)
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            mma_f16_ts(d + 128u * w, a + 128u * w + 8u * k, x0 + (k >> 2) * (S::kHalf >> 4) + (k & 3) * 2u, idesc, !(begins && k == 0));
+                    // one event ends the group for everybody: the stage may be refilled, the A buffer rewritten, D read
+                    tc_commit(done(s));
+                    if (kScaled && ends) tc_commit(d_full);  // (a parity wait cannot look past the next phase of done(s))
+                    if (ends) ++dn;
+                    if (++s == kStages) s = 0;
+                }
+            }
+            if (!ok) {  // gave up: nothing may still write TMEM when it is freed
+                tc_commit(drained);
+                mbar_wait(drained, 0);
+            }
+        }
+    } else if (warp >= 8 && warp < 16) {
+        // ---- widen: thread = weight row ----------------------------------------------------------------------------
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsWiden));
+        const int w = (warp >> 2) & 1, row = tid & 127;
+        const uint32_t to0 = tmem + (static_cast<uint32_t>(warp & 3) << 21) + kColA + 128u * w;
+        const uint32_t from0 = stage0 + w * (kCodeBytes / 2) + row * 128u, swz = row & 7;
+        const int gk = p.K / p.group;
+        int s = 0, it = 0, s2 = kStages - 2;       // s2, ph2: stage and phase of group it - 2, the last user of this A buffer
+        uint32_t ph = 0, ph2 = 1;
+        bool ok = true;
+        for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
+            const __half* sc = nullptr;
+            __half next = __half(), scale = __half();
+            if (kScaled) {
+                const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
+                sc = p.scale + (static_cast<int64_t>(t.e) * p.N + min((w ? t.row1 : t.row0) + row, p.N - 1)) * gk;
+                next = __ldg(sc);
+            }
+            for (int g = 0; g < groups; ++g, ++it) {
+                const int b = it & 1;
+                if (kScaled) {
+                    scale = next;
+                    if (g + 1 < groups) next = __ldg(sc + ((g + 1) << 7) / p.group);
+                }
+                if (!(ok = warp_wait(full(s), ph, abort) && warp_wait(done(s2), ph2, abort))) break;
+                tc_fence_after();
+                const uint32_t from = from0 + static_cast<uint32_t>(s) * S::kStage, to = to0 + 64u * b;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    uint32_t a[16];
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) widen16<kScaled>(lds128(from + ((static_cast<uint32_t>(2 * h + c) ^ swz) << 4)), scale, a + 8 * c);
+                    tmem_st16(to + 16u * h, a);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                warp_arrive(a_full(b));
+                if (++s == kStages) { s = 0; ph ^= 1; }
+                if (++s2 == kStages) { s2 = 0; ph2 ^= 1; }
+            }
+        }
+    } else if (warp < 8) {
+        // ---- collect: thread = weight row --------------------------------------------------------------------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCollect));
+        const int w = warp >> 2, row = tid & 127;
+        const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;  // TMEM lane field
+        const int half_rows = p.N / 2, gk = p.K / p.group;
+        int it = 0, round = 0, s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x, ++round) {
+            const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
+            const int lim = p.gate_up ? half_rows : p.N;                 // rows of this tile's kind
+            const int mrow = (p.gate_up ? t.row0 : (w ? t.row1 : t.row0)) + row;  // gate/up: both tiles count gate rows
+            const int wrow = (w ? t.row1 : t.row0) + row;
+            const bool live = mrow < lim;
+            if constexpr (kScaled) {
+                // the sums are complete: take them out of TMEM as fp16, hand the columns back, then store
+                constexpr int H = NT / 2;
+                const bool gu = p.gate_up;
+                const int j0 = gu ? w * H : 0, nj = max(0, min(t.n - j0, gu ? H : NT));  // this warpgroup's tokens
+                if (!(ok = warp_wait(d_full, round & 1, abort))) break;
+                tc_fence_after();
+                __half2 out[H];
+#pragma unroll
+                for (int c = 0; c < NT; c += 16) {
+                    if (c < nj) {
+                        uint32_t r[16];
+                        tmem_ld16(r, tmem + lanes + (gu ? 0u : 128u * w) + j0 + c);
+                        if (gu) {
+                            uint32_t u[16];
+                            tmem_ld16(u, tmem + lanes + 128u + j0 + c);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const float gate = __uint_as_float(r[j]);
+                                r[j] = __float_as_uint(gate * (1.0f / (1.0f + expf(-gate))) * __uint_as_float(u[j]));
+                            }
+                        } else {
+                            tmem_wait_ld();
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; j += 2) out[(c + j) / 2] = __floats2half2_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+                    }
+                }
+                tc_fence_before();
+                warp_arrive(d_free(0));
+                if (live) {
+                    const int64_t ld = gu ? half_rows : p.N;
+                    __half* y = p.y + static_cast<int64_t>(t.t0 + j0) * ld + mrow;
+                    const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * ld + mrow : nullptr;
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) {
+                        if (j < nj) {
+                            __half v = j & 1 ? __high2half(out[j / 2]) : __low2half(out[j / 2]);
+                            if (res) v = __hadd(v, res[j * ld]);
+                            y[j * ld] = v;
+                        }
+                    }
+                }
+            } else {
+            const __half* sc = p.scale + (static_cast<int64_t>(t.e) * p.N + min(wrow, p.N - 1)) * gk;
+            float acc[NT];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) acc[j] = 0.f;
+
+            float scale = __half2float(__ldg(sc));
+            for (int g = 0; g < groups; ++g, ++it) {
+                const int db = it & 1;
+                const float next = g + 1 < groups ? __half2float(__ldg(sc + ((g + 1) << 7) / p.group)) : 0.f;
+                if (!(ok = warp_wait(done(s), ph, abort))) break;
+                tc_fence_after();
+                const uint32_t d = tmem + lanes + 128u * w + 64u * db;
+#pragma unroll
+                for (int c = 0; c < NT; c += 16) {
+                    if (c < t.n) {
+                        uint32_t r[16];
+                        tmem_ld16(r, d + c);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(scale, __uint_as_float(r[j]), acc[c + j]);
+                    }
+                }
+                tc_fence_before();
+                // gate/up: the last sums' columns carry the exchange below and are freed after it
+                if (!p.gate_up || g + 1 < groups) warp_arrive(d_free(db));
+                scale = next;
+                if (++s == kStages) { s = 0; ph ^= 1; }
+            }
+            if (!ok) break;
+            const int dl = (it - 1) & 1;  // buffer of the last group
+            if (p.gate_up) {
+                // SwiGLU: the gate tile's threads finish the first half of the tokens, the up tile's the second; what the other
+                // needs goes through the accumulators' own columns of TMEM (same lanes, so no shared memory)
+                constexpr int H = NT / 2;
+                uint32_t r[16];
+#pragma unroll
+                for (int c = 0; c < H; c += 16) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) r[j] = c + j < H ? __float_as_uint(w ? acc[c + j < H ? c + j : 0] : acc[H + (c + j < H ? c + j : 0)]) : 0u;
+                    tmem_st16(tmem + lanes + 128u * w + 64u * dl + c, r);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                warp_arrive(ex);
+                if (!(ok = warp_wait(ex, round & 1, abort))) break;
+                tc_fence_after();
+                const uint32_t d_other = tmem + lanes + 128u * (w ^ 1) + 64u * dl;
+                const int first = w ? H : 0;
+#pragma unroll
+                for (int c = 0; c < H; c += 16) {
+                    if (first + c < t.n) {
+                        tmem_ld16(r, d_other + c);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16 && c + j < H; ++j) {
+                            const float mine = w ? acc[H + c + j] : acc[c + j], other = __uint_as_float(r[j]);
+                            const float gate = w ? other : mine, up = w ? mine : other;
+                            if (live && first + c + j < t.n)
+                                p.y[static_cast<int64_t>(t.t0 + first + c + j) * half_rows + mrow] = __float2half_rn(gate * (1.0f / (1.0f + expf(-gate))) * up);
+                        }
+                    }
+                }
+                tc_fence_before();
+                warp_arrive(d_free(dl));
+            } else if (live) {
+                __half* y = p.y + static_cast<int64_t>(t.t0) * p.N + mrow;
+                const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * p.N + mrow : nullptr;
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    if (j < t.n) {
+                        __half v = __float2half_rn(acc[j]);
+                        if (res) v = __hadd(v, res[static_cast<int64_t>(j) * p.N]);
+                        y[static_cast<int64_t>(j) * p.N] = v;
+                    }
+                }
+            }
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && s_abort && p.err_flag) atomicOr(p.err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+    if (warp == 17) {
+        tc_fence_after();
+        tmem_free(tmem, 512);
+    }
+}
+
+template <int NT>
+int launch_nt(const GemmShape& p, const __half* x, const int8_t* codes, const LaunchCfg& lc) {
+    CUtensorMap map_w, map_x;
+    if (int rc = encode_rows_map(&map_w, codes, 1, static_cast<int64_t>(p.E) * p.N, p.K, 128)) return rc;
+    if (int rc = encode_rows_map(&map_x, x, 2, p.T, p.K, Shape<NT>::kBox)) return rc;
+    {  // per device and idempotent; not a stream operation, so legal under capture
+        const cudaError_t err = cudaFuncSetAttribute(w8_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<NT>::kSmem));
+        if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
+    }
+    const int64_t mt = p.gate_up ? (p.N / 2 + 127) / 128 : (p.N + kTileRows - 1) / kTileRows;
+    const int64_t most = mt * (p.seg ? p.T / NT + std::min<int64_t>(p.E, p.T) : (p.T + NT - 1) / NT);  // tiles, at most
+    const int grid = static_cast<int>(std::min<int64_t>(sm_count(), std::max<int64_t>(most, 1)));
+    return launch_kernel(w8_gemm_kernel<NT>, dim3(grid), dim3(kThreads), Shape<NT>::kSmem, lc, map_w, map_x, p);
+}
+
+}  // namespace
+
+int launch_w8_gemm(const W8GemmParams& g, const LaunchCfg& lc) {
+    GemmShape p;
+    p.T = g.T; p.N = g.N; p.K = g.K; p.group = g.group_size; p.E = g.E; p.gate_up = g.gate_up ? 1 : 0;
+    p.seg = g.seg; p.scale = g.scale; p.resid = g.resid; p.y = g.y; p.err_flag = g.err_flag;
+    // NT bounds the tokens of a tile, the MMA's N follows the real count: a small NT only saves registers and stage bytes, a
+    // large one saves widening the same codes again for a second token tile.  Twice the mean per expert covers nearly all.
+    const int64_t want = g.seg ? 2 * ((static_cast<int64_t>(g.T) + g.E - 1) / g.E) : g.T;
+    if (want <= 16) return launch_nt<16>(p, g.x, g.codes, lc);
+    if (want <= 32) return launch_nt<32>(p, g.x, g.codes, lc);
+    if (want <= kExactTokens || g.exact) return launch_nt<kExactTokens>(p, g.x, g.codes, lc);
+    return launch_nt<kScaledTokens>(p, g.x, g.codes, lc);
+}
+
+}  // namespace lemoq
+
+using namespace lemoq;
+
+extern "C" int lemoq_w8_gemm(const void* x, int T, const int8_t* codes, const void* scale, int N, int K, int group_size, const int32_t* seg_offsets,
+                             int E, int gate_up, int exact, const void* resid, void* y, int* err_flag, void* stream) {
+    LEMOQ_REQUIRE(T >= 0 && N > 0 && K > 0 && E >= 1, LEMOQ_ERR_INVALID, "w8_gemm: bad shape");
+    LEMOQ_REQUIRE(!gate_up || N % 2 == 0, LEMOQ_ERR_UNSUPPORTED, "w8_gemm: gate/up needs an even number of rows");
+    LEMOQ_REQUIRE(K % 128 == 0, LEMOQ_ERR_UNSUPPORTED, "w8_gemm: K=%d must be a multiple of 128", K);
+    LEMOQ_REQUIRE(group_size > 0 && K % group_size == 0, LEMOQ_ERR_INVALID, "w8_gemm: bad group_size %d", group_size);
+    LEMOQ_REQUIRE(group_size % 128 == 0, LEMOQ_ERR_UNSUPPORTED, "w8_gemm: group_size=%d must be a multiple of 128", group_size);
+    LEMOQ_REQUIRE(E == 1 || seg_offsets, LEMOQ_ERR_INVALID, "w8_gemm: several experts need segment offsets");
+    LEMOQ_REQUIRE(E <= kMaxExperts, LEMOQ_ERR_UNSUPPORTED, "w8_gemm: E=%d above %d", E, kMaxExperts);
+    LEMOQ_REQUIRE(!(gate_up && resid), LEMOQ_ERR_UNSUPPORTED, "w8_gemm: no residual in gate/up mode");
+    LEMOQ_REQUIRE(static_cast<int64_t>(E) * N <= 0x7fffffff, LEMOQ_ERR_UNSUPPORTED, "w8_gemm: too many rows");
+    if (T == 0) return LEMOQ_OK;
+    LEMOQ_REQUIRE(x && codes && scale && y && aligned16(x) && aligned16(codes), LEMOQ_ERR_INVALID, "w8_gemm: null or unaligned pointer");
+    W8GemmParams g;
+    g.x = reinterpret_cast<const __half*>(x);
+    g.codes = codes;
+    g.scale = reinterpret_cast<const __half*>(scale);
+    g.seg = seg_offsets;
+    g.resid = reinterpret_cast<const __half*>(resid);
+    g.y = reinterpret_cast<__half*>(y);
+    g.T = T; g.N = N; g.K = K; g.group_size = group_size; g.E = E; g.gate_up = gate_up != 0;
+    g.exact = exact != 0;
+    g.err_flag = err_flag;
+    LaunchCfg lc;
+    lc.stream = static_cast<cudaStream_t>(stream);
+    return launch_w8_gemm(g, lc);
+}

@@ -67,6 +67,7 @@ _SIGNATURES = {
     "lemoq_w8_quantise_tokens": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "lemoq_w8_rows_tokens": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int,
                                      c_void_p, c_void_p]),
+    "lemoq_w8_gemm": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "lemoq_ep_dispatch": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p]),
     "lemoq_ep_regroup": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
@@ -95,6 +96,8 @@ _SIGNATURES = {
     "lemoq_step_topk_ids": (c_void_p, [c_void_p]),
     "lemoq_step_router_logits": (c_void_p, [c_void_p]),
     "lemoq_step_phase_stamps": (c_void_p, [c_void_p]),
+    "lemoq_prompt_workspace_bytes": (c_size_t, [POINTER(StepDesc), c_int]),
+    "lemoq_prompt_run": (c_int, [POINTER(StepDesc), POINTER(LayerDesc), c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "lemoq_step_engine": (ctypes.c_char_p, [c_void_p]),
 }
 

@@ -256,12 +256,18 @@ class OlmoeForCausalLM(nn.Module):
     def forward(self, input_ids: Any, attention_mask: Any = None, past_key_values: Any = None, use_cache: bool = False,
                 cache_position: Any = None, position_ids: Any = None, **kwargs: Any) -> Any:
         m = self.model
-        x = m.embed_tokens(input_ids)
         bsz, q_len = input_ids.shape
         if cache_position is None:
-            cache_position = torch.arange(q_len, device=x.device)
+            cache_position = torch.arange(q_len, device=input_ids.device)
         if position_ids is None:
             position_ids = cache_position.unsqueeze(0)
+        if q_len > 1 and past_key_values is not None and (attention_mask is None or attention_mask.dim() != 4):
+            from lemoq.prompt import run_prompt
+
+            logits = run_prompt(self, input_ids, past_key_values, cache_position, position_ids)
+            if logits is not None:
+                return SimpleNamespace(logits=logits, past_key_values=past_key_values)
+        x = m.embed_tokens(input_ids)
         max_len = past_key_values.max_cache_len if past_key_values is not None else None
         cos, sin = m.rotary_emb(x, position_ids, max_len=max_len)
         mask4 = None

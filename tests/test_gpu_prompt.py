@@ -1,0 +1,89 @@
+"""The tensor-core kernels for many tokens at the edges of their tiles, and a whole prompt through ``lemoq_prompt_run``, against the CPU
+oracle."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from gpu_util import PER_KERNEL_REL_TOL, install_canonical, lemoq_model_from_oracle, rel_err
+from oracle import lemoq_oracle as ops
+from oracle import olmoe_decode_oracle as glue
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _w8(n, k, seed, experts=0):
+    w = torch.randn(*((experts,) if experts else ()), n, k, generator=torch.Generator().manual_seed(seed)) * 0.02
+    return ops.rtn_quantize_w8(w, 128)
+
+
+def _gemm(x, codes, scale, *, seg=None, gate_up=False, exact=True, resid=None):
+    from lemoq import _cabi
+
+    n, k = codes.shape[-2:]
+    y = torch.full((x.shape[0], n // 2 if gate_up else n), float("nan"), dtype=torch.float16, device=DEV)
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    _cabi.call("lemoq_w8_gemm", _cabi.ptr(x), x.shape[0], _cabi.ptr(codes), _cabi.ptr(scale), n, k, 128, _cabi.ptr(seg),
+               codes.shape[0] if codes.dim() == 3 else 1, int(gate_up), int(exact), _cabi.ptr(resid), _cabi.ptr(y), _cabi.ptr(flag), _cabi.current_stream())
+    assert int(flag) == 0
+    return y
+
+
+# one token; either side of the 16-, 32-, 64- and 128-token tiles; rows that leave a tile of 256 half empty or spill over it; one
+# group of codes, and an odd number of them
+@pytest.mark.parametrize("tokens,n,k,exact", [(1, 2, 128, True), (16, 256, 128, True), (17, 130, 384, True), (33, 258, 256, True), (64, 514, 640, True),
+                                              (65, 256, 128, True), (65, 258, 384, False), (128, 128, 256, False), (129, 770, 128, False), (300, 256, 640, False)])
+def test_w8_gemm_edges(tokens, n, k, exact):
+    codes, scale = _w8(n, k, tokens + n)
+    x = torch.randn(tokens, k, generator=torch.Generator().manual_seed(k)).half()
+    resid = torch.randn(tokens, n, generator=torch.Generator().manual_seed(n)).half()
+    ref = ops.dense_w8_gemv(x, codes, scale, 128)
+    args = (x.to(DEV), codes.to(DEV), scale.to(DEV))
+    assert rel_err(_gemm(*args, exact=exact), ref) < PER_KERNEL_REL_TOL
+    assert rel_err(_gemm(*args, exact=exact, resid=resid.to(DEV)), ref.half() + resid) < PER_KERNEL_REL_TOL
+    gate, up = ref.float()[:, : n // 2], ref.float()[:, n // 2:]
+    assert rel_err(_gemm(*args, exact=exact, gate_up=True), gate * torch.sigmoid(gate) * up) < 2 * PER_KERNEL_REL_TOL
+
+
+@pytest.mark.parametrize("counts,exact", [((0, 1, 16, 17, 0), True), ((70, 0, 3), True), ((128, 129, 0, 257, 1), False)])
+def test_w8_gemm_segments(counts, exact):
+    n, k, rows = 258, 256, sum(counts)
+    codes, scale = _w8(n, k, rows, experts=len(counts))
+    x = torch.randn(rows + 3, k, generator=torch.Generator().manual_seed(rows)).half()
+    seg = torch.tensor([sum(counts[:e]) for e in range(len(counts) + 1)], dtype=torch.int32)
+    got = _gemm(x.to(DEV), codes.to(DEV), scale.to(DEV), seg=seg.to(DEV), exact=exact)
+    ref = torch.cat([ops.dense_w8_gemv(x[seg[e]: seg[e + 1]], codes[e], scale[e], 128) for e in range(len(counts)) if counts[e]])
+    assert rel_err(got[:rows], ref) < PER_KERNEL_REL_TOL
+    assert bool(got[rows:].isnan().all())  # rows of no expert are left alone
+
+
+# prompts shorter than a tile of 128 query rows, one row into the second tile and into the second block; hidden 256 .. 512, 8 and 128 experts
+@pytest.mark.parametrize("tokens,spec", [(2, dict(hidden=256, heads=2, experts=8, top_k=2, ffn=128)), (129, dict(hidden=256, heads=2, experts=8, top_k=2, ffn=128)),
+                                         (257, dict(hidden=512, heads=4, experts=128, top_k=16, ffn=256))])
+def test_prompt_matches_oracle(tokens, spec):
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+
+    spec = glue.OlmoeSpec(layers=2, head_dim=128, vocab=512, **spec)
+    wf = glue.random_float_weights(spec, seed=tokens, dtype=torch.float16, std=0.05, norm_weight_jitter=0.1)
+    # a dominant residual stream and a decisive router: no top-k choice hangs on the last bit of an fp16 sum
+    wf.embed.mul_(20.0)
+    for layer in wf.layers:
+        layer.router.mul_(5.0)
+    wq = glue.quantize_weights(wf)
+    model = lemoq_model_from_oracle(wf)
+    install_canonical(model, tokens, 4)
+    prompt = torch.tensor([[(11 * i * i + 3) % spec.vocab for i in range(tokens)]])
+    state = glue.new_state(spec, tokens + 4)
+    first = glue.prefill(wq, state, prompt[0])
+    session = StaticCacheDecodeSession(model, prompt.to(DEV), ctx=tokens, max_new_tokens=4, engine="ops")
+    assert "_lemoq_prompt_plan" in session.cache.__dict__ and int(session.cache._lemoq_prompt_plan["flags"]) == 0
+    for i, slot in enumerate(session.cache.layers):
+        assert rel_err(slot.keys[:, :, :tokens], state.keys[i][:, :, :tokens]) < 2e-2
+        assert rel_err(slot.values[:, :, :tokens], state.values[i][:, :, :tokens]) < 2e-2
+        assert not slot.keys[:, :, tokens:].any()
+    logits = session.prefill().logits
+    assert tuple(logits.shape) == (1, tokens, spec.vocab)
+    assert rel_err(logits[0, -1], first) < 2e-2
+    assert session.seed_token_id == int(first.float().argmax())
