@@ -306,6 +306,7 @@ static int launch_attn_d(const AttnParams& p, bool int8_kv, bool fused, const La
 }
 
 int launch_attn_decode(const AttnParams& p, bool int8_kv, bool fused, const LaunchCfg& lc) {
+    if (int8_kv && !fused && attn_i8_eligible(p)) return launch_attn_i8(p, lc);
     if (p.D == 128) return launch_attn_d<128>(p, int8_kv, fused, lc);
     if (p.D == 64) return launch_attn_d<64>(p, int8_kv, fused, lc);
     return set_error(LEMOQ_ERR_UNSUPPORTED, "head_dim %d: the attention kernel is built for 64 and 128", p.D);

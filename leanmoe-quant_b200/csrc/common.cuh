@@ -103,16 +103,29 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 }
 
 // ---- int8 / fp16 unpacking -----------------------------------------------------
+// 4 int8 codes to fp32, exactly: bytes with the sign flipped dropped into 0x64__ are 1024 + 128 + c in fp16; one subtraction
+// gives two codes, then they are widened.  (The int -> float conversion runs at a quarter of the rate: attention over 64 x 16
+// heads at 2048 int8 positions was bound by it.)
+__device__ __forceinline__ void codes4_f32(uint32_t w, float (&f)[4]) {
+    const uint32_t u = w ^ 0x80808080u, off = 0x64806480u;  // (1152, 1152)
+    const uint32_t lo = __byte_perm(u, 0x64646464u, 0x4140), hi = __byte_perm(u, 0x64646464u, 0x4342);
+    const float2 a = __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&lo), *reinterpret_cast<const __half2*>(&off)));
+    const float2 b = __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&hi), *reinterpret_cast<const __half2*>(&off)));
+    f[0] = a.x;
+    f[1] = a.y;
+    f[2] = b.x;
+    f[3] = b.y;
+}
 // Dot product of 16 int8 codes (one 128-bit word) with 16 fp32 activations.
 __device__ __forceinline__ float dot16_s8(const uint4& w, const float* x) {
     const uint32_t u[4] = {w.x, w.y, w.z, w.w};
     float a = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        a = fmaf(static_cast<float>(static_cast<int8_t>(u[i] & 0xffu)), x[4 * i + 0], a);
-        a = fmaf(static_cast<float>(static_cast<int8_t>((u[i] >> 8) & 0xffu)), x[4 * i + 1], a);
-        a = fmaf(static_cast<float>(static_cast<int8_t>((u[i] >> 16) & 0xffu)), x[4 * i + 2], a);
-        a = fmaf(static_cast<float>(static_cast<int8_t>(u[i] >> 24)), x[4 * i + 3], a);
+        float f[4];
+        codes4_f32(u[i], f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a = fmaf(f[j], x[4 * i + j], a);
     }
     return a;
 }
@@ -121,10 +134,10 @@ __device__ __forceinline__ void axpy16_s8(const uint4& w, float s, float* acc) {
     const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        acc[4 * i + 0] = fmaf(s, static_cast<float>(static_cast<int8_t>(u[i] & 0xffu)), acc[4 * i + 0]);
-        acc[4 * i + 1] = fmaf(s, static_cast<float>(static_cast<int8_t>((u[i] >> 8) & 0xffu)), acc[4 * i + 1]);
-        acc[4 * i + 2] = fmaf(s, static_cast<float>(static_cast<int8_t>((u[i] >> 16) & 0xffu)), acc[4 * i + 2]);
-        acc[4 * i + 3] = fmaf(s, static_cast<float>(static_cast<int8_t>(u[i] >> 24)), acc[4 * i + 3]);
+        float f[4];
+        codes4_f32(u[i], f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[4 * i + j] = fmaf(s, f[j], acc[4 * i + j]);
     }
 }
 // 8 fp16 values (one 128-bit word) to fp32.

@@ -147,6 +147,8 @@ struct AttnParams {
     int* err_flag = nullptr;
 };
 int launch_attn_decode(const AttnParams& p, bool int8_kv, bool fused, const LaunchCfg& lc);
+bool attn_i8_eligible(const AttnParams& p);  // tensor-core form (attn_i8.cu): int8 mirror, finished q, head_dim 128, heads back to back
+int launch_attn_i8(const AttnParams& p, const LaunchCfg& lc);
 
 // ---- small ops ---------------------------------------------------------------------
 int launch_rms_norm(const __half* x, const __half* w, __half* y, int64_t rows, int H, float eps, const LaunchCfg& lc);

@@ -30,6 +30,18 @@ __device__ __forceinline__ bool elect_one() {
     return r != 0;
 }
 
+// Power-of-two scale of a group of fp32 values and its inverse: |x| / scale < 2^20, so x is three 7-bit digits
+// d2 * 2^14 + d1 * 2^7 + d0 (fp16 values within 2^9 of the maximum are exact, the rest good to 2^-20 of it).
+__device__ __forceinline__ void digit_scale(float amax, float& sx, float& inv) {
+    const int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu);  // biased exponent
+    const int k = amax > 0.f && e > 20 ? e - 19 : 2;  // zero or denormal range: a fixed tiny scale keeps the arithmetic exact
+    sx = __uint_as_float(static_cast<uint32_t>(k) << 23);
+    inv = __uint_as_float(static_cast<uint32_t>(254 - k) << 23);
+}
+__device__ __forceinline__ int digit_round(float x, float inv) {  // round to nearest even, |x| * inv < 2^20
+    return static_cast<int>(__float_as_uint(fmaf(x, inv, 12582912.0f)) - 0x4B400000u);
+}
+
 // One arrival for the warp.
 __device__ __forceinline__ void warp_arrive(uint32_t bar) {
     __syncwarp();
@@ -80,7 +92,22 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d, uint64_t a, uint64_t b, u
                  : "memory");
 }
 
+// Instruction descriptor of kind::i8 with signed operands and int32 accumulators: M x N, B K-major, A K- or MN-major.  K = 32.
+__device__ __forceinline__ constexpr uint32_t idesc_i8(int m, int n, bool a_mn_major) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | (a_mn_major ? 1u << 15 : 0u) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+__device__ __forceinline__ void mma_i8_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a),
+                 "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u)
+                 : "memory");
+}
+// Shared-memory stores of this thread become visible to the tensor core (async proxy) once it has also arrived somewhere.
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 // Warp w of a warpgroup reads / writes lanes [32 w, 32 w + 32) of TMEM, one lane per thread, n consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_ld4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t addr) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -88,30 +115,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t addr) {
           "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(addr));
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t (&r)[32], uint32_t addr) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,"
-        "%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-          "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-          "=r"(r[31])
-        : "r"(addr));
-}
 __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
         "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
         "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,"
-        "%27,%28,%29,%30,%31,%32};" ::"r"(addr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
-        "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
 

@@ -1,0 +1,43 @@
+"""The tensor-core decode attention over the int8 mirror at the edges of its tiles of 128 positions, its splits and its persistent grid."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from gpu_util import PER_KERNEL_REL_TOL, rel_err
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# nothing filled; one position; either side of a tile; a last tile of one position in a split of its own; more heads than two blocks per SM
+@pytest.mark.parametrize("heads,capacity,filled,splits", [(3, 40, 0, 1), (3, 40, 0, 4), (2, 40, 1, 3), (2, 200, 127, 2), (2, 200, 128, 2), (2, 200, 129, 2),
+                                                          (5, 700, 641, 19), (5, 700, 700, 6), (300, 300, 259, 4), (700, 131, 131, 1)])
+def test_attn_i8_edges(heads, capacity, filled, splits):
+    from lemoq import _cabi
+
+    g = torch.Generator().manual_seed(heads + filled)
+    q = torch.randn(heads, 128, generator=g).half()
+    kc, vc = (torch.randint(-127, 128, (heads, capacity, 128), generator=g, dtype=torch.int8) for _ in range(2))
+    ks, vs = ((torch.rand(heads, capacity, generator=g) * 0.02 + 0.001).half() for _ in range(2))
+    ks[:, filled:] = float("nan")  # scales behind the filled length need not be numbers
+    vs[:, filled:] = float("nan")
+    q[0] = 0
+    dev = [t.to(DEV) for t in (q, kc, ks, vc, vs)]
+    out = torch.full((heads, 128), float("nan"), dtype=torch.float16, device=DEV)
+    ws = torch.zeros(int(_cabi.lib().lemoq_attn_workspace_bytes(heads, 128, splits)), dtype=torch.uint8, device=DEV)
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    length = torch.tensor([filled], dtype=torch.int32, device=DEV)
+    runs = []
+    for _ in range(2):  # the second launch finds the arrival counters as the first left them
+        _cabi.call("lemoq_attn_decode_int8", *(_cabi.ptr(t) for t in dev), capacity * 128, _cabi.ptr(length), _cabi.ptr(out), heads, capacity, 128, splits,
+                   128 ** -0.5, _cabi.ptr(ws), _cabi.ptr(flag), _cabi.current_stream())
+        runs.append(out.clone())
+    assert int(flag) == 0 and torch.equal(runs[0], runs[1])
+    if filled == 0:
+        assert not out.any()
+        return
+    k, v = (c[:, :filled].double() * s[:, :filled].double()[..., None] for c, s in ((kc, ks), (vc, vs)))
+    weights = torch.softmax(torch.einsum("hd,hsd->hs", q.double(), k) * 128 ** -0.5, dim=-1)
+    assert rel_err(out, torch.einsum("hs,hsd->hd", weights, v)) < PER_KERNEL_REL_TOL
