@@ -403,6 +403,19 @@ LEMOQ_API size_t lemoq_prompt_workspace_bytes(const lemoq_step_desc* desc, int T
 LEMOQ_API int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens,
                      const int64_t* positions, int T, void* logits, void* workspace, size_t workspace_bytes, int* err_flag, void* stream);
 
+/* One token of each of T sequences through the whole model, all at cache slot *position
+ * (lockstep batch decoding): row t's K and V are quantised into slot *position of its own
+ * int8 caches - layers[i].kc / .vc (T * heads, max_len, 128), .ks / .vs (T * heads, max_len) -
+ * and it attends to slots [0, *filled) of them; logits (T, vocab) fp16.  No counterpart in the
+ * reference, which is batch 1 (ref for the layer: src/lemoq/kernels/attn_decode.py:836).
+ * Shapes as above; the workspace is zeroed once by the caller and not shared by launches that
+ * overlap.  position, filled: device scalars, so a captured graph follows them.
+ */
+LEMOQ_API size_t lemoq_lockstep_workspace_bytes(const lemoq_step_desc* desc, int T);
+LEMOQ_API int lemoq_lockstep_run(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens,
+                       const int64_t* position, const int32_t* filled, int T, void* logits, void* workspace,
+                       size_t workspace_bytes, int* err_flag, void* stream);
+
 #define LEMOQ_FLAG_BAD_POSITION 1
 #define LEMOQ_FLAG_BAD_LENGTH 2
 #define LEMOQ_FLAG_BAD_EXPERT 4

@@ -294,6 +294,7 @@ class ExpertParallelDecoder:
     def __init__(self, model: Any, session: Any, *, sequences: int, world: int, rank: int, group: Any = None,
                  attn_splits: int = 4, static_exchange: bool = False, exchange_kernels: bool = True) -> None:
         from lemoq import _cabi
+        from lemoq.prompt import lockstep_plan
 
         if sequences % world != 0:
             raise ValueError("sequences=%d must divide evenly over %d ranks" % (sequences, world))
@@ -336,6 +337,8 @@ class ExpertParallelDecoder:
         self.pos_t = torch.zeros(1, dtype=torch.int64, device=self.device)
         self.filled_t = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.err = torch.zeros(1, dtype=torch.int32, device=self.device)
+        # on one rank nothing leaves the device: the whole step is one native call
+        self.native = lockstep_plan(model, self.kv, self.b, self.max_len) if world == 1 and static_exchange else None
         self.sections = None  # name -> list of (start, end) CUDA events while a timing split is being taken
 
     def _section(self, name: str) -> Any:
@@ -422,6 +425,10 @@ class ExpertParallelDecoder:
         self.graph = graph
 
     def _forward(self, tokens: Any) -> Any:
+        if self.native is not None and self.sections is None:
+            from lemoq.prompt import run_lockstep
+
+            return run_lockstep(self.native, tokens.contiguous(), self.pos_t, self.filled_t, self.cfg.vocab_size, self.err)
         from lemoq import _cabi
         from lemoq.kernels.batched_w8 import w8_linear_tokens
         from lemoq.kernels.dequant_gemv import dequant_gemm_fused

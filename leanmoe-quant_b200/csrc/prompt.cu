@@ -1,8 +1,12 @@
-// A whole prompt through the model: T tokens, all layers, logits of every row, the K/V rows left in the fp16 caches.
+// Many tokens through the whole model, all layers, logits of every row:
+//   lemoq_prompt_run    a prompt: T rows of one sequence, K/V rows left in its fp16 caches, causal attention over them
+//   lemoq_lockstep_run  one token of each of T sequences, all at the same slot: K/V rows quantised into each sequence's int8 caches,
+//                       decode attention over those
 //
 // Eleven kernels per layer, launched from here with programmatic dependent launch: the prompt of a short question is
 // bound by the 6.9 GB of weights all experts together have (1.1 ms), so a launch gap or a host call per expert is what it
-// must not pay; a long prompt is bound by the tensor cores (w8_gemm.cu, prompt_attn.cu).
+// must not pay; a long prompt is bound by the tensor cores (w8_gemm.cu, prompt_attn.cu); a lockstep step by the weights and its
+// sequences' caches (attn_i8.cu).
 #include <algorithm>
 
 #include "prompt.h"
@@ -63,14 +67,15 @@ int validate_prompt(const lemoq_step_desc& d) {
 
 using namespace lemoq;
 
-extern "C" size_t lemoq_prompt_workspace_bytes(const lemoq_step_desc* desc, int T) {
-    if (!desc || T <= 0 || validate_prompt(*desc) != LEMOQ_OK) return 0;
-    return carve_prompt(*desc, T, nullptr, nullptr);
-}
+namespace {
 
-extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens, const int64_t* positions, int T, void* logits,
-                                void* workspace, size_t workspace_bytes, int* err_flag, void* stream) {
-    LEMOQ_REQUIRE(desc && layers && tokens && positions && logits && workspace, LEMOQ_ERR_INVALID, "prompt: null pointer");
+constexpr int kLockstepSplits = 16;  // at most (two or three sequences: 32 heads and few SMs busy without splits)
+size_t attn_scratch_bytes(int heads) { return lemoq_attn_workspace_bytes(heads, 128, kLockstepSplits); }
+
+// `filled` == nullptr: a prompt, positions (T).  Otherwise a lockstep step, positions and filled are device scalars.
+int run_rows(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens, const int64_t* positions, const int32_t* filled, int T, void* logits,
+             void* workspace, size_t workspace_bytes, int* err_flag, void* stream) {
+    LEMOQ_REQUIRE(desc && layers && tokens && logits && workspace, LEMOQ_ERR_INVALID, "prompt: null pointer");
     const lemoq_step_desc& d = *desc;
     if (int rc = validate_prompt(d)) return rc;
     LEMOQ_REQUIRE(T > 0 && static_cast<int64_t>(T) * d.top_k <= (1 << 24), LEMOQ_ERR_INVALID, "prompt: T=%d out of range", T);
@@ -78,7 +83,8 @@ extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_d
                   "prompt: null pointer in descriptor");
     LEMOQ_REQUIRE(aligned16(logits) && aligned16(workspace), LEMOQ_ERR_INVALID, "prompt: logits and workspace must be 16-byte aligned");
     PromptBuffers b;
-    const size_t need = carve_prompt(d, T, static_cast<char*>(workspace), &b);
+    const bool lockstep = filled != nullptr;
+    const size_t rows_bytes = carve_prompt(d, T, static_cast<char*>(workspace), &b), need = rows_bytes + (lockstep ? attn_scratch_bytes(T * d.heads) : 0);
     LEMOQ_REQUIRE(workspace_bytes >= need, LEMOQ_ERR_INVALID, "prompt: workspace of %zu bytes, needs %zu", workspace_bytes, need);
 
     LaunchCfg lc;
@@ -91,7 +97,7 @@ extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_d
     auto gemm = [&](const __half* x, int rows, const int8_t* codes, const void* scale, int N, int K, const __half* resid, __half* y) {
         W8GemmParams g;
         g.x = x; g.T = rows; g.codes = codes; g.scale = half(scale); g.N = N; g.K = K; g.group_size = d.group_size;
-        g.resid = resid; g.y = y; g.exact = false; g.err_flag = err_flag;
+        g.resid = resid; g.y = y; g.exact = lockstep; g.err_flag = err_flag;
         return launch_w8_gemm(g, chained);
     };
 #define LEMOQ_TRY(call)            \
@@ -105,13 +111,30 @@ extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_d
         LEMOQ_TRY(gemm(b.h, T, L.qkv_codes, L.qkv_scale, 3 * A, d.hidden, nullptr, b.qkv));
         QkvRows r;
         r.qkv = b.qkv; r.q_norm = half(L.q_norm); r.k_norm = half(L.k_norm); r.rope_cos = half(d.rope_cos); r.rope_sin = half(d.rope_sin);
-        r.pos = positions; r.q = b.q; r.keys = reinterpret_cast<__half*>(L.keys); r.values = reinterpret_cast<__half*>(L.values);
+        r.pos = positions; r.q = b.q;
+        if (lockstep) {
+            r.kc = L.kc; r.vc = L.vc; r.ks = reinterpret_cast<__half*>(L.ks); r.vs = reinterpret_cast<__half*>(L.vs);
+        } else {
+            r.keys = reinterpret_cast<__half*>(L.keys); r.values = reinterpret_cast<__half*>(L.values);
+        }
         r.eps = d.eps; r.T = T; r.heads = d.heads; r.S = d.max_len; r.err_flag = err_flag;
         LEMOQ_TRY(launch_qkv_rows(r, chained));
-        PromptAttn a;
-        a.q = b.q; a.keys = half(L.keys); a.values = half(L.values); a.pos = positions; a.out = b.ctx;
-        a.T = T; a.heads = d.heads; a.S = d.max_len; a.scale = 1.0f / sqrtf(128.0f); a.err_flag = err_flag;
-        LEMOQ_TRY(launch_prompt_attn(a, chained));
+        if (lockstep) {
+            AttnParams a;
+            a.q = b.q; a.k = L.kc; a.v = L.vc; a.ks = r.ks; a.vs = r.vs; a.kv_head_stride = static_cast<int64_t>(d.max_len) * 128; a.filled = filled; a.out = b.ctx;
+            a.heads = T * d.heads; a.S = d.max_len; a.D = 128; a.num_splits = std::min(kLockstepSplits, (2 * sm_count() + a.heads - 1) / a.heads);
+            a.qk_scale_log2 = 1.4426950408889634f / sqrtf(128.0f); a.err_flag = err_flag;
+            char* scratch = static_cast<char*>(workspace) + rows_bytes;
+            a.counters = reinterpret_cast<unsigned int*>(scratch);
+            a.part = reinterpret_cast<float*>(scratch + up256(sizeof(unsigned int) * a.heads));
+            LEMOQ_REQUIRE(attn_i8_eligible(a), LEMOQ_ERR_UNSUPPORTED, "lockstep: %d sequences x %d heads x %d slots are too many", T, d.heads, d.max_len);
+            LEMOQ_TRY(launch_attn_i8(a, chained));
+        } else {
+            PromptAttn a;
+            a.q = b.q; a.keys = half(L.keys); a.values = half(L.values); a.pos = positions; a.out = b.ctx;
+            a.T = T; a.heads = d.heads; a.S = d.max_len; a.scale = 1.0f / sqrtf(128.0f); a.err_flag = err_flag;
+            LEMOQ_TRY(launch_prompt_attn(a, chained));
+        }
         LEMOQ_TRY(gemm(b.ctx, T, L.o_codes, L.o_scale, d.hidden, A, b.x, b.x1));
         LEMOQ_TRY(launch_combine_norm(nullptr, nullptr, nullptr, T, 0, b.x1, d.hidden, half(L.ln2), d.eps, nullptr, b.h, chained));
         LEMOQ_TRY(launch_route_rows(b.h, half(L.router), T, d.hidden, d.experts, d.top_k, d.norm_topk_prob, nullptr, b.top_w, b.top_i, chained));
@@ -119,7 +142,7 @@ extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_d
         LEMOQ_TRY(launch_gather_rows(b.h, b.pair_of, P, d.top_k, d.hidden, b.pairs, chained));
         W8GemmParams g;
         g.x = b.pairs; g.T = P; g.codes = L.gu_codes; g.scale = half(L.gu_scale); g.N = 2 * d.ffn; g.K = d.hidden; g.group_size = d.group_size;
-        g.seg = b.seg; g.E = d.experts; g.gate_up = true; g.y = b.act; g.exact = false; g.err_flag = err_flag;
+        g.seg = b.seg; g.E = d.experts; g.gate_up = true; g.y = b.act; g.exact = lockstep; g.err_flag = err_flag;
         LEMOQ_TRY(launch_w8_gemm(g, chained));
         g.x = b.act; g.codes = L.dn_codes; g.scale = half(L.dn_scale); g.N = d.hidden; g.K = d.ffn; g.gate_up = false; g.y = b.pairs;
         LEMOQ_TRY(launch_w8_gemm(g, chained));
@@ -129,4 +152,28 @@ extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_d
     LEMOQ_TRY(gemm(b.h, T, d.lm_head_codes, d.lm_head_scale, d.vocab, d.hidden, nullptr, reinterpret_cast<__half*>(logits)));
 #undef LEMOQ_TRY
     return LEMOQ_OK;
+}
+
+}  // namespace
+
+extern "C" size_t lemoq_prompt_workspace_bytes(const lemoq_step_desc* desc, int T) {
+    if (!desc || T <= 0 || validate_prompt(*desc) != LEMOQ_OK) return 0;
+    return carve_prompt(*desc, T, nullptr, nullptr);
+}
+
+extern "C" int lemoq_prompt_run(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens, const int64_t* positions, int T, void* logits,
+                                void* workspace, size_t workspace_bytes, int* err_flag, void* stream) {
+    LEMOQ_REQUIRE(positions, LEMOQ_ERR_INVALID, "prompt: null pointer");
+    return run_rows(desc, layers, tokens, positions, nullptr, T, logits, workspace, workspace_bytes, err_flag, stream);
+}
+
+extern "C" size_t lemoq_lockstep_workspace_bytes(const lemoq_step_desc* desc, int T) {
+    const size_t rows = lemoq_prompt_workspace_bytes(desc, T);
+    return rows ? rows + attn_scratch_bytes(T * desc->heads) : 0;
+}
+
+extern "C" int lemoq_lockstep_run(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const int64_t* tokens, const int64_t* position,
+                                  const int32_t* filled, int T, void* logits, void* workspace, size_t workspace_bytes, int* err_flag, void* stream) {
+    LEMOQ_REQUIRE(position && filled, LEMOQ_ERR_INVALID, "lockstep: null pointer");
+    return run_rows(desc, layers, tokens, position, filled, T, logits, workspace, workspace_bytes, err_flag, stream);
 }

@@ -15,9 +15,11 @@ struct QkvRows {
     const __half* qkv = nullptr;     // (T, 3A)
     const __half *q_norm = nullptr, *k_norm = nullptr;        // (A)
     const __half *rope_cos = nullptr, *rope_sin = nullptr;    // (S, 128)
-    const int64_t* pos = nullptr;    // (T) cache slot of each row
+    const int64_t* pos = nullptr;    // (T) cache slot of each row; with kc: one slot for all
     __half* q = nullptr;             // (T, A)
     __half *keys = nullptr, *values = nullptr;                // (heads, S, 128)
+    int8_t *kc = nullptr, *vc = nullptr;                      // instead of keys / values: (T * heads, S, 128) codes ...
+    __half *ks = nullptr, *vs = nullptr;                      // ... and (T * heads, S) scales
     float eps = 0.f;
     int T = 0, heads = 0, S = 0;
     int* err_flag = nullptr;

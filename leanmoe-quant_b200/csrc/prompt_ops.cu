@@ -95,8 +95,28 @@ __global__ void __launch_bounds__(kRowThreads) combine_norm_kernel(const __half*
     norm_row_store(f, H, w, eps, h + t * H, red);
 }
 
-// One block per token, A = heads * 128 <= 4096.  qkv (T, 3A) -> q (T, A) normalised and rotated; the k and v rows go into
-// slot pos[t] of the fp16 caches (heads, S, 128).
+// Per-token symmetric int8 of a head's 128 values, eight in each of 16 neighbouring lanes (fp32 amax, true division, half to even; the
+// scale is stored as fp16).
+__device__ __forceinline__ void quantise_head_store(const __half* x, int8_t* codes, __half* scale, bool first_lane) {
+    float f[8], amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        f[j] = __half2float(x[j]);
+        amax = fmaxf(amax, fabsf(f[j]));
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(threadIdx.x & 16 ? 0xffff0000u : 0x0000ffffu, amax, o, 16));
+    const float s = amax > 0.f ? __fdiv_rn(amax, 127.0f) : 1.0f;
+    __align__(8) int8_t c[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c[j] = static_cast<int8_t>(static_cast<int>(fminf(fmaxf(rintf(__fdiv_rn(f[j], s)), -127.0f), 127.0f)));
+    *reinterpret_cast<uint2*>(codes) = *reinterpret_cast<const uint2*>(c);
+    if (first_lane) *scale = __float2half_rn(s);
+}
+
+// One block per token, A = heads * 128 <= 4096.  qkv (T, 3A) -> q (T, A) normalised and rotated.  The k and v rows go into slot pos[t] of
+// the fp16 caches (heads, S, 128), or (INT8, lockstep decoding) quantised into slot *pos of the row's own caches (T * heads, S, 128).
+template <bool INT8>
 __global__ void __launch_bounds__(kRowThreads) qkv_rows_kernel(const QkvRows p) {
     __shared__ float red[40];
     __shared__ __align__(16) __half row[2][kRowThreads * 8 * kRowVecs];
@@ -104,7 +124,7 @@ __global__ void __launch_bounds__(kRowThreads) qkv_rows_kernel(const QkvRows p) 
     pdl_trigger();
     const int64_t t = blockIdx.x;
     const int A = p.heads * 128, tid = threadIdx.x;
-    int64_t pos = p.pos[t];
+    int64_t pos = p.pos[INT8 ? 0 : t];
     if (pos < 0 || pos >= p.S) {
         if (p.err_flag && tid == 0) atomicOr(p.err_flag, LEMOQ_FLAG_BAD_POSITION);
         pos = pos < 0 ? 0 : p.S - 1;
@@ -150,7 +170,7 @@ __global__ void __launch_bounds__(kRowThreads) qkv_rows_kernel(const QkvRows p) 
             float c[8], s[8];
             unpack8_h(__ldg(reinterpret_cast<const uint4*>(cos + d)), c);
             unpack8_h(__ldg(reinterpret_cast<const uint4*>(sin + d)), s);
-            const int64_t slot = (static_cast<int64_t>(i >> 7) * p.S + pos) * 128 + d;
+            const int64_t row_at = (INT8 ? t * p.heads + (i >> 7) : static_cast<int64_t>(i >> 7)) * p.S + pos, slot = row_at * 128 + d;
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 float a[8], b[8];
@@ -159,10 +179,18 @@ __global__ void __launch_bounds__(kRowThreads) qkv_rows_kernel(const QkvRows p) 
                 __align__(16) __half o[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) o[j] = __float2half_rn(__fadd_rn(__fmul_rn(a[j], c[j]), __fmul_rn(sign * b[j], s[j])));
-                __half* dst = m ? p.keys + slot : p.q + t * A + i;
-                *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
+                if (INT8 && m) {
+                    quantise_head_store(o, p.kc + slot, p.ks + row_at, d == 0);
+                } else {
+                    __half* dst = m ? p.keys + slot : p.q + t * A + i;
+                    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
+                }
             }
-            *reinterpret_cast<uint4*>(p.values + slot) = ld_cg16(src + 2 * A + i);
+            const uint4 v4 = ld_cg16(src + 2 * A + i);
+            if (INT8)
+                quantise_head_store(reinterpret_cast<const __half*>(&v4), p.vc + slot, p.vs + row_at, d == 0);
+            else
+                *reinterpret_cast<uint4*>(p.values + slot) = v4;
         }
     }
 }
@@ -349,7 +377,10 @@ int launch_combine_norm(const __half* y, const int32_t* place, const float* top_
     return launch_kernel(combine_norm_kernel, dim3(T), dim3(kRowThreads), 0, lc, y, place, top_w, K, x1, H, w, eps, x2, h);
 }
 
-int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc) { return launch_kernel(qkv_rows_kernel, dim3(p.T), dim3(kRowThreads), 0, lc, p); }
+int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc) {
+    return p.kc ? launch_kernel(qkv_rows_kernel<true>, dim3(p.T), dim3(kRowThreads), 0, lc, p)
+                : launch_kernel(qkv_rows_kernel<false>, dim3(p.T), dim3(kRowThreads), 0, lc, p);
+}
 
 int launch_route_rows(const __half* h, const __half* router, int T, int H, int E, int top_k, int norm, __half* logits, float* top_w, int32_t* top_i,
                       const LaunchCfg& lc) {

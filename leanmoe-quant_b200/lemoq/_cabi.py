@@ -98,6 +98,8 @@ _SIGNATURES = {
     "lemoq_step_phase_stamps": (c_void_p, [c_void_p]),
     "lemoq_prompt_workspace_bytes": (c_size_t, [POINTER(StepDesc), c_int]),
     "lemoq_prompt_run": (c_int, [POINTER(StepDesc), POINTER(LayerDesc), c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "lemoq_lockstep_workspace_bytes": (c_size_t, [POINTER(StepDesc), c_int]),
+    "lemoq_lockstep_run": (c_int, [POINTER(StepDesc), POINTER(LayerDesc), c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "lemoq_step_engine": (ctypes.c_char_p, [c_void_p]),
 }
 

@@ -1,6 +1,8 @@
-"""A prompt through the whole model in one native call (``lemoq_prompt_run``), for models in the canonical W8 form.
+"""Many tokens through the whole model in one native call, for models in the canonical W8 form: a prompt (``lemoq_prompt_run``), or one
+token of each of many sequences (``lemoq_lockstep_run``).
 
-The module tree's own forward stays the path of everything else; :func:`run_prompt` returns None for a call it does not take.
+The module tree's own forward stays the path of everything else; :func:`run_prompt` and :func:`lockstep_plan` return None for
+what the native path does not take.
 """
 
 from __future__ import annotations
@@ -46,34 +48,41 @@ def _signature(model: Any) -> tuple | None:
     return (lm, model.model.embed_tokens.weight, *parts)
 
 
-def _make_plan(model: Any, cache: Any, signature: tuple) -> dict:
+def _describe(model: Any, signature: tuple, max_len: int, caches: list[dict]) -> dict:
+    """The model and one set of cache tensors per layer (named as in ``LayerDesc``) for the C side: pointers only."""
     cfg, m = model.config, model.model
     device = m.embed_tokens.weight.device
-    heads, dim = cfg.num_attention_heads, cfg.head_dim
-    cos, sin = m.rotary_emb.tables(cache.max_cache_len, torch.float16, device)
+    cos, sin = m.rotary_emb.tables(max_len, torch.float16, device)
     layers = (_cabi.LayerDesc * len(m.layers))()
     keep: list[Any] = [cos, sin]
-    for d, layer, (attn, mlp, packed, o_proj, stacks), slot in zip(layers, m.layers, signature[2:], cache.layers):
-        if not slot.is_initialized:
-            slot.lazy_initialization(torch.empty((1, heads, 1, dim), dtype=torch.float16, device=device))
+    for d, layer, (attn, mlp, packed, o_proj, stacks), slots in zip(layers, m.layers, signature[2:], caches):
         router = mlp._static_router.contiguous()
-        keep.append(router)
+        keep += [router, slots]
         tensors = {"ln1": layer.input_layernorm.weight, "ln2": layer.post_attention_layernorm.weight, "q_norm": attn.q_norm.weight,
                    "k_norm": attn.k_norm.weight, "qkv_codes": packed.packed, "qkv_scale": packed.scale, "o_codes": o_proj.packed,
                    "o_scale": o_proj.scale, "router": router, "gu_codes": stacks.packed_gate_up, "gu_scale": stacks.scale_gate_up,
-                   "dn_codes": stacks.packed_down, "dn_scale": stacks.scale_down, "keys": slot.keys, "values": slot.values}
+                   "dn_codes": stacks.packed_down, "dn_scale": stacks.scale_down, **slots}
         for name, t in tensors.items():
             setattr(d, name, _cabi.ptr(t))
     desc = _cabi.StepDesc()
-    desc.layers, desc.hidden, desc.heads, desc.head_dim = len(m.layers), cfg.hidden_size, heads, dim
+    desc.layers, desc.hidden, desc.heads, desc.head_dim = len(m.layers), cfg.hidden_size, cfg.num_attention_heads, cfg.head_dim
     desc.experts, desc.top_k, desc.ffn, desc.vocab = cfg.num_experts, cfg.num_experts_per_tok, cfg.intermediate_size, cfg.vocab_size
-    desc.group_size, desc.max_len, desc.eps = int(model.lm_head.group_size), cache.max_cache_len, float(cfg.rms_norm_eps)
+    desc.group_size, desc.max_len, desc.eps = int(model.lm_head.group_size), max_len, float(cfg.rms_norm_eps)
     desc.norm_topk_prob = int(bool(cfg.norm_topk_prob))
     desc.embed, desc.final_norm = _cabi.ptr(m.embed_tokens.weight), _cabi.ptr(m.norm.weight)
     desc.lm_head_codes, desc.lm_head_scale = _cabi.ptr(model.lm_head.packed), _cabi.ptr(model.lm_head.scale)
     desc.rope_cos, desc.rope_sin = _cabi.ptr(cos), _cabi.ptr(sin)
-    return {"signature": signature, "caches": tuple(s.keys for s in cache.layers), "desc": desc, "layers": layers, "keep": keep,
-            "flags": torch.zeros(1, dtype=torch.int32, device=device)}
+    return {"signature": signature, "desc": desc, "layers": layers, "keep": keep}
+
+
+def _prompt_plan(model: Any, cache: Any, signature: tuple) -> dict:
+    cfg, device = model.config, model.model.embed_tokens.weight.device
+    for slot in cache.layers:
+        if not slot.is_initialized:
+            slot.lazy_initialization(torch.empty((1, cfg.num_attention_heads, 1, cfg.head_dim), dtype=torch.float16, device=device))
+    plan = _describe(model, signature, cache.max_cache_len, [{"keys": s.keys, "values": s.values} for s in cache.layers])
+    plan.update(caches=tuple(s.keys for s in cache.layers), flags=torch.zeros(1, dtype=torch.int32, device=device))
+    return plan
 
 
 def _same(a: tuple, b: tuple) -> bool:
@@ -96,7 +105,7 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
         return None
     plan = cache.__dict__.get(_PLAN)
     if plan is None or not _same(plan["signature"], signature) or any(s.keys is not k for s, k in zip(cache.layers, plan["caches"])):
-        plan = cache.__dict__[_PLAN] = _make_plan(model, cache, signature)
+        plan = cache.__dict__[_PLAN] = _prompt_plan(model, cache, signature)
     tokens = int(input_ids.shape[1])
     size = int(_cabi.lib().lemoq_prompt_workspace_bytes(plan["desc"], tokens))
     if size == 0:
@@ -106,4 +115,27 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     _cabi.call("lemoq_prompt_run", plan["desc"], plan["layers"], _cabi.ptr(ids), _cabi.ptr(cache_position), tokens, _cabi.ptr(logits),
                _cabi.ptr(workspace), size, _cabi.ptr(plan["flags"]), _cabi.current_stream(device))
+    return logits
+
+
+def lockstep_plan(model: Any, kv: list[dict], sequences: int, max_len: int) -> Any:
+    """What :func:`run_lockstep` needs for ``sequences`` sequences with the int8 caches ``kv`` (per layer ``kc/vc (B*heads, S, D)``,
+    ``ks/vs (B*heads, S)``), or None when the model is not in the canonical form."""
+    signature = _signature(model) if _cabi.available() and model.model.embed_tokens.weight.dtype == torch.float16 else None
+    if signature is None:
+        return None
+    plan = _describe(model, signature, max_len, kv)
+    size = int(_cabi.lib().lemoq_lockstep_workspace_bytes(plan["desc"], sequences))
+    if size == 0:
+        return None
+    plan["workspace"] = torch.zeros(size, dtype=torch.uint8, device=model.model.embed_tokens.weight.device)
+    return plan
+
+
+def run_lockstep(plan: dict, tokens: Any, position: Any, filled: Any, vocab: int, flags: Any) -> Any:
+    """Logits ``(B, V)`` of one token per sequence; ``position`` and ``filled`` are device scalars."""
+    rows, workspace = int(tokens.shape[0]), plan["workspace"]
+    logits = torch.empty((rows, vocab), dtype=torch.float16, device=tokens.device)
+    _cabi.call("lemoq_lockstep_run", plan["desc"], plan["layers"], _cabi.ptr(tokens), _cabi.ptr(position), _cabi.ptr(filled), rows, _cabi.ptr(logits),
+               _cabi.ptr(workspace), workspace.numel(), _cabi.ptr(flags), _cabi.current_stream(tokens.device))
     return logits

@@ -87,3 +87,34 @@ def test_prompt_matches_oracle(tokens, spec):
     assert tuple(logits.shape) == (1, tokens, spec.vocab)
     assert rel_err(logits[0, -1], first) < 2e-2
     assert session.seed_token_id == int(first.float().argmax())
+
+
+# one sequence; more sequences than a tile of tokens takes exactly; more heads than SMs
+@pytest.mark.parametrize("sequences", [1, 5, 67])
+def test_lockstep_matches_the_step_by_parts(sequences):
+    """The native lockstep step against the same step written with the per-operator kernels."""
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+    from benchmarks.expert_parallel import ExpertParallelDecoder
+
+    spec = glue.OlmoeSpec(layers=2, hidden=512, heads=4, head_dim=128, experts=16, top_k=4, ffn=256, vocab=512)
+    wf = glue.random_float_weights(spec, seed=sequences, dtype=torch.float16, std=0.05, norm_weight_jitter=0.1)
+    wf.embed.mul_(20.0)
+    for layer in wf.layers:
+        layer.router.mul_(5.0)
+    model = lemoq_model_from_oracle(wf)
+    ctx = 140
+    install_canonical(model, ctx, 8)
+    prompt = torch.tensor([[(7 * i * i + 1) % spec.vocab for i in range(ctx)]], device=DEV)
+    session = StaticCacheDecodeSession(model, prompt, ctx=ctx, max_new_tokens=8, engine="ops")
+    decoders = [ExpertParallelDecoder(model, session, sequences=sequences, world=1, rank=0, static_exchange=True) for _ in range(2)]
+    assert decoders[0].native is not None
+    decoders[1].native = None
+    tokens = (torch.arange(sequences, device=DEV) * 37 + 5) % spec.vocab
+    with torch.no_grad():
+        for _ in range(3):
+            got, ref = (d.step(tokens) for d in decoders)
+            assert rel_err(got, ref) < 1e-2
+            tokens = ref.float().argmax(dim=-1)
+    for a, b in zip(decoders[0].kv, decoders[1].kv):
+        assert float((a["kc"] != b["kc"]).float().mean()) < 1e-2 and rel_err(a["vs"], b["vs"]) < 1e-2
+    assert decoders[0].error_flags() == 0
