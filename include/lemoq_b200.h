@@ -280,6 +280,17 @@ LEMOQ_API int lemoq_moe_grouped_w8(const void* x, const int8_t* gu_codes, const 
                          const void* dn_scale, const int64_t* ids, const void* top_w, int T, int K, int E, int H,
                          int F, int group_size, void* act, void* out, int* err_flag, void* stream);
 
+/* The same layer for several tokens: every expert that is needed streams its weights once for
+ * all of its tokens (pairs sorted by expert, tensor-core GEMM).  out[t] as above; act is internal.
+ * ref: src/lemoq/kernels/moe_grouped_quant.py:411 applied to T tokens.
+ * H, F multiples of 128, group_size a multiple of 128.  workspace:
+ * lemoq_moe_tokens_workspace_bytes(T, K, E, H, F) bytes, need not be cleared.
+ */
+LEMOQ_API size_t lemoq_moe_tokens_workspace_bytes(int T, int K, int E, int H, int F);
+LEMOQ_API int lemoq_moe_tokens_w8(const void* x, const int8_t* gu_codes, const void* gu_scale, const int8_t* dn_codes,
+                        const void* dn_scale, const int64_t* ids, const void* top_w, int T, int K, int E, int H, int F,
+                        int group_size, void* out, void* workspace, size_t workspace_bytes, int* err_flag, void* stream);
+
 /* The two launches of lemoq_moe_grouped_w8 on their own (same arguments; gate_up reads x and
  * writes act, down reads act and writes out).
  * ref: src/lemoq/kernels/_grouped_triton.py:249 (_gate_up_act_kernel_q) and

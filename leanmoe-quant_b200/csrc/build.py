@@ -1,9 +1,9 @@
-"""Build liblemoq_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Build liblemoq_b200.so (the C-ABI library) in-tree with nvcc for sm_100a, and the Python binding of its short operators.
 
     python leanmoe-quant_b200/csrc/build.py [--verbose]
 
 The library has no dependency on torch or Python: it links against the CUDA runtime
-only.  Objects are rebuilt when a source or header is newer than the object.
+only.  ``lemoq/_bind.so`` (bind.cpp, g++) links against the library, torch and Python.  Objects are rebuilt when a source or header is newer than the object.
 """
 
 from __future__ import annotations
@@ -28,6 +28,31 @@ FLAGS = [
 
 def _newer(src: str, dst: str) -> bool:
     return not os.path.exists(dst) or os.path.getmtime(src) > os.path.getmtime(dst)
+
+
+BIND_SOURCE, BIND = os.path.join(HERE, "bind.cpp"), os.path.join(os.path.dirname(HERE), "lemoq", "_bind.so")
+
+
+def build_bind(verbose: bool = False) -> str:
+    """The binding for the running interpreter and its torch; it finds the library next to it (rpath)."""
+    import sysconfig
+
+    import torch
+
+    if not any(_newer(src, BIND) for src in (BIND_SOURCE, HEADERS[-1], __file__)):
+        return BIND
+    root = os.path.dirname(torch.__file__)
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+               os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), *("-isystem" + d for d in include), BIND_SOURCE, "-o", BIND, LIB,
+           "-Wl,-rpath,$ORIGIN/../csrc", "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for %s" % BIND_SOURCE)
+    return BIND
 
 
 def build(verbose: bool = False) -> str:
@@ -55,11 +80,12 @@ def build(verbose: bool = False) -> str:
             if r.returncode != 0:
                 raise RuntimeError("nvcc failed for %s" % cmd[-3])
     if jobs or not os.path.exists(LIB):
-        cmd = [NVCC, "-shared", "-o", LIB, *objs, "-cudart", "static"]
+        cmd = [NVCC, "-shared", "-o", LIB, *objs, "-cudart", "static", "-Xlinker", "-soname=liblemoq_b200.so"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_bind(verbose)
     return LIB
 
 

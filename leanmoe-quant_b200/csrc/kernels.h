@@ -108,6 +108,7 @@ struct W8GemmParams {
     const __half* scale = nullptr;   // (E, N, K / group_size)
     const int32_t* seg = nullptr;    // (E + 1) token offsets on the device, or null: one segment [0, T)
     const __half* resid = nullptr;   // optional (T, N): y = fp16(acc) + resid
+    float* y32 = nullptr;            // exact form without gate_up and resid: (T, N) in fp32 instead of y
     __half* y = nullptr;             // (T, N); gate/up: (T, N / 2) = silu(row n) * row N / 2 + n
     int T = 0, N = 0, K = 0, group_size = 128, E = 1;
     bool gate_up = false;

@@ -138,8 +138,7 @@ int run_rows(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const 
         LEMOQ_TRY(gemm(b.ctx, T, L.o_codes, L.o_scale, d.hidden, A, b.x, b.x1));
         LEMOQ_TRY(launch_combine_norm(nullptr, nullptr, nullptr, T, 0, b.x1, d.hidden, half(L.ln2), d.eps, nullptr, b.h, chained));
         LEMOQ_TRY(launch_route_rows(b.h, half(L.router), T, d.hidden, d.experts, d.top_k, d.norm_topk_prob, nullptr, b.top_w, b.top_i, chained));
-        LEMOQ_TRY(launch_pair_plan(b.top_i, P, d.experts, b.place, b.pair_of, b.seg, chained));
-        LEMOQ_TRY(launch_gather_rows(b.h, b.pair_of, P, d.top_k, d.hidden, b.pairs, chained));
+        LEMOQ_TRY(launch_pairs(b.top_i, P, d.experts, b.h, d.top_k, d.hidden, b.place, b.pair_of, b.seg, b.pairs, nullptr, chained));
         W8GemmParams g;
         g.x = b.pairs; g.T = P; g.codes = L.gu_codes; g.scale = half(L.gu_scale); g.N = 2 * d.ffn; g.K = d.hidden; g.group_size = d.group_size;
         g.seg = b.seg; g.E = d.experts; g.gate_up = true; g.y = b.act; g.exact = lockstep; g.err_flag = err_flag;
@@ -150,11 +149,70 @@ int run_rows(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const 
                                       half(i + 1 < d.layers ? layers[i + 1].ln1 : d.final_norm), d.eps, b.x, b.h, chained));
     }
     LEMOQ_TRY(gemm(b.h, T, d.lm_head_codes, d.lm_head_scale, d.vocab, d.hidden, nullptr, reinterpret_cast<__half*>(logits)));
-#undef LEMOQ_TRY
     return LEMOQ_OK;
 }
 
+struct MoeBuffers {
+    __half *x, *act;
+    float* y;
+    int32_t *place, *pair_of, *seg;
+};
+
+size_t carve_moe(int T, int K, int E, int H, int F, char* base, MoeBuffers* b) {
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char* at = base + off;
+        off += up256(bytes);
+        return at;
+    };
+    const size_t P = static_cast<size_t>(T) * K;
+    MoeBuffers o;
+    o.x = reinterpret_cast<__half*>(take(2 * P * H));
+    o.act = reinterpret_cast<__half*>(take(2 * P * F));
+    o.y = reinterpret_cast<float*>(take(4 * P * H));
+    o.place = reinterpret_cast<int32_t*>(take(4 * P));
+    o.pair_of = reinterpret_cast<int32_t*>(take(4 * P));
+    o.seg = reinterpret_cast<int32_t*>(take(4 * (static_cast<size_t>(E) + 1)));
+    if (b) *b = o;
+    return off;
+}
+
 }  // namespace
+
+extern "C" size_t lemoq_moe_tokens_workspace_bytes(int T, int K, int E, int H, int F) {
+    if (T <= 0 || K <= 0 || E <= 0 || H <= 0 || F <= 0) return 0;
+    return carve_moe(T, K, E, H, F, nullptr, nullptr);
+}
+
+extern "C" int lemoq_moe_tokens_w8(const void* x, const int8_t* gu_codes, const void* gu_scale, const int8_t* dn_codes, const void* dn_scale, const int64_t* ids,
+                                   const void* top_w, int T, int K, int E, int H, int F, int group_size, void* out, void* workspace, size_t workspace_bytes,
+                                   int* err_flag, void* stream) {
+    LEMOQ_REQUIRE(T >= 0 && K > 0 && E > 0 && H > 0 && F > 0, LEMOQ_ERR_INVALID, "moe_tokens_w8: bad shape");
+    LEMOQ_REQUIRE(static_cast<int64_t>(T) * K <= (1 << 24) && E <= kMaxExperts, LEMOQ_ERR_UNSUPPORTED, "moe_tokens_w8: T=%d x K=%d pairs or E=%d experts above the limit", T, K, E);
+    LEMOQ_REQUIRE(H % 128 == 0 && F % 128 == 0, LEMOQ_ERR_UNSUPPORTED, "moe_tokens_w8: hidden and ffn must be multiples of 128");
+    LEMOQ_REQUIRE(group_size > 0 && group_size % 128 == 0 && H % group_size == 0 && F % group_size == 0, LEMOQ_ERR_UNSUPPORTED,
+                  "moe_tokens_w8: group_size=%d must be a multiple of 128 that divides hidden and ffn", group_size);
+    if (T == 0) return LEMOQ_OK;
+    LEMOQ_REQUIRE(x && gu_codes && gu_scale && dn_codes && dn_scale && ids && top_w && out && workspace, LEMOQ_ERR_INVALID, "moe_tokens_w8: null pointer");
+    LEMOQ_REQUIRE(aligned16(x) && aligned16(gu_codes) && aligned16(dn_codes) && aligned16(out) && aligned16(workspace), LEMOQ_ERR_INVALID,
+                  "moe_tokens_w8: pointers must be 16-byte aligned");
+    MoeBuffers b;
+    const size_t need = carve_moe(T, K, E, H, F, static_cast<char*>(workspace), &b);
+    LEMOQ_REQUIRE(workspace_bytes >= need, LEMOQ_ERR_INVALID, "moe_tokens_w8: workspace of %zu bytes, needs %zu", workspace_bytes, need);
+    LaunchCfg lc;
+    lc.stream = static_cast<cudaStream_t>(stream);
+    LaunchCfg chained = lc;
+    chained.pdl = true;
+    LEMOQ_TRY(launch_pairs(ids, T * K, E, reinterpret_cast<const __half*>(x), K, H, b.place, b.pair_of, b.seg, b.x, err_flag, lc));
+    W8GemmParams g;
+    g.x = b.x; g.T = T * K; g.codes = gu_codes; g.scale = reinterpret_cast<const __half*>(gu_scale); g.N = 2 * F; g.K = H; g.group_size = group_size;
+    g.seg = b.seg; g.E = E; g.gate_up = true; g.y = b.act; g.err_flag = err_flag;
+    LEMOQ_TRY(launch_w8_gemm(g, chained));
+    g.x = b.act; g.codes = dn_codes; g.scale = reinterpret_cast<const __half*>(dn_scale); g.N = H; g.K = F; g.gate_up = false; g.y = nullptr; g.y32 = b.y;
+    LEMOQ_TRY(launch_w8_gemm(g, chained));
+    return launch_weighted_sum(b.y, b.place, reinterpret_cast<const __half*>(top_w), T, K, H, reinterpret_cast<__half*>(out), chained);
+}
+#undef LEMOQ_TRY
 
 extern "C" size_t lemoq_prompt_workspace_bytes(const lemoq_step_desc* desc, int T) {
     if (!desc || T <= 0 || validate_prompt(*desc) != LEMOQ_OK) return 0;

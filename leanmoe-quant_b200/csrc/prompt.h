@@ -29,9 +29,13 @@ int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc);
 // logits (T, E) fp16 = h . router^T, softmax + top-k of every row.  E a multiple of 16, <= 128; H a multiple of 64.
 int launch_route_rows(const __half* h, const __half* router, int T, int H, int E, int top_k, int norm, __half* logits, float* top_w, int32_t* top_i,
                       const LaunchCfg& lc);
-// Stable sort of the P = T * K pairs by expert: place[p] = row of pair p in expert order, pair_of[row] = p, seg[e] = first row of e.
-int launch_pair_plan(const int32_t* top_i, int P, int E, int32_t* place, int32_t* pair_of, int32_t* seg, const LaunchCfg& lc);
-int launch_gather_rows(const __half* h, const int32_t* pair_of, int P, int K, int H, __half* x_sorted, const LaunchCfg& lc);
+// Stable sort of the P = T * K pairs by expert: place[p] = row of pair p in expert order, pair_of[row] = p, seg[e] = first row of e,
+// x_sorted[row] = h[pair_of[row] / K].  Ids outside [0, E) are clamped and flagged.
+int launch_pairs(const int32_t* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,
+                 const LaunchCfg& lc);
+int launch_pairs(const int64_t* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,
+                 const LaunchCfg& lc);
+int launch_weighted_sum(const float* y, const int32_t* place, const __half* top_w, int T, int K, int H, __half* out, const LaunchCfg& lc);
 
 struct PromptAttn {
     const __half* q = nullptr;       // (T, heads * 128)

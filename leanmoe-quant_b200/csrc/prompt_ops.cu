@@ -6,7 +6,7 @@
 //   qkv_rows       q/k RMSNorm over the projection width, RoPE, rows into the caches one block per token
 //   route_rows     router logits (fp16 mma), softmax, top-k                         one block per 16 tokens
 //   pair_plan      stable counting sort of the (token, slot) pairs by expert         one block per expert
-//   gather_rows    activations into expert order                                    one block per pair
+//   gather_rows    activations into expert order (few pairs: done by pair_plan)     one block per pair
 //   combine_norm   routing-weighted sum in slot order (fp32) + residual, next norm   one block per token
 #include "prompt.h"
 #include "stream.cuh"
@@ -314,15 +314,28 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_rows_kernel(const __ha
 // ---- pairs into expert order ----------------------------------------------------------------------------------------------
 constexpr int kPlanThreads = 512;
 
-// One block per expert: counts the pairs of lower experts, then gives its own pairs their rows in pair order.
-__global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const int32_t* __restrict__ top_i, int P, int E, int32_t* __restrict__ place,
-                                                                 int32_t* __restrict__ pair_of, int32_t* __restrict__ seg) {
+template <typename ID>
+__device__ __forceinline__ int expert_of(const ID* __restrict__ ids, int p, int E, int* err) {
+    const ID e = ids[p];
+    if (e >= 0 && e < E) return static_cast<int>(e);
+    if (err) atomicOr(err, LEMOQ_FLAG_BAD_EXPERT);
+    return e < 0 ? 0 : E - 1;
+}
+
+// One block per expert: counts the pairs of lower experts, then gives its own pairs their rows in pair order.  GATHER: it also copies
+// the activations of its pairs (up to kGatherPairs of them in all: a launch less; with more pairs a block per row is faster).
+constexpr int kGatherPairs = 1024;
+template <typename ID, bool GATHER>
+__global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const ID* __restrict__ top_i, int P, int E, int32_t* __restrict__ place,
+                                                                 int32_t* __restrict__ pair_of, int32_t* __restrict__ seg, const __half* __restrict__ h, int K, int H,
+                                                                 __half* __restrict__ x_sorted, int* err) {
     __shared__ int s_warp[kPlanThreads / 32 + 1];
+    __shared__ int s_mine[GATHER ? kGatherPairs : 1];
     const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     pdl_wait();
     pdl_trigger();
     int below = 0;
-    for (int p = threadIdx.x; p < P; p += kPlanThreads) below += top_i[p] < e;
+    for (int p = threadIdx.x; p < P; p += kPlanThreads) below += expert_of(top_i, p, E, e == 0 ? err : nullptr) < e;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
     if (lane == 0) s_warp[warp] = below;
@@ -332,9 +345,10 @@ __global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const int32_t* 
     for (int w = 0; w < kPlanThreads / 32; ++w) base += s_warp[w];
     __syncthreads();
     if (threadIdx.x == 0) seg[e] = base;
+    const int row0 = base;
     for (int p0 = 0; p0 < P; p0 += kPlanThreads) {
         const int p = p0 + threadIdx.x;
-        const bool hit = p < P && top_i[p] == e;
+        const bool hit = p < P && expert_of<ID>(top_i, p, E, nullptr) == e;
         const unsigned m = __ballot_sync(0xffffffffu, hit);
         if (lane == 0) s_warp[warp] = __popc(m);
         __syncthreads();
@@ -349,11 +363,42 @@ __global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const int32_t* 
             const int row = base + before + __popc(m & ((1u << lane) - 1u));
             place[p] = row;
             pair_of[row] = p;
+            if (GATHER) s_mine[row - row0] = p;
         }
         base += all;
         __syncthreads();
     }
     if (e == E - 1 && threadIdx.x == 0) seg[E] = base;
+    if (GATHER) {
+        const int vecs = H / 8;
+        for (int u = threadIdx.x; u < (base - row0) * vecs; u += kPlanThreads) {
+            const int r = u / vecs, i = 8 * (u - r * vecs);
+            *reinterpret_cast<uint4*>(x_sorted + static_cast<int64_t>(row0 + r) * H + i) = ld_cg16(h + static_cast<int64_t>(s_mine[r] / K) * H + i);
+        }
+    }
+}
+
+// out[t] = fp16(sum_k w[t, k] * y[place[t, k]]), products and sums in slot order in fp32, y not rounded before.
+__global__ void __launch_bounds__(kRowThreads) weighted_sum_kernel(const float* __restrict__ y, const int32_t* __restrict__ place, const __half* __restrict__ top_w, int K,
+                                                                   int H, __half* __restrict__ out) {
+    pdl_wait();
+    pdl_trigger();
+    const int64_t t = blockIdx.x;
+    for (int i = 4 * (threadIdx.x + kRowThreads * blockIdx.y); i < H; i += 4 * kRowThreads * gridDim.y) {
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < K; ++k) {
+            const float w = __half2float(__ldg(top_w + t * K + k));
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(y + static_cast<int64_t>(__ldg(place + t * K + k)) * H + i));
+            a[0] = fmaf(w, v.x, a[0]);
+            a[1] = fmaf(w, v.y, a[1]);
+            a[2] = fmaf(w, v.z, a[2]);
+            a[3] = fmaf(w, v.w, a[3]);
+        }
+        __align__(8) __half o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = __float2half_rn(a[j]);
+        *reinterpret_cast<uint2*>(out + t * H + i) = *reinterpret_cast<const uint2*>(o);
+    }
 }
 
 __global__ void __launch_bounds__(kRowThreads) gather_rows_kernel(const __half* __restrict__ h, const int32_t* __restrict__ pair_of, int K, int H,
@@ -392,12 +437,27 @@ int launch_route_rows(const __half* h, const __half* router, int T, int H, int E
     return launch_kernel(route_rows_kernel<16>, grid, block, smem, lc, h, router, T, H, E, top_k, norm, logits, top_w, top_i);
 }
 
-int launch_pair_plan(const int32_t* top_i, int P, int E, int32_t* place, int32_t* pair_of, int32_t* seg, const LaunchCfg& lc) {
-    return launch_kernel(pair_plan_kernel, dim3(E), dim3(kPlanThreads), 0, lc, top_i, P, E, place, pair_of, seg);
+template <typename ID>
+static int plan_and_gather(const ID* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,
+                           const LaunchCfg& lc) {
+    if (P <= kGatherPairs)
+        return launch_kernel(pair_plan_kernel<ID, true>, dim3(E), dim3(kPlanThreads), 0, lc, ids, P, E, place, pair_of, seg, h, K, H, x_sorted, err);
+    if (int rc = launch_kernel(pair_plan_kernel<ID, false>, dim3(E), dim3(kPlanThreads), 0, lc, ids, P, E, place, pair_of, seg, h, K, H, x_sorted, err)) return rc;
+    return launch_kernel(gather_rows_kernel, dim3(P), dim3(kRowThreads), 0, lc, h, pair_of, K, H, x_sorted);
 }
 
-int launch_gather_rows(const __half* h, const int32_t* pair_of, int P, int K, int H, __half* x_sorted, const LaunchCfg& lc) {
-    return launch_kernel(gather_rows_kernel, dim3(P), dim3(kRowThreads), 0, lc, h, pair_of, K, H, x_sorted);
+int launch_pairs(const int32_t* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,
+                 const LaunchCfg& lc) {
+    return plan_and_gather(ids, P, E, h, K, H, place, pair_of, seg, x_sorted, err, lc);
+}
+
+int launch_pairs(const int64_t* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,
+                 const LaunchCfg& lc) {
+    return plan_and_gather(ids, P, E, h, K, H, place, pair_of, seg, x_sorted, err, lc);
+}
+
+int launch_weighted_sum(const float* y, const int32_t* place, const __half* top_w, int T, int K, int H, __half* out, const LaunchCfg& lc) {
+    return launch_kernel(weighted_sum_kernel, dim3(T, (H / 4 + kRowThreads - 1) / kRowThreads), dim3(kRowThreads), 0, lc, y, place, top_w, K, H, out);
 }
 
 }  // namespace lemoq

@@ -85,6 +85,7 @@ struct GemmShape {
     const __half* scale;   // (E, N, K / group)
     const __half* resid;   // (T, N) or null
     __half* y;             // (T, N), or (T, N / 2) in gate/up mode
+    float* y32;            // or: (T, N) in fp32
     int* err_flag;
 };
 
@@ -434,10 +435,15 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 warp_arrive(d_free(dl));
             } else if (live) {
                 __half* y = p.y + static_cast<int64_t>(t.t0) * p.N + mrow;
+                float* y32 = p.y32 + static_cast<int64_t>(t.t0) * p.N + mrow;
                 const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * p.N + mrow : nullptr;
 #pragma unroll
                 for (int j = 0; j < NT; ++j) {
                     if (j < t.n) {
+                        if (p.y32) {
+                            y32[static_cast<int64_t>(j) * p.N] = acc[j];
+                            continue;
+                        }
                         __half v = __float2half_rn(acc[j]);
                         if (res) v = __hadd(v, res[static_cast<int64_t>(j) * p.N]);
                         y[static_cast<int64_t>(j) * p.N] = v;
@@ -475,7 +481,7 @@ int launch_nt(const GemmShape& p, const __half* x, const int8_t* codes, const La
 int launch_w8_gemm(const W8GemmParams& g, const LaunchCfg& lc) {
     GemmShape p;
     p.T = g.T; p.N = g.N; p.K = g.K; p.group = g.group_size; p.E = g.E; p.gate_up = g.gate_up ? 1 : 0;
-    p.seg = g.seg; p.scale = g.scale; p.resid = g.resid; p.y = g.y; p.err_flag = g.err_flag;
+    p.seg = g.seg; p.scale = g.scale; p.resid = g.resid; p.y = g.y; p.y32 = g.y32; p.err_flag = g.err_flag;
     // NT bounds the tokens of a tile, the MMA's N follows the real count: a small NT only saves registers and stage bytes, a
     // large one saves widening the same codes again for a second token tile.  Twice the mean per expert covers nearly all.
     const int64_t want = g.seg ? 2 * ((static_cast<int64_t>(g.T) + g.E - 1) / g.E) : g.T;

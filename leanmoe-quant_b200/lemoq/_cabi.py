@@ -82,6 +82,9 @@ _SIGNATURES = {
                             c_void_p]),
     "lemoq_moe_grouped_w8": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                      c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "lemoq_moe_tokens_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "lemoq_moe_tokens_w8": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                                    c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "lemoq_moe_gate_up_w8": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                      c_void_p, c_void_p, c_void_p]),
     "lemoq_moe_down_w8": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,

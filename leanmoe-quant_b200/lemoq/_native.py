@@ -1,0 +1,16 @@
+"""The native call path of the short operators (``csrc/bind.cpp``): ``attention``, ``linear``, ``experts``.  Each returns None for a call it
+does not take; the callers then go their Python way, which raises the error or serves the call.  Without the built module they always do."""
+
+from __future__ import annotations
+
+try:
+    import torch  # noqa: F401  (the module links against torch's libraries)
+
+    from lemoq._bind import attention, experts, linear
+except ImportError:  # not built: same results through ctypes
+    def _absent(*args: object) -> None:
+        return None
+
+    attention = experts = linear = _absent
+
+__all__ = ["attention", "experts", "linear"]

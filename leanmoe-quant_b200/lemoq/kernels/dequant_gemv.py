@@ -11,7 +11,7 @@ from typing import Any
 
 import torch
 
-from lemoq import _cabi
+from lemoq import _cabi, _native
 
 __all__ = ["DEQUANT_GEMM_CONFIGS", "dequant_gemm_fused", "fused_available", "unavailable_reason", "warm"]
 
@@ -42,6 +42,10 @@ def dequant_gemm_fused(x: Any, qweight: Any, scale: Any, zero: Any = None, *, gr
 
     ``out_dtype=None`` returns fp32 like the reference.  All tensors must be contiguous.
     """
+    if out_dtype is torch.float16 and symmetric and zero is None and not mxfp4 and bits in (None, 8) and x.dim() == 2:
+        y = _native.linear(x, qweight, scale, group_size, True)
+        if y is not None:
+            return y
     if x.dim() != 2:
         raise ValueError("x 必须是 (M, K) 二维，得到 %r" % (tuple(x.shape),))
     if qweight.dim() != 2:

@@ -12,7 +12,7 @@ from typing import Any
 
 import torch
 
-from lemoq import _cabi
+from lemoq import _cabi, _native
 from lemoq.kernels.moe_grouped import _MAX_OFFSET, PARITY_GATE, launch_plan, merged_config  # noqa: F401
 
 __all__ = ["QuantFusedExperts", "dequantize_fused_experts", "grouped_moe_forward_quant", "quant_launch_plan",
@@ -146,6 +146,10 @@ def quant_launch_plan(q: QuantFusedExperts, *, top_k: int, config: dict[str, Any
 def grouped_moe_forward_quant(x: Any, q: QuantFusedExperts, ids: Any, top_w: Any, *,
                               config: dict[str, Any] | None = None, backend: str = "auto") -> Any:
     """``(H,)`` hidden state + ``(K,)`` expert ids + ``(K,)`` routing weights -> ``(H,)`` fp16."""
+    if config is None and backend in ("auto", "cuda", "triton") and x.dim() == 1 and q.bits == 8:
+        out = _native.experts(x, q.packed_gate_up, q.scale_gate_up, q.packed_down, q.scale_down, ids, top_w, q.group_size)
+        if out is not None:
+            return out
     if backend == "oracle":
         raise RuntimeError("backend='oracle' is not part of this package (the CPU oracle is test infrastructure)")
     if backend not in ("auto", "cuda", "triton"):
@@ -183,8 +187,11 @@ def grouped_moe_forward_quant(x: Any, q: QuantFusedExperts, ids: Any, top_w: Any
 
 
 def grouped_moe_forward_quant_tokens(x: Any, q: QuantFusedExperts, ids: Any, top_w: Any) -> Any:
-    """Batched form for the grouped-GEMV microbenchmark: ``x (T, H)``, ``ids/top_w (T, K)`` ->
-    ``(T, H)``.  Each token is an independent one-token problem."""
+    """Batched form: ``x (T, H)``, ``ids/top_w (T, K)`` -> ``(T, H)``.  Several tokens go through the tensor-core experts, which stream an
+    expert's weights once for all of its tokens; shapes those do not take, as T independent one-token problems."""
+    out = _native.experts(x, q.packed_gate_up, q.scale_gate_up, q.packed_down, q.scale_down, ids, top_w, q.group_size) if x.dim() == 2 else None
+    if out is not None:
+        return out
     t, hidden = int(x.shape[0]), int(x.shape[1])
     k = int(ids.shape[1])
     dt = q.scale_gate_up.dtype

@@ -1,0 +1,54 @@
+"""The native call path of the short operators: same results as the path it shortcuts, at the token counts where the kernel changes."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+from torch import nn
+
+from gpu_util import PER_KERNEL_REL_TOL, rel_err
+from oracle import lemoq_oracle as ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# one expert for all tokens and experts without any; the sort's own gather (up to 1024 pairs) and the separate one behind it; ids out of range
+@pytest.mark.parametrize("tokens,top_k,experts", [(1, 2, 4), (2, 1, 3), (5, 3, 7), (17, 8, 16), (130, 8, 16)])
+def test_experts_for_several_tokens(tokens, top_k, experts):
+    from lemoq.kernels.moe_grouped_quant import QuantFusedExperts, grouped_moe_forward_quant, grouped_moe_forward_quant_tokens
+
+    hidden, ffn = 256, 384
+    g = torch.Generator().manual_seed(tokens)
+    gu, dn = (ops.rtn_quantize_w8(torch.randn(experts, *s, generator=g) * 0.05, 128) for s in ((2 * ffn, hidden), (hidden, ffn)))
+    q = ops.QuantExperts(*gu, *dn, 128)
+    x = torch.randn(tokens, hidden, generator=g).half()
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)])
+    ids[0] = ids[0, 0]
+    weights = torch.rand(tokens, top_k, generator=g).half()
+    ref = torch.stack([ops.grouped_moe_w8(x[t], q, ids[t], weights[t])[0] for t in range(tokens)])
+    ids[0] = torch.where(ids[0] == experts - 1, experts + 5, ids[0])  # clamped back to the last expert
+    own = QuantFusedExperts(*(t.to(DEV) for t in (*gu, *dn)), 8, 128)
+    args = x.to(DEV), own, ids.to(DEV), weights.to(DEV)
+    got = grouped_moe_forward_quant_tokens(*args) if tokens > 1 else grouped_moe_forward_quant(args[0][0], own, args[2][0], args[3][0])
+    assert rel_err(got, ref) < PER_KERNEL_REL_TOL
+
+
+@pytest.mark.parametrize("mode", ["fused", "separate"])
+@pytest.mark.parametrize("shape", [(256,), (1, 1, 256), (1, 3, 256), (70, 256)])
+def test_quant_linear_native_and_fallback_agree(mode, shape):
+    from lemoq.quant.linear import QuantLinear, SchemeSpec
+
+    torch.manual_seed(len(shape))
+    dense = nn.Linear(256, 130, bias=True, device=DEV, dtype=torch.float16)
+    linear = QuantLinear(dense, SchemeSpec.from_flags("w8a16", 128, dequant=mode))
+    x = torch.randn(*shape, device=DEV).half()
+    with torch.no_grad():
+        got = linear(x)
+        ref = torch.nn.functional.linear(x, linear.dequantized_weight(dtype=torch.float16), linear.bias)
+        strided = linear(torch.cat([x, x], dim=-1)[..., :256])  # not contiguous: the Python way
+    assert got.shape == ref.shape and rel_err(got, ref) < PER_KERNEL_REL_TOL and rel_err(strided, ref) < PER_KERNEL_REL_TOL
+    single = x.numel() == 256
+    assert linear._counters["fused_calls"] == (2 if single and mode == "fused" else 0)
+    assert linear._counters["separate_calls"] == (0 if single and mode == "fused" else 2)
+    assert linear._counters["fallbacks"] == ({"multi_token": 2} if mode == "fused" and not single else {})
