@@ -15,6 +15,7 @@ constexpr int kMaxTopK = 64;
 struct LaunchCfg {
     cudaStream_t stream = nullptr;
     bool pdl = false;        // attach the programmatic-stream-serialization attribute
+    int cluster = 1;         // blocks of a thread-block cluster along x
     int* launch_count = nullptr;
 };
 
@@ -26,12 +27,17 @@ int launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, 
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = lc.stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
     if (lc.pdl) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (lc.cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = static_cast<unsigned>(lc.cluster);
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
     }
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(err));

@@ -65,7 +65,7 @@ constexpr int kExactTokens = 64, kScaledTokens = 128;  // most tokens of a tile
 constexpr int kRegsCollect = 144, kRegsWiden = 56, kRegsIssue = 72;
 constexpr int kTileRows = 256;      // weight rows of a tile (two M tiles of 128)
 constexpr int kCodeBytes = 2 * 128 * 128;
-constexpr int kSegCap = kMaxExperts + 1;
+constexpr int kScaleStride = 36;    // bytes of a row's group scales in shared memory: 16 of them and a pad against bank conflicts
 constexpr uint32_t kColA = 256;     // first TMEM column of the widened codes
 
 template <int NT>
@@ -76,7 +76,7 @@ struct Shape {
     static constexpr bool kScaled = NT > kExactTokens;
     static constexpr int kDBufs = kScaled ? 1 : 2;                      // accumulator buffers per M tile
     static constexpr int kStages = NT >= 128 ? 3 : (NT == 64 ? 4 : 5);
-    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + 1024;
+    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + 1024;  // + 8 (E + 1) bytes of tile table
 };
 
 struct GemmShape {
@@ -87,6 +87,8 @@ struct GemmShape {
     __half* y;             // (T, N), or (T, N / 2) in gate/up mode
     float* y32;            // or: (T, N) in fp32
     int* err_flag;
+    int parts;             // SPLIT: blocks of a cluster that share a tile's groups
+    int scale_vecs;        // 16-byte vectors of a row's scales when they fit the shared rows (1 or 2), else 0
 };
 
 struct Tile {
@@ -97,7 +99,8 @@ struct Tile {
 // Tiles before expert e: first[e].  A tile number -> expert by binary search, then (M tile pair, token tile): neighbours in
 // the order share their weight rows and meet in L2.  The tokens of an expert are split evenly.
 template <int NT>
-__device__ __forceinline__ Tile tile_at(int i, const int* first, const int* tok, const GemmShape& p, int mt) {
+__device__ __forceinline__ Tile tile_at(int i, const int* first, const int* tok, const GemmShape& p) {
+    if (i >= first[p.E]) return Tile{0, 0, 0, 0, 0};
     int lo = 0, hi = p.E;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -130,19 +133,65 @@ __device__ __forceinline__ void widen16(const uint4& w, __half scale, uint32_t* 
     }
 }
 
-template <int NT>
+// The group scales of one weight row: the thread of the row asks for those of its next tile a tile ahead (a load takes up to three
+// groups under load), keeps them in registers until the tile is done and then leaves them in its own row of shared memory.
+struct RowScales {
+    uint4 ahead[2];
+    const __half* row;
+    uint32_t at;
+    __device__ __forceinline__ void ask(const GemmShape& p, const Tile& t, int wrow) {
+        row = p.scale + (static_cast<int64_t>(t.e) * p.N + min(wrow, p.N - 1)) * (p.K / p.group);
+        if (p.scale_vecs > 0) ahead[0] = __ldg(reinterpret_cast<const uint4*>(row));
+        if (p.scale_vecs > 1) ahead[1] = __ldg(reinterpret_cast<const uint4*>(row) + 1);
+    }
+    __device__ __forceinline__ void keep(const GemmShape& p) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            if (v < p.scale_vecs) {
+                const uint32_t u[4] = {ahead[v].x, ahead[v].y, ahead[v].z, ahead[v].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + 16u * v + 4u * i), "r"(u[i]) : "memory");
+            }
+        }
+    }
+    // `mine`: the row this tile works on (the one asked for last belongs to the next tile)
+    __device__ __forceinline__ __half get(const GemmShape& p, const __half* mine, int g) const {
+        const int k = p.group == 128 ? g : (g << 7) / p.group;
+        if (p.scale_vecs == 0) return __ldg(mine + k);
+        unsigned short h;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(at + 2u * k));
+        return __ushort_as_half(h);
+    }
+};
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_peer(uint32_t addr, int rank) {
+    uint32_t there;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(there) : "memory");
+    return v;
+}
+
+// SPLIT (exact form, dense, fewer tiles than SMs): the blocks of a cluster take a part of the groups each, one tile per cluster; every
+// block leaves its sums in its own shared memory and finishes a part of the tokens from those of all, in rank order.
+template <int NT, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                               const GemmShape p) {
     using S = Shape<NT>;
     constexpr int kStages = S::kStages;
     extern __shared__ uint8_t raw[];
     __shared__ __align__(8) uint64_t s_bar[2 * kStages + 7];
-    __shared__ int s_first[kSegCap], s_tok[kSegCap];
+    __shared__ __align__(16) uint8_t s_scale[kTileRows * kScaleStride];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage0 = (smem_u32(raw) + 1023u) & ~1023u;
+    int* s_first = reinterpret_cast<int*>(raw + (stage0 - smem_u32(raw)) + static_cast<size_t>(kStages) * S::kStage);
+    int* s_tok = s_first + p.E + 1;
     const uint32_t bars = smem_u32(s_bar);
     auto full = [&](int s) { return bars + 8u * s; };
     auto done = [&](int s) { return bars + 8u * (kStages + s); };
@@ -172,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
         tma_prefetch_map(&map_w);
         tma_prefetch_map(&map_x);
     }
-    pdl_wait();  // the segments and the tokens come from earlier kernels
+    if (p.seg) pdl_wait();  // segments and tokens come from earlier kernels; without segments only the token loads wait
     pdl_trigger();
     const int mt = p.gate_up ? (p.N / 2 + 127) / 128 : (p.N + kTileRows - 1) / kTileRows;
     if (warp == 0) {  // tokens and tiles before each expert
@@ -204,31 +253,48 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
     const uint32_t tmem = s_tmem;
     const int tiles = s_first[p.E], groups = p.K >> 7;
     volatile int* abort = &s_abort;
+    // this block's tiles and, of each, its groups
+    const int rank = SPLIT ? blockIdx.x % p.parts : 0, tile0 = SPLIT ? blockIdx.x / p.parts : blockIdx.x, stride = SPLIT ? tiles : gridDim.x;
+    const int g0 = SPLIT ? rank * groups / p.parts : 0, g1 = SPLIT ? (rank + 1) * groups / p.parts : groups;
+    auto tile = [&](int i) { return tile_at<NT>(i, s_first, s_tok, p); };
 
     if (warp >= 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
     if (warp == 16) {
         // ---- TMA: one thread ---------------------------------------------------------------------------------------
         if (elect_one()) {
-            int s = 0, issued = 0;
+            int s = 0, issued = 0, early = 0;
             uint32_t ph = 1;
             bool ok = true;
-            for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
-                const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
-                const int boxes = (t.n + S::kBox - 1) / S::kBox, base = t.e * p.N;
-                const uint32_t bytes = kCodeBytes + 2u * boxes * S::kBox * 128u;
-                for (int g = 0; g < groups; ++g) {
-                    if (!(ok = thread_wait(done(s), ph, abort))) break;
-                    const uint32_t at = stage0 + static_cast<uint32_t>(s) * S::kStage, bar = full(s);
-                    mbar_expect_tx(bar, bytes);
-                    tma_load_2d(at, &map_w, g * 128, base + t.row0, bar);
-                    tma_load_2d(at + kCodeBytes / 2, &map_w, g * 128, base + t.row1, bar);
-                    for (int b = 0; b < boxes; ++b) {
-                        tma_load_2d(at + kCodeBytes + b * S::kBox * 128, &map_x, g * 128, t.t0 + b * S::kBox, bar);
-                        tma_load_2d(at + kCodeBytes + S::kHalf + b * S::kBox * 128, &map_x, g * 128 + 64, t.t0 + b * S::kBox, bar);
+            Tile t = tile(tile0);
+            auto stage_at = [&](int k) { return stage0 + static_cast<uint32_t>(k) * S::kStage; };
+            auto bytes_of = [&](const Tile& x) { return kCodeBytes + 2u * ((x.n + S::kBox - 1) / S::kBox) * S::kBox * 128u; };
+            auto load_codes = [&](const Tile& x, int g, int k) {
+                mbar_expect_tx(full(k), bytes_of(x));
+                tma_load_2d(stage_at(k), &map_w, g * 128, x.e * p.N + x.row0, full(k));
+                tma_load_2d(stage_at(k) + kCodeBytes / 2, &map_w, g * 128, x.e * p.N + x.row1, full(k));
+            };
+            if (!p.seg) {  // the codes of the first stages do not depend on earlier kernels: on their way while those finish
+                if (tile0 < tiles)
+                    for (; early < min(kStages, g1 - g0); ++early) load_codes(t, g0 + early, early);
+                pdl_wait();
+            }
+            for (int i = tile0; i < tiles && ok; i += stride) {
+                Tile next = t;
+                for (int g = g0; g < g1; ++g) {
+                    if (issued >= early) {
+                        if (!(ok = thread_wait(done(s), ph, abort))) break;
+                        load_codes(t, g, s);
+                    }
+                    const uint32_t at = stage_at(s) + kCodeBytes;
+                    for (int b = 0; b * S::kBox < t.n; ++b) {
+                        tma_load_2d(at + b * S::kBox * 128, &map_x, g * 128, t.t0 + b * S::kBox, full(s));
+                        tma_load_2d(at + S::kHalf + b * S::kBox * 128, &map_x, g * 128 + 64, t.t0 + b * S::kBox, full(s));
                     }
                     ++issued;
                     if (++s == kStages) { s = 0; ph ^= 1; }
+                    if (g == g0) next = tile(i + stride);
                 }
+                t = next;
             }
             if (!ok) {  // gave up: the copies in flight still land in this block's shared memory
                 for (int j = max(0, issued - kStages); j < issued; ++j) mbar_wait(full(j % kStages), (j / kStages) & 1);
@@ -239,12 +305,12 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
         if (elect_one()) {
             int s = 0, it = 0, dn = 0;  // dn counts the accumulations: one per group (exact) or per tile (scaled)
             bool ok = true;
-            for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
-                const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
+            Tile t = tile(tile0);
+            for (int i = tile0; i < tiles && ok; i += stride) {
                 const uint32_t idesc = idesc_f16(128, max(16, (t.n + 15) & ~15), false);
-                for (int g = 0; g < groups; ++g, ++it) {
+                for (int g = g0; g < g1; ++g, ++it) {
                     const int b = it & 1, db = kD == 2 ? dn & 1 : 0;
-                    const bool begins = !kScaled || g == 0, ends = !kScaled || g + 1 == groups;
+                    const bool begins = !kScaled || g == g0, ends = !kScaled || g + 1 == g1;
                     // a widening warp has seen the stage's copies land before it arrives: no wait on full(s) here
                     if (!(ok = thread_wait(a_full(b), (it >> 1) & 1, abort))) break;
                     if (begins && !(ok = thread_wait(d_free(db), ((kD == 2 ? dn >> 1 : dn) & 1) ^ 1, abort))) break;
@@ -261,6 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                     if (kScaled && ends) tc_commit(d_full);  // (a parity wait cannot look past the next phase of done(s))
                     if (ends) ++dn;
                     if (++s == kStages) s = 0;
+                    if (g + 1 == g1) t = tile(i + stride);
                 }
             }
             if (!ok) {  // gave up: nothing may still write TMEM when it is freed
@@ -274,24 +341,21 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
         const int w = (warp >> 2) & 1, row = tid & 127;
         const uint32_t to0 = tmem + (static_cast<uint32_t>(warp & 3) << 21) + kColA + 128u * w;
         const uint32_t from0 = stage0 + w * (kCodeBytes / 2) + row * 128u, swz = row & 7;
-        const int gk = p.K / p.group;
         int s = 0, it = 0, s2 = kStages - 2;       // s2, ph2: stage and phase of group it - 2, the last user of this A buffer
         uint32_t ph = 0, ph2 = 1;
         bool ok = true;
-        for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
-            const __half* sc = nullptr;
-            __half next = __half(), scale = __half();
-            if (kScaled) {
-                const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
-                sc = p.scale + (static_cast<int64_t>(t.e) * p.N + min((w ? t.row1 : t.row0) + row, p.N - 1)) * gk;
-                next = __ldg(sc);
-            }
-            for (int g = 0; g < groups; ++g, ++it) {
+        RowScales sc;
+        sc.at = smem_u32(s_scale) + (w * 128 + row) * kScaleStride;
+        if (kScaled && tile0 < tiles) {
+            const Tile t = tile(tile0);
+            sc.ask(p, t, (w ? t.row1 : t.row0) + row);
+        }
+        for (int i = tile0; i < tiles && ok; i += stride) {
+            const __half* mine = sc.row;
+            if (kScaled) sc.keep(p);
+            for (int g = g0; g < g1; ++g, ++it) {
                 const int b = it & 1;
-                if (kScaled) {
-                    scale = next;
-                    if (g + 1 < groups) next = __ldg(sc + ((g + 1) << 7) / p.group);
-                }
+                const __half scale = kScaled ? sc.get(p, mine, g) : __half();
                 if (!(ok = warp_wait(full(s), ph, abort) && warp_wait(done(s2), ph2, abort))) break;
                 tc_fence_after();
                 const uint32_t from = from0 + static_cast<uint32_t>(s) * S::kStage, to = to0 + 64u * b;
@@ -307,28 +371,37 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 warp_arrive(a_full(b));
                 if (++s == kStages) { s = 0; ph ^= 1; }
                 if (++s2 == kStages) { s2 = 0; ph2 ^= 1; }
+                if (kScaled && g == g0 && i + stride < tiles) {
+                    const Tile t = tile(i + stride);
+                    sc.ask(p, t, (w ? t.row1 : t.row0) + row);
+                }
             }
         }
     } else if (warp < 8) {
         // ---- collect: thread = weight row --------------------------------------------------------------------------
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCollect));
+        pdl_wait();  // the residual is an earlier kernel's, and y may still be read by one
         const int w = warp >> 2, row = tid & 127;
         const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;  // TMEM lane field
-        const int half_rows = p.N / 2, gk = p.K / p.group;
+        const int half_rows = p.N / 2;
         int it = 0, round = 0, s = 0;
         uint32_t ph = 0;
         bool ok = true;
-        for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x, ++round) {
-            const Tile t = tile_at<NT>(i, s_first, s_tok, p, mt);
+        Tile t = tile(tile0);
+        RowScales sc;
+        sc.at = smem_u32(s_scale) + (w * 128 + row) * kScaleStride;
+        if (!kScaled && tile0 < tiles) sc.ask(p, t, (w ? t.row1 : t.row0) + row);
+        for (int i = tile0; i < tiles && ok; i += stride, ++round) {
             const int lim = p.gate_up ? half_rows : p.N;                 // rows of this tile's kind
             const int mrow = (p.gate_up ? t.row0 : (w ? t.row1 : t.row0)) + row;  // gate/up: both tiles count gate rows
-            const int wrow = (w ? t.row1 : t.row0) + row;
             const bool live = mrow < lim;
+            Tile next = t;
             if constexpr (kScaled) {
                 // the sums are complete: take them out of TMEM as fp16, hand the columns back, then store
                 constexpr int H = NT / 2;
                 const bool gu = p.gate_up;
                 const int j0 = gu ? w * H : 0, nj = max(0, min(t.n - j0, gu ? H : NT));  // this warpgroup's tokens
+                next = tile(i + stride);
                 if (!(ok = warp_wait(d_full, round & 1, abort))) break;
                 tc_fence_after();
                 __half2 out[H];
@@ -369,89 +442,120 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                     }
                 }
             } else {
-            const __half* sc = p.scale + (static_cast<int64_t>(t.e) * p.N + min(wrow, p.N - 1)) * gk;
-            float acc[NT];
+                float acc[NT];
 #pragma unroll
-            for (int j = 0; j < NT; ++j) acc[j] = 0.f;
+                for (int j = 0; j < NT; ++j) acc[j] = 0.f;
+                const __half* mine = sc.row;
+                sc.keep(p);
+                for (int g = g0; g < g1; ++g, ++it) {
+                    const int db = it & 1;
+                    const float scale = __half2float(sc.get(p, mine, g));
+                    if (!(ok = warp_wait(done(s), ph, abort))) break;
+                    tc_fence_after();
+                    const uint32_t d = tmem + lanes + 128u * w + 64u * db;
+#pragma unroll
+                    for (int c = 0; c < NT; c += 16) {
+                        if (c < t.n) {
+                            uint32_t r[16];
+                            tmem_ld16(r, d + c);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(scale, __uint_as_float(r[j]), acc[c + j]);
+                        }
+                    }
+                    tc_fence_before();
+                    // gate/up: the last sums' columns carry the exchange below and are freed after it
+                    if (!p.gate_up || g + 1 < g1) warp_arrive(d_free(db));
+                    if (++s == kStages) { s = 0; ph ^= 1; }
+                    if (g == g0) {
+                        next = tile(i + stride);
+                        if (i + stride < tiles) sc.ask(p, next, (w ? next.row1 : next.row0) + row);
+                    }
+                }
+                if (!ok) break;
+                const int dl = (it - 1) & 1;  // buffer of the last group
 
-            float scale = __half2float(__ldg(sc));
-            for (int g = 0; g < groups; ++g, ++it) {
-                const int db = it & 1;
-                const float next = g + 1 < groups ? __half2float(__ldg(sc + ((g + 1) << 7) / p.group)) : 0.f;
-                if (!(ok = warp_wait(done(s), ph, abort))) break;
-                tc_fence_after();
-                const uint32_t d = tmem + lanes + 128u * w + 64u * db;
+                if (SPLIT) {
+                    // every group of this block has been read: the stages are free for its sums, [token][row]
+                    const uint32_t at = stage0 + 4u * (w * 128 + row);
 #pragma unroll
-                for (int c = 0; c < NT; c += 16) {
-                    if (c < t.n) {
-                        uint32_t r[16];
-                        tmem_ld16(r, d + c);
-                        tmem_wait_ld();
+                    for (int j = 0; j < NT; ++j)
+                        if (j < t.n) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 4u * kTileRows * j), "f"(acc[j]) : "memory");
+                } else if (p.gate_up) {
+                    // SwiGLU: the gate tile's threads finish the first half of the tokens, the up tile's the second; what the other
+                    // needs goes through the accumulators' own columns of TMEM (same lanes, so no shared memory)
+                    constexpr int H = NT / 2;
+                    uint32_t r[16];
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(scale, __uint_as_float(r[j]), acc[c + j]);
+                    for (int c = 0; c < H; c += 16) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r[j] = c + j < H ? __float_as_uint(w ? acc[c + j < H ? c + j : 0] : acc[H + (c + j < H ? c + j : 0)]) : 0u;
+                        tmem_st16(tmem + lanes + 128u * w + 64u * dl + c, r);
                     }
-                }
-                tc_fence_before();
-                // gate/up: the last sums' columns carry the exchange below and are freed after it
-                if (!p.gate_up || g + 1 < groups) warp_arrive(d_free(db));
-                scale = next;
-                if (++s == kStages) { s = 0; ph ^= 1; }
-            }
-            if (!ok) break;
-            const int dl = (it - 1) & 1;  // buffer of the last group
-            if (p.gate_up) {
-                // SwiGLU: the gate tile's threads finish the first half of the tokens, the up tile's the second; what the other
-                // needs goes through the accumulators' own columns of TMEM (same lanes, so no shared memory)
-                constexpr int H = NT / 2;
-                uint32_t r[16];
+                    tmem_wait_st();
+                    tc_fence_before();
+                    warp_arrive(ex);
+                    if (!(ok = warp_wait(ex, round & 1, abort))) break;
+                    tc_fence_after();
+                    const uint32_t d_other = tmem + lanes + 128u * (w ^ 1) + 64u * dl;
+                    const int first = w ? H : 0;
 #pragma unroll
-                for (int c = 0; c < H; c += 16) {
+                    for (int c = 0; c < H; c += 16) {
+                        if (first + c < t.n) {
+                            tmem_ld16(r, d_other + c);
+                            tmem_wait_ld();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) r[j] = c + j < H ? __float_as_uint(w ? acc[c + j < H ? c + j : 0] : acc[H + (c + j < H ? c + j : 0)]) : 0u;
-                    tmem_st16(tmem + lanes + 128u * w + 64u * dl + c, r);
-                }
-                tmem_wait_st();
-                tc_fence_before();
-                warp_arrive(ex);
-                if (!(ok = warp_wait(ex, round & 1, abort))) break;
-                tc_fence_after();
-                const uint32_t d_other = tmem + lanes + 128u * (w ^ 1) + 64u * dl;
-                const int first = w ? H : 0;
+                            for (int j = 0; j < 16 && c + j < H; ++j) {
+                                const float own = w ? acc[H + c + j] : acc[c + j], other = __uint_as_float(r[j]);
+                                const float gate = w ? other : own, up = w ? own : other;
+                                if (live && first + c + j < t.n)
+                                    p.y[static_cast<int64_t>(t.t0 + first + c + j) * half_rows + mrow] = __float2half_rn(gate * (1.0f / (1.0f + expf(-gate))) * up);
+                            }
+                        }
+                    }
+                    tc_fence_before();
+                    warp_arrive(d_free(dl));
+                } else if (live) {
+                    __half* y = p.y + static_cast<int64_t>(t.t0) * p.N + mrow;
+                    float* y32 = p.y32 + static_cast<int64_t>(t.t0) * p.N + mrow;
+                    const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * p.N + mrow : nullptr;
 #pragma unroll
-                for (int c = 0; c < H; c += 16) {
-                    if (first + c < t.n) {
-                        tmem_ld16(r, d_other + c);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int j = 0; j < 16 && c + j < H; ++j) {
-                            const float mine = w ? acc[H + c + j] : acc[c + j], other = __uint_as_float(r[j]);
-                            const float gate = w ? other : mine, up = w ? mine : other;
-                            if (live && first + c + j < t.n)
-                                p.y[static_cast<int64_t>(t.t0 + first + c + j) * half_rows + mrow] = __float2half_rn(gate * (1.0f / (1.0f + expf(-gate))) * up);
+                    for (int j = 0; j < NT; ++j) {
+                        if (j < t.n) {
+                            if (p.y32) {
+                                y32[static_cast<int64_t>(j) * p.N] = acc[j];
+                                continue;
+                            }
+                            __half v = __float2half_rn(acc[j]);
+                            if (res) v = __hadd(v, res[static_cast<int64_t>(j) * p.N]);
+                            y[static_cast<int64_t>(j) * p.N] = v;
                         }
                     }
                 }
-                tc_fence_before();
-                warp_arrive(d_free(dl));
-            } else if (live) {
-                __half* y = p.y + static_cast<int64_t>(t.t0) * p.N + mrow;
-                float* y32 = p.y32 + static_cast<int64_t>(t.t0) * p.N + mrow;
-                const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * p.N + mrow : nullptr;
-#pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    if (j < t.n) {
-                        if (p.y32) {
-                            y32[static_cast<int64_t>(j) * p.N] = acc[j];
-                            continue;
-                        }
-                        __half v = __float2half_rn(acc[j]);
-                        if (res) v = __hadd(v, res[static_cast<int64_t>(j) * p.N]);
-                        y[static_cast<int64_t>(j) * p.N] = v;
-                    }
-                }
             }
+            t = next;
+        }
+    }
+    if (SPLIT) {
+        __syncwarp();
+        cluster_sync();
+        const Tile t = tile(tile0);
+        const int mrow = t.row0 + tid;  // row1 follows row0 (dense)
+        if (warp < 8 && mrow < p.N) {
+            const int per = (t.n + p.parts - 1) / p.parts, j1 = min(t.n, (rank + 1) * per);
+            for (int j = rank * per; j < j1; ++j) {
+                float part[8], sum = 0.f;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) part[r] = r < p.parts ? ld_peer(stage0 + 4u * (kTileRows * j + tid), r) : 0.f;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) sum += part[r];
+                const int64_t o = static_cast<int64_t>(t.t0 + j) * p.N + mrow;
+                __half v = __float2half_rn(sum);
+                if (p.resid) v = __hadd(v, p.resid[o]);
+                p.y[o] = v;
             }
         }
+        cluster_sync();  // nobody leaves while its sums are read
     }
     __syncthreads();
     if (tid == 0 && s_abort && p.err_flag) atomicOr(p.err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
@@ -461,25 +565,46 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
     }
 }
 
+// Per device and idempotent; not a stream operation, so legal under capture.
+template <typename K>
+int allow_smem(K kernel, size_t bytes) {
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    return err == cudaSuccess ? LEMOQ_OK : set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
+}
+
 template <int NT>
-int launch_nt(const GemmShape& p, const __half* x, const int8_t* codes, const LaunchCfg& lc) {
+int launch_nt(GemmShape p, const __half* x, const int8_t* codes, const LaunchCfg& lc) {
     CUtensorMap map_w, map_x;
     if (int rc = encode_rows_map(&map_w, codes, 1, static_cast<int64_t>(p.E) * p.N, p.K, 128)) return rc;
     if (int rc = encode_rows_map(&map_x, x, 2, p.T, p.K, Shape<NT>::kBox)) return rc;
-    {  // per device and idempotent; not a stream operation, so legal under capture
-        const cudaError_t err = cudaFuncSetAttribute(w8_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Shape<NT>::kSmem));
-        if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
-    }
+    const size_t smem = Shape<NT>::kSmem + 8 * (static_cast<size_t>(p.E) + 1);
+    const int gk = p.K / p.group;
+    p.scale_vecs = aligned16(p.scale) && (gk == 8 || gk == 16) ? gk / 8 : 0;
     const int64_t mt = p.gate_up ? (p.N / 2 + 127) / 128 : (p.N + kTileRows - 1) / kTileRows;
     const int64_t most = mt * (p.seg ? p.T / NT + std::min<int64_t>(p.E, p.T) : (p.T + NT - 1) / NT);  // tiles, at most
-    const int grid = static_cast<int>(std::min<int64_t>(sm_count(), std::max<int64_t>(most, 1)));
-    return launch_kernel(w8_gemm_kernel<NT>, dim3(grid), dim3(kThreads), Shape<NT>::kSmem, lc, map_w, map_x, p);
+    const int sms = sm_count();
+    if constexpr (NT <= kExactTokens) {
+        // A linear of few rows is a tile on every sixth SM or fewer (2048 rows: 8 tiles), each a chain of K / 128 groups of half a
+        // microsecond: its groups are shared out over a cluster while that leaves every block two of them and an SM of its own.
+        int parts = 1;
+        while (parts < 8 && most * 2 * parts <= sms && 4 * parts <= p.K >> 7) parts *= 2;
+        if (parts > 1 && !p.seg && !p.gate_up && !p.y32 && p.T <= NT) {
+            if (int rc = allow_smem(w8_gemm_kernel<NT, true>, smem)) return rc;
+            p.parts = parts;
+            LaunchCfg clustered = lc;
+            clustered.cluster = parts;
+            return launch_kernel(w8_gemm_kernel<NT, true>, dim3(static_cast<unsigned>(most) * parts), dim3(kThreads), smem, clustered, map_w, map_x, p);
+        }
+    }
+    if (int rc = allow_smem(w8_gemm_kernel<NT, false>, smem)) return rc;
+    const int grid = static_cast<int>(std::min<int64_t>(sms, std::max<int64_t>(most, 1)));
+    return launch_kernel(w8_gemm_kernel<NT, false>, dim3(grid), dim3(kThreads), smem, lc, map_w, map_x, p);
 }
 
 }  // namespace
 
 int launch_w8_gemm(const W8GemmParams& g, const LaunchCfg& lc) {
-    GemmShape p;
+    GemmShape p = {};
     p.T = g.T; p.N = g.N; p.K = g.K; p.group = g.group_size; p.E = g.E; p.gate_up = g.gate_up ? 1 : 0;
     p.seg = g.seg; p.scale = g.scale; p.resid = g.resid; p.y = g.y; p.y32 = g.y32; p.err_flag = g.err_flag;
     // NT bounds the tokens of a tile, the MMA's N follows the real count: a small NT only saves registers and stage bytes, a

@@ -34,7 +34,9 @@ def _gemm(x, codes, scale, *, seg=None, gate_up=False, exact=True, resid=None):
 # one token; either side of the 16-, 32-, 64- and 128-token tiles; rows that leave a tile of 256 half empty or spill over it; one
 # group of codes, and an odd number of them
 @pytest.mark.parametrize("tokens,n,k,exact", [(1, 2, 128, True), (16, 256, 128, True), (17, 130, 384, True), (33, 258, 256, True), (64, 514, 640, True),
-                                              (65, 256, 128, True), (65, 258, 384, False), (128, 128, 256, False), (129, 770, 128, False), (300, 256, 640, False)])
+                                              (65, 256, 128, True), (65, 258, 384, False), (128, 128, 256, False), (129, 770, 128, False), (300, 256, 640, False),
+                                              # groups shared out over a cluster: evenly, unevenly, more parts than tokens
+                                              (64, 514, 2048, True), (33, 2048, 1152, True), (3, 130, 1024, True)])
 def test_w8_gemm_edges(tokens, n, k, exact):
     codes, scale = _w8(n, k, tokens + n)
     x = torch.randn(tokens, k, generator=torch.Generator().manual_seed(k)).half()
