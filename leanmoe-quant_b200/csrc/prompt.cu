@@ -3,7 +3,7 @@
 //   lemoq_lockstep_run  one token of each of T sequences, all at the same slot: K/V rows quantised into each sequence's int8 caches,
 //                       decode attention over those
 //
-// Eleven kernels per layer, launched from here with programmatic dependent launch: the prompt of a short question is
+// Nine kernels per layer (ten with more than a thousand routed pairs), launched from here with programmatic dependent launch: the prompt of a short question is
 // bound by the 6.9 GB of weights all experts together have (1.1 ms), so a launch gap or a host call per expert is what it
 // must not pay; a long prompt is bound by the tensor cores (w8_gemm.cu, prompt_attn.cu); a lockstep step by the weights and its
 // sequences' caches (attn_i8.cu).
@@ -136,8 +136,7 @@ int run_rows(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const 
             LEMOQ_TRY(launch_prompt_attn(a, chained));
         }
         LEMOQ_TRY(gemm(b.ctx, T, L.o_codes, L.o_scale, d.hidden, A, b.x, b.x1));
-        LEMOQ_TRY(launch_combine_norm(nullptr, nullptr, nullptr, T, 0, b.x1, d.hidden, half(L.ln2), d.eps, nullptr, b.h, chained));
-        LEMOQ_TRY(launch_route_rows(b.h, half(L.router), T, d.hidden, d.experts, d.top_k, d.norm_topk_prob, nullptr, b.top_w, b.top_i, chained));
+        LEMOQ_TRY(launch_norm_route(b.x1, half(L.ln2), d.eps, half(L.router), T, d.hidden, d.experts, d.top_k, d.norm_topk_prob, b.h, b.top_w, b.top_i, chained));
         LEMOQ_TRY(launch_pairs(b.top_i, P, d.experts, b.h, d.top_k, d.hidden, b.place, b.pair_of, b.seg, b.pairs, nullptr, chained));
         W8GemmParams g;
         g.x = b.pairs; g.T = P; g.codes = L.gu_codes; g.scale = half(L.gu_scale); g.N = 2 * d.ffn; g.K = d.hidden; g.group_size = d.group_size;

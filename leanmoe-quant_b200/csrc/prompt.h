@@ -7,7 +7,6 @@ namespace lemoq {
 
 int launch_embed_norm(const int64_t* tokens, const __half* embed, int64_t vocab, int T, int H, const __half* w, float eps, __half* x, __half* h, int* err,
                       const LaunchCfg& lc);
-// y == nullptr: h = norm(x1) only
 int launch_combine_norm(const __half* y, const int32_t* place, const float* top_w, int T, int K, const __half* x1, int H, const __half* w, float eps, __half* x2,
                         __half* h, const LaunchCfg& lc);
 
@@ -26,9 +25,9 @@ struct QkvRows {
 };
 int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc);
 
-// logits (T, E) fp16 = h . router^T, softmax + top-k of every row.  E a multiple of 16, <= 128; H a multiple of 64.
-int launch_route_rows(const __half* h, const __half* router, int T, int H, int E, int top_k, int norm, __half* logits, float* top_w, int32_t* top_i,
-                      const LaunchCfg& lc);
+// h = RMSNorm(x); logits fp16(h . router^T), softmax + top-k of every row.  E a multiple of 8, <= 128; H a multiple of 64, <= 4096.
+int launch_norm_route(const __half* x, const __half* norm_w, float eps, const __half* router, int T, int H, int E, int top_k, int norm, __half* h, float* top_w,
+                      int32_t* top_i, const LaunchCfg& lc);
 // Stable sort of the P = T * K pairs by expert: place[p] = row of pair p in expert order, pair_of[row] = p, seg[e] = first row of e,
 // x_sorted[row] = h[pair_of[row] / K].  Ids outside [0, E) are clamped and flagged.
 int launch_pairs(const int32_t* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,

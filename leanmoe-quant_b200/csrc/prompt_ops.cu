@@ -1,15 +1,17 @@
 // Row operations between the tensor-core kernels when many tokens go through a layer at once.  All of them are bounded by
 // the rows they read and write (L2-resident up to some thousand tokens); each does everything that touches its rows in one
-// pass, so that a layer is eleven launches:
+// pass, so that a layer is nine launches (four of them GEMMs, one attention):
 //
 //   embed_norm     embedding row, input RMSNorm                                   one block per token
 //   qkv_rows       q/k RMSNorm over the projection width, RoPE, rows into the caches one block per token
-//   route_rows     router logits (fp16 mma), softmax, top-k                         one block per 16 tokens
+//   norm_route     post-attention RMSNorm, router logits (fp16 mma), softmax, top-k  one block per 16 tokens
 //   pair_plan      stable counting sort of the (token, slot) pairs by expert         one block per expert
 //   gather_rows    activations into expert order (few pairs: done by pair_plan)     one block per pair
 //   combine_norm   routing-weighted sum in slot order (fp32) + residual, next norm   one block per token
 #include "prompt.h"
 #include "stream.cuh"
+
+#include <algorithm>
 
 namespace lemoq {
 namespace {
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(kRowThreads) embed_norm_kernel(const int64_t* 
     norm_row_store(f, H, w, eps, h + t * H, red);
 }
 
-// out[t] = fp16(sum_k w[t, k] * y[place[t, k]]) + x1[t]; then the next RMSNorm of it.  Without y: only the norm of x1.
+// out[t] = fp16(sum_k w[t, k] * y[place[t, k]]) + x1[t]; then the next RMSNorm of it.
 __global__ void __launch_bounds__(kRowThreads) combine_norm_kernel(const __half* __restrict__ y, const int32_t* __restrict__ place, const float* __restrict__ top_w,
                                                                    int K, const __half* __restrict__ x1, int H, const __half* __restrict__ w, float eps,
                                                                    __half* __restrict__ x2, __half* __restrict__ h) {
@@ -76,19 +78,18 @@ __global__ void __launch_bounds__(kRowThreads) combine_norm_kernel(const __half*
         for (int j = 0; j < 8; ++j) f[v][j] = 0.f;
         if (i < H) {
             uint4 r = ld_cg16(x1 + t * H + i);
-            if (y) {
-                for (int k = 0; k < K; ++k) {
-                    const float wk = __half2float(__float2half_rn(__ldg(top_w + t * K + k)));
-                    float g[8];
-                    unpack8_h(ld_cg16(y + static_cast<int64_t>(__ldg(place + t * K + k)) * H + i), g);
+#pragma unroll 4
+            for (int k = 0; k < K; ++k) {
+                const float wk = __half2float(__float2half_rn(__ldg(top_w + t * K + k)));
+                float g[8];
+                unpack8_h(ld_cg16(y + static_cast<int64_t>(__ldg(place + t * K + k)) * H + i), g);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) f[v][j] = __fadd_rn(f[v][j], __fmul_rn(g[j], wk));
-                }
-                __half* rh = reinterpret_cast<__half*>(&r);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) rh[j] = __hadd(__float2half_rn(f[v][j]), rh[j]);
-                *reinterpret_cast<uint4*>(x2 + t * H + i) = r;
+                for (int j = 0; j < 8; ++j) f[v][j] = __fadd_rn(f[v][j], __fmul_rn(g[j], wk));
             }
+            __half* rh = reinterpret_cast<__half*>(&r);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) rh[j] = __hadd(__float2half_rn(f[v][j]), rh[j]);
+            *reinterpret_cast<uint4*>(x2 + t * H + i) = r;
             unpack8_h(r, f[v]);
         }
     }
@@ -202,37 +203,79 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-constexpr int kRouteWarps = 8;
+constexpr int kRouteWarps = 16;
 constexpr int kRouteTokens = 16;
 
-// 16 tokens x all experts per block.  The warps split H; their partial sums meet in shared memory and are added in warp
-// order.  With 0.27 GFLOP per thousand tokens the work is too small for a tcgen05 pipeline to fill: what counts is one round
-// of loads.  A and B use the same permutation of k inside 32 values, so that 128-bit loads feed the fragments.
+// A warp normalises one of the block's 16 rows; then the warps split H for the logits of all 16 rows and all experts.  Their partial
+// sums meet in shared memory (over the rows) and are added in warp order.  With 0.27 GFLOP per thousand tokens the work is too small for
+// a tcgen05 pipeline to fill: what counts is one round of loads.  The router does not depend on earlier kernels: it is asked into L2
+// while those finish.  A and B use the same permutation of k inside 32 values, so that 128-bit loads feed the fragments.
+// (As a norm kernel and a router kernel of eight warps with all loads in turn: 3.5 + 19 us at 64 tokens.)
 template <int TILES>  // expert tiles of 8
-__global__ void __launch_bounds__(kRouteWarps * 32) route_rows_kernel(const __half* __restrict__ h, const __half* __restrict__ router, int T, int H, int E, int top_k,
-                                                                      int norm, __half* __restrict__ logits, float* __restrict__ top_w, int32_t* __restrict__ top_i) {
-    extern __shared__ float part[];  // [warp][16 tokens][E]
+__global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __half* __restrict__ x, const __half* __restrict__ norm_w, float eps,
+                                                                      const __half* __restrict__ router, int T, int H, int E, int top_k, int norm,
+                                                                      __half* __restrict__ h, float* __restrict__ top_w, int32_t* __restrict__ top_i) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    float* part = reinterpret_cast<float*>(smem);    // [warp][16 tokens][E], after the rows
+    __half* rows = reinterpret_cast<__half*>(smem);  // [16][H + 8]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
-    const int t0 = blockIdx.x * kRouteTokens, tiles = E >> 3;
+    const int t0 = blockIdx.x * kRouteTokens, tiles = E >> 3, pitch = H + 8;
+    for (int i = (blockIdx.x % 4) * kRouteWarps * 32 + threadIdx.x; i < E * H / 64; i += 4 * kRouteWarps * 32)  // four blocks share it
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(router + 64 * static_cast<int64_t>(i)));
     pdl_wait();
     pdl_trigger();
+    {
+        const int t = t0 + warp;
+        __half* mine = rows + warp * pitch;
+        if (t < T) {
+            const __half* src = x + static_cast<int64_t>(t) * H;
+            float ss = 0.f;
+            for (int i = 8 * lane; i < H; i += 256) {
+                const uint4 v = ld_cg16(src + i);
+                *reinterpret_cast<uint4*>(mine + i) = v;
+                float f[8];
+                unpack8_h(v, f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+            }
+            const float rstd = 1.0f / sqrtf(warp_sum(ss) / static_cast<float>(H) + eps);
+            for (int i = 8 * lane; i < H; i += 256) {
+                const uint4 v = *reinterpret_cast<const uint4*>(mine + i), wv = __ldg(reinterpret_cast<const uint4*>(norm_w + i));
+                const __half *vh = reinterpret_cast<const __half*>(&v), *wh = reinterpret_cast<const __half*>(&wv);
+                __align__(16) __half o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(__half2float(vh[j]) * rstd), wh[j]);
+                *reinterpret_cast<uint4*>(mine + i) = *reinterpret_cast<const uint4*>(o);
+                *reinterpret_cast<uint4*>(h + static_cast<int64_t>(t) * H + i) = *reinterpret_cast<const uint4*>(o);
+            }
+        } else {
+            for (int i = 8 * lane; i < H; i += 256) *reinterpret_cast<uint4*>(mine + i) = make_uint4(0, 0, 0, 0);
+        }
+    }
+    __syncthreads();
     float c[TILES][4];
 #pragma unroll
     for (int n = 0; n < TILES; ++n) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
-    const __half* lo = h + static_cast<int64_t>(min(t0 + g, T - 1)) * H + 8 * q;
-    const __half* hi = h + static_cast<int64_t>(min(t0 + g + 8, T - 1)) * H + 8 * q;
     const __half* wr = router + static_cast<int64_t>(g) * H + 8 * q;
+#pragma unroll(TILES <= 8 ? 2 : 1)
     for (int k = 32 * warp; k < H; k += 32 * kRouteWarps) {
-        const uint4 a = ld_cg16(lo + k), b = ld_cg16(hi + k);
+        const uint4 a = *reinterpret_cast<const uint4*>(rows + g * pitch + 8 * q + k), b = *reinterpret_cast<const uint4*>(rows + (g + 8) * pitch + 8 * q + k);
 #pragma unroll
-        for (int n = 0; n < TILES; ++n) {
-            if (n < tiles) {
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(8 * n) * H + k));
-                mma_f16(c[n], a.x, b.x, a.y, b.y, w.x, w.y);
-                mma_f16(c[n], a.z, b.z, a.w, b.w, w.z, w.w);
+        for (int n0 = 0; n0 < TILES; n0 += 8) {
+            uint4 w[8];
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+                if (n0 + n < tiles) w[n] = __ldg(reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(8 * (n0 + n)) * H + k));
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                if (n0 + n < tiles) {
+                    mma_f16(c[n0 + n], a.x, b.x, a.y, b.y, w[n].x, w[n].y);
+                    mma_f16(c[n0 + n], a.z, b.z, a.w, b.w, w[n].z, w[n].w);
+                }
             }
         }
     }
+    __syncthreads();
     float* mine = part + warp * kRouteTokens * E;
 #pragma unroll
     for (int n = 0; n < TILES; ++n) {
@@ -256,9 +299,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_rows_kernel(const __ha
                 float v = 0.f;
 #pragma unroll
                 for (int w = 0; w < kRouteWarps; ++w) v += part[(w * kRouteTokens + j) * E + e];
-                const __half r = __float2half_rn(v);
-                if (logits) logits[static_cast<int64_t>(t) * E + e] = r;
-                p[i] = __half2float(r);
+                p[i] = __half2float(__float2half_rn(v));  // the logits are fp16 values
             }
             mx = fmaxf(mx, p[i]);
         }
@@ -371,9 +412,19 @@ __global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const ID* __res
     if (e == E - 1 && threadIdx.x == 0) seg[E] = base;
     if (GATHER) {
         const int vecs = H / 8;
-        for (int u = threadIdx.x; u < (base - row0) * vecs; u += kPlanThreads) {
-            const int r = u / vecs, i = 8 * (u - r * vecs);
-            *reinterpret_cast<uint4*>(x_sorted + static_cast<int64_t>(row0 + r) * H + i) = ld_cg16(h + static_cast<int64_t>(s_mine[r] / K) * H + i);
+        const int total = (base - row0) * vecs;
+        for (int u0 = threadIdx.x; u0 < total; u0 += 4 * kPlanThreads) {  // four loads in flight
+            uint4 v[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int u = u0 + b * kPlanThreads, r = u / vecs;
+                if (u < total) v[b] = ld_cg16(h + static_cast<int64_t>(s_mine[r] / K) * H + 8 * (u - r * vecs));
+            }
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int u = u0 + b * kPlanThreads, r = u / vecs;
+                if (u < total) *reinterpret_cast<uint4*>(x_sorted + static_cast<int64_t>(row0 + r) * H + 8 * (u - r * vecs)) = v[b];
+            }
         }
     }
 }
@@ -427,14 +478,16 @@ int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc) {
                 : launch_kernel(qkv_rows_kernel<false>, dim3(p.T), dim3(kRowThreads), 0, lc, p);
 }
 
-int launch_route_rows(const __half* h, const __half* router, int T, int H, int E, int top_k, int norm, __half* logits, float* top_w, int32_t* top_i,
-                      const LaunchCfg& lc) {
+int launch_norm_route(const __half* x, const __half* norm_w, float eps, const __half* router, int T, int H, int E, int top_k, int norm, __half* h, float* top_w,
+                      int32_t* top_i, const LaunchCfg& lc) {
     const dim3 grid((T + kRouteTokens - 1) / kRouteTokens), block(kRouteWarps * 32);
-    const size_t smem = static_cast<size_t>(kRouteWarps) * kRouteTokens * E * sizeof(float);
-    if (E <= 64) return launch_kernel(route_rows_kernel<8>, grid, block, smem, lc, h, router, T, H, E, top_k, norm, logits, top_w, top_i);
-    const cudaError_t err = cudaFuncSetAttribute(route_rows_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
-    return launch_kernel(route_rows_kernel<16>, grid, block, smem, lc, h, router, T, H, E, top_k, norm, logits, top_w, top_i);
+    const size_t smem = std::max(static_cast<size_t>(kRouteWarps) * kRouteTokens * E * sizeof(float), static_cast<size_t>(kRouteTokens) * (H + 8) * sizeof(__half));
+    auto run = [&](auto* kernel) {
+        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
+        return launch_kernel(kernel, grid, block, smem, lc, x, norm_w, eps, router, T, H, E, top_k, norm, h, top_w, top_i);
+    };
+    return E <= 64 ? run(norm_route_kernel<8>) : run(norm_route_kernel<16>);
 }
 
 template <typename ID>
