@@ -3,22 +3,23 @@
 // One block = one head x 256 query rows, as two tiles of 128 that take turns: while the warpgroup of one tile is in its softmax,
 // the tensor pipe works for the other.  Per 128 cache slots and tile:
 //   S = Q K^T   A, B from shared memory, 128 x 128 fp32 in TMEM
-//   softmax     one thread per row, in base 2: two passes over its row in TMEM (maximum; exp2, fp16, back into TMEM over S)
+//   softmax     one thread per row, in base 2: its row in registers, maximum, exp2, fp16, back into TMEM over S
 //   PV          A = the fp16 weights from TMEM, B = V (d is the contiguous side: MN-major), 128 x 128 fp32 in TMEM
-//   O           in registers: O = O * alpha + PV, so nothing in TMEM is ever rescaled
+//   O           accumulates in TMEM.  The maximum a row's weights are taken against follows the true one only when that has grown by more
+//               than 2^8 (the weights stay below 256, the sum of them in fp32): then, which is rare after the first steps, O is rescaled.
 // Blocks are handed out longest first.  No S x S matrix exists anywhere.
 //
-// Bounded by the issue slots of the softmax warps (about 700 per 128 x 128 tile and scheduler, of which 128 exp2) against 1024 cycles of
-// MMAs; the two tiles overlap them.
+// Bounded by exp2 (16 per SM and clock: 2048 cycles for the two tiles of a step) and the MMAs (2048 cycles as well), which the two tiles
+// overlap.  (With O in registers, 128 of them beside a row of S, the kernel spilled: 412 us at 4096 rows and 16 heads
+// instead of 111.)
 #include "prompt.h"
 #include "tc.cuh"
 
 namespace lemoq {
 namespace {
 
-constexpr int kThreads = 384;     // two softmax warpgroups, a third with the TMA warp and the MMA warp
-// Registers: 384 threads are launched with 168 each (64,512); 256 x 216 + 128 x 64 = 63,488 afterwards.
-constexpr int kRegsSoftmax = 216, kRegsIssue = 64;
+constexpr int kThreads = 320;     // two softmax warpgroups, the TMA warp, the MMA warp
+constexpr float kSlack = 8.f;     // log2 of how far the true maximum may run ahead of the one in use
 constexpr int kRows = 128;        // query rows of a tile
 constexpr int kSlots = 128;       // cache slots of a step
 constexpr int kHalf = 128 * 128;  // bytes of 128 rows x 64 values
@@ -34,6 +35,13 @@ struct AttnShape {
     int* err_flag;
 };
 
+// 2^x, 0 below 2^-126 (exp2f would keep those, for three more instructions an element)
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                                                   const __grid_constant__ CUtensorMap map_v, const AttnShape p) {
     extern __shared__ uint8_t raw[];
@@ -42,7 +50,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_c
     __shared__ volatile int s_abort;
     __shared__ int s_most[2];  // last slot any row of the tile sees
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t q_smem = (smem_u32(raw) + 1023u) & ~1023u, k_smem = q_smem + 2 * kTile, v_smem = k_smem + kKvStages * kTile;
     const uint32_t bars = smem_u32(s_bar);
     const uint32_t q_full = bars;
@@ -90,11 +98,6 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_c
     const int live = t0 + kRows < p.T ? 2 : 1;
     const int steps = max(s_most[0], s_most[1]) / kSlots + 1;  // both tiles run over the same slots
 
-    if (warp >= 8) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
-    } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
-    }
     if (warp == 8) {
         if (elect_one()) {
             mbar_expect_tx(q_full, live * kTile);
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_c
                     tc_fence_after();
                     const uint64_t v = smem_desc_sw128(v_smem + s * kTile, 1024, kHalf);
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) mma_f16_ts(tmem + 256u + 128u * i, tmem + 128u * i + 8u * k, v + k * (16u * 128u >> 4), id_o, k != 0);
+                    for (int k = 0; k < 8; ++k) mma_f16_ts(tmem + 256u + 128u * i, tmem + 128u * i + 8u * k, v + k * (16u * 128u >> 4), id_o, j > 0 || k > 0);
                     tc_commit(o_full(i));
                     if (j + 1 < steps) scores(i, sn);
                 }
@@ -162,86 +165,95 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_c
                 mbar_wait(drained, 0);
             }
         }
-    } else if (warp < 8 && warp >> 2 < live) {
+    } else if (warp >> 2 < live) {
         const int i = warp >> 2;
         const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
         const uint32_t s_at = tmem + lanes + 128u * i, o_at = tmem + lanes + 256u + 128u * i;
-        float o[128];
-#pragma unroll
-        for (int d = 0; d < 128; ++d) o[d] = 0.f;
-        float m = -INFINITY, l = 0.f, alpha_prev = 1.f;
+        float m = -INFINITY, l = 0.f;  // the maximum in use (times the scale, in base 2)
         bool ok = true;
-        auto take_o = [&](int j, float alpha) {  // O = O * alpha + PV of step j
-            if (!warp_wait(o_full(i), j & 1, abort)) return false;
-            tc_fence_after();
-#pragma unroll
-            for (int c = 0; c < 128; c += 16) {
-                uint32_t r[16];
-                tmem_ld16(r, o_at + c);
-                tmem_wait_ld();
-#pragma unroll
-                for (int d = 0; d < 16; ++d) o[c + d] = fmaf(o[c + d], alpha, __uint_as_float(r[d]));
-            }
-            return true;
-        };
         for (int j = 0; j < steps; ++j) {
             if (!(ok = warp_wait(s_full(i), j & 1, abort))) break;
             tc_fence_after();
-            const int first = j * kSlots, seen = my_pos - first;  // slots [0, seen] of this step are visible
+            const int seen = my_pos - j * kSlots;  // slots [0, seen] of this step are visible
             const bool all = __all_sync(0xffffffffu, seen >= kSlots - 1);
-            float top = -INFINITY;
+            uint32_t r[4][32];  // the row stays in registers for both passes
 #pragma unroll
-            for (int c = 0; c < kSlots; c += 16) {
-                uint32_t r[16];
-                tmem_ld16(r, s_at + c);
-                tmem_wait_ld();
+            for (int c = 0; c < 4; ++c) tmem_ld32(r[c], s_at + 32 * c);
+            tmem_wait_ld();
+            if (!all) {
 #pragma unroll
-                for (int d = 0; d < 16; ++d) top = fmaxf(top, all || c + d <= seen ? __uint_as_float(r[d]) : -INFINITY);
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int d = 0; d < 32; ++d)
+                        if (32 * c + d > seen) r[c][d] = 0xff800000u;  // -inf: weight 0
             }
+            float tops[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                tops[c] = __uint_as_float(r[c][0]);
+#pragma unroll
+                for (int d = 1; d < 31; d += 2) tops[c] = fmaxf(fmaxf(tops[c], __uint_as_float(r[c][d])), __uint_as_float(r[c][d + 1]));
+                tops[c] = fmaxf(tops[c], __uint_as_float(r[c][31]));
+            }
+            const float top = fmaxf(fmaxf(tops[0], tops[1]), fmaxf(tops[2], tops[3]));
             const float m_new = fmaxf(m, top * p.scale_log2);
-            const float shift = m_new > -INFINITY ? m_new : 0.f;
-            const float alpha = exp2f(m - shift);
-            float sum = 0.f;
+            const bool grown = m_new > m + kSlack;  // the first visible slot of a row always is
+            if (__any_sync(0xffffffffu, grown)) {
+                const float alpha = grown ? exp2f(m - m_new) : 1.f;
+                if (grown) m = m_new;
+                l *= alpha;
+                if (j > 0) {
+                    if (!(ok = warp_wait(o_full(i), (j - 1) & 1, abort))) break;
+                    tc_fence_after();
 #pragma unroll
-            for (int c = 0; c < kSlots; c += 32) {
-                uint32_t w[16];
+                    for (int c = 0; c < 128; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld16(v, o_at + c);
+                        tmem_wait_ld();
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    uint32_t r[16];
-                    tmem_ld16(r, s_at + c + 16 * b);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int d = 0; d < 16; d += 2) {
-                        float e[2];
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) {
-                            e[u] = all || c + 16 * b + d + u <= seen ? exp2f(fmaf(__uint_as_float(r[d + u]), p.scale_log2, -shift)) : 0.f;
-                            sum += e[u];
-                        }
-                        const __half2 h = __floats2half2_rn(e[0], e[1]);
-                        w[8 * b + d / 2] = *reinterpret_cast<const uint32_t*>(&h);
+                        for (int d = 0; d < 16; ++d) v[d] = __float_as_uint(__uint_as_float(v[d]) * alpha);
+                        tmem_st16(o_at + c, v);
                     }
                 }
-                tmem_st16(s_at + c / 2, w);  // over columns this thread has already read
             }
+            const float shift = m > -INFINITY ? m : 0.f;
+            float sums[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                uint32_t w[16];
+#pragma unroll
+                for (int d = 0; d < 32; d += 2) {
+                    const float e0 = ex2(fmaf(__uint_as_float(r[c][d]), p.scale_log2, -shift)), e1 = ex2(fmaf(__uint_as_float(r[c][d + 1]), p.scale_log2, -shift));
+                    sums[d & 2] += e0;
+                    sums[(d & 2) + 1] += e1;
+                    const __half2 h = __floats2half2_rn(e0, e1);
+                    w[d / 2] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                tmem_st16(s_at + 16 * c, w);  // over columns this thread has read
+            }
+            l += (sums[0] + sums[1]) + (sums[2] + sums[3]);
             tmem_wait_st();
-            l = fmaf(l, alpha, sum);
-            // the sums of the step before leave TMEM before this step's product may overwrite them
-            if (j > 0 && !(ok = take_o(j - 1, alpha_prev))) break;
-            alpha_prev = alpha;
-            m = m_new;
             tc_fence_before();
             warp_arrive(p_full(i));
         }
-        if (ok && (ok = take_o(steps - 1, alpha_prev)) && t0 + tid < p.T) {
+        if (ok && (ok = warp_wait(o_full(i), (steps - 1) & 1, abort))) {
+            tc_fence_after();
             const float inv = 1.f / l;
             __half* dst = p.out + (static_cast<int64_t>(t0 + tid) * p.heads + head) * 128;
 #pragma unroll
-            for (int c = 0; c < 128; c += 8) {
-                __align__(16) __half h[8];
+            for (int c = 0; c < 128; c += 32) {
+                uint32_t r[32];
+                tmem_ld32(r, o_at + c);
+                tmem_wait_ld();
+                if (t0 + tid < p.T) {
 #pragma unroll
-                for (int d = 0; d < 8; ++d) h[d] = __float2half_rn(o[c + d] * inv);
-                *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(h);
+                    for (int e = 0; e < 32; e += 8) {
+                        __align__(16) __half h[8];
+#pragma unroll
+                        for (int d = 0; d < 8; ++d) h[d] = __float2half_rn(__uint_as_float(r[e + d]) * inv);
+                        *reinterpret_cast<uint4*>(dst + c + e) = *reinterpret_cast<const uint4*>(h);
+                    }
+                }
             }
         }
         tc_fence_before();
