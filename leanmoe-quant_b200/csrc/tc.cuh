@@ -142,8 +142,20 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
         : "memory");
 }
 
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait of one thread; `abort` as below.
 __device__ __forceinline__ bool thread_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
+    if (mbar_test(bar, parity)) return true;
     for (uint32_t i = 0; i < kWaitLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((i & 1023u) == 1023u && *abort) return false;
@@ -154,7 +166,7 @@ __device__ __forceinline__ bool thread_wait(uint32_t bar, uint32_t parity, volat
 // Bounded wait of a whole warp: the same outcome in every lane.  `abort` is a flag in shared memory: a warp that gave up
 // sets it, and every later wait in the block ends at once.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
-    bool ok = mbar_try_wait(bar, parity);
+    bool ok = mbar_test(bar, parity);
     for (uint32_t i = 0; !__all_sync(0xffffffffu, ok) && i < kWaitLimit; ++i) {
         if ((i & 1023u) == 1023u && __any_sync(0xffffffffu, *abort)) break;
         ok = ok || mbar_try_wait(bar, parity);

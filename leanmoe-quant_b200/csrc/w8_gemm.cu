@@ -15,7 +15,7 @@
 // x up to NT tokens of one expert:
 //   warp 16      TMA: per group of 128 k the codes (2 x 128 rows x 128 bytes) and the tokens (two halves of 64 k), swizzled
 //   warps 8-15   a warpgroup per M tile, thread = weight row: widen the codes of a group into TMEM (two buffers)
-//   warp 17      issues the MMAs: A = widened codes from TMEM, B = tokens from shared memory, D in TMEM
+//   warps 17, 18 issue the MMAs, one warp per M tile: A = widened codes from TMEM, B = tokens from shared memory, D in TMEM
 //   warps 0-7    a warpgroup per M tile, thread = weight row: collect the sums (per group / at the end), finish the rows
 // TMEM: D of tile w at column 128 w (exact: two buffers of 64), A of tile w, buffer b at 256 + 128 w + 64 b.
 //
@@ -24,7 +24,8 @@
 // codes in shared memory would add a write and a read of twice the codes' size.  Widening and collecting are different warps
 // because either is a chain of waits, and the TMA and MMA loops are one thread each because a vote after every wait cost
 // that warp 160 cycles (exact, NT = 16: 3200 cycles per group with both by the same warps and `lane == 0` issue, 1700 with
-// separate warps and elect.sync).
+// separate warps and elect.sync).  One MMA thread for both tiles left the tensor pipe idle for a quarter of the time (a wait
+// that is over costs it 200 cycles): with two, one waits while the other's MMAs run.
 #include "tc.cuh"
 
 #include <algorithm>
@@ -76,7 +77,8 @@ struct Shape {
     static constexpr bool kScaled = NT > kExactTokens;
     static constexpr int kDBufs = kScaled ? 1 : 2;                      // accumulator buffers per M tile
     static constexpr int kStages = NT >= 128 ? 3 : (NT == 64 ? 4 : 5);
-    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + 1024;  // + 8 (E + 1) bytes of tile table
+    static constexpr int kTurn = kScaled ? 8 * 32 * 32 * 2 : 0;         // a collecting warp's 32 rows x 32 tokens, turned for wide stores
+    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + kTurn + 1024;  // + 8 (E + 1) bytes of tile table
 };
 
 struct GemmShape {
@@ -115,6 +117,15 @@ __device__ __forceinline__ Tile tile_at(int i, const int* first, const int* tok,
     t.row0 = p.gate_up ? m * 128 : m * kTileRows;
     t.row1 = p.gate_up ? p.N / 2 + m * 128 : m * kTileRows + 128;
     return t;
+}
+
+// silu(gate) * up of two pairs, for fp16 results: exp and the quotients to about 2^-21, one reciprocal for both.  Below -43 the exponential is
+// held at e^43 (its square is finite): such a gate gives less than 1e-12 whatever `up` is.  (With expf and rounded divisions the epilogue of a
+// gate/up tile of 128 tokens took 9900 cycles, half as long as its MMAs.)
+__device__ __forceinline__ void swiglu2(float g0, float u0, float g1, float u1, float& y0, float& y1) {
+    const float a = 1.0f + __expf(-fmaxf(g0, -43.f)), b = 1.0f + __expf(-fmaxf(g1, -43.f)), r = __fdividef(1.0f, a * b);
+    y0 = g0 * (r * b) * u0;
+    y1 = g1 * (r * a) * u1;
 }
 
 // 16 codes -> 8 words of two exact fp16 each: bytes with the sign flipped dropped into 0x64__ are 1024 + 128 + c.
@@ -183,21 +194,22 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
     using S = Shape<NT>;
     constexpr int kStages = S::kStages;
     extern __shared__ uint8_t raw[];
-    __shared__ __align__(8) uint64_t s_bar[2 * kStages + 7];
+    __shared__ __align__(8) uint64_t s_bar[2 * kStages + 10];
     __shared__ __align__(16) uint8_t s_scale[kTileRows * kScaleStride];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage0 = (smem_u32(raw) + 1023u) & ~1023u;
-    int* s_first = reinterpret_cast<int*>(raw + (stage0 - smem_u32(raw)) + static_cast<size_t>(kStages) * S::kStage);
+    int* s_first = reinterpret_cast<int*>(raw + (stage0 - smem_u32(raw)) + static_cast<size_t>(kStages) * S::kStage + S::kTurn);
     int* s_tok = s_first + p.E + 1;
     const uint32_t bars = smem_u32(s_bar);
     auto full = [&](int s) { return bars + 8u * s; };
     auto done = [&](int s) { return bars + 8u * (kStages + s); };
-    auto a_full = [&](int b) { return bars + 8u * (2 * kStages + b); };
-    auto d_free = [&](int b) { return bars + 8u * (2 * kStages + 2 + b); };
-    const uint32_t ex = bars + 8u * (2 * kStages + 4), drained = ex + 8u, d_full = ex + 16u;
+    auto a_full = [&](int w, int b) { return bars + 8u * (2 * kStages + 2 * w + b); };
+    auto d_free = [&](int b) { return bars + 8u * (2 * kStages + 4 + b); };
+    const uint32_t ex = bars + 8u * (2 * kStages + 6), d_full = ex + 8u;
+    auto drained = [&](int w) { return ex + 16u + 8u * w; };
     constexpr int kD = S::kDBufs;
     constexpr bool kScaled = S::kScaled;
 
@@ -205,15 +217,16 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
         s_abort = 0;
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full(s), 1);
-            mbar_init(done(s), 1);
+            mbar_init(done(s), 2);  // the MMAs of both tiles
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(a_full(b), 8);
+            mbar_init(a_full(0, b), 4);
+            mbar_init(a_full(1, b), 4);
             mbar_init(d_free(b), 8);
+            mbar_init(drained(b), 1);
         }
         mbar_init(ex, 8);
-        mbar_init(drained, 1);
-        mbar_init(d_full, 1);
+        mbar_init(d_full, 2);
         mbar_fence_init();
     }
     if (warp == 17) tmem_alloc(smem_u32(&s_tmem), 512);
@@ -300,9 +313,10 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 for (int j = max(0, issued - kStages); j < issued; ++j) mbar_wait(full(j % kStages), (j / kStages) & 1);
             }
         }
-    } else if (warp == 17) {
-        // ---- MMA: one thread ---------------------------------------------------------------------------------------
+    } else if (warp == 17 || warp == 18) {
+        // ---- MMA: one thread per M tile ------------------------------------------------------------------------------
         if (elect_one()) {
+            const int w = warp - 17;
             int s = 0, it = 0, dn = 0;  // dn counts the accumulations: one per group (exact) or per tile (scaled)
             bool ok = true;
             Tile t = tile(tile0);
@@ -312,16 +326,13 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                     const int b = it & 1, db = kD == 2 ? dn & 1 : 0;
                     const bool begins = !kScaled || g == g0, ends = !kScaled || g + 1 == g1;
                     // a widening warp has seen the stage's copies land before it arrives: no wait on full(s) here
-                    if (!(ok = thread_wait(a_full(b), (it >> 1) & 1, abort))) break;
+                    if (!(ok = thread_wait(a_full(w, b), (it >> 1) & 1, abort))) break;
                     if (begins && !(ok = thread_wait(d_free(db), ((kD == 2 ? dn >> 1 : dn) & 1) ^ 1, abort))) break;
                     tc_fence_after();
                     const uint64_t x0 = smem_desc_sw128(stage0 + static_cast<uint32_t>(s) * S::kStage + kCodeBytes, 1024);
-                    const uint32_t a = tmem + kColA + 64u * b, d = tmem + 64u * db;
+                    const uint32_t a = tmem + kColA + 128u * w + 64u * b, d = tmem + 128u * w + 64u * db;
 #pragma unroll
-                    for (int w = 0; w < 2; ++w)
-#pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            mma_f16_ts(d + 128u * w, a + 128u * w + 8u * k, x0 + (k >> 2) * (S::kHalf >> 4) + (k & 3) * 2u, idesc, !(begins && k == 0));
+                    for (int k = 0; k < 8; ++k) mma_f16_ts(d, a + 8u * k, x0 + (k >> 2) * (S::kHalf >> 4) + (k & 3) * 2u, idesc, !(begins && k == 0));
                     // one event ends the group for everybody: the stage may be refilled, the A buffer rewritten, D read
                     tc_commit(done(s));
                     if (kScaled && ends) tc_commit(d_full);  // (a parity wait cannot look past the next phase of done(s))
@@ -331,8 +342,8 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 }
             }
             if (!ok) {  // gave up: nothing may still write TMEM when it is freed
-                tc_commit(drained);
-                mbar_wait(drained, 0);
+                tc_commit(drained(w));
+                mbar_wait(drained(w), 0);
             }
         }
     } else if (warp >= 8 && warp < 16) {
@@ -368,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 }
                 tmem_wait_st();
                 tc_fence_before();
-                warp_arrive(a_full(b));
+                warp_arrive(a_full(w, b));
                 if (++s == kStages) { s = 0; ph ^= 1; }
                 if (++s2 == kStages) { s2 = 0; ph2 ^= 1; }
                 if (kScaled && g == g0 && i + stride < tiles) {
@@ -405,39 +416,85 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 if (!(ok = warp_wait(d_full, round & 1, abort))) break;
                 tc_fence_after();
                 __half2 out[H];
+                if (gu) {
 #pragma unroll
-                for (int c = 0; c < NT; c += 16) {
-                    if (c < nj) {
-                        uint32_t r[16];
-                        tmem_ld16(r, tmem + lanes + (gu ? 0u : 128u * w) + j0 + c);
-                        if (gu) {
-                            uint32_t u[16];
-                            tmem_ld16(u, tmem + lanes + 128u + j0 + c);
+                    for (int c = 0; c < H; c += 32) {
+                        if (c < nj) {
+                            uint32_t r[32], u[32];
+                            tmem_ld32(r, tmem + lanes + j0 + c);
+                            tmem_ld32(u, tmem + lanes + 128u + j0 + c);
                             tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const float gate = __uint_as_float(r[j]);
-                                r[j] = __float_as_uint(gate * (1.0f / (1.0f + expf(-gate))) * __uint_as_float(u[j]));
+                            if (c + 32 >= nj) {  // everything has left TMEM: the next tile may begin
+                                tc_fence_before();
+                                warp_arrive(d_free(0));
                             }
-                        } else {
-                            tmem_wait_ld();
-                        }
 #pragma unroll
-                        for (int j = 0; j < 16; j += 2) out[(c + j) / 2] = __floats2half2_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+                            for (int j = 0; j < 32; j += 2) {
+                                float y0, y1;
+                                swiglu2(__uint_as_float(r[j]), __uint_as_float(u[j]), __uint_as_float(r[j + 1]), __uint_as_float(u[j + 1]), y0, y1);
+                                out[(c + j) / 2] = __floats2half2_rn(y0, y1);
+                            }
+                        }
                     }
+                    if (nj == 0) {
+                        tc_fence_before();
+                        warp_arrive(d_free(0));
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < NT; c += 32) {
+                        if (c < nj) {
+                            uint32_t r[32];
+                            tmem_ld32(r, tmem + lanes + 128u * w + c);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int j = 0; j < 32; j += 2) out[(c + j) / 2] = __floats2half2_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+                        }
+                    }
+                    tc_fence_before();
+                    warp_arrive(d_free(0));
                 }
-                tc_fence_before();
-                warp_arrive(d_free(0));
-                if (live) {
-                    const int64_t ld = gu ? half_rows : p.N;
-                    __half* y = p.y + static_cast<int64_t>(t.t0 + j0) * ld + mrow;
-                    const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * ld + mrow : nullptr;
+                const int64_t ld = gu ? half_rows : p.N;
+                __half* y = p.y + static_cast<int64_t>(t.t0 + j0) * ld;
+                const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * ld : nullptr;
+                if (ld % 8 == 0 && mrow - lane + 32 <= lim) {
+                    // A thread has one row of many tokens; turned over in shared memory 32 x 32 at a time, a lane stores eight rows of a token
+                    // (two bytes a lane instead: a down tile of 128 tokens spent longer in its stores than in its MMAs).
+                    const uint32_t turn = stage0 + kStages * S::kStage + warp * 2048u;
+#pragma unroll
+                    for (int c = 0; c < NT; c += 32) {
+                        if (c < nj) {
+                            __syncwarp();
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) {
+                                const __half v = j & 1 ? __high2half(out[(c + j) / 2]) : __low2half(out[(c + j) / 2]);
+                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(turn + 64u * j + 2u * lane), "h"(__half_as_ushort(v)) : "memory");
+                            }
+                            __syncwarp();
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                const int j = 8 * k + (lane >> 2), at = mrow - lane + 8 * (lane & 3);
+                                if (c + j < nj) {
+                                    uint4 v = lds128(turn + 64u * j + 16u * (lane & 3));
+                                    if (res) {
+                                        const uint4 r4 = __ldcg(reinterpret_cast<const uint4*>(res + (c + j) * ld + at));
+                                        __half2* vh = reinterpret_cast<__half2*>(&v);
+                                        const __half2* rh = reinterpret_cast<const __half2*>(&r4);
+#pragma unroll
+                                        for (int e = 0; e < 4; ++e) vh[e] = __hadd2(vh[e], rh[e]);
+                                    }
+                                    *reinterpret_cast<uint4*>(y + (c + j) * ld + at) = v;
+                                }
+                            }
+                        }
+                    }
+                } else if (live) {
 #pragma unroll
                     for (int j = 0; j < NT; ++j) {
                         if (j < nj) {
                             __half v = j & 1 ? __high2half(out[j / 2]) : __low2half(out[j / 2]);
-                            if (res) v = __hadd(v, res[j * ld]);
-                            y[j * ld] = v;
+                            if (res) v = __hadd(v, res[j * ld + mrow]);
+                            y[j * ld + mrow] = v;
                         }
                     }
                 }
@@ -505,11 +562,15 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                             tmem_ld16(r, d_other + c);
                             tmem_wait_ld();
 #pragma unroll
-                            for (int j = 0; j < 16 && c + j < H; ++j) {
-                                const float own = w ? acc[H + c + j] : acc[c + j], other = __uint_as_float(r[j]);
-                                const float gate = w ? other : own, up = w ? own : other;
-                                if (live && first + c + j < t.n)
-                                    p.y[static_cast<int64_t>(t.t0 + first + c + j) * half_rows + mrow] = __float2half_rn(gate * (1.0f / (1.0f + expf(-gate))) * up);
+                            for (int j = 0; j < 16 && c + j < H; j += 2) {
+                                float y[2];
+                                const float o0 = __uint_as_float(r[j]), o1 = __uint_as_float(r[j + 1]);
+                                if (w) swiglu2(o0, acc[H + c + j], o1, acc[H + c + j + 1], y[0], y[1]);
+                                else swiglu2(acc[c + j], o0, acc[c + j + 1], o1, y[0], y[1]);
+#pragma unroll
+                                for (int v = 0; v < 2; ++v)
+                                    if (live && first + c + j + v < t.n)
+                                        p.y[static_cast<int64_t>(t.t0 + first + c + j + v) * half_rows + mrow] = __float2half_rn(y[v]);
                             }
                         }
                     }

@@ -115,7 +115,8 @@ def test_lockstep_matches_the_step_by_parts(sequences):
     with torch.no_grad():
         for _ in range(3):
             got, ref = (d.step(tokens) for d in decoders)
-            assert rel_err(got, ref) < 1e-2
+            # over all rows: now and then a sequence has another, nearly equal expert in its last slot
+            assert float((got.float() - ref.float()).norm() / ref.float().norm()) < 5e-3
             tokens = ref.float().argmax(dim=-1)
     for a, b in zip(decoders[0].kv, decoders[1].kv):
         assert float((a["kc"] != b["kc"]).float().mean()) < 1e-2 and rel_err(a["vs"], b["vs"]) < 1e-2
