@@ -1357,6 +1357,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                         p.top_w[lane] = __float2half_rn(w);
                     }
                     __threadfence_block();
+                    __syncwarp();  // the lanes may leave the top-k apart: lane 0 must not announce ids that others still hold
                     if (lane == 0) S.ready_layer = l;  // the producers may start the expert tiles of this layer
                 }
                 consumer_sync();
