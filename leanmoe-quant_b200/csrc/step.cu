@@ -50,9 +50,11 @@ namespace lemoq {
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// words of the flagged exchange buffers: x 4*2048, q.k.v 2*6144, sums of squares 2*2048, logits 2*128, activations 2*4096
+// words of the flagged exchange buffers: x 4*2048, q.k.v 2*6144, sums of squares 2*2048, logits 2*128, activations 2*4096,
+// attention outputs 2*1024, attention partials of at most 16 heads x 9 splits, 132 words each, twice
 constexpr size_t kFlX = 0, kFlQkv = kFlX + 4 * 2048, kFlStats = kFlQkv + 2 * 6144, kFlLogits = kFlStats + 2 * 2048,
-                 kFlAct = kFlLogits + 2 * 128, kFlaggedWords = kFlAct + 2 * 4096;
+                 kFlAct = kFlLogits + 2 * 128, kFlAttn = kFlAct + 2 * 4096, kFlPart = kFlAttn + 2 * 1024,
+                 kFlaggedWords = kFlPart + 2 * 16 * 9 * 132;
 
 static int resolve_splits(const lemoq_step_desc& d) {
     if (d.attn_splits > 0) return d.attn_splits;
@@ -288,8 +290,9 @@ extern "C" int lemoq_step_run(lemoq_step* s, void* stream, int* launches) {
         p.err_flag = s->err_flag; p.bar_counter = s->bar_counter; p.bar_epoch = s->bar_epoch;
         p.fl_x = s->flagged + kFlX; p.fl_qkv = s->flagged + kFlQkv; p.fl_stats = s->flagged + kFlStats;
         p.fl_logits = s->flagged + kFlLogits; p.fl_act = s->flagged + kFlAct;
+        p.fl_attn = s->flagged + kFlAttn; p.fl_part = s->flagged + kFlPart;
         p.router_logits = s->router_logits; p.top_w = s->top_w; p.top_i = s->top_i; p.attn_part = s->attn_part;
-        p.barriers_per_launch = d.layers + 1;  // attention -> o_proj in every layer, and the end of the step
+        p.barriers_per_launch = 1;  // the end of the step
         p.stamps = s->stamps;
         if (int rc = launch_step_tile(p, s->whole_grid, static_cast<cudaStream_t>(stream))) return rc;
         if (launches) *launches = 1;

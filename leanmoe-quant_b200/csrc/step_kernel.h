@@ -41,7 +41,7 @@ struct StepParams {
     // flagged-word buffers (8-byte words {data, tag}), two parities each: layer outputs [2][2048] then post-attention
     // streams [2][2048]; q.k.v rows [2][3*2048]; q/k sums of squares per block [2][2][1024]; router logits [2][128];
     // expert activations, two per word [2][4096]
-    unsigned long long *fl_x, *fl_qkv, *fl_stats, *fl_logits, *fl_act;
+    unsigned long long *fl_x, *fl_qkv, *fl_stats, *fl_logits, *fl_act, *fl_attn, *fl_part;
     int64_t* top_i;
     float* attn_part;            // (m, l, acc[D]) partial of every (head, split) unit; at the end the per-block greedy candidates
     int barriers_per_launch;

@@ -2,21 +2,25 @@
 // int8 tensor-core dot product.
 //
 // One block per SM stays resident for the whole step.  All weights move as TILES: 8 whole rows and the rows'
-// group scales, brought into a 16.9 KB shared-memory stage by three to six bulk asynchronous copies, each issued by
-// a lane of its own: the codes in runs of four rows (adjacent in memory; every run lands 64 bytes further than its
+// group scales, brought into a 16.9 KB shared-memory stage by three to six bulk asynchronous copies: the codes in runs of four rows (adjacent in memory; every run lands 64 bytes further than its
 // natural place, so that the 16-byte reads of rows r and r + 4, which one request of a quarter warp combines, hit
 // different banks), the scales in one or two runs.  The block has ten stages.  Ten CONSUMER warps own one stage
-// each and do all the arithmetic; five PRODUCER warps do nothing but issue copies: each keeps two stages filled,
-// walking the block's tile sequence of the WHOLE STEP in order (a copy instruction occupies the issuing warp for
-// well over a thousand cycles, which is why the consumers do not issue their own).  A stage is handed back and
+// each and do all the arithmetic; one elected thread of each of five PRODUCER warps does nothing but issue copies: it keeps
+// two stages filled, walking the block's tile sequence of the WHOLE STEP in order.  A stage is handed back and
 // forth through a full/empty pair of shared-memory barriers.  The producers run ahead across phases and layers:
 // q.k.v, KV-cache, o_proj, router and lm_head tiles do not depend on activations, so they land while the
 // consumers still work on the phase before; only the expert tiles wait, on the block's own top-k.
 //
 // Between phases the blocks exchange small vectors (the residual stream, q.k.v, router logits, the SwiGLU
 // activations) through global memory as flagged 8-byte words that the readers poll, see "flagged words" below.
-// The one place where every block needs everything every other block wrote in bulk - the attention partials
-// before o_proj - is a grid barrier: one per layer, plus one at the end of the step.
+// The attention partials of a head's splits go the same way to one block, which merges them and publishes the head.
+// The only grid barrier is the one at the end of the step.
+//
+// What bounds it: the chain of these exchanges, two to three L2 round trips each, then the burst of the expert tiles that
+// can start only when a layer's routing is known.  The code of a layer is kept compact and free of register spills: with
+// 220 KB of shared memory in use a spilled register comes back from L2 (a spilling build: 780 us a step, 568 without, at
+// 1024 cached positions), and code beyond the first-level instruction cache runs at a third of the speed.  With the
+// barrier in every layer, fp32 partials read by all blocks and three copies of the tile product the step took 646 us.
 //
 // Arithmetic: the activation vector of a phase is turned once per block into three planes of signed
 // 7-bit digits with one power-of-two scale per group of 128 (x = sx * (d2*2^14 + d1*2^7 + d0)).  The
@@ -38,9 +42,9 @@
 // Phases per layer (what a block waits for -> what it publishes):
 //   A  q.k.v tiles          flagged x of the layer before; planes of RMSNorm(x)   -> flagged qkv + sum-of-squares partials
 //   B  attention            flagged qkv; one (head, split) per block, KV tiles of 16, 32 or 64 positions through the
-//                           same stages; q/k norm + RoPE + KV row write fused     -> (m, l, acc) partial per unit
-//      grid barrier
-//   C  o_proj tiles         splits of each head merged while the planes are built; + residual -> flagged x1
+//                           same stages; q/k norm + RoPE + KV row write fused     -> flagged (m, l, acc) per unit;
+//                           split 0 of a head merges the others                        -> flagged attention output
+//   C  o_proj tiles         flagged attention output; + residual                       -> flagged x1
 //   D  router tiles (fp16)  flagged x1; planes of h2 = RMSNorm(x1) stay in shared memory for E -> flagged logits
 //   E  expert gate/up       flagged logits; one warp per block derives the top-k; SwiGLU -> flagged act
 //   F  expert down          flagged act; routing-weighted sum + residual          -> flagged x2
@@ -70,6 +74,7 @@ constexpr int kMaxLayers = 33;
 constexpr int kMaxSplits = 9;
 constexpr int kHeadDim = 128;
 constexpr int kQPlaneStride = kHeadDim + kPad;
+constexpr int kPartWords = kHeadDim + 4;  // a unit's attention partial: acc[128], m, l, two words unused
 constexpr int kPartFloats = 1024;       // partial sums of the down phase (8 per tile)
 constexpr uint32_t kBarrierSpinLimit = 1u << 24;
 
@@ -96,9 +101,10 @@ __device__ __forceinline__ uint2 ld_cg8(const void* p) {
 // (unique over launches).  8-byte accesses are single-copy atomic, so a reader that sees the tag it waits for (or
 // a later one) holds the data that was stored with it: it polls the very words it needs and starts as soon as
 // they are there - one memory round trip behind the producer's store, where a barrier costs an arrival, a poll
-// and then the load.  Buffers alternate with the layer's parity; the one grid barrier per layer that remains
-// (attention -> o_proj) keeps every block within one layer of every other, so no word is overwritten while
-// somebody still waits for its previous content.
+// and then the load.  Buffers alternate with the layer's parity, and no word is overwritten while somebody still waits for
+// its previous content: a head's output is published only after the sums of squares of ALL blocks have come in, and every
+// block stores its sum when it is through with phase A, so a block that works on o_proj or later of a layer knows that every
+// other block has left the layer before.
 constexpr uint32_t kFlagSpinLimit = 1u << 21;  // default of the limit below
 // Polls of a flagged word before a wait gives up (raising LEMOQ_FLAG_WAIT_TIMEOUT; the step then goes on with what the
 // word held).  lemoq_set_tuning key 5 changes it on the current device: the time-out path can be tested by making it 1.
@@ -129,40 +135,24 @@ __device__ __forceinline__ bool others_gave_up(const int* err_flag, uint32_t it)
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(err_flag) : "memory");
     return (v & LEMOQ_FLAG_WAIT_TIMEOUT) != 0;
 }
-// N words of this thread (src[0..N), used where on[i]) until all carry the tag: data[i] = their data.  Bounded.
-template <int N>
-__device__ __forceinline__ bool flag_wait(const unsigned long long* src, const bool (&on)[N], uint32_t tag, uint32_t (&data)[N],
-                                          const int* err_flag) {
+// Four neighbouring words of this thread (32-byte aligned) until all carry the tag: d = their data.  Bounded; the lanes
+// of a warp may leave apart.
+__device__ __forceinline__ bool tags_reached(const unsigned long long (&w)[4], uint32_t tag) {
+    return tag_reached(w[0], tag) && tag_reached(w[1], tag) && tag_reached(w[2], tag) && tag_reached(w[3], tag);
+}
+__device__ __forceinline__ bool flag_wait4(const unsigned long long* src, uint32_t tag, uint32_t (&d)[4], const int* err_flag) {
     const uint32_t limit = c_flag_spin_limit;
-    bool have[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        have[i] = !on[i];
-        data[i] = 0;
-    }
+    bool good = false;
+    unsigned long long w[4];
 #pragma unroll 1  // one look per trip: an unrolled poll loop multiplies the traffic of everybody who waits
     for (uint32_t it = 0; it < limit; ++it) {
-        bool ok = true;
-        static_assert(N % 4 == 0, "words are looked at four at a time");
-#pragma unroll
-        for (int i = 0; i < N; i += 4) {
-            if (!(have[i] && have[i + 1] && have[i + 2] && have[i + 3])) {  // only sectors with a word still missing
-                unsigned long long w[4];
-                flag_load4(src + i, w);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (!have[i + j]) {
-                        have[i + j] = tag_reached(w[j], tag);
-                        data[i + j] = static_cast<uint32_t>(w[j]);
-                    }
-                    ok = ok && have[i + j];
-                }
-            }
-        }
-        if (ok) return true;
-        if (others_gave_up(err_flag, it)) return false;
+        flag_load4(src, w);
+        good = tags_reached(w, tag);
+        if (good || others_gave_up(err_flag, it)) break;
     }
-    return false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] = static_cast<uint32_t>(w[i]);
+    return good;
 }
 
 // Block barrier of the consumer warps (the producer warps never take part in it).
@@ -268,6 +258,7 @@ __device__ __forceinline__ void plane_weights(int t, bool one_vector, float (&pw
 template <int NB>
 __device__ __forceinline__ float tile_s8_steps(const unsigned char* alo, const unsigned char* ahi, const unsigned char* bp, const float* sx,
                                                const __half* sc, int gh, int gs0, const float (&pw)[4], float acc) {
+    static_assert(NB == 2 || NB == 4, "");
     int c[NB][4];
 #pragma unroll
     for (int u = 0; u < NB; ++u) c[u][0] = c[u][1] = c[u][2] = c[u][3] = 0;
@@ -286,11 +277,24 @@ __device__ __forceinline__ float tile_s8_steps(const unsigned char* alo, const u
 #pragma unroll
         for (int u = 0; u < NB; ++u) mma_s8(c[u], a[u].z, b[u].z, a[u].w, b[u].w, x[u].z, x[u].w);
     }
+    // scales of the NB groups of either half: the row's (fp16) and the vector's, a load each
+    __half2 h_lo[NB / 2], h_hi[NB / 2];
+    float x_lo[NB], x_hi[NB];
+    if constexpr (NB == 4) {
+        *reinterpret_cast<uint2*>(h_lo) = *reinterpret_cast<const uint2*>(sc + gs0);
+        *reinterpret_cast<uint2*>(h_hi) = *reinterpret_cast<const uint2*>(sc + gh + gs0);
+        *reinterpret_cast<float4*>(x_lo) = *reinterpret_cast<const float4*>(sx + gs0);
+        *reinterpret_cast<float4*>(x_hi) = *reinterpret_cast<const float4*>(sx + gh + gs0);
+    } else {
+        h_lo[0] = *reinterpret_cast<const __half2*>(sc + gs0);
+        h_hi[0] = *reinterpret_cast<const __half2*>(sc + gh + gs0);
+        *reinterpret_cast<float2*>(x_lo) = *reinterpret_cast<const float2*>(sx + gs0);
+        *reinterpret_cast<float2*>(x_hi) = *reinterpret_cast<const float2*>(sx + gh + gs0);
+    }
 #pragma unroll
     for (int u = 0; u < NB; ++u) {
-        const int gs = gs0 + u;
-        const float s_lo = __half2float(sc[gs]) * sx[gs];
-        const float s_hi = __half2float(sc[gh + gs]) * sx[gh + gs];
+        const float s_lo = __half2float(u & 1 ? __high2half(h_lo[u / 2]) : __low2half(h_lo[u / 2])) * x_lo[u];
+        const float s_hi = __half2float(u & 1 ? __high2half(h_hi[u / 2]) : __low2half(h_hi[u / 2])) * x_hi[u];
         acc = fmaf(fmaf(static_cast<float>(c[u][1]), pw[1], static_cast<float>(c[u][0]) * pw[0]), s_lo, acc);
         acc = fmaf(fmaf(static_cast<float>(c[u][3]), pw[3], static_cast<float>(c[u][2]) * pw[2]), s_hi, acc);
     }
@@ -298,15 +302,17 @@ __device__ __forceinline__ float tile_s8_steps(const unsigned char* alo, const u
 }
 
 // One int8 tile: 8 rows of K codes in a stage (tile row r at r * K + (r >> 2) * kRunPad) against the plane segments
-// of a vector.  r: the tile row of this lane's instruction row (tile_row()).  bp: this lane's segment pointer (+ t*16
-// applied here).  sx: the K/128 group scales of the vector.  sc: the K/128 fp16 group scales of row r.  Returns the
-// lane's share of row r (to be added over the 4 lanes of a group).
-__device__ __forceinline__ float tile_s8(const unsigned char* st, int K, int r, int t, const unsigned char* bp, const float* sx,
-                                         const __half* sc, const float (&pw)[4]) {
+// of a vector.  r: the tile row of this lane's instruction row.  bp: this lane's segment pointer (+ t*16
+// applied here).  sx: the K/128 group scales of the vector.  sc: the K/128 fp16 group scales of row r.  Returns row r
+// (the same value in the 4 lanes of a group).  One copy of this code for all phases: what a layer runs should fit the
+// first-level instruction cache.
+__device__ __forceinline__ float tile_s8(const unsigned char* st, int K, int r, int t, const unsigned char* bp, const float* sx, const __half* sc) {
     const int half_k = K >> 1, gh = K >> 8;  // bytes per half row, groups per half
     const unsigned char* alo = st + r * K + (r >> 2) * kRunPad + t * 16;
     const unsigned char* ahi = alo + half_k;
     bp += t * 16;
+    float pw[4];
+    plane_weights(t, false, pw);
     float acc = 0.f;
     if (gh >= 4) {
 #pragma unroll 1
@@ -314,6 +320,8 @@ __device__ __forceinline__ float tile_s8(const unsigned char* st, int K, int r, 
     } else {
         acc = tile_s8_steps<2>(alo, ahi, bp, sx, sc, gh, 0, pw, acc);
     }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
     return acc;
 }
 
@@ -368,6 +376,8 @@ struct AttnSm {
     __align__(16) uint2 newk16[32];
     __align__(16) uint2 newv16[32];
     float p32[kStreamWarps][32];
+    // the partials of the head's other splits, as its first split collects them: acc[128], m, l (a row: kPartWords)
+    __align__(16) float other[kMaxSplits - 1][kPartWords];
 };
 
 // Sizes, shifts and this block's place in the grid (all row widths are powers of two between 512 and 2048).
@@ -399,7 +409,7 @@ struct Smem {
     __align__(8) unsigned long long empty_bars[kStreamWarps];  // the consumer is done with the stage
     volatile int ready_layer;                                  // the routing of layers <= this is in route_id
     __align__(128) unsigned char xplanes[kXPlaneBytes];
-    float xsx[16];
+    __align__(16) float xsx[16];
     __align__(128) unsigned char xh[4 * (1024 + kPad)];  // fp16 copy of the normalised vector, in quarters (router rows)
     __align__(128) unsigned char big[kBigBytes > static_cast<int>(sizeof(AttnSm)) ? kBigBytes : static_cast<int>(sizeof(AttnSm))];
     float part[kPartFloats];
@@ -416,91 +426,100 @@ __device__ __forceinline__ int udiv_small(int q, int magic) { return (q * magic)
 // ---------------------------------------------------------------------------------------------
 // per-warp tile stream
 // ---------------------------------------------------------------------------------------------
-// The bulk copies of tile (layer, kind, lt) of this block into a stage (a few large copies: starting a copy costs
-// a warp some hundred cycles).  Global tile index of local tile lt: b + lt * G (down phase: row block b + j * G with
-// the top_k routed experts as consecutive tiles).
-__device__ __noinline__ void issue_tile(const Smem& S, int layer, int kind, int lt, uint32_t stage, uint32_t bar) {
-    const Geo& geo = S.geo;
+// Where tile (layer, kind, lt) of this block lies in memory.  Global tile index of local tile lt: b + lt * G (down
+// phase: row block b + j * G with the top_k routed experts as consecutive tiles).  An int8 weight tile is one or two
+// pairs of code runs (a run: four rows, adjacent in memory; the second run of a pair `run_step` bytes after the first)
+// and one or two runs of group scales.
+struct TileSource {
+    const char* codes[2];
+    const char* scales[2];
+    uint32_t K, run_step, scale_bytes;  // bytes of a code row, of the step between the runs of a pair, of a run of scales
+    int pairs, scale_runs;
+};
+__device__ __forceinline__ TileSource weight_tile(const Smem& S, const Geo& geo, const StepLayer& L, int kind, int lt) {
+    TileSource w;
+    w.pairs = w.scale_runs = 1;
+    w.codes[1] = w.scales[1] = nullptr;
+    if (kind == KF) {  // 8 down rows of one routed expert, or of two
+        const uint32_t K = geo.F, sb = (K >> 7) * 2;
+        const int j = udiv_small(lt, geo.f_magic), pp = lt - j * geo.ftiles;
+        const uint32_t first = (geo.b + j * geo.G) * 8;
+        const int slot = geo.fpair ? 2 * pp : pp;
+        const size_t r0 = static_cast<size_t>(S.route_id[slot]) * geo.H + first;
+        w.codes[0] = reinterpret_cast<const char*>(L.dn_codes) + r0 * K;
+        w.scales[0] = reinterpret_cast<const char*>(L.dn_scale) + r0 * sb;
+        if (geo.fpair && slot + 1 < geo.K) {
+            const size_t r1 = static_cast<size_t>(S.route_id[slot + 1]) * geo.H + first;
+            w.codes[1] = reinterpret_cast<const char*>(L.dn_codes) + r1 * K;
+            w.scales[1] = reinterpret_cast<const char*>(L.dn_scale) + r1 * sb;
+            w.pairs = w.scale_runs = 2;
+        }
+        w.K = K;
+        w.run_step = 4 * K;
+        w.scale_bytes = 8 * sb;
+        return w;
+    }
+    const int tg = geo.b + lt * geo.G;
+    if (kind == KE) {  // 4 gate rows + 4 up rows of one routed expert
+        const uint32_t K = geo.H, sb = (K >> 7) * 2;
+        const int slot = tg >> geo.shF4, n0 = (tg - (slot << geo.shF4)) * 4;
+        const size_t row = static_cast<size_t>(S.route_id[slot]) * 2 * geo.F + n0;
+        w.codes[0] = reinterpret_cast<const char*>(L.gu_codes) + row * K;
+        w.scales[0] = reinterpret_cast<const char*>(L.gu_scale) + row * sb;
+        w.scales[1] = w.scales[0] + static_cast<size_t>(geo.F) * sb;
+        w.scale_runs = 2;
+        w.K = K;
+        w.run_step = geo.F * K;
+        w.scale_bytes = 4 * sb;
+        return w;
+    }
+    // 8 consecutive rows of q.k.v / lm_head (KA) or o_proj (KC)
+    const uint32_t K = kind == KA ? geo.H : geo.A, sb = (K >> 7) * 2;
+    w.codes[0] = reinterpret_cast<const char*>(kind == KA ? L.qkv_codes : L.o_codes) + static_cast<size_t>(tg) * 8 * K;
+    w.scales[0] = reinterpret_cast<const char*>(kind == KA ? L.qkv_scale : L.o_scale) + static_cast<size_t>(tg) * 8 * sb;
+    w.K = K;
+    w.run_step = 4 * K;
+    w.scale_bytes = 8 * sb;
+    return w;
+}
+
+// The bulk copies of a tile into a stage, by ONE thread (inside elect_one(): with the copies spread over the lanes of
+// a warp, each with an address of its own, the compiler issues them lane by lane, some 1700 cycles a tile).
+__device__ __forceinline__ void issue_tile(const Smem& S, const Geo& geo, int layer, int kind, int lt, uint32_t stage, uint32_t bar) {
     const StepLayer& L = S.layers[layer];
-    const int lane = threadIdx.x & 31;
-    const char* src = nullptr;
-    uint32_t bytes = 0, dst = 0, tx = 0;
     if (kind == KB) {  // cached positions of this block's head: keys and values (int8: the consumer reads the scales itself)
         const int first = (geo.tile0 + lt) * geo.kvt;
         const uint32_t npos = static_cast<uint32_t>(min(geo.kvt, geo.S - first));  // the last tile of a head may be short
-        const uint32_t p0 = static_cast<uint32_t>(geo.h * geo.S + first);
-        const uint32_t row = geo.kv16 ? 2 * kHeadDim : kHeadDim;  // bytes of a position
-        tx = 2 * npos * row;
-        if (lane < 2) {
-            const void* base = geo.kv16 ? static_cast<const void*>(lane == 0 ? L.keys : L.values) : static_cast<const void*>(lane == 0 ? L.kc : L.vc);
-            src = reinterpret_cast<const char*>(base) + static_cast<size_t>(p0) * row;
-            bytes = npos * row;
-            dst = lane * kKvTile * kHeadDim;
-        }
-    } else if (kind == KD) {  // 4 router rows (fp16) in one copy; fewer than 4 experts left: only those
-        const int row0 = (geo.b + lt * geo.G) * 4;
-        const uint32_t nrows = static_cast<uint32_t>(min(4, geo.E - row0));
-        tx = nrows * 2 * geo.H;
-        if (lane == 0) {
-            src = reinterpret_cast<const char*>(L.router) + static_cast<size_t>(row0) * 2 * geo.H;
-            bytes = tx;
-        }
-    } else {
-        // The code rows of a tile land in runs of four, each run 64 bytes further than its natural place (tile row r at
-        // r * K + (r >> 2) * 64): the eight lanes that read 16 bytes each of tile rows r and r + 4 in one request then
-        // hit different banks.  Lanes 0-3 copy one run of codes each, lanes 4-5 the group scales (rows of a run are
-        // consecutive in memory; gate/up: the gate run and the up run; down: the runs of one routed expert or of two).
-        const int tg = geo.b + lt * geo.G;
-        const uint32_t run = lane & 3, half = lane & 1;  // code lanes: run of four rows; scale lanes 4, 5: first / second part
-        uint32_t K = geo.H;          // row width
-        uint32_t crow = 0, srow = 0; // first row of this lane's run of codes / part of the scales
-        uint32_t nruns = 2;          // runs of four code rows in the tile
-        uint32_t sparts = 1, srows = 8;  // parts of the scales and rows per part
-        const char* cbase;
-        const char* sbase;
-        if (kind == KE) {  // 4 gate rows + 4 up rows of one routed expert
-            const int slot = tg >> geo.shF4, n0 = (tg - (slot << geo.shF4)) * 4;
-            crow = srow = static_cast<uint32_t>(S.route_id[slot]) * 2 * geo.F + n0 + (half ? geo.F : 0);
-            sparts = 2;
-            srows = 4;
-            cbase = reinterpret_cast<const char*>(L.gu_codes);
-            sbase = reinterpret_cast<const char*>(L.gu_scale);
-        } else if (kind == KF) {  // 8 down rows of one routed expert, or of two (runs 2-3 and scale part 1: the second one)
-            const int j = udiv_small(lt, geo.f_magic), pp = lt - j * geo.ftiles;
-            const bool two = geo.fpair && 2 * pp + 1 < geo.K;
-            const uint32_t first = (geo.b + j * geo.G) * 8;
-            const int cslot = geo.fpair ? 2 * pp + static_cast<int>(run >> 1) : pp, sslot = geo.fpair ? 2 * pp + static_cast<int>(half) : pp;
-            crow = static_cast<uint32_t>(S.route_id[min(cslot, geo.K - 1)]) * geo.H + first + (run & 1) * 4;
-            srow = static_cast<uint32_t>(S.route_id[min(sslot, geo.K - 1)]) * geo.H + first;
-            nruns = two ? 4 : 2;
-            sparts = two ? 2 : 1;
-            K = geo.F;
-            cbase = reinterpret_cast<const char*>(L.dn_codes);
-            sbase = reinterpret_cast<const char*>(L.dn_scale);
-        } else {  // 8 consecutive rows of q.k.v / lm_head (KA) or o_proj (KC)
-            crow = tg * 8 + run * 4;
-            srow = tg * 8;
-            K = kind == KA ? geo.H : geo.A;
-            cbase = reinterpret_cast<const char*>(kind == KA ? L.qkv_codes : L.o_codes);
-            sbase = reinterpret_cast<const char*>(kind == KA ? L.qkv_scale : L.o_scale);
-        }
-        const uint32_t sb = (K >> 7) * 2;  // bytes of one row of group scales
-        tx = nruns * 4u * (K + sb);
-        if (lane < 4) {
-            if (run < nruns) {
-                src = cbase + static_cast<size_t>(crow) * K;
-                bytes = 4 * K;
-                dst = run * (4 * K + kRunPad);
-            }
-        } else if (lane < 6 && half < sparts) {
-            src = sbase + static_cast<size_t>(srow) * sb;
-            bytes = srows * sb;
-            dst = kScaleOff + half * srows * sb;
-        }
+        const uint32_t row = geo.kv16 ? 2 * kHeadDim : kHeadDim;                    // bytes of a position
+        const size_t at = (static_cast<size_t>(geo.h) * geo.S + first) * row;
+        const char* keys = geo.kv16 ? reinterpret_cast<const char*>(L.keys) : reinterpret_cast<const char*>(L.kc);
+        const char* values = geo.kv16 ? reinterpret_cast<const char*>(L.values) : reinterpret_cast<const char*>(L.vc);
+        mbar_expect_tx(bar, 2 * npos * row);
+        bulk_g2s(stage, keys + at, npos * row, bar);
+        bulk_g2s(stage + kKvTile * kHeadDim, values + at, npos * row, bar);
+        return;
     }
-    if (lane == 0) mbar_expect_tx(bar, tx);
-    __syncwarp();
-    if (bytes != 0) bulk_g2s(stage + dst, src, bytes, bar);
+    if (kind == KD) {  // 4 router rows (fp16) in one copy; fewer than 4 experts left: only those
+        const int row0 = (geo.b + lt * geo.G) * 4;
+        const uint32_t bytes = static_cast<uint32_t>(min(4, geo.E - row0)) * 2 * geo.H;
+        mbar_expect_tx(bar, bytes);
+        bulk_g2s(stage, reinterpret_cast<const char*>(L.router) + static_cast<size_t>(row0) * 2 * geo.H, bytes, bar);
+        return;
+    }
+    // The code rows of a tile land in runs of four, each run 64 bytes further than its natural place (tile row r at
+    // r * K + (r >> 2) * 64): the eight lanes that read 16 bytes each of tile rows r and r + 4 in one request then
+    // hit different banks.
+    const TileSource w = weight_tile(S, geo, L, kind, lt);
+    const uint32_t run = 4 * w.K;
+    mbar_expect_tx(bar, 2 * w.pairs * run + w.scale_runs * w.scale_bytes);
+    bulk_g2s(stage, w.codes[0], run, bar);
+    bulk_g2s(stage + run + kRunPad, w.codes[0] + w.run_step, run, bar);
+    if (w.pairs == 2) {
+        bulk_g2s(stage + 2 * (run + kRunPad), w.codes[1], run, bar);
+        bulk_g2s(stage + 3 * (run + kRunPad), w.codes[1] + w.run_step, run, bar);
+    }
+    bulk_g2s(stage + kScaleOff, w.scales[0], w.scale_bytes, bar);
+    if (w.scale_runs == 2) bulk_g2s(stage + kScaleOff + w.scale_bytes, w.scales[1], w.scale_bytes, bar);
 }
 
 // Place in the block's tile sequence of the tiles that go through one stage.  The tiles of a block form one
@@ -536,31 +555,25 @@ struct Cursor {
     }
 };
 
-// A producer warp: fills its two stages in sequence order for the whole step.  A stage is refilled as soon as its
-// consumer gives it back, whatever phase the consumers are in; only the expert tiles wait for the routing of
-// their layer.  Every wait is bounded: a producer that gives up raises the flag word and stops, and the consumers
-// then run into their own bounded waits.
-__device__ __noinline__ void producer_loop(Smem& S, int* err_flag, int first_stage) {
+// One thread of a producer warp: fills the warp's two stages in sequence order for the whole step.  A stage is
+// refilled as soon as its consumer gives it back, whatever phase the consumers are in; only the expert tiles wait for
+// the routing of their layer.  Every wait is bounded: a producer that gives up raises the flag word and stops, and the
+// consumers then run into their own bounded waits.
+__device__ __forceinline__ void producer_loop(Smem& S, int* err_flag, int first_stage) {
     const Geo& geo = S.geo;
-    const int lane = threadIdx.x & 31;
-    Cursor c0, c1;
-    c0.start(geo, first_stage);
-    c1.start(geo, first_stage + 1);
-    uint32_t used0 = 0, used1 = 0;  // fills of each stage so far
+    Cursor c, other;  // the stage whose turn it is, and the other one
+    c.start(geo, first_stage);
+    other.start(geo, first_stage + 1);
+    int stage = first_stage;
+    uint32_t used = 0, other_used = 0;  // fills of each stage so far
     bool ok = true;
 #pragma unroll 1
-    while (ok && (c0.kind != KEND || c1.kind != KEND)) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            Cursor& c = i == 0 ? c0 : c1;
-            uint32_t& used = i == 0 ? used0 : used1;
-            if (!ok || c.kind == KEND) continue;
-            const int stage = first_stage + i;
+    while (ok && (c.kind != KEND || other.kind != KEND)) {
+        if (c.kind != KEND) {
             if (c.kind >= KE) {  // expert tiles: the routing of the layer must be known
                 uint32_t n = 0;
                 while (S.ready_layer < c.layer) {
-                    __nanosleep(64);
-                    if (++n > (1u << 22)) {
+                    if (++n > (1u << 24)) {
                         ok = false;
                         break;
                     }
@@ -568,23 +581,28 @@ __device__ __noinline__ void producer_loop(Smem& S, int* err_flag, int first_sta
                 __threadfence_block();
             }
             if (ok && used > 0) ok = mbar_wait(smem_u32(&S.empty_bars[stage]), (used - 1) & 1u);
-            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
-            issue_tile(S, c.layer, c.kind, c.lt, smem_u32(S.ring) + static_cast<uint32_t>(stage) * kStageBytes, smem_u32(&S.full_bars[stage]));
+            issue_tile(S, geo, c.layer, c.kind, c.lt, smem_u32(S.ring) + static_cast<uint32_t>(stage) * kStageBytes, smem_u32(&S.full_bars[stage]));
             ++used;
             c.lt += kStreamWarps;
             c.normalise(geo, stage);
         }
+        const Cursor turn = c;
+        c = other;
+        other = turn;
+        const uint32_t n = used;
+        used = other_used;
+        other_used = n;
+        stage ^= 1;
     }
-    if (!ok && err_flag && lane == 0) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+    if (!ok && err_flag) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
 }
 
-// Consumer side of a stage: wait for the tile (warp-uniform result; false on time-out), give the stage back.
-__device__ __forceinline__ bool stage_acquire(uint32_t full_bar, uint32_t parity, int* err_flag) {
-    bool ok = mbar_wait(full_bar, parity);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok && err_flag && (threadIdx.x & 31) == 0) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
-    return ok;
+// Consumer side of a stage: wait for the tile, give the stage back.  A wait that gives up raises the flag word and the
+// step goes on with what the stage holds (no vote: the lanes need not agree, and a vote costs as much as the wait).
+__device__ __forceinline__ void stage_acquire(uint32_t full_bar, uint32_t parity, int* err_flag) {
+    if (!mbar_wait(full_bar, parity) && err_flag) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+    __syncwarp();
 }
 __device__ __forceinline__ void stage_release(uint32_t empty_bar) {
     __syncwarp();
@@ -679,153 +697,95 @@ __device__ __noinline__ void warp_topk(const unsigned long long* logits, uint32_
 // ---------------------------------------------------------------------------------------------
 // block-wide preparation of a phase's activation vectors
 // ---------------------------------------------------------------------------------------------
-// ngroups groups of 128 fp16 values (contiguous at src; vectors of K values each) -> plane segments (vector v at
-// planes + v * 6 * (K/2 + 64)) and group scales sx[group].  With nw (one vector of at most 2048 values) the values
-// are RMS-normalised first; xh, when given, receives them as fp16 in quarters.  A half warp handles a group (eight
-// values per lane), the block twenty groups per pass (at most four passes, all requested before any is worked on).
-// The values come from a plain fp16 vector (src) or from flagged words (fsrc: `pack` values per word, waited for
-// until they carry `tag`).
-__device__ __noinline__ void prepare(float eps, const __half* __restrict__ src, const unsigned long long* fsrc, uint32_t tag, int pack,
-                                     const __half* __restrict__ nw, int K, int ngroups, unsigned char* planes, float* sx,
-                                     unsigned char* xh, float* red, int* err_flag) {
+// One vector of K <= 2048 fp16 values -> plane segments and group scales sx[group].  With nw the values are
+// RMS-normalised first; xh, when given, receives them as fp16 in quarters.  A half warp handles a group of 128 (eight
+// values per lane).  The values come from a plain fp16 vector (src) or from flagged words (fsrc: two values per word,
+// waited for until they carry `tag`).
+__device__ __noinline__ void prepare_vector(float eps, const __half* __restrict__ src, const unsigned long long* fsrc, uint32_t tag,
+                                            const __half* __restrict__ nw, int K, unsigned char* planes, float* sx, unsigned char* xh,
+                                            float* red, int* err_flag) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lane16 = lane & 15;
-    constexpr int kPerPass = 2 * kStreamWarps, kMaxPass = 4;
-    const int gi0 = warp * 2 + (lane >> 4);
-    // the raw fp16 values of this half warp's groups (pass q: group gi0 + 20 q), eight per lane
-    uint4 raw[kMaxPass];
-    bool good = true;
-    if (fsrc == nullptr) {  // plain fp16 vector (the embedding row)
-#pragma unroll
-        for (int q = 0; q < kMaxPass; ++q) {
-            const int gi = gi0 + q * kPerPass;
-            raw[q] = gi < ngroups ? *reinterpret_cast<const uint4*>(src + gi * 128 + lane16 * 8) : make_uint4(0u, 0u, 0u, 0u);
-        }
-    } else if (pack == 1) {  // one value per flagged word
-#pragma unroll
-        for (int q = 0; q < kMaxPass; ++q) {
-            const int gi = gi0 + q * kPerPass;
-            uint32_t d[8];
-            const bool act = gi < ngroups;
-            const bool on[8] = {act, act, act, act, act, act, act, act};
-            good = flag_wait<8>(fsrc + (act ? gi : 0) * 128 + lane16 * 8, on, tag, d, err_flag) && good;
-            raw[q] = make_uint4((d[0] & 0xffffu) | (d[1] << 16), (d[2] & 0xffffu) | (d[3] << 16), (d[4] & 0xffffu) | (d[5] << 16),
-                                (d[6] & 0xffffu) | (d[7] << 16));
-            if (q == 0 && ngroups <= kPerPass) break;
-        }
-    } else {  // two values per flagged word
-#pragma unroll
-        for (int q = 0; q < kMaxPass; ++q) {
-            const int gi = gi0 + q * kPerPass;
-            uint32_t d[4];
-            const bool act = gi < ngroups;
-            const bool on[4] = {act, act, act, act};
-            good = flag_wait<4>(fsrc + (act ? gi : 0) * 64 + lane16 * 4, on, tag, d, err_flag) && good;
-            raw[q] = make_uint4(d[0], d[1], d[2], d[3]);
-        }
+    const int gi = warp * 2 + (lane >> 4);
+    const bool on = gi < (K >> 7);
+    const int at = (on ? gi : 0) * 128 + lane16 * 8;
+    uint4 wv = make_uint4(0u, 0u, 0u, 0u), raw = make_uint4(0u, 0u, 0u, 0u);
+    if (nw != nullptr) wv = *reinterpret_cast<const uint4*>(nw + at);
+    if (src != nullptr) {
+        raw = *reinterpret_cast<const uint4*>(src + at);
+    } else if (on) {
+        uint32_t d[4];
+        if (!flag_wait4(fsrc + (at >> 1), tag, d, err_flag) && err_flag) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+        raw = make_uint4(d[0], d[1], d[2], d[3]);
     }
-    if (!good && err_flag) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
     __syncwarp();
-    uint4 wv = make_uint4(0u, 0u, 0u, 0u);
-    float rstd = 0.f;
-    if (nw != nullptr) {  // one pass: at most 16 groups
-        if (gi0 < ngroups) wv = *reinterpret_cast<const uint4*>(nw + gi0 * 128 + lane16 * 8);
-        float xf[8];
-        unpack8_h(gi0 < ngroups ? raw[0] : make_uint4(0u, 0u, 0u, 0u), xf);
+    float f[8];
+    unpack8_h(raw, f);
+    if (nw != nullptr) {
         float ss = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss = fmaf(xf[j], xf[j], ss);
-        ss = warp_sum(ss);
+        for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+        ss = warp_sum(on ? ss : 0.f);
         if (lane == 0) red[warp] = ss;
         consumer_sync();
         float tot = 0.f;
 #pragma unroll
         for (int w = 0; w < kStreamWarps; ++w) tot += red[w];
-        rstd = 1.0f / sqrtf(tot / static_cast<float>(K) + eps);
-    }
-    const int kshift = 31 - __clz(K);
-#pragma unroll
-    for (int q = 0; q < kMaxPass; ++q) {
-        const int gi = gi0 + q * kPerPass;
-        if (q * kPerPass >= ngroups) break;
-        const __half* xv = reinterpret_cast<const __half*>(&raw[q]);
+        const float rstd = 1.0f / sqrtf(tot / static_cast<float>(K) + eps);
+        const __half* xv = reinterpret_cast<const __half*>(&raw);
         const __half* wh = reinterpret_cast<const __half*>(&wv);
-        float f[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = nw != nullptr ? norm_elem(xv[j], rstd, wh[j]) : __half2float(xv[j]);
-        const bool on = gi < ngroups;
-        const int v = (gi * 128) >> kshift, k0 = gi * 128 - (v << kshift);
-        const float s = store_group_planes(f, planes + v * 6 * ((K >> 1) + kPad), K, k0, lane16, on);
-        if (on && lane16 == 0) sx[gi] = s;
-        if (xh != nullptr && on) {
-            uint4 o;
-            __half2 h;
-            h = __floats2half2_rn(f[0], f[1]); o.x = *reinterpret_cast<uint32_t*>(&h);
-            h = __floats2half2_rn(f[2], f[3]); o.y = *reinterpret_cast<uint32_t*>(&h);
-            h = __floats2half2_rn(f[4], f[5]); o.z = *reinterpret_cast<uint32_t*>(&h);
-            h = __floats2half2_rn(f[6], f[7]); o.w = *reinterpret_cast<uint32_t*>(&h);
-            const int qv = K >> 2, qq = k0 >> (kshift - 2);  // values per quarter, quarter of this group
-            *reinterpret_cast<uint4*>(xh + qq * (2 * qv + kPad) + (k0 - qq * qv) * 2 + lane16 * 16) = o;
-        }
+        for (int j = 0; j < 8; ++j) f[j] = norm_elem(xv[j], rstd, wh[j]);
+    }
+    const float s = store_group_planes(f, planes, K, gi * 128, lane16, on);
+    if (on && lane16 == 0) sx[gi] = s;
+    if (xh != nullptr && on) {
+        uint4 o;
+        __half2 h;
+        h = __floats2half2_rn(f[0], f[1]); o.x = *reinterpret_cast<uint32_t*>(&h);
+        h = __floats2half2_rn(f[2], f[3]); o.y = *reinterpret_cast<uint32_t*>(&h);
+        h = __floats2half2_rn(f[4], f[5]); o.z = *reinterpret_cast<uint32_t*>(&h);
+        h = __floats2half2_rn(f[6], f[7]); o.w = *reinterpret_cast<uint32_t*>(&h);
+        const int kshift = 31 - __clz(K), k0 = gi * 128;
+        const int qv = K >> 2, qq = k0 >> (kshift - 2);  // values per quarter, quarter of this group
+        *reinterpret_cast<uint4*>(xh + qq * (2 * qv + kPad) + (k0 - qq * qv) * 2 + lane16 * 16) = o;
     }
     consumer_sync();
 }
 
-// The attention output as the o_proj input: a half warp merges the splits of one head (partials (m, l, acc[128]) of
-// the (head, split) units, taken four splits at a time in split order), rounds to fp16 and builds the planes of the
-// head's group.  Lane i of the half warp holds dimensions 8i .. 8i+7.
-__device__ __noinline__ void prepare_attention_output(const StepParams& p, Smem& S) {
-    constexpr int D = kHeadDim;
+// The activations of the routed experts (ngroups <= 64 groups of 128 values, vectors of K values each, flagged words with
+// two values each) -> plane segments (vector v at planes + v * 6 * (K/2 + 64)) and group scales.  Twenty groups per pass
+// of the block, waited for in order (looking at the words of all passes at once multiplies the polling).
+__device__ __noinline__ void prepare_activations(const unsigned long long* fsrc, uint32_t tag, int K, int ngroups, unsigned char* planes,
+                                                 float* sx, int* err_flag) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lane16 = lane & 15;
-    const int head = warp * 2 + (lane >> 4);
-    const bool on = head < p.heads;
-    const int hd = on ? head : 0;
-    const float* hacc = p.attn_part + static_cast<int64_t>(hd) * p.splits * D + lane16 * 8;
-    const float* hml = p.attn_part + static_cast<int64_t>(p.heads) * p.splits * D + static_cast<int64_t>(hd) * p.splits * 2;
-    float big = -INFINITY, den = 0.f;
-    float num[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-    for (int j0 = 0; j0 < p.splits; j0 += 4) {
-        float4 a0[4], a1[4];
-        float2 mv[4];
+    constexpr int kPerPass = 2 * kStreamWarps, kMaxPass = 4;
+    const int gi0 = warp * 2 + (lane >> 4);
+    uint4 raw[kMaxPass];
+    bool good = true;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (j0 + j < p.splits) {
-                a0[j] = __ldcg(reinterpret_cast<const float4*>(hacc + (j0 + j) * D));
-                a1[j] = __ldcg(reinterpret_cast<const float4*>(hacc + (j0 + j) * D + 4));
-                mv[j] = __ldcg(reinterpret_cast<const float2*>(hml + 2 * (j0 + j)));
-            } else {
-                a0[j] = a1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                mv[j] = make_float2(-INFINITY, 0.f);
-            }
+    for (int q = 0; q < kMaxPass; ++q) {
+        const int gi = gi0 + q * kPerPass;
+        raw[q] = make_uint4(0u, 0u, 0u, 0u);
+        if (gi < ngroups) {
+            uint32_t d[4];
+            good = flag_wait4(fsrc + gi * 64 + lane16 * 4, tag, d, err_flag) && good;
+            raw[q] = make_uint4(d[0], d[1], d[2], d[3]);
         }
-        float nb = big;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) nb = fmaxf(nb, mv[j].x);
-        const float ref = nb > -INFINITY ? nb : 0.f;
-        const float keep = exp2f(big - ref);  // 0 for the first batch (big = -inf)
-        den *= keep;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) num[i] *= keep;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float w = exp2f(mv[j].x - ref);
-            den = fmaf(mv[j].y, w, den);
-            num[0] = fmaf(a0[j].x, w, num[0]);
-            num[1] = fmaf(a0[j].y, w, num[1]);
-            num[2] = fmaf(a0[j].z, w, num[2]);
-            num[3] = fmaf(a0[j].w, w, num[3]);
-            num[4] = fmaf(a1[j].x, w, num[4]);
-            num[5] = fmaf(a1[j].y, w, num[5]);
-            num[6] = fmaf(a1[j].z, w, num[6]);
-            num[7] = fmaf(a1[j].w, w, num[7]);
-        }
-        big = nb;
     }
-    float f[8];
+    if (!good && err_flag) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+    __syncwarp();
+    const int kshift = 31 - __clz(K);
+#pragma unroll 1
+    for (int gi = gi0; gi - gi0 < ngroups; gi += kPerPass) {  // all warps make the same trips: the groups meet in shuffles
+        float f[8];
+        unpack8_h(raw[0], f);
+        const bool on = gi < ngroups;
+        const int v = (gi * 128) >> kshift, k0 = gi * 128 - (v << kshift);
+        const float s = store_group_planes(f, planes + v * 6 * ((K >> 1) + kPad), K, k0, lane16, on);
+        if (on && lane16 == 0) sx[gi] = s;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = __half2float(__float2half_rn(den > 0.f ? num[j] / den : num[j]));
-    const float s = store_group_planes(f, S.xplanes, p.heads * D, hd * D, lane16, on);
-    if (on && lane16 == 0) S.xsx[hd] = s;
+        for (int q = 0; q + 1 < kMaxPass; ++q) raw[q] = raw[q + 1];
+    }
     consumer_sync();
 }
 
@@ -845,8 +805,7 @@ __device__ __noinline__ void attention_prologue(const StepParams& p, const StepL
         const int A = geo.A, h = geo.h;
         // this lane's four values of the head's q (k, v) row: flagged words written by the q.k.v phase
         uint32_t d4[4];
-        const bool on4[4] = {true, true, true, true};
-        bool good = flag_wait<4>(fqkv + warp * A + h * D + lane * 4, on4, tag, d4, p.err_flag);
+        bool good = flag_wait4(fqkv + warp * A + h * D + lane * 4, tag, d4, p.err_flag);
         const uint2 raw = make_uint2((d4[0] & 0xffffu) | (d4[1] << 16), (d4[2] & 0xffffu) | (d4[3] << 16));
         const __half* rh = reinterpret_cast<const __half*>(&raw);
         float f[4];
@@ -1106,32 +1065,64 @@ __device__ __forceinline__ void attention_tile16(unsigned char* st, AttnSm& sm, 
     __syncwarp();
 }
 
-// Merge of the block's warps into the unit's partial (m, l, acc[128]).
-__device__ __noinline__ void attention_partial(const StepParams& p, Smem& S) {
+// End of a (head, split) unit: the block's warps are merged into its partial (m, l, acc[128]).  The splits of a head hand
+// theirs to the block of its first split as flagged words; that block merges them in split order and publishes the
+// head's 128 outputs, rounded to fp16, two to a flagged word.  (All 148 blocks reading the fp32 partials of all units
+// behind a grid barrier took 7,500 cycles from the last unit's end to the planes of o_proj: 50 KB a block.)
+__device__ __noinline__ void attention_finish(const StepParams& p, Smem& S, unsigned long long* part, unsigned long long* f_attn, uint32_t tag) {
     constexpr int D = kHeadDim;
     AttnSm& sm = *reinterpret_cast<AttnSm*>(S.big);
     const Geo& geo = S.geo;
     const int tid = threadIdx.x;
-    // partial layout: acc[(h*splits + split)*D + d], then the (m, l) pairs
-    if (tid < D) {
-        constexpr int nactive = kStreamWarps;  // warps without a tile hold (-inf, 0, 0)
-        float big = -INFINITY;
-#pragma unroll 1
-        for (int w = 0; w < nactive; ++w) big = fmaxf(big, sm.wm[w]);
-        const float bs = big > -INFINITY ? big : 0.f;
-        float a = 0.f, l = 0.f;
-#pragma unroll 1
-        for (int w = 0; w < nactive; ++w) {
-            const float wt = exp2f(sm.wm[w] - bs);
+    const int others = p.splits - 1;
+    float big = -INFINITY, a = 0.f, l = 0.f;
+    if (tid < D) {  // warps without a tile hold (-inf, 0, 0)
+        float m[kStreamWarps];
+#pragma unroll
+        for (int w = 0; w < kStreamWarps; ++w) {
+            m[w] = sm.wm[w];
+            big = fmaxf(big, m[w]);
+        }
+        const float ref = big > -INFINITY ? big : 0.f;
+#pragma unroll
+        for (int w = 0; w < kStreamWarps; ++w) {
+            const float wt = exp2f(m[w] - ref);
             a = fmaf(sm.wacc[w][tid], wt, a);
             l = fmaf(sm.wl[w], wt, l);
         }
-        p.attn_part[(static_cast<int64_t>(geo.h) * p.splits + geo.split) * D + tid] = a;
-        if (tid == 0) {
-            float* ml = p.attn_part + static_cast<int64_t>(p.heads) * p.splits * D + (static_cast<int64_t>(geo.h) * p.splits + geo.split) * 2;
-            ml[0] = big;
-            ml[1] = l;
+    }
+    unsigned long long* const mine = part + static_cast<size_t>(geo.h * p.splits + geo.split) * kPartWords;
+    if (geo.split != 0) {
+        if (tid < D) flag_store(mine + tid, __float_as_uint(a), tag);
+        if (tid < 4) flag_store(mine + D + tid, tid == 0 ? __float_as_uint(big) : __float_as_uint(tid == 1 ? l : 0.f), tag);
+        return;
+    }
+    if (others > 0) {  // a thread collects four words: at most 8 x 33 of the 320 threads
+        static_assert((kMaxSplits - 1) * (kPartWords / 4) <= kConsumerThreads, "");
+        const int j = tid / (kPartWords / 4), q = tid - j * (kPartWords / 4);
+        if (j < others) {
+            uint32_t d[4];
+            if (!flag_wait4(mine + (j + 1) * kPartWords + q * 4, tag, d, p.err_flag) && p.err_flag) atomicOr(p.err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+            *reinterpret_cast<uint4*>(&sm.other[j][q * 4]) = make_uint4(d[0], d[1], d[2], d[3]);
         }
+        consumer_sync();
+    }
+    if (tid < D) {
+        float m = big;
+#pragma unroll 1
+        for (int j = 0; j < others; ++j) m = fmaxf(m, sm.other[j][D]);
+        const float ref = m > -INFINITY ? m : 0.f;
+        const float own = exp2f(big - ref);
+        float num = a * own, den = l * own;
+#pragma unroll 1
+        for (int j = 0; j < others; ++j) {
+            const float w = exp2f(sm.other[j][D] - ref);
+            den = fmaf(sm.other[j][D + 1], w, den);
+            num = fmaf(sm.other[j][tid], w, num);
+        }
+        const uint32_t out = __half_as_ushort(__float2half_rn(den > 0.f ? num / den : num));
+        const uint32_t next = __shfl_down_sync(0xffffffffu, out, 1);
+        if ((tid & 1) == 0) flag_store(f_attn + ((geo.h * D + tid) >> 1), out | (next << 16), tag);
     }
 }
 
@@ -1237,7 +1228,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
     }
     __syncthreads();  // the one barrier of all warps: from here on producers and consumers only meet at the stages
     if (warp >= kStreamWarps) {
-        producer_loop(S, p.err_flag, 2 * (warp - kStreamWarps));
+        if (elect_one()) producer_loop(S, p.err_flag, 2 * (warp - kStreamWarps));
         return;
     }
     const Geo& geo = S.geo;
@@ -1250,9 +1241,8 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
     unsigned int bar_target = epoch * static_cast<unsigned int>(p.barriers_per_launch) * gridDim.x;
     const uint32_t tag0 = epoch * 64u;  // tag of layer l's exchanges: tag0 + l + 1 (at most 33 layers per launch)
     const __half* const embed_row = p.embed + tok * static_cast<int64_t>(p.H);
-    float pw1v[4], pw2v[4];
+    float pw1v[4];
     plane_weights(t, true, pw1v);
-    plane_weights(t, false, pw2v);
     const int bseg = g < 6 ? g : (g & 1);  // plane segment this lane feeds to B: first half planes 0-2, second half planes 0-2
     float* const fsx = reinterpret_cast<float*>(S.big + kBigPlaneBytes);  // group scales of the routed experts' activations
     float pick_v = -INFINITY;
@@ -1295,54 +1285,58 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
         unsigned long long* const f_stats = p.fl_stats + par * 2048;
         unsigned long long* const f_logits = p.fl_logits + par * 128;
         unsigned long long* const f_act = p.fl_act + par * 4096;
+        unsigned long long* const f_attn = p.fl_attn + par * 1024;
         float sq = 0.f, sk = 0.f;  // phase A: sums of squares of the q / k values this lane stored
 
         if (ph == 1) {
             if (geo.has_unit) {
                 AttnSm& sm = *reinterpret_cast<AttnSm*>(S.big);
+                // the scales of a tile's positions, two per lane; those of the warp's first tile are requested before the
+                // query is waited for
+                float kscale[2], vscale[2];
+                auto load_scales = [&](int lt) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int pos = (geo.tile0 + lt) * geo.kvt + 32 * r + lane;
+                        const bool in = lt < ntiles && !geo.kv16 && 32 * r + lane < geo.kvt && pos < geo.nf;
+                        const int64_t at = static_cast<int64_t>(geo.h) * geo.S + pos;
+                        kscale[r] = in ? __half2float(__ldcg(L.ks + at)) : 0.f;
+                        vscale[r] = in ? __half2float(__ldcg(L.vs + at)) : 0.f;
+                    }
+                };
+                load_scales(lt0);
                 attention_prologue(p, L, S, f_qkv, f_stats, tag);
-                {
-                    float m_i = -INFINITY, l_i = 0.f;
-                    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                float m_i = -INFINITY, l_i = 0.f;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-                    for (int lt = lt0; lt < ntiles; lt += kStreamWarps) {
-                        if (geo.kv16) {
-                            if (!stage_acquire(full_bar, c_par, p.err_flag)) break;
-                            c_par ^= 1u;
-                            attention_tile16(my_stage, sm, geo, lt, lane, warp, p.qk_scale_log2, m_i, l_i, acc);
-                            stage_release(empty_bar);
-                            continue;
-                        }
-                        // the scales of the tile's positions (two per lane), requested before the wait for the codes
-                        float kscale[2], vscale[2];
+                for (int lt = lt0; lt < ntiles; lt += kStreamWarps) {
+                    if (lt != lt0) load_scales(lt);
+                    if (geo.owner && !geo.kv16) {  // the new token: the scales this block has just derived
 #pragma unroll
                         for (int r = 0; r < 2; ++r) {
-                            const int pos = (geo.tile0 + lt) * geo.kvt + 32 * r + lane;
-                            const bool in = 32 * r + lane < geo.kvt && pos < geo.nf;
-                            const int64_t at = static_cast<int64_t>(geo.h) * geo.S + (in ? pos : 0);
-                            const bool fresh = geo.owner && pos == geo.pos;  // the new token: the scales this block has just derived
-                            kscale[r] = fresh ? __half2float(__ushort_as_half(sm.newks)) : (in ? __half2float(__ldcg(L.ks + at)) : 0.f);
-                            vscale[r] = fresh ? __half2float(__ushort_as_half(sm.newvs)) : (in ? __half2float(__ldcg(L.vs + at)) : 0.f);
+                            if ((geo.tile0 + lt) * geo.kvt + 32 * r + lane == geo.pos && 32 * r + lane < geo.kvt) {
+                                kscale[r] = __half2float(__ushort_as_half(sm.newks));
+                                vscale[r] = __half2float(__ushort_as_half(sm.newvs));
+                            }
                         }
-                        if (!stage_acquire(full_bar, c_par, p.err_flag)) break;
-                        c_par ^= 1u;
-                        if (geo.kvt == 16) attention_tile<16>(my_stage, sm, geo, lt, lane, warp, pw1v, kscale, vscale, m_i, l_i, acc);
-                        else if (geo.kvt == 32) attention_tile<32>(my_stage, sm, geo, lt, lane, warp, pw1v, kscale, vscale, m_i, l_i, acc);
-                        else attention_tile<kKvTile>(my_stage, sm, geo, lt, lane, warp, pw1v, kscale, vscale, m_i, l_i, acc);
-                        stage_release(empty_bar);
                     }
-                    *reinterpret_cast<float4*>(&sm.wacc[warp][lane * 4]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                    if (lane == 0) {
-                        sm.wm[warp] = m_i;
-                        sm.wl[warp] = l_i;
-                    }
+                    stage_acquire(full_bar, c_par, p.err_flag);
+                    c_par ^= 1u;
+                    if (geo.kv16) attention_tile16(my_stage, sm, geo, lt, lane, warp, p.qk_scale_log2, m_i, l_i, acc);
+                    else if (geo.kvt == 16) attention_tile<16>(my_stage, sm, geo, lt, lane, warp, pw1v, kscale, vscale, m_i, l_i, acc);
+                    else if (geo.kvt == 32) attention_tile<32>(my_stage, sm, geo, lt, lane, warp, pw1v, kscale, vscale, m_i, l_i, acc);
+                    else attention_tile<kKvTile>(my_stage, sm, geo, lt, lane, warp, pw1v, kscale, vscale, m_i, l_i, acc);
+                    stage_release(empty_bar);
+                }
+                *reinterpret_cast<float4*>(&sm.wacc[warp][lane * 4]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                if (lane == 0) {
+                    sm.wm[warp] = m_i;
+                    sm.wl[warp] = l_i;
                 }
                 consumer_sync();
-                attention_partial(p, S);
+                attention_finish(p, S, p.fl_part + static_cast<size_t>(par) * p.heads * p.splits * kPartWords, f_attn, tag);
+                consumer_sync();
             }
-            // the one grid barrier of the layer: the o_proj phase of every block merges the partials of all units
-            consumer_sync();
-            grid_arrive();
         } else {
             // ---- block-wide preparation of the phase -----------------------------------------------------
             if (ph == 4) {
@@ -1362,8 +1356,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                 }
                 consumer_sync();
             } else if (ph == 2) {
-                grid_wait();
-                prepare_attention_output(p, S);
+                prepare_vector(p.eps, nullptr, f_attn, tag, nullptr, A, S.xplanes, S.xsx, nullptr, S.red, p.err_flag);
             } else if (ph == 0) {
                 if (!last && geo.has_unit && !geo.kv16) {
                     // the scales of this warp's first KV tile of the coming attention phase, towards the L2 cache
@@ -1379,11 +1372,11 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                         }
                     }
                 }
-                prepare(p.eps, embed_row, l == 0 ? nullptr : f_xin, tag - 1, 2, L.ln1, p.H, p.H >> 7, S.xplanes, S.xsx, nullptr, S.red, p.err_flag);
+                prepare_vector(p.eps, l == 0 ? embed_row : nullptr, f_xin, tag - 1, L.ln1, p.H, S.xplanes, S.xsx, nullptr, S.red, p.err_flag);
             } else if (ph == 3) {
-                prepare(p.eps, nullptr, f_xa, tag, 2, L.ln2, p.H, p.H >> 7, S.xplanes, S.xsx, S.xh, S.red, p.err_flag);
+                prepare_vector(p.eps, nullptr, f_xa, tag, L.ln2, p.H, S.xplanes, S.xsx, S.xh, S.red, p.err_flag);
             } else {
-                prepare(p.eps, nullptr, f_act, tag, 2, nullptr, p.F, (p.K * p.F) >> 7, S.big, fsx, nullptr, S.red, p.err_flag);
+                prepare_activations(f_act, tag, p.F, (p.K * p.F) >> 7, S.big, fsx, p.err_flag);
             }
             // ---- this warp's tiles of the phase: a warp finishes the rows of its tile by itself ------------------
             {
@@ -1396,34 +1389,33 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                         const int n = tg * 8 + gr;
                         resid = l == 0 ? embed_row[n] : __ushort_as_half(static_cast<unsigned short>((flag_load(f_xin + (n >> 1)) >> (16 * (n & 1))) & 0xffffu));
                     }
-                    if (!stage_acquire(full_bar, c_par, p.err_flag)) break;
+                    stage_acquire(full_bar, c_par, p.err_flag);
                     c_par ^= 1u;
                     float val;
                     if (ph == 3) {
                         val = tile_f16(my_stage, p.H, g, t, S.xh);
                         val += __shfl_xor_sync(0xffffffffu, val, 1);
                         val += __shfl_xor_sync(0xffffffffu, val, 16);
-                    } else if (ph == 5) {
-                        // one or two routed experts' rows of the same 8 outputs: each against its own activation planes
-                        const int j = udiv_small(lt, geo.f_magic), pp = lt - j * geo.ftiles;
-                        const int seg = (K >> 1) + kPad, slot = geo.fpair ? 2 * pp : pp;
-                        const __half* sc = reinterpret_cast<const __half*>(my_stage + kScaleOff) + gr * (K >> 7);
-                        val = tile_s8(my_stage, K, gr, t, S.big + slot * 6 * seg + bseg * seg, fsx + slot * (K >> 7), sc, pw2v);
-                        val += __shfl_xor_sync(0xffffffffu, val, 1);
-                        val += __shfl_xor_sync(0xffffffffu, val, 2);
-                        if (t == 0) S.part[(j * p.K + slot) * 8 + gr] = val;
-                        if (geo.fpair && slot + 1 < p.K) {  // tile rows 8-15: two runs further
-                            val = tile_s8(my_stage + 8 * K + 2 * kRunPad, K, gr, t, S.big + (slot + 1) * 6 * seg + bseg * seg, fsx + (slot + 1) * (K >> 7),
-                                          sc + 8 * (K >> 7), pw2v);
-                            val += __shfl_xor_sync(0xffffffffu, val, 1);
-                            val += __shfl_xor_sync(0xffffffffu, val, 2);
-                            if (t == 0) S.part[(j * p.K + slot + 1) * 8 + gr] = val;
-                        }
                     } else {
-                        val = tile_s8(my_stage, K, gr, t, S.xplanes + bseg * ((K >> 1) + kPad), S.xsx,
-                                      reinterpret_cast<const __half*>(my_stage + kScaleOff) + gr * (K >> 7), pw2v);
-                        val += __shfl_xor_sync(0xffffffffu, val, 1);
-                        val += __shfl_xor_sync(0xffffffffu, val, 2);
+                        // down phase: one or two routed experts' rows of the same 8 outputs, each against its own planes
+                        const int j = ph == 5 ? udiv_small(lt, geo.f_magic) : 0, pp = ph == 5 ? lt - j * geo.ftiles : 0;
+                        const int seg = (K >> 1) + kPad, slot = geo.fpair ? 2 * pp : pp;
+                        const unsigned char* st = my_stage;
+                        const unsigned char* planes = (ph == 5 ? S.big + slot * 6 * seg : S.xplanes) + bseg * seg;
+                        const float* sx = ph == 5 ? fsx + slot * (K >> 7) : S.xsx;
+                        const __half* sc = reinterpret_cast<const __half*>(my_stage + kScaleOff) + gr * (K >> 7);
+                        const bool two = ph == 5 && geo.fpair && slot + 1 < p.K;
+                        float* const part = S.part + (j * p.K + slot) * 8 + gr;
+#pragma unroll 1
+                        for (int i = 0;; ++i) {
+                            val = tile_s8(st, K, gr, t, planes, sx, sc);
+                            if (ph == 5 && t == 0) part[8 * i] = val;
+                            if (!two || i == 1) break;
+                            st += 8 * K + 2 * kRunPad;  // tile rows 8-15: two runs further
+                            planes += 6 * seg;
+                            sx += K >> 7;
+                            sc += 8 * (K >> 7);
+                        }
                     }
                     stage_release(empty_bar);
                     if (ph == 0) {
@@ -1478,7 +1470,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                     uint32_t mine = 0;
                     if (on) {
                         float out = 0.f;
-#pragma unroll 1
+#pragma unroll 4
                         for (int slot = 0; slot < p.K; ++slot) out = fmaf(S.route_w[slot], S.part[(j * p.K + slot) * 8 + r], out);
                         // the residual: this block has seen the tag of every word of the stream in the router phase
                         const __half resid = __ushort_as_half(static_cast<unsigned short>((flag_load(f_xa + (n >> 1)) >> (16 * (n & 1))) & 0xffffu));
@@ -1575,7 +1567,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
             *p.next_token = pick;
             if (p.token_log != nullptr) p.token_log[geo.pos] = pick;
             if (p.self_feed) {
-                // every block read the three step scalars before its first grid barrier, long ago: the next launch
+                // every block read the three step scalars long before it arrived at the barrier: the next launch
                 // finds the picked token, the next slot and the next length
                 *const_cast<int64_t*>(p.token) = pick;
                 *const_cast<int64_t*>(p.cache_position) += 1;

@@ -22,13 +22,6 @@ __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// One lane of a converged warp.  elect.sync instead of `lane == 0`: the compiler then knows that a single thread issues the
-// tcgen05 / TMA instruction and does not wrap it in a loop over the active lanes (8 MMAs: 300 cycles instead of 900).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-    return r != 0;
-}
 
 // Power-of-two scale of a group of fp32 values and its inverse: |x| / scale < 2^20, so x is three 7-bit digits
 // d2 * 2^14 + d1 * 2^7 + d0 (fp16 values within 2^9 of the maximum are exact, the rest good to 2^-20 of it).
