@@ -382,6 +382,12 @@ LEMOQ_API void lemoq_step_destroy(lemoq_step* step);
 /* Enqueue one decode step.  Returns the number of kernels launched through
  * *launches when it is not NULL. */
 LEMOQ_API int lemoq_step_run(lemoq_step* step, void* stream, int* launches);
+/* One captured step from the host's side in one call: the four step scalars
+ * (token, position, position, position + 1; device int64[4]) are copied in, the
+ * instantiated graph is launched, the pick (device int64) is copied to
+ * *pick_host (pinned) and the stream is waited for. */
+LEMOQ_API int lemoq_step_replay(void* graph_exec, void* stream, void* scalars, int64_t token, int64_t position,
+                                const int64_t* pick, int64_t* pick_host);
 /* Device int32 inside the workspace: 0, or a bit mask of LEMOQ_FLAG_* set by a
  * kernel that had to clamp a position, a length or an expert id. */
 LEMOQ_API int* lemoq_step_error_flag(lemoq_step* step);

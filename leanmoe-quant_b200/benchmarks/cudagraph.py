@@ -243,6 +243,8 @@ class StaticCacheDecodeSession:
         self.engine = None
         self._step = None         # plan of the native step engine (built after the first prefill)
         self._chain_host = None   # pinned buffer of replay_chained
+        self._graph_exec = None   # handle of the instantiated graph, where the native step engine replays it
+        self._pick_host = None    # pinned word the step's pick is read into
         self.after_prefill = None  # optional callable(session), run at the end of every prefill
         # graph state
         self.graph = self.stream = self.logits = None
@@ -618,6 +620,9 @@ class StaticCacheDecodeSession:
             raise CudaGraphCaptureError("capture", exc) from exc
         self.graph = graph
         self._captured_mask_independent = self._decode_mask_independent()
+        if self._step is not None and self.capture_info.get("engine") == "step" and hasattr(graph, "raw_cuda_graph_exec"):
+            self._graph_exec = int(graph.raw_cuda_graph_exec())
+            self._pick_host = torch.zeros(1, dtype=torch.int64).pin_memory()
         self.capture_info.update(capture_success=True, stream="dedicated CUDA stream",
                                  mask_independent_decode=self._captured_mask_independent)
         return dict(self.capture_info)
@@ -634,6 +639,10 @@ class StaticCacheDecodeSession:
         without, it only queues the step (same inputs next time)."""
         self._captured("replay")
         try:
+            if synchronize and self._graph_exec is not None and self._replay_skip_mask():
+                self._replay_native()
+                self.capture_info["replay_success"] = True
+                return self.logits
             with self.torch.cuda.stream(self.stream), self.torch.no_grad():
                 self._set_step_inputs(skip_mask=self._replay_skip_mask())
                 self.graph.replay()
@@ -644,6 +653,19 @@ class StaticCacheDecodeSession:
             raise CudaGraphCaptureError("replay", exc) from exc
         self.capture_info["replay_success"] = True
         return self.logits
+
+    def _replay_native(self) -> None:
+        """Inputs in, replay, pick out and the wait in one native call (the native step engine needs no mask)."""
+        from lemoq import _cabi
+
+        token = self._seeded_token("decode")
+        self._room_for(1)
+        pick = self._pick_host
+        _cabi.check(_cabi.lib().lemoq_step_replay(self._graph_exec, self.stream.cuda_stream, self.buffers.packed.data_ptr(), int(token),
+                                                  self.position, self._step["next_token"].data_ptr(), pick.data_ptr()),
+                    "lemoq_step_replay")
+        self.current_token_id = int(pick[0])
+        self.position += 1
 
     def replay_chained(self, steps: int) -> list[int]:
         """``steps`` greedy decode steps with no host work in between (native step engine only): the step inputs go to
@@ -725,3 +747,4 @@ class StaticCacheDecodeSession:
 
             _cabi.lib().lemoq_step_destroy(self._step["handle"])
             self._step = None
+            self._graph_exec = None

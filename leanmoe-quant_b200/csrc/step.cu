@@ -259,6 +259,22 @@ extern "C" const char* lemoq_step_engine(lemoq_step* s) {
 }
 extern "C" const unsigned long long* lemoq_step_phase_stamps(lemoq_step* s) { return (s && s->whole_grid > 0) ? s->stamps : nullptr; }
 
+// What a generated token costs beside the step kernel is host work and small copies; as four fills, a graph launch, a wait
+// and a read-back from Python it was 65 us of a 625 us step at 48 cached positions, here it is 17.
+extern "C" int lemoq_step_replay(void* graph_exec, void* stream, void* scalars, int64_t token, int64_t position, const int64_t* pick,
+                                 int64_t* pick_host) {
+    LEMOQ_REQUIRE(graph_exec && scalars && pick && pick_host, LEMOQ_ERR_INVALID, "step_replay: null pointer");
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int64_t words[4] = {token, position, position, position + 1};  // pageable: the driver takes its copy before the call returns
+    cudaError_t err = cudaMemcpyAsync(scalars, words, sizeof(words), cudaMemcpyHostToDevice, s);
+    if (err == cudaSuccess) err = cudaGraphLaunch(static_cast<cudaGraphExec_t>(graph_exec), s);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(pick_host, pick, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    const cudaError_t waited = cudaStreamSynchronize(s);  // in any case: `words` and pick_host are the caller's again
+    if (err == cudaSuccess) err = waited;
+    if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "step_replay: %s", cudaGetErrorString(err));
+    return LEMOQ_OK;
+}
+
 extern "C" int lemoq_step_run(lemoq_step* s, void* stream, int* launches) {
     LEMOQ_REQUIRE(s, LEMOQ_ERR_INVALID, "step_run: null step");
     const lemoq_step_desc& d = s->d;

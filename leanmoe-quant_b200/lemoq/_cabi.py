@@ -95,6 +95,7 @@ _SIGNATURES = {
     "lemoq_step_create": (c_int, [POINTER(StepDesc), POINTER(LayerDesc), POINTER(c_void_p)]),
     "lemoq_step_destroy": (None, [c_void_p]),
     "lemoq_step_run": (c_int, [c_void_p, c_void_p, POINTER(c_int)]),
+    "lemoq_step_replay": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
     "lemoq_step_error_flag": (c_void_p, [c_void_p]),
     "lemoq_step_topk_ids": (c_void_p, [c_void_p]),
     "lemoq_step_router_logits": (c_void_p, [c_void_p]),
