@@ -21,6 +21,8 @@
 // 220 KB of shared memory in use a spilled register comes back from L2 (a spilling build: 780 us a step, 568 without, at
 // 1024 cached positions), and code beyond the first-level instruction cache runs at a third of the speed.  With the
 // barrier in every layer, fp32 partials read by all blocks and three copies of the tile product the step took 646 us.
+// Keeping the block's own residual rows in shared memory and inlining the attention code (its calls saved registers on the
+// stack) made 553 of the 568.
 //
 // Arithmetic: the activation vector of a phase is turned once per block into three planes of signed
 // 7-bit digits with one power-of-two scale per group of 128 (x = sx * (d2*2^14 + d1*2^7 + d0)).  The
@@ -413,6 +415,7 @@ struct Smem {
     __align__(128) unsigned char xh[4 * (1024 + kPad)];  // fp16 copy of the normalised vector, in quarters (router rows)
     __align__(128) unsigned char big[kBigBytes > static_cast<int>(sizeof(AttnSm)) ? kBigBytes : static_cast<int>(sizeof(AttnSm))];
     float part[kPartFloats];
+    __half xres[kPartFloats];  // residual stream, the rows of this block's o_proj and down tiles (the same rows): row j * 8 + r
     float red[64];
     float cs[2 * kHeadDim];
     int route_id[32];
@@ -570,10 +573,14 @@ __device__ __forceinline__ void producer_loop(Smem& S, int* err_flag, int first_
 #pragma unroll 1
     while (ok && (c.kind != KEND || other.kind != KEND)) {
         if (c.kind != KEND) {
-            if (c.kind >= KE) {  // expert tiles: the routing of the layer must be known
+            if (c.kind >= KE) {
+                // expert tiles: the routing of the layer must be known.  (A word and not a barrier: a producer need not have
+                // tiles in every layer, so it may come two phases late.  Asleep between looks: looking all the time costs the
+                // consumer warps of the block 2 % of the step.)
                 uint32_t n = 0;
                 while (S.ready_layer < c.layer) {
-                    if (++n > (1u << 24)) {
+                    __nanosleep(64);
+                    if (++n > (1u << 22)) {
                         ok = false;
                         break;
                     }
@@ -795,7 +802,7 @@ __device__ __noinline__ void prepare_activations(const unsigned long long* fsrc,
 // Warp 0: q (RMSNorm over all heads, RoPE, softmax scale, digit planes).  Warp 1 / warp 2 of the block that owns
 // the new position: the new K row (norm, RoPE) / V row into the fp16 cache and, quantised, into the int8 mirror
 // and shared memory.  Lane i holds dimensions 4i .. 4i+3; the RoPE partner (d +- 64) lives 16 lanes away.
-__device__ __noinline__ void attention_prologue(const StepParams& p, const StepLayer& L, Smem& S, const unsigned long long* fqkv,
+__device__ __forceinline__ void attention_prologue(const StepParams& p, const StepLayer& L, Smem& S, const unsigned long long* fqkv,
                                                 const unsigned long long* fstats, uint32_t tag) {
     constexpr int D = kHeadDim;
     AttnSm& sm = *reinterpret_cast<AttnSm*>(S.big);
@@ -1069,7 +1076,7 @@ __device__ __forceinline__ void attention_tile16(unsigned char* st, AttnSm& sm, 
 // theirs to the block of its first split as flagged words; that block merges them in split order and publishes the
 // head's 128 outputs, rounded to fp16, two to a flagged word.  (All 148 blocks reading the fp32 partials of all units
 // behind a grid barrier took 7,500 cycles from the last unit's end to the planes of o_proj: 50 KB a block.)
-__device__ __noinline__ void attention_finish(const StepParams& p, Smem& S, unsigned long long* part, unsigned long long* f_attn, uint32_t tag) {
+__device__ __forceinline__ void attention_finish(const StepParams& p, Smem& S, unsigned long long* part, unsigned long long* f_attn, uint32_t tag) {
     constexpr int D = kHeadDim;
     AttnSm& sm = *reinterpret_cast<AttnSm*>(S.big);
     const Geo& geo = S.geo;
@@ -1385,10 +1392,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                 for (int lt = lt0; lt < ntiles; lt += kStreamWarps) {
                     const int tg = b + lt * G;  // global tile index (not in the down phase)
                     __half resid = __float2half_rn(0.f);
-                    if (ph == 2) {  // the residual of this lane's row (this block has seen the tag of every word in phase A)
-                        const int n = tg * 8 + gr;
-                        resid = l == 0 ? embed_row[n] : __ushort_as_half(static_cast<unsigned short>((flag_load(f_xin + (n >> 1)) >> (16 * (n & 1))) & 0xffffu));
-                    }
+                    if (ph == 2) resid = l == 0 ? embed_row[tg * 8 + gr] : S.xres[lt * 8 + gr];
                     stage_acquire(full_bar, c_par, p.err_flag);
                     c_par ^= 1u;
                     float val;
@@ -1438,7 +1442,9 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                     } else if (ph == 2) {
                         // the residual stream travels two values per word: tile rows r and r + 1 meet in the even row's lane
                         // (the lanes of tile row r + 1 are those of instruction row g + 2)
-                        const uint32_t mine = __half_as_ushort(__hadd(__float2half_rn(val), resid));
+                        const __half sum = __hadd(__float2half_rn(val), resid);
+                        if (t == 0) S.xres[lt * 8 + gr] = sum;
+                        const uint32_t mine = __half_as_ushort(sum);
                         const uint32_t next = __shfl_down_sync(0xffffffffu, mine, 8);
                         if (t == 0 && (gr & 1) == 0) flag_store(f_xa + ((tg * 8 + gr) >> 1), mine | (next << 16), tag);
                     } else if (ph == 3) {
@@ -1472,9 +1478,9 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                         float out = 0.f;
 #pragma unroll 4
                         for (int slot = 0; slot < p.K; ++slot) out = fmaf(S.route_w[slot], S.part[(j * p.K + slot) * 8 + r], out);
-                        // the residual: this block has seen the tag of every word of the stream in the router phase
-                        const __half resid = __ushort_as_half(static_cast<unsigned short>((flag_load(f_xa + (n >> 1)) >> (16 * (n & 1))) & 0xffffu));
-                        mine = __half_as_ushort(__hadd(__float2half_rn(out), resid));
+                        const __half sum = __hadd(__float2half_rn(out), S.xres[i]);
+                        S.xres[i] = sum;
+                        mine = __half_as_ushort(sum);
                     }
                     const uint32_t next = __shfl_down_sync(0xffffffffu, mine, 1);  // row n + 1: the neighbouring thread
                     if (on && (r & 1) == 0) flag_store(f_x2 + (n >> 1), mine | (next << 16), tag);
