@@ -15,6 +15,7 @@ produce that forward:
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 import os
@@ -661,9 +662,11 @@ class StaticCacheDecodeSession:
         token = self._seeded_token("decode")
         self._room_for(1)
         pick = self._pick_host
-        _cabi.check(_cabi.lib().lemoq_step_replay(self._graph_exec, self.stream.cuda_stream, self.buffers.packed.data_ptr(), int(token),
-                                                  self.position, self._step["next_token"].data_ptr(), pick.data_ptr()),
-                    "lemoq_step_replay")
+        home = self.stream.device.index
+        with contextlib.nullcontext() if self.torch.cuda.current_device() == home else self.torch.cuda.device(home):
+            rc = _cabi.lib().lemoq_step_replay(self._graph_exec, self.stream.cuda_stream, self.buffers.packed.data_ptr(), int(token),
+                                               self.position, self._step["next_token"].data_ptr(), pick.data_ptr())
+        _cabi.check(rc, "lemoq_step_replay")
         self.current_token_id = int(pick[0])
         self.position += 1
 
