@@ -93,11 +93,6 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
 __device__ __forceinline__ void red_release_add(unsigned int* p, unsigned int v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ uint2 ld_cg8(const void* p) {
-    uint2 v;
-    asm volatile("ld.global.cg.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
 // ---- flagged words: how the blocks hand small vectors to each other without a grid barrier --------------------
 // A value travels as one 8-byte word {32 bits of data, 32-bit tag}; the tag is the sequence number of the layer
 // (unique over launches).  8-byte accesses are single-copy atomic, so a reader that sees the tag it waits for (or
