@@ -362,7 +362,7 @@ class StaticCacheDecodeSession:
         kv_int8 = fusion_enabled("kv_int8")
         max_len = self.config.max_cache_len
         cos, sin = m.model.rotary_emb.tables(max_len, self.dtype, self.device)
-        keep: list[Any] = [cos, sin]
+        keep: list[Any] = [cos, sin]  # the plan reads these for as long as it lives, also when the model is given other tensors
         layers = (_cabi.LayerDesc * cfg.num_hidden_layers)()
         for i, layer in enumerate(m.model.layers):
             attn, mlp = layer.self_attn, layer.mlp
@@ -375,10 +375,10 @@ class StaticCacheDecodeSession:
             d.q_norm, d.k_norm = _cabi.ptr(attn.q_norm.weight), _cabi.ptr(attn.k_norm.weight)
             d.qkv_codes, d.qkv_scale = _cabi.ptr(pk.packed), _cabi.ptr(pk.scale)
             d.o_codes, d.o_scale = _cabi.ptr(attn.o_proj.packed), _cabi.ptr(attn.o_proj.scale)
-            router = mlp._static_router
-            if not router.is_contiguous():
-                router = router.contiguous()
-                keep.append(router)
+            router = mlp._static_router.contiguous()
+            keep += [t.detach() for t in (layer.input_layernorm.weight, layer.post_attention_layernorm.weight, attn.q_norm.weight, attn.k_norm.weight, router,
+                                          pk.packed, pk.scale, attn.o_proj.packed, attn.o_proj.scale, ex.packed_gate_up, ex.scale_gate_up, ex.packed_down,
+                                          ex.scale_down, cl.keys, cl.values)]
             d.router = _cabi.ptr(router)
             d.gu_codes, d.gu_scale = _cabi.ptr(ex.packed_gate_up), _cabi.ptr(ex.scale_gate_up)
             d.dn_codes, d.dn_scale = _cabi.ptr(ex.packed_down), _cabi.ptr(ex.scale_down)
@@ -392,6 +392,8 @@ class StaticCacheDecodeSession:
 
                 attn._lemoq_kv_int8_src_cache_ref = weakref.ref(self.cache)
                 d.kc, d.ks, d.vc, d.vs = (_cabi.ptr(bufs[n]) for n in ("kc", "ks", "vc", "vs"))
+                keep += [bufs[n] for n in ("kc", "ks", "vc", "vs")]
+        keep += [t.detach() for t in (m.model.embed_tokens.weight, m.model.norm.weight, m.lm_head.packed, m.lm_head.scale)]
         desc = _cabi.StepDesc()
         desc.layers, desc.hidden, desc.heads, desc.head_dim = cfg.num_hidden_layers, cfg.hidden_size, cfg.num_attention_heads, cfg.head_dim
         desc.experts, desc.top_k, desc.ffn, desc.vocab = cfg.num_experts, cfg.num_experts_per_tok, cfg.intermediate_size, cfg.vocab_size

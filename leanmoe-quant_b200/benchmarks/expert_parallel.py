@@ -423,12 +423,17 @@ class ExpertParallelDecoder:
         with torch.cuda.graph(graph, capture_error_mode="thread_local"):
             self.static_logits = self._forward(self.static_tokens)
         self.graph = graph
+        # the graph reads the weights where they were: they live as long as it does, also when the model is given others
+        weights = (self.native or {}).get("weights")
+        self.graph_weights = [] if weights is None else [t.detach() for t in weights.tensors()]
 
     def _forward(self, tokens: Any) -> Any:
         if self.native is not None and self.sections is None:
             from lemoq.prompt import run_lockstep
 
-            return run_lockstep(self.native, tokens.contiguous(), self.pos_t, self.filled_t, self.cfg.vocab_size, self.err)
+            logits = run_lockstep(self.native, tokens.contiguous(), self.pos_t, self.filled_t, self.cfg.vocab_size, self.err)
+            if logits is not None:
+                return logits
         from lemoq import _cabi
         from lemoq.kernels.batched_w8 import w8_linear_tokens
         from lemoq.kernels.dequant_gemv import dequant_gemm_fused

@@ -1,92 +1,89 @@
 """Many tokens through the whole model in one native call, for models in the canonical W8 form: a prompt (``lemoq_prompt_run``), or one
 token of each of many sequences (``lemoq_lockstep_run``).
 
-The module tree's own forward stays the path of everything else; :func:`run_prompt` and :func:`lockstep_plan` return None for
-what the native path does not take.
+The module tree's own forward stays the path of everything else; :func:`run_prompt`, :func:`lockstep_plan` and :func:`run_lockstep` return
+None for what the native path does not take.  The model is read anew at every call, as its modules' forwards would read it: nothing of a
+call is kept for the next by the address or identity of a tensor or module.
 """
 
 from __future__ import annotations
 
-from typing import Any
+from array import array
+from typing import Any, NamedTuple
 
 import torch
 import torch.nn.functional as F
 
 from lemoq import _cabi
 
-_PLAN = "_lemoq_prompt_plan"  # on the cache object: descriptors of one model over that cache
+_PLAN = "_lemoq_prompt_plan"  # on the cache object: what the last native call over that cache was given
+
+# the weights of a layer, in the order of ``LayerDesc``; behind them come the cache tensors
+_LAYER_WEIGHTS = ("ln1", "ln2", "q_norm", "k_norm", "qkv_codes", "qkv_scale", "o_codes", "o_scale", "router", "gu_codes", "gu_scale", "dn_codes", "dn_scale")
+_CACHES = ("keys", "values", "kc", "ks", "vc", "vs")
+assert _LAYER_WEIGHTS + _CACHES == tuple(name for name, _ in _cabi.LayerDesc._fields_)
 
 
-def _layer_parts(layer: Any) -> tuple | None:
-    """The quantised pieces of a decoder layer, or None when a piece is not in the form the native path knows."""
+class Weights(NamedTuple):
+    """The tensors of a model in the canonical form."""
+
+    own: dict      # field of ``StepDesc`` -> tensor
+    layers: list   # per layer, in the order of ``_LAYER_WEIGHTS``
+
+    def tensors(self) -> list:
+        return [*self.own.values(), *(t for layer in self.layers for t in layer)]
+
+
+def read_weights(model: Any) -> Weights | None:
+    """The tensors that the model's forwards would use now; None when a piece is not in the form the native path knows.  (Through the
+    modules' own dictionaries: 300 attribute look-ups of ``nn.Module`` would take longer than the launches of a short prompt.)"""
     from lemoq.kernels.attn_decode import _decode_forward_impl
     from lemoq.kernels.moe_grouped_quant import QuantFusedExperts
-    from lemoq.model import OlmoeAttention
+    from lemoq.model import OlmoeAttention, OlmoeDecoderLayer
     from lemoq.quant.linear import QuantLinear
 
-    attn, mlp = layer.self_attn, layer.mlp
-    here = attn.__dict__
-    packed, o_proj = here.get("_lemoq_packed_qkv"), attn.o_proj
-    stacks = mlp.__dict__.get("_static_experts")
-    plain = getattr(here.get("_lemoq_original_forward"), "__func__", None)
-    ok = (packed is not None and isinstance(o_proj, QuantLinear) and o_proj.bias is None and isinstance(stacks, QuantFusedExperts)
-          and getattr(here.get("forward"), "__func__", None) is _decode_forward_impl and plain is OlmoeAttention.forward
-          and attn.num_key_value_groups == 1 and mlp._static_act in (None, F.silu))
-    return (attn, mlp, packed, o_proj, stacks) if ok else None
-
-
-def _signature(model: Any) -> tuple | None:
-    """The objects a plan was made from; None when the model is not in the canonical form."""
-    from lemoq.quant.linear import QuantLinear
-
-    cfg, lm = model.config, model.lm_head
-    if not isinstance(lm, QuantLinear) or lm.bias is not None or cfg.clip_qkv is not None:
+    m, lm = model.model, model.lm_head
+    if type(lm) is not QuantLinear or lm.bias is not None or model.config.clip_qkv is not None or not len(m.layers):
         return None
-    parts = [_layer_parts(layer) for layer in model.model.layers]
-    if not parts or any(p is None for p in parts):
-        return None
-    return (lm, model.model.embed_tokens.weight, *parts)
+    layers = []
+    for layer in m.layers:
+        if type(layer) is not OlmoeDecoderLayer:
+            return None
+        parts = layer._modules
+        attn, mlp = parts["self_attn"], parts["mlp"]
+        inner, here, moe = attn._modules, attn.__dict__, mlp.__dict__
+        packed, o_proj, stacks = here.get("_lemoq_packed_qkv"), inner.get("o_proj"), moe.get("_static_experts")
+        if (packed is None or type(o_proj) is not QuantLinear or o_proj._buffers["bias"] is not None or not isinstance(stacks, QuantFusedExperts)
+                or getattr(here.get("forward"), "__func__", None) is not _decode_forward_impl
+                or getattr(here.get("_lemoq_original_forward"), "__func__", None) is not OlmoeAttention.forward
+                or here["num_key_value_groups"] != 1 or moe["_static_act"] not in (None, F.silu)):
+            return None
+        norms = [norm._parameters.get("weight") for norm in (parts["input_layernorm"], parts["post_attention_layernorm"], inner["q_norm"], inner["k_norm"])]
+        if any(t is None for t in norms):
+            return None
+        layers.append((*norms, packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"], moe["_static_router"].contiguous(),
+                       stacks.packed_gate_up, stacks.scale_gate_up, stacks.packed_down, stacks.scale_down))
+    return Weights({"embed": m.embed_tokens.weight, "final_norm": m.norm.weight, "lm_head_codes": lm.packed, "lm_head_scale": lm.scale}, layers)
 
 
-def _describe(model: Any, signature: tuple, max_len: int, caches: list[dict]) -> dict:
-    """The model and one set of cache tensors per layer (named as in ``LayerDesc``) for the C side: pointers only."""
+def describe(model: Any, weights: Weights, max_len: int, caches: list[dict]) -> tuple[Any, Any]:
+    """``(StepDesc, LayerDesc array)`` of the model over one set of cache tensors per layer (named as in ``LayerDesc``): pointers only, the
+    caller keeps the tensors for as long as the C side may read them."""
     cfg, m = model.config, model.model
-    device = m.embed_tokens.weight.device
-    cos, sin = m.rotary_emb.tables(max_len, torch.float16, device)
-    layers = (_cabi.LayerDesc * len(m.layers))()
-    keep: list[Any] = [cos, sin]
-    for d, layer, (attn, mlp, packed, o_proj, stacks), slots in zip(layers, m.layers, signature[2:], caches):
-        router = mlp._static_router.contiguous()
-        keep += [router, slots]
-        tensors = {"ln1": layer.input_layernorm.weight, "ln2": layer.post_attention_layernorm.weight, "q_norm": attn.q_norm.weight,
-                   "k_norm": attn.k_norm.weight, "qkv_codes": packed.packed, "qkv_scale": packed.scale, "o_codes": o_proj.packed,
-                   "o_scale": o_proj.scale, "router": router, "gu_codes": stacks.packed_gate_up, "gu_scale": stacks.scale_gate_up,
-                   "dn_codes": stacks.packed_down, "dn_scale": stacks.scale_down, **slots}
-        for name, t in tensors.items():
-            setattr(d, name, _cabi.ptr(t))
+    cos, sin = m.rotary_emb.tables(max_len, torch.float16, m.embed_tokens.weight.device)
+    words = array("Q")
+    for layer, slots in zip(weights.layers, caches):
+        words.extend([t.data_ptr() for t in layer])
+        words.extend([0 if slots.get(name) is None else slots[name].data_ptr() for name in _CACHES])
     desc = _cabi.StepDesc()
     desc.layers, desc.hidden, desc.heads, desc.head_dim = len(m.layers), cfg.hidden_size, cfg.num_attention_heads, cfg.head_dim
     desc.experts, desc.top_k, desc.ffn, desc.vocab = cfg.num_experts, cfg.num_experts_per_tok, cfg.intermediate_size, cfg.vocab_size
     desc.group_size, desc.max_len, desc.eps = int(model.lm_head.group_size), max_len, float(cfg.rms_norm_eps)
     desc.norm_topk_prob = int(bool(cfg.norm_topk_prob))
-    desc.embed, desc.final_norm = _cabi.ptr(m.embed_tokens.weight), _cabi.ptr(m.norm.weight)
-    desc.lm_head_codes, desc.lm_head_scale = _cabi.ptr(model.lm_head.packed), _cabi.ptr(model.lm_head.scale)
-    desc.rope_cos, desc.rope_sin = _cabi.ptr(cos), _cabi.ptr(sin)
-    return {"signature": signature, "desc": desc, "layers": layers, "keep": keep}
-
-
-def _prompt_plan(model: Any, cache: Any, signature: tuple) -> dict:
-    cfg, device = model.config, model.model.embed_tokens.weight.device
-    for slot in cache.layers:
-        if not slot.is_initialized:
-            slot.lazy_initialization(torch.empty((1, cfg.num_attention_heads, 1, cfg.head_dim), dtype=torch.float16, device=device))
-    plan = _describe(model, signature, cache.max_cache_len, [{"keys": s.keys, "values": s.values} for s in cache.layers])
-    plan.update(caches=tuple(s.keys for s in cache.layers), flags=torch.zeros(1, dtype=torch.int32, device=device))
-    return plan
-
-
-def _same(a: tuple, b: tuple) -> bool:
-    return len(a) == len(b) and all(x is y or (isinstance(x, tuple) and _same(x, y)) for x, y in zip(a, b))
+    for name, t in weights.own.items():
+        setattr(desc, name, t.data_ptr())
+    desc.rope_cos, desc.rope_sin = cos.data_ptr(), sin.data_ptr()
+    return desc, (_cabi.LayerDesc * len(m.layers)).from_buffer(words)
 
 
 def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, position_ids: Any) -> Any:
@@ -100,42 +97,52 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
             or position_ids.data_ptr() != cache_position.data_ptr() or position_ids.numel() != cache_position.numel() or not cache_position.is_contiguous()
             or len(cache.layers) != len(model.model.layers) or not _cabi.available()):
         return None
-    signature = _signature(model)
-    if signature is None:
+    weights = read_weights(model)
+    if weights is None:
         return None
-    plan = cache.__dict__.get(_PLAN)
-    if plan is None or not _same(plan["signature"], signature) or any(s.keys is not k for s, k in zip(cache.layers, plan["caches"])):
-        plan = cache.__dict__[_PLAN] = _prompt_plan(model, cache, signature)
+    cfg, device = model.config, weight.device
+    for slot in cache.layers:
+        if not slot.is_initialized:
+            slot.lazy_initialization(torch.empty((1, cfg.num_attention_heads, 1, cfg.head_dim), dtype=torch.float16, device=device))
+    desc, layers = describe(model, weights, cache.max_cache_len, [{"keys": s.keys, "values": s.values} for s in cache.layers])
     tokens = int(input_ids.shape[1])
-    size = int(_cabi.lib().lemoq_prompt_workspace_bytes(plan["desc"], tokens))
+    size = int(_cabi.lib().lemoq_prompt_workspace_bytes(desc, tokens))
     if size == 0:
         return None
-    ids, device = input_ids.contiguous(), weight.device
-    logits = torch.empty((1, tokens, model.config.vocab_size), dtype=torch.float16, device=device)
+    plan = cache.__dict__.setdefault(_PLAN, {})
+    if plan.get("flags") is None:
+        plan["flags"] = torch.zeros(1, dtype=torch.int32, device=device)
+    ids = input_ids.contiguous()
+    logits = torch.empty((1, tokens, cfg.vocab_size), dtype=torch.float16, device=device)
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
-    _cabi.call("lemoq_prompt_run", plan["desc"], plan["layers"], _cabi.ptr(ids), _cabi.ptr(cache_position), tokens, _cabi.ptr(logits),
+    _cabi.call("lemoq_prompt_run", desc, layers, _cabi.ptr(ids), _cabi.ptr(cache_position), tokens, _cabi.ptr(logits),
                _cabi.ptr(workspace), size, _cabi.ptr(plan["flags"]), _cabi.current_stream(device))
     return logits
 
 
-def lockstep_plan(model: Any, kv: list[dict], sequences: int, max_len: int) -> Any:
-    """What :func:`run_lockstep` needs for ``sequences`` sequences with the int8 caches ``kv`` (per layer ``kc/vc (B*heads, S, D)``,
-    ``ks/vs (B*heads, S)``), or None when the model is not in the canonical form."""
-    signature = _signature(model) if _cabi.available() and model.model.embed_tokens.weight.dtype == torch.float16 else None
-    if signature is None:
+def lockstep_plan(model: Any, kv: list[dict], sequences: int, max_len: int) -> dict | None:
+    """What :func:`run_lockstep` keeps from step to step for ``sequences`` sequences with the int8 caches ``kv`` (per layer ``kc/vc
+    (B*heads, S, D)``, ``ks/vs (B*heads, S)``), or None when the model is not in the canonical form."""
+    weights = read_weights(model) if _cabi.available() and model.model.embed_tokens.weight.dtype == torch.float16 else None
+    if weights is None:
         return None
-    plan = _describe(model, signature, max_len, kv)
-    size = int(_cabi.lib().lemoq_lockstep_workspace_bytes(plan["desc"], sequences))
+    size = int(_cabi.lib().lemoq_lockstep_workspace_bytes(describe(model, weights, max_len, kv)[0], sequences))
     if size == 0:
         return None
-    plan["workspace"] = torch.zeros(size, dtype=torch.uint8, device=model.model.embed_tokens.weight.device)
-    return plan
+    workspace = torch.zeros(size, dtype=torch.uint8, device=model.model.embed_tokens.weight.device)
+    return {"model": model, "kv": kv, "max_len": max_len, "workspace": workspace}
 
 
 def run_lockstep(plan: dict, tokens: Any, position: Any, filled: Any, vocab: int, flags: Any) -> Any:
-    """Logits ``(B, V)`` of one token per sequence; ``position`` and ``filled`` are device scalars."""
+    """Logits ``(B, V)`` of one token per sequence; ``position`` and ``filled`` are device scalars.  None when the model has left the
+    canonical form.  ``plan["weights"]``: the tensors this call reads (a captured step's graph reads them at every replay)."""
+    weights = read_weights(plan["model"])
+    if weights is None:
+        return None
+    desc, layers = describe(plan["model"], weights, plan["max_len"], plan["kv"])
     rows, workspace = int(tokens.shape[0]), plan["workspace"]
     logits = torch.empty((rows, vocab), dtype=torch.float16, device=tokens.device)
-    _cabi.call("lemoq_lockstep_run", plan["desc"], plan["layers"], _cabi.ptr(tokens), _cabi.ptr(position), _cabi.ptr(filled), rows, _cabi.ptr(logits),
+    _cabi.call("lemoq_lockstep_run", desc, layers, _cabi.ptr(tokens), _cabi.ptr(position), _cabi.ptr(filled), rows, _cabi.ptr(logits),
                _cabi.ptr(workspace), workspace.numel(), _cabi.ptr(flags), _cabi.current_stream(tokens.device))
+    plan["weights"] = weights
     return logits

@@ -121,3 +121,32 @@ def test_lockstep_matches_the_step_by_parts(sequences):
     for a, b in zip(decoders[0].kv, decoders[1].kv):
         assert float((a["kc"] != b["kc"]).float().mean()) < 1e-2 and rel_err(a["vs"], b["vs"]) < 1e-2
     assert decoders[0].error_flags() == 0
+
+
+def test_replaced_weights_are_the_ones_a_prompt_uses():
+    """The tensors of a model may be exchanged between two prompts of a session, and between a step and its capture."""
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+    from benchmarks.expert_parallel import ExpertParallelDecoder
+
+    spec = glue.OlmoeSpec(layers=2, hidden=256, heads=2, head_dim=128, experts=8, top_k=2, ffn=128, vocab=512)
+    wf = glue.random_float_weights(spec, seed=3, dtype=torch.float16, std=0.05, norm_weight_jitter=0.1)
+    model, tokens = lemoq_model_from_oracle(wf), 40
+    install_canonical(model, tokens, 4)
+    prompt = torch.tensor([[(11 * i * i + 3) % spec.vocab for i in range(tokens)]], device=DEV)
+    session = StaticCacheDecodeSession(model, prompt, ctx=tokens, max_new_tokens=4, engine="ops")
+    decoder = ExpertParallelDecoder(model, session, sequences=2, world=1, rank=0, static_exchange=True)
+    first = session.prefill().logits.clone()
+    step = lambda d: (setattr(d, "position", tokens), d.step(torch.tensor([1, 2], device=DEV)).clone())[1]  # noqa: E731
+    stepped = step(decoder)
+    lm, norm = model.lm_head, model.model.layers[1].input_layernorm
+    kept = norm.weight, lm.scale
+    norm.weight, lm.scale = torch.nn.Parameter(-norm.weight.detach()), lm.scale * 2
+    other, other_step = session.prefill().logits.clone(), step(decoder)
+    fresh = StaticCacheDecodeSession(model, prompt, ctx=tokens, max_new_tokens=4, engine="ops")
+    assert torch.equal(other, fresh.prefill().logits) and rel_err(other, first) > 0.5 and rel_err(other_step, stepped) > 0.5
+    decoder.capture()
+    assert torch.equal(step(decoder), other_step)
+    norm.weight, lm.scale = kept
+    torch.empty(1 << 20, dtype=torch.uint8, device=DEV).fill_(255)  # would land on freed weights
+    assert torch.equal(step(decoder), other_step)  # a captured graph goes on with the weights it was captured with
+    assert torch.equal(session.prefill().logits, first)

@@ -1,0 +1,77 @@
+"""How the native paths read a model (no GPU)."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import lemoq_oracle as ops
+
+
+@pytest.fixture
+def canonical(monkeypatch):
+    """Builder of a small canonical model on the CPU; ``experts``: group size of the experts' scales."""
+    import lemoq.quant.rtn as rtn
+    from lemoq.kernels.attn_decode import replace_attention_cores
+    from lemoq.kernels.moe_grouped_quant import QuantFusedExperts
+    from lemoq.kernels.moe_static import fuse_experts, replace_moe_blocks
+    from lemoq.kernels.packed_qkv import install_packed_qkv
+    from lemoq.kernels.rmsnorm import replace_rms_norms
+    from lemoq.model import OlmoeConfig, OlmoeForCausalLM
+    from lemoq.quant.linear import SchemeSpec, quantize_model
+
+    monkeypatch.setattr(rtn, "quantize_w8", lambda w, g=128: ops.rtn_quantize_w8(w.detach().float(), g))
+
+    def build(experts=128):
+        torch.manual_seed(0)
+        cfg = OlmoeConfig(vocab_size=64, hidden_size=256, intermediate_size=256, num_hidden_layers=2, num_attention_heads=2,
+                          num_key_value_heads=2, num_experts=8, num_experts_per_tok=2)
+        model = OlmoeForCausalLM(cfg).to(torch.float16).eval()
+        packed = {}
+        for i, layer in enumerate(model.model.layers):
+            fused = fuse_experts(layer.mlp.experts)
+            packed[i] = QuantFusedExperts(*ops.rtn_quantize_w8(fused.gate_up.float(), experts), *ops.rtn_quantize_w8(fused.down.float(), experts), 8, experts)
+        replace_rms_norms(model, "fused")
+        replace_moe_blocks(model, impl="grouped", prequantized=packed)
+        quantize_model(model, SchemeSpec.from_flags("w8a16", 128, targets=("attention", "experts", "lm_head"), keep_lm_head_fp16=False))
+        replace_attention_cores(model, backend="cuda")
+        install_packed_qkv(model)
+        return model
+
+    return build
+
+
+def test_a_description_follows_the_tensors_of_the_model(canonical):
+    """Nothing is kept by a module's identity: whatever replaces a parameter or a buffer is what the next call is given."""
+    from lemoq.prompt import describe, read_weights
+
+    model = canonical()
+    caches = [{"keys": torch.zeros(1, 2, 8, 128, dtype=torch.float16), "values": torch.zeros(1, 2, 8, 128, dtype=torch.float16)} for _ in range(2)]
+
+    def pointers():
+        desc, layers = describe(model, read_weights(model), 8, caches)
+        return [getattr(desc, n) for n in ("embed", "final_norm", "lm_head_codes", "lm_head_scale")], [[getattr(d, n) for n, _ in d._fields_] for d in layers]
+
+    def moved():
+        """Fields of the model and of the last layer that are given other tensors than before."""
+        nonlocal before
+        after = pointers()
+        names = [n for n, a, b in zip(("embed", "final_norm", "lm_head_codes", "lm_head_scale"), before[0], after[0]) if a != b]
+        names += [n for (n, _), a, b in zip(type(describe(model, read_weights(model), 8, caches)[1][0])._fields_, before[1][-1], after[1][-1]) if a != b]
+        before = after
+        return names
+
+    before, last = pointers(), model.model.layers[-1]
+    keep = []  # nothing may land where the old tensor was
+    for change, expected in ((lambda: setattr(last.input_layernorm, "weight", torch.nn.Parameter(last.input_layernorm.weight.clone())), ["ln1"]),
+                             (lambda: setattr(last.self_attn.q_norm.weight, "data", last.self_attn.q_norm.weight.data.clone()), ["q_norm"]),
+                             (lambda: setattr(last.self_attn.o_proj, "packed", last.self_attn.o_proj.packed.clone()), ["o_codes"]),
+                             (lambda: setattr(last.mlp._static_experts, "scale_down", last.mlp._static_experts.scale_down.clone()), ["dn_scale"]),
+                             (lambda: model.lm_head.load_state_dict({k: v.clone() for k, v in model.lm_head.state_dict().items()}, assign=True),
+                              ["lm_head_codes", "lm_head_scale"]),
+                             (lambda: caches[-1].update(keys=caches[-1]["keys"].clone()), ["keys"])):
+        keep.append([t.detach() for t in read_weights(model).tensors()] + [c["keys"] for c in caches])
+        change()
+        assert moved() == expected
+    last.self_attn.o_proj.bias = torch.zeros(256)
+    assert read_weights(model) is None  # and what it no longer describes is not taken
