@@ -335,7 +335,9 @@ class StaticCacheDecodeSession:
                 return "layer %d: GQA" % i
             if getattr(m.config, "clip_qkv", None) is not None:
                 return "clip_qkv is set"
-        return None
+        from lemoq.prompt import form_blocker
+
+        return form_blocker(m)  # group sizes, top_k, shapes: one description for all layers
 
     def _select_engine(self) -> str:
         if self.engine is not None:

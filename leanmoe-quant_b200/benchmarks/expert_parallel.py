@@ -463,11 +463,10 @@ class ExpertParallelDecoder:
         for i, layer in enumerate(self.model.model.layers):
             attn, mlp = layer.self_attn, layer.mlp
             pk = attn._lemoq_packed_qkv
-            gs = int(pk.group_size)
             dense = sec("dense + attention")
             dense.__enter__()
             h1 = rms_norm_fused(x, layer.input_layernorm.weight, eps)
-            qkv = linear(h1, pk.packed, pk.scale, gs)  # (b, 3A)
+            qkv = linear(h1, pk.packed, pk.scale, int(pk.group_size))  # (b, 3A)
             q = rms_norm_fused(qkv[:, :a].contiguous(), attn.q_norm.weight, eps)
             k = rms_norm_fused(qkv[:, a:2 * a].contiguous(), attn.k_norm.weight, eps)
             v = qkv[:, 2 * a:].contiguous()
@@ -483,11 +482,11 @@ class ExpertParallelDecoder:
             _cabi.call("lemoq_attn_decode_int8", _cabi.ptr(q_r), _cabi.ptr(kv["kc"]), _cabi.ptr(kv["ks"]), _cabi.ptr(kv["vc"]),
                        _cabi.ptr(kv["vs"]), self.max_len * dim, _cabi.ptr(self.filled_t), _cabi.ptr(ctx_out), b * heads,
                        self.max_len, dim, self.splits, 1.0 / math.sqrt(dim), _cabi.ptr(self.attn_ws), _cabi.ptr(self.err), stream)
-            o = linear(ctx_out, attn.o_proj.packed, attn.o_proj.scale, gs)
+            o = linear(ctx_out, attn.o_proj.packed, attn.o_proj.scale, int(attn.o_proj.group_size))
             x1 = o + x
             h2 = rms_norm_fused(x1, layer.post_attention_layernorm.weight, eps)
             logits = torch.matmul(h2, mlp._static_router.t())  # (b, E) fp16: a plain library GEMM
-            top_w, top_i = routing_softmax_topk(logits, top_k=cfg.num_experts_per_tok, norm_topk_prob=bool(cfg.norm_topk_prob))
+            top_w, top_i = routing_softmax_topk(logits, top_k=mlp._static_top_k, norm_topk_prob=mlp._static_norm)
             dense.__exit__(None, None, None)
             moe = moe_fn(h2, top_w.to(torch.float16), top_i, experts=cfg.num_experts, world=self.world,
                          rank=self.rank, expert_fn=self.local[i], group=self.group, section=sec)

@@ -12,6 +12,7 @@
 #include <cmath>
 #include <map>
 #include <tuple>
+#include <vector>
 
 #include "../../include/lemoq_b200.h"
 
@@ -170,6 +171,53 @@ PyObject* experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return rc ? raise(rc) : THPVariable_Wrap(out);
 }
 
+// ---- a model's tensors ----------------------------------------------------------------------------------------------------
+// pointers(tensors, forms, device): the addresses of the tensors as bytes, 64 bits each (None: 0).  Tensor i has the form forms[i % n], a tuple
+// (0 for fp16 or 1 for int8, *sizes).  None when one is not contiguous, 16-byte aligned, of its form and on the device (-1: the CPU).  A prompt
+// asks this of some 250 tensors: 2 us here, 200 us as Python expressions.
+PyObject* pointers(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 3 || !PyList_Check(args[0]) || !PyTuple_Check(args[1])) return none();
+    const Py_ssize_t count = PyList_GET_SIZE(args[0]), period = PyTuple_GET_SIZE(args[1]);
+    const long device = PyLong_AsLong(args[2]);
+    if (period == 0 || (device == -1 && PyErr_Occurred())) {
+        PyErr_Clear();
+        return none();
+    }
+    struct Form {
+        at::ScalarType type;
+        c10::DimVector sizes;
+    };
+    std::vector<Form> forms;
+    for (Py_ssize_t i = 0; i < period; ++i) {
+        PyObject* f = PyTuple_GET_ITEM(args[1], i);
+        if (!PyTuple_Check(f) || PyTuple_GET_SIZE(f) < 1) return none();
+        Form form;
+        for (Py_ssize_t d = 0; d < PyTuple_GET_SIZE(f); ++d) {
+            const int64_t v = PyLong_AsLongLong(PyTuple_GET_ITEM(f, d));
+            if (v == -1 && PyErr_Occurred()) {
+                PyErr_Clear();
+                return none();
+            }
+            if (d == 0) form.type = v ? at::kChar : at::kHalf;
+            else form.sizes.push_back(v);
+        }
+        forms.push_back(std::move(form));
+    }
+    std::vector<uint64_t> words(static_cast<size_t>(count), 0);
+    for (Py_ssize_t i = 0; i < count; ++i) {
+        PyObject* o = PyList_GET_ITEM(args[0], i);
+        if (o == Py_None) continue;
+        if (!THPVariable_Check(o)) return none();
+        const at::Tensor& t = THPVariable_Unpack(o);
+        const Form& form = forms[static_cast<size_t>(i % period)];
+        if (t.scalar_type() != form.type || t.sizes() != at::IntArrayRef(form.sizes) || !t.is_contiguous()) return none();
+        if (device < 0 ? !t.device().is_cpu() : !t.is_cuda() || t.get_device() != device) return none();
+        words[static_cast<size_t>(i)] = reinterpret_cast<uint64_t>(t.data_ptr());
+        if (words[static_cast<size_t>(i)] & 15) return none();
+    }
+    return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(words.data()), static_cast<Py_ssize_t>(8 * words.size()));
+}
+
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     try {
@@ -184,6 +232,7 @@ PyMethodDef kMethods[] = {
     {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<attention>)), METH_FASTCALL, "decode attention, or None"},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<linear>)), METH_FASTCALL, "W8 linear, or None"},
     {"experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<experts>)), METH_FASTCALL, "routed W8 experts, or None"},
+    {"pointers", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<pointers>)), METH_FASTCALL, "addresses of tensors of given forms, or None"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_bind", "native call path of the lemoq operators", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -14,7 +14,7 @@ from typing import Any, NamedTuple
 import torch
 import torch.nn.functional as F
 
-from lemoq import _cabi
+from lemoq import _cabi, _native
 
 _PLAN = "_lemoq_prompt_plan"  # on the cache object: what the last native call over that cache was given
 
@@ -34,56 +34,120 @@ class Weights(NamedTuple):
         return [*self.own.values(), *(t for layer in self.layers for t in layer)]
 
 
-def read_weights(model: Any) -> Weights | None:
-    """The tensors that the model's forwards would use now; None when a piece is not in the form the native path knows.  (Through the
-    modules' own dictionaries: 300 attribute look-ups of ``nn.Module`` would take longer than the launches of a short prompt.)"""
+def _read(model: Any) -> tuple[Weights | None, str | None]:
+    """The tensors that the model's forwards would use now, or None and the reason why one ``StepDesc`` does not stand for the model: it has
+    ONE group size, top_k, eps and so on, so what every block was really built with is compared here.  (Through the modules' own
+    dictionaries: 300 attribute look-ups of ``nn.Module`` would take longer than the launches of a short prompt.)"""
     from lemoq.kernels.attn_decode import _decode_forward_impl
     from lemoq.kernels.moe_grouped_quant import QuantFusedExperts
     from lemoq.model import OlmoeAttention, OlmoeDecoderLayer
     from lemoq.quant.linear import QuantLinear
 
-    m, lm = model.model, model.lm_head
-    if type(lm) is not QuantLinear or lm.bias is not None or model.config.clip_qkv is not None or not len(m.layers):
-        return None
+    cfg, m, lm = model.config, model.model, model.lm_head
+    if type(lm) is not QuantLinear or lm.bias is not None:
+        return None, "lm_head is not a W8 linear without bias"
+    if cfg.clip_qkv is not None or not len(m.layers):
+        return None, "clip_qkv is set, or there are no layers"
+    group, eps, routing = lm.group_size, cfg.rms_norm_eps, (cfg.num_experts_per_tok, bool(cfg.norm_topk_prob))
+    if getattr(m.norm, "variance_epsilon", None) != eps:
+        return None, "the final norm has an eps of its own"
     layers = []
-    for layer in m.layers:
+    for i, layer in enumerate(m.layers):
         if type(layer) is not OlmoeDecoderLayer:
-            return None
+            return None, "layer %d is a %s" % (i, type(layer).__name__)
         parts = layer._modules
         attn, mlp = parts["self_attn"], parts["mlp"]
         inner, here, moe = attn._modules, attn.__dict__, mlp.__dict__
         packed, o_proj, stacks = here.get("_lemoq_packed_qkv"), inner.get("o_proj"), moe.get("_static_experts")
-        if (packed is None or type(o_proj) is not QuantLinear or o_proj._buffers["bias"] is not None or not isinstance(stacks, QuantFusedExperts)
-                or getattr(here.get("forward"), "__func__", None) is not _decode_forward_impl
-                or getattr(here.get("_lemoq_original_forward"), "__func__", None) is not OlmoeAttention.forward
-                or here["num_key_value_groups"] != 1 or moe["_static_act"] not in (None, F.silu)):
-            return None
-        norms = [norm._parameters.get("weight") for norm in (parts["input_layernorm"], parts["post_attention_layernorm"], inner["q_norm"], inner["k_norm"])]
-        if any(t is None for t in norms):
-            return None
-        layers.append((*norms, packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"], moe["_static_router"].contiguous(),
+        if packed is None or type(o_proj) is not QuantLinear or o_proj._buffers["bias"] is not None:
+            return None, "layer %d: packed q/k/v not installed, or o_proj is not a W8 linear without bias" % i
+        if not isinstance(stacks, QuantFusedExperts) or stacks.bits != 8 or moe["_static_act"] not in (None, F.silu):
+            return None, "layer %d: experts are not W8 with SiLU" % i
+        if (getattr(here.get("forward"), "__func__", None) is not _decode_forward_impl or here["num_key_value_groups"] != 1
+                or getattr(here.get("_lemoq_original_forward"), "__func__", None) is not OlmoeAttention.forward):
+            return None, "layer %d: attention core not replaced, or GQA" % i
+        if not packed.group_size == o_proj.group_size == stacks.group_size == group:
+            return None, ("layer %d: group sizes %d (q.k.v), %d (o_proj), %d (experts) beside %d (lm_head)"
+                          % (i, packed.group_size, o_proj.group_size, stacks.group_size, group))
+        if (moe["_static_top_k"], moe["_static_norm"]) != routing:
+            return None, "layer %d: top_k %d (normalised: %s) is not the configuration's" % (i, moe["_static_top_k"], moe["_static_norm"])
+        weights = []
+        for norm in (parts["input_layernorm"], parts["post_attention_layernorm"], inner["q_norm"], inner["k_norm"]):
+            if "weight" not in norm._parameters or getattr(norm, "variance_epsilon", None) != eps:
+                return None, "layer %d: a norm is not RMSNorm with the configuration's eps" % i
+            weights.append(norm._parameters["weight"])
+        layers.append((*weights, packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"], moe["_static_router"].contiguous(),
                        stacks.packed_gate_up, stacks.scale_gate_up, stacks.packed_down, stacks.scale_down))
-    return Weights({"embed": m.embed_tokens.weight, "final_norm": m.norm.weight, "lm_head_codes": lm.packed, "lm_head_scale": lm.scale}, layers)
+    return Weights({"embed": m.embed_tokens.weight, "final_norm": m.norm.weight, "lm_head_codes": lm.packed, "lm_head_scale": lm.scale}, layers), None
 
 
-def describe(model: Any, weights: Weights, max_len: int, caches: list[dict]) -> tuple[Any, Any]:
-    """``(StepDesc, LayerDesc array)`` of the model over one set of cache tensors per layer (named as in ``LayerDesc``): pointers only, the
-    caller keeps the tensors for as long as the C side may read them."""
+def read_weights(model: Any) -> Weights | None:
+    return _read(model)[0]
+
+
+_HALF, _CODE = 0, 1  # element types of a form: (type, *shape)
+
+
+def _forms(model: Any) -> tuple[tuple, tuple]:
+    """What the C side takes the model's own tensors and those of a layer to be: it computes every offset from the sizes alone."""
+    cfg, g = model.config, int(model.lm_head.group_size)
+    h, a, f, e, v = cfg.hidden_size, cfg.num_attention_heads * cfg.head_dim, cfg.intermediate_size, cfg.num_experts, cfg.vocab_size
+    own = ((_HALF, v, h), (_HALF, h), (_CODE, v, h), (_HALF, v, h // g))
+    return own, ((_HALF, h), (_HALF, h), (_HALF, a), (_HALF, a), (_CODE, 3 * a, h), (_HALF, 3 * a, h // g), (_CODE, h, a), (_HALF, h, a // g), (_HALF, e, h),
+                 (_CODE, e, 2 * f, h), (_HALF, e, 2 * f, h // g), (_CODE, e, h, f), (_HALF, e, h, f // g))
+
+
+def _misfit(tensors: list, forms: tuple, names: tuple, device: Any) -> str | None:
+    """The first tensor (None: absent) that is not contiguous, 16-byte aligned, on ``device`` and of its form."""
+    for i, t in enumerate(tensors):
+        form, name = forms[i % len(forms)], names[i % len(names)]
+        if t is not None and (t.dtype is not (torch.float16, torch.int8)[form[0]] or tuple(t.shape) != form[1:] or t.device != device):
+            return "%s is %s %s on %s" % (name, tuple(t.shape), t.dtype, t.device)
+        if t is not None and (not t.is_contiguous() or t.data_ptr() & 15):
+            return "%s is not contiguous and 16-byte aligned" % name
+    return None
+
+
+def _pointers(tensors: list, forms: tuple, names: tuple, device: Any) -> bytes | bytearray | None:
+    """The tensors' addresses, 64 bits each; None when one of them misfits."""
+    words = _native.pointers(tensors, forms, -1 if device.index is None else device.index)
+    if words is None and _misfit(tensors, forms, names, device) is None:
+        words = array("Q", [0 if t is None else t.data_ptr() for t in tensors]).tobytes()
+    return words
+
+
+def form_blocker(model: Any) -> str | None:
+    """Why the native paths' one set of sizes does not describe the model (None: it does)."""
+    weights, reason = _read(model)
+    if weights is None:
+        return reason
+    if any(n % model.lm_head.group_size for n in (model.config.hidden_size, model.config.intermediate_size)):
+        return "group size %d does not divide every row" % model.lm_head.group_size
+    own, layer = _forms(model)
+    device = weights.own["embed"].device
+    return (_misfit(list(weights.own.values()), own, tuple(weights.own), device)
+            or _misfit([t for tensors in weights.layers for t in tensors], layer, _LAYER_WEIGHTS, device))
+
+
+def describe(model: Any, weights: Weights, max_len: int, caches: list[dict], cache_forms: dict) -> tuple[Any, Any] | None:
+    """``(StepDesc, LayerDesc array)`` of the model over one set of cache tensors per layer (named as in ``LayerDesc``, each with its form):
+    pointers only, the caller keeps the tensors for as long as the C side may read them.  None when a tensor misfits."""
     cfg, m = model.config, model.model
-    cos, sin = m.rotary_emb.tables(max_len, torch.float16, m.embed_tokens.weight.device)
-    words = array("Q")
-    for layer, slots in zip(weights.layers, caches):
-        words.extend([t.data_ptr() for t in layer])
-        words.extend([0 if slots.get(name) is None else slots[name].data_ptr() for name in _CACHES])
+    device, (own_forms, layer_forms) = weights.own["embed"].device, _forms(model)
+    own = _pointers(list(weights.own.values()), own_forms, tuple(weights.own), device)
+    words = _pointers([t for layer, slots in zip(weights.layers, caches) for t in (*layer, *map(slots.get, _CACHES))],
+                      layer_forms + tuple(cache_forms.get(name, (_HALF,)) for name in _CACHES), _LAYER_WEIGHTS + _CACHES, device)
+    if own is None or words is None:
+        return None
+    cos, sin = m.rotary_emb.tables(max_len, torch.float16, device)
     desc = _cabi.StepDesc()
     desc.layers, desc.hidden, desc.heads, desc.head_dim = len(m.layers), cfg.hidden_size, cfg.num_attention_heads, cfg.head_dim
     desc.experts, desc.top_k, desc.ffn, desc.vocab = cfg.num_experts, cfg.num_experts_per_tok, cfg.intermediate_size, cfg.vocab_size
     desc.group_size, desc.max_len, desc.eps = int(model.lm_head.group_size), max_len, float(cfg.rms_norm_eps)
     desc.norm_topk_prob = int(bool(cfg.norm_topk_prob))
-    for name, t in weights.own.items():
-        setattr(desc, name, t.data_ptr())
+    desc.embed, desc.final_norm, desc.lm_head_codes, desc.lm_head_scale = array("Q", own)
     desc.rope_cos, desc.rope_sin = cos.data_ptr(), sin.data_ptr()
-    return desc, (_cabi.LayerDesc * len(m.layers)).from_buffer(words)
+    return desc, (_cabi.LayerDesc * len(m.layers)).from_buffer_copy(words)
 
 
 def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, position_ids: Any) -> Any:
@@ -104,7 +168,11 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
     for slot in cache.layers:
         if not slot.is_initialized:
             slot.lazy_initialization(torch.empty((1, cfg.num_attention_heads, 1, cfg.head_dim), dtype=torch.float16, device=device))
-    desc, layers = describe(model, weights, cache.max_cache_len, [{"keys": s.keys, "values": s.values} for s in cache.layers])
+    slots = (_HALF, 1, cfg.num_attention_heads, cache.max_cache_len, cfg.head_dim)
+    described = describe(model, weights, cache.max_cache_len, [{"keys": s.keys, "values": s.values} for s in cache.layers], {"keys": slots, "values": slots})
+    if described is None:
+        return None
+    desc, layers = described
     tokens = int(input_ids.shape[1])
     size = int(_cabi.lib().lemoq_prompt_workspace_bytes(desc, tokens))
     if size == 0:
@@ -120,26 +188,34 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
     return logits
 
 
+def _lockstep_forms(model: Any, sequences: int, max_len: int) -> dict:
+    heads, dim = sequences * model.config.num_attention_heads, model.config.head_dim
+    return {"kc": (_CODE, heads, max_len, dim), "vc": (_CODE, heads, max_len, dim), "ks": (_HALF, heads, max_len), "vs": (_HALF, heads, max_len)}
+
+
 def lockstep_plan(model: Any, kv: list[dict], sequences: int, max_len: int) -> dict | None:
     """What :func:`run_lockstep` keeps from step to step for ``sequences`` sequences with the int8 caches ``kv`` (per layer ``kc/vc
     (B*heads, S, D)``, ``ks/vs (B*heads, S)``), or None when the model is not in the canonical form."""
-    weights = read_weights(model) if _cabi.available() and model.model.embed_tokens.weight.dtype == torch.float16 else None
-    if weights is None:
+    weights = read_weights(model) if _cabi.available() else None
+    described = None if weights is None else describe(model, weights, max_len, kv, _lockstep_forms(model, sequences, max_len))
+    if described is None:
         return None
-    size = int(_cabi.lib().lemoq_lockstep_workspace_bytes(describe(model, weights, max_len, kv)[0], sequences))
+    size = int(_cabi.lib().lemoq_lockstep_workspace_bytes(described[0], sequences))
     if size == 0:
         return None
     workspace = torch.zeros(size, dtype=torch.uint8, device=model.model.embed_tokens.weight.device)
-    return {"model": model, "kv": kv, "max_len": max_len, "workspace": workspace}
+    return {"model": model, "kv": kv, "max_len": max_len, "workspace": workspace, "sequences": sequences}
 
 
 def run_lockstep(plan: dict, tokens: Any, position: Any, filled: Any, vocab: int, flags: Any) -> Any:
     """Logits ``(B, V)`` of one token per sequence; ``position`` and ``filled`` are device scalars.  None when the model has left the
     canonical form.  ``plan["weights"]``: the tensors this call reads (a captured step's graph reads them at every replay)."""
-    weights = read_weights(plan["model"])
-    if weights is None:
+    model, max_len = plan["model"], plan["max_len"]
+    weights = read_weights(model)
+    described = None if weights is None else describe(model, weights, max_len, plan["kv"], _lockstep_forms(model, plan["sequences"], max_len))
+    if described is None:
         return None
-    desc, layers = describe(plan["model"], weights, plan["max_len"], plan["kv"])
+    desc, layers = described
     rows, workspace = int(tokens.shape[0]), plan["workspace"]
     logits = torch.empty((rows, vocab), dtype=torch.float16, device=tokens.device)
     _cabi.call("lemoq_lockstep_run", desc, layers, _cabi.ptr(tokens), _cabi.ptr(position), _cabi.ptr(filled), rows, _cabi.ptr(logits),

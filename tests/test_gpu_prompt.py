@@ -150,3 +150,36 @@ def test_replaced_weights_are_the_ones_a_prompt_uses():
     torch.empty(1 << 20, dtype=torch.uint8, device=DEV).fill_(255)  # would land on freed weights
     assert torch.equal(step(decoder), other_step)  # a captured graph goes on with the weights it was captured with
     assert torch.equal(session.prefill().logits, first)
+
+
+# the experts' scales are finer or coarser than the rest of the model's; the sizes are such that every kernel would take them
+@pytest.mark.parametrize("group", [64, 256])
+def test_experts_of_another_group_size_match_oracle(group):
+    """Not a model that one native description fits: prompt, decode and lockstep step follow the experts' own group size all the same."""
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+    from benchmarks.expert_parallel import ExpertParallelDecoder
+    from benchmarks.runner import install_replacements
+    from lemoq.kernels.moe_grouped_quant import QuantFusedExperts
+
+    spec = glue.OlmoeSpec(layers=2, hidden=512, heads=4, head_dim=128, experts=8, top_k=2, ffn=512, vocab=512)
+    wf = glue.random_float_weights(spec, seed=group, dtype=torch.float16, std=0.05, norm_weight_jitter=0.1)
+    wf.embed.mul_(20.0)
+    for layer in wf.layers:
+        layer.router.mul_(5.0)
+    wq, model, packed, tokens = glue.quantize_weights(wf), lemoq_model_from_oracle(wf), {}, 33
+    for i, (lq, lw) in enumerate(zip(wq.layers, wf.layers)):
+        parts = (*ops.rtn_quantize_w8(lw.gate_up_w, group), *ops.rtn_quantize_w8(lw.down_w, group))
+        lq.experts = ops.QuantExperts(*parts, group)
+        packed[i] = QuantFusedExperts(*(t.to(DEV).contiguous() for t in parts), 8, group)
+    install_replacements(model, attn="kernel", moe="grouped", quant_cfg={"bit_width": "w8a16", "dequant": "fused", "group_size": 128}, rmsnorm="fused",
+                         ctx=tokens, max_new_tokens=4, prequantized=packed)
+    prompt = torch.tensor([[(11 * i * i + 3) % spec.vocab for i in range(tokens)]])
+    state = glue.new_state(spec, tokens + 4)
+    first = glue.prefill(wq, state, prompt[0])
+    session = StaticCacheDecodeSession(model, prompt.to(DEV), ctx=tokens, max_new_tokens=4)
+    assert rel_err(session.prefill().logits[0, -1], first) < 2e-2 and session.seed_token_id == int(first.float().argmax())
+    decoder = ExpertParallelDecoder(model, session, sequences=1, world=1, rank=0, static_exchange=group % 128 == 0)
+    glue.build_int8_mirror(state)
+    ref = glue.decode_step(wq, state, session.seed_token_id, tokens)
+    assert rel_err(decoder.step(torch.tensor([session.seed_token_id], device=DEV))[0], ref) < 2e-2
+    assert rel_err(session.decode_eager().reshape(-1), ref) < 2e-2

@@ -1,4 +1,4 @@
-"""How the native paths read a model (no GPU)."""
+"""How the native paths read a model (no GPU), and which they leave to the module tree."""
 
 from __future__ import annotations
 
@@ -43,13 +43,13 @@ def canonical(monkeypatch):
 
 def test_a_description_follows_the_tensors_of_the_model(canonical):
     """Nothing is kept by a module's identity: whatever replaces a parameter or a buffer is what the next call is given."""
-    from lemoq.prompt import describe, read_weights
+    from lemoq.prompt import _HALF, describe, read_weights
 
-    model = canonical()
+    model, forms = canonical(), dict.fromkeys(("keys", "values"), (_HALF, 1, 2, 8, 128))
     caches = [{"keys": torch.zeros(1, 2, 8, 128, dtype=torch.float16), "values": torch.zeros(1, 2, 8, 128, dtype=torch.float16)} for _ in range(2)]
 
     def pointers():
-        desc, layers = describe(model, read_weights(model), 8, caches)
+        desc, layers = describe(model, read_weights(model), 8, caches, forms)
         return [getattr(desc, n) for n in ("embed", "final_norm", "lm_head_codes", "lm_head_scale")], [[getattr(d, n) for n, _ in d._fields_] for d in layers]
 
     def moved():
@@ -57,7 +57,7 @@ def test_a_description_follows_the_tensors_of_the_model(canonical):
         nonlocal before
         after = pointers()
         names = [n for n, a, b in zip(("embed", "final_norm", "lm_head_codes", "lm_head_scale"), before[0], after[0]) if a != b]
-        names += [n for (n, _), a, b in zip(type(describe(model, read_weights(model), 8, caches)[1][0])._fields_, before[1][-1], after[1][-1]) if a != b]
+        names += [n for (n, _), a, b in zip(type(describe(model, read_weights(model), 8, caches, forms)[1][0])._fields_, before[1][-1], after[1][-1]) if a != b]
         before = after
         return names
 
@@ -75,3 +75,48 @@ def test_a_description_follows_the_tensors_of_the_model(canonical):
         assert moved() == expected
     last.self_attn.o_proj.bias = torch.zeros(256)
     assert read_weights(model) is None  # and what it no longer describes is not taken
+
+
+@pytest.mark.parametrize("group", [64, 256])
+def test_experts_of_another_group_size_are_not_one_description(canonical, group):
+    from lemoq.prompt import form_blocker
+
+    assert form_blocker(canonical()) is None
+    assert "group sizes 128 (q.k.v), 128 (o_proj), %d (experts) beside 128" % group in form_blocker(canonical(experts=group))
+
+
+def test_every_block_is_compared_with_the_configuration(canonical):
+    from lemoq.prompt import form_blocker
+
+    model = canonical()
+    first, last = model.model.layers
+    for owner, name, value, told in ((last.mlp, "_static_top_k", 3, "top_k 3"), (last.mlp, "_static_norm", True, "normalised: True"),
+                                     (first.mlp, "_static_act", torch.relu, "SiLU"), (last.self_attn.q_norm, "variance_epsilon", 1e-6, "eps"),
+                                     (model.lm_head, "bias", torch.zeros(64), "bias"), (first.self_attn.o_proj, "bias", torch.zeros(256), "bias"),
+                                     (first.mlp, "_static_router", first.mlp._static_router[:4], "router"),
+                                     (last.self_attn._lemoq_packed_qkv, "scale", last.self_attn._lemoq_packed_qkv.scale.float(), "qkv_scale"),
+                                     (last.mlp._static_experts, "scale_down", torch.zeros(8 * 256 * 2 + 1, dtype=torch.float16)[1:].view(8, 256, 2), "aligned")):
+        kept = getattr(owner, name)
+        setattr(owner, name, value)
+        assert told in form_blocker(model), name
+        setattr(owner, name, kept)
+    assert form_blocker(model) is None
+
+
+@pytest.mark.parametrize("bound", [True, False])
+def test_a_tensor_of_another_form_is_not_described(canonical, bound, monkeypatch):
+    """The binding and the Python expressions it stands for refuse the same."""
+    from lemoq import _native
+    from lemoq.prompt import _HALF, describe, read_weights
+
+    if not bound:
+        monkeypatch.setattr(_native, "pointers", lambda *a: None)
+    model, forms = canonical(), dict.fromkeys(("keys", "values"), (_HALF, 1, 2, 8, 128))
+    cache = lambda n: [{"keys": torch.zeros(1, 2, n, 128, dtype=torch.float16), "values": torch.zeros(1, 2, 8, 128, dtype=torch.float16)} for _ in range(2)]  # noqa: E731
+    assert describe(model, read_weights(model), 8, cache(8), forms) is not None and describe(model, read_weights(model), 8, cache(9), forms) is None
+    mlp = model.model.layers[1].mlp
+    whole = mlp._static_experts.packed_down
+    for other in (whole[:7], whole.to(torch.int16), whole.to("meta"), whole.transpose(1, 2).contiguous().transpose(1, 2),
+                  torch.zeros(whole.numel() + 1, dtype=torch.int8)[1:].view_as(whole)):
+        mlp._static_experts.packed_down = other
+        assert describe(model, read_weights(model), 8, cache(8), forms) is None
