@@ -236,6 +236,8 @@ class StaticCacheDecodeSession:
         self.cache = StaticCache(config=model.config, max_cache_len=capacity)
         self.buffers = GraphBuffers.allocate(self.device, batch=1, max_cache_len=capacity, dtype=self.dtype)
         self.cache._lemoq_filled_len = self.buffers.filled_len  # the attention modules find the device length here
+        self._error_word = torch.zeros((), dtype=torch.long, device=self.device)  # what a native prompt flags; prefill reads it
+        self.cache._lemoq_error_word = self._error_word.view(1).view(torch.int32)[:1]  # (the low half)
         # engine choice: an explicit argument wins; "auto" listens to LEMOQ_STEP_ENGINE (1 = step, else ops)
         forced = os.environ.get("LEMOQ_STEP_ENGINE")
         self._engine_request = engine if engine != "auto" or forced is None else ("step" if forced == "1" else "ops")
@@ -263,14 +265,21 @@ class StaticCacheDecodeSession:
 
     def prefill(self) -> Any:
         """Run the prompt through the model eagerly into the emptied static cache; the arg-max of the last position
-        seeds the decode."""
+        seeds the decode.  A prompt with a token id outside the vocabulary raises ``RuntimeError``."""
+        from lemoq import _cabi
+
         torch, ctx = self.torch, self.config.ctx
+        self.current_token_id = None
         self._clear_cache()
         slots = torch.arange(ctx, dtype=torch.long, device=self.device)
         with torch.no_grad():
             output = self.model(self.prompt_ids, attention_mask=torch.ones_like(slots).unsqueeze(0), past_key_values=self.cache,
                                 use_cache=True, cache_position=slots, position_ids=slots.unsqueeze(0))
-        self.current_token_id, self.position = int(output.logits[0, -1].argmax().item()), ctx
+        picked, flags = torch.stack((output.logits[0, -1].argmax(), self._error_word)).tolist()  # one read-back
+        if flags:
+            self._error_word.zero_()
+            _cabi.check_flags(flags, "prefill")
+        self.current_token_id, self.position = picked, ctx
         if self.after_prefill is not None:
             self.after_prefill(self)
         self._requantize_mirror()

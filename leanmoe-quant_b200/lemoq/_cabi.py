@@ -19,7 +19,9 @@ LIB_PATH = os.path.join(os.path.dirname(_HERE), "csrc", "liblemoq_b200.so")
 
 OK, ERR_INVALID, ERR_UNSUPPORTED, ERR_CUDA = 0, 1, 2, 3
 DTYPE_F16, DTYPE_F32 = 0, 1
-FLAG_BAD_POSITION, FLAG_BAD_LENGTH, FLAG_BAD_EXPERT = 1, 2, 4
+FLAG_BAD_POSITION, FLAG_BAD_LENGTH, FLAG_BAD_EXPERT, FLAG_WAIT_TIMEOUT, FLAG_BAD_TOKEN = 1, 2, 4, 8, 16
+_FLAG_TEXT = {FLAG_BAD_POSITION: "a position outside the cache", FLAG_BAD_LENGTH: "a length outside the cache", FLAG_BAD_EXPERT: "an expert id out of range",
+              FLAG_WAIT_TIMEOUT: "a kernel's wait ran out", FLAG_BAD_TOKEN: "a token id outside the vocabulary"}
 
 _lib = None
 _load_error: str | None = None
@@ -166,6 +168,12 @@ def check(status: int, what: str = "") -> None:
 
 def call(name: str, *args: Any) -> None:
     check(getattr(lib(), name)(*args), name)
+
+
+def check_flags(word: int, what: str) -> None:
+    """Raise ``RuntimeError`` for an error word that a kernel has left (its results are void)."""
+    if word:
+        raise RuntimeError("%s: %s" % (what, ", ".join(text for bit, text in _FLAG_TEXT.items() if word & bit) or "flags %d" % word))
 
 
 def ptr(t: Any) -> int | None:

@@ -152,7 +152,8 @@ def describe(model: Any, weights: Weights, max_len: int, caches: list[dict], cac
 
 def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, position_ids: Any) -> Any:
     """Logits ``(1, T, V)`` of the prompt ``input_ids (1, T)``, with its K/V rows written into ``cache`` - or None when the
-    model, the cache or the call is not of the kind the native path takes."""
+    model, the cache or the call is not of the kind the native path takes.  A token id outside the vocabulary, a position outside the cache
+    and a wait that ran out raise ``RuntimeError`` (the kernels clamp and flag; the call waits for the flag unless the cache's owner does)."""
     from lemoq.model import StaticCache
 
     weight = model.model.embed_tokens.weight
@@ -177,14 +178,17 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
     size = int(_cabi.lib().lemoq_prompt_workspace_bytes(desc, tokens))
     if size == 0:
         return None
-    plan = cache.__dict__.setdefault(_PLAN, {})
-    if plan.get("flags") is None:
-        plan["flags"] = torch.zeros(1, dtype=torch.int32, device=device)
+    # the error word: the one the cache carries, whose owner reads it, or one of this call's own
+    carried = cache.__dict__.get("_lemoq_error_word")
+    flags = torch.zeros(1, dtype=torch.int32, device=device) if carried is None else carried
+    cache.__dict__[_PLAN] = {"flags": flags}
     ids = input_ids.contiguous()
     logits = torch.empty((1, tokens, cfg.vocab_size), dtype=torch.float16, device=device)
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     _cabi.call("lemoq_prompt_run", desc, layers, _cabi.ptr(ids), _cabi.ptr(cache_position), tokens, _cabi.ptr(logits),
-               _cabi.ptr(workspace), size, _cabi.ptr(plan["flags"]), _cabi.current_stream(device))
+               _cabi.ptr(workspace), size, _cabi.ptr(flags), _cabi.current_stream(device))
+    if carried is None and not torch.cuda.is_current_stream_capturing():
+        _cabi.check_flags(int(flags), "prompt")
     return logits
 
 

@@ -183,3 +183,30 @@ def test_experts_of_another_group_size_match_oracle(group):
     ref = glue.decode_step(wq, state, session.seed_token_id, tokens)
     assert rel_err(decoder.step(torch.tensor([session.seed_token_id], device=DEV))[0], ref) < 2e-2
     assert rel_err(session.decode_eager().reshape(-1), ref) < 2e-2
+
+
+def test_a_flagged_prompt_raises():
+    """The kernels clamp a token id or a position that is out of range and flag it: the call says so and seeds nothing."""
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+    from lemoq.model import StaticCache
+
+    spec = glue.OlmoeSpec(layers=1, hidden=256, heads=2, head_dim=128, experts=8, top_k=2, ffn=128, vocab=512)
+    model = lemoq_model_from_oracle(glue.random_float_weights(spec, seed=4, dtype=torch.float16))
+    install_canonical(model, 20, 4)
+    prompt = torch.arange(20, device=DEV).unsqueeze(0)
+    session = StaticCacheDecodeSession(model, prompt.clone(), ctx=20, max_new_tokens=4, engine="ops")
+    first = session.prefill().logits.clone()
+    for bad in (spec.vocab, -1):
+        session.prompt_ids[0, 7] = bad
+        with pytest.raises(RuntimeError, match="token id outside the vocabulary"):
+            session.prefill()
+        with pytest.raises(RuntimeError, match="prefill must run"):
+            session.seed_token_id
+    session.prompt_ids[0, 7] = 7
+    assert torch.equal(session.prefill().logits, first)  # the word is clean again
+    with torch.no_grad():
+        cache, slots = StaticCache(model.config, 24), torch.arange(20, device=DEV)
+        assert torch.equal(model(prompt, past_key_values=cache, cache_position=slots).logits, first)
+        for ids, at, told in ((prompt + spec.vocab, slots, "token id"), (prompt, slots + 5, "position")):
+            with pytest.raises(RuntimeError, match=told):
+                model(ids, past_key_values=cache, cache_position=at)
