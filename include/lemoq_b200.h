@@ -49,6 +49,13 @@ extern "C" {
 LEMOQ_API const char* lemoq_version(void);
 LEMOQ_API const char* lemoq_last_error(void);
 
+/* The current device's status word: an int in pinned host memory, allocated at the first call on the device (64 bytes, for
+ * good; NULL when that fails) and from then on the place where a call whose err_flag is NULL, or that has none, has its
+ * LEMOQ_FLAG_* left.  The host may read it at any time without waiting; it is final for a launch once its stream has been
+ * waited for, and stays set until the host stores 0.  lemoq_attn_decode_int8_static does not use it.  No counterpart in
+ * the reference. */
+LEMOQ_API int* lemoq_status_word(void);
+
 /* Kernel tuning knobs for benchmarking (process-wide, not thread-safe; defaults are the measured
  * best).  Returns LEMOQ_ERR_INVALID for an unknown key or a value out of range.
  *   key 0  int8 dot-product variant of the streaming GEMV kernels: 0 fp32 magic number, 1 exact fp16

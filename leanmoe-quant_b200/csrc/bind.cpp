@@ -26,6 +26,16 @@ PyObject* raise(int status) {
     return nullptr;
 }
 
+// The kernels of these calls leave their flags in the device's status word (the calls pass no error word).  A wait that ran out in an earlier
+// call has voided its results: that is said here, at the next call, as the CUDA runtime does with errors of its own.
+bool healthy() {
+    volatile int* word = lemoq_status_word();
+    if (!word || !(*word & LEMOQ_FLAG_WAIT_TIMEOUT)) return true;
+    *word = *word & ~LEMOQ_FLAG_WAIT_TIMEOUT;
+    PyErr_SetString(PyExc_RuntimeError, "a wait ran out in the kernel of an earlier attention, linear or experts call: its results are void");
+    return false;
+}
+
 // Is the first argument a CUDA tensor?  (Asked before anything that needs a CUDA device.)
 bool on_cuda(PyObject* o) { return THPVariable_Check(o) && THPVariable_Unpack(o).is_cuda(); }
 
@@ -68,6 +78,7 @@ void* attn_scratch(int device, const c10::cuda::CUDAStream& stream, int64_t head
 // attention(q, k, ks | None, v, vs | None, filled, scale | None): the default split count, as resolve_num_splits gives it
 PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 7 || !on_cuda(args[0])) return none();
+    if (!healthy()) return nullptr;
     const int device = c10::cuda::current_device();
     const bool int8 = args[2] != Py_None;
     const at::Tensor *q = cuda_tensor(args[0], device), *k = cuda_tensor(args[1], device), *v = cuda_tensor(args[3], device), *filled = cuda_tensor(args[5], device);
@@ -110,6 +121,7 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // linear(x (..., K), codes (N, K), scale (N, K / group), group, exact): one token through the GEMV, several through the tensor-core GEMM
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 5 || !on_cuda(args[0])) return none();
+    if (!healthy()) return nullptr;
     const int device = c10::cuda::current_device();
     const at::Tensor *x = cuda_tensor(args[0], device), *codes = cuda_tensor(args[1], device), *scale = cuda_tensor(args[2], device);
     if (!x || x->scalar_type() != at::kHalf || x->dim() < 1 || !x->is_contiguous() || !rows(codes, at::kChar, 2) || !rows(scale, at::kHalf, 2)) return none();
@@ -135,6 +147,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // experts(x (T, H) | (H), gate_up, gate_up_scale, down, down_scale, ids (T, K) | (K), weights, group)
 PyObject* experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 8 || !on_cuda(args[0])) return none();
+    if (!healthy()) return nullptr;
     const int device = c10::cuda::current_device();
     const at::Tensor* a[7];
     for (int i = 0; i < 7; ++i)

@@ -2,6 +2,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <mutex>
 
 #include "kernels.h"
 
@@ -29,6 +30,13 @@ int sm_count() {
     return n;
 }
 
+static std::atomic<int*> g_status[64];  // by device
+
+int* status_word() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? g_status[dev].load(std::memory_order_acquire) : nullptr;
+}
+
 static LaunchCfg cfg_of(void* stream) {
     LaunchCfg lc;
     lc.stream = static_cast<cudaStream_t>(stream);
@@ -41,6 +49,24 @@ using namespace lemoq;
 
 extern "C" const char* lemoq_version(void) { return "lemoq_b200 0.1 (sm_100a)"; }
 extern "C" const char* lemoq_last_error(void) { return g_err; }
+extern "C" int* lemoq_status_word(void) {
+    static std::mutex guard;
+    if (int* known = status_word()) return known;
+    int dev = 0;
+    std::lock_guard<std::mutex> lock(guard);
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    if (int* known = g_status[dev].load(std::memory_order_acquire)) return known;
+    // not a stream operation, so it may happen while a capture runs
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+    void* word = nullptr;
+    const cudaError_t err = cudaHostAlloc(&word, 64, cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (err != cudaSuccess) return nullptr;
+    *static_cast<int*>(word) = 0;
+    g_status[dev].store(static_cast<int*>(word), std::memory_order_release);
+    return static_cast<int*>(word);
+}
 extern "C" int lemoq_set_tuning(int key, int value) { return set_stream_tuning(key, value); }
 
 extern "C" int lemoq_rtn_quantize_w8(const void* w, int w_dtype, int64_t rows, int in_features, int group_size,
@@ -80,6 +106,7 @@ extern "C" int lemoq_dequant_gemv_w8(const void* x, int M, const int8_t* codes, 
     p.group_size = group_size;
     p.y = y;
     p.y_stride = N;
+    p.err_flag = status_word();
     return launch_gemv_w8(p, M, false, false, out_dtype == LEMOQ_DTYPE_F32, cfg_of(stream));
 }
 
@@ -160,7 +187,7 @@ static int attn_common(AttnParams& p, const void* q, const int32_t* filled, void
     const size_t counters = (sizeof(unsigned int) * heads + 255) / 256 * 256;
     p.counters = reinterpret_cast<unsigned int*>(workspace);
     p.part = reinterpret_cast<float*>(static_cast<char*>(workspace) + counters);
-    p.err_flag = err_flag;
+    p.err_flag = err_flag ? err_flag : status_word();
     return LEMOQ_OK;
 }
 
@@ -250,7 +277,7 @@ static int moe_common(MoeParams& p, const void* x, const int64_t* ids, const voi
     p.F = F;
     p.act = reinterpret_cast<__half*>(act);
     p.out = reinterpret_cast<__half*>(out);
-    p.err_flag = err_flag;
+    p.err_flag = err_flag ? err_flag : status_word();
     return LEMOQ_OK;
 }
 

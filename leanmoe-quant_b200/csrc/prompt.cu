@@ -86,6 +86,7 @@ int run_rows(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const 
     const bool lockstep = filled != nullptr;
     const size_t rows_bytes = carve_prompt(d, T, static_cast<char*>(workspace), &b), need = rows_bytes + (lockstep ? attn_scratch_bytes(T * d.heads) : 0);
     LEMOQ_REQUIRE(workspace_bytes >= need, LEMOQ_ERR_INVALID, "prompt: workspace of %zu bytes, needs %zu", workspace_bytes, need);
+    if (!err_flag) err_flag = status_word();
 
     LaunchCfg lc;
     lc.stream = static_cast<cudaStream_t>(stream);
@@ -198,6 +199,7 @@ extern "C" int lemoq_moe_tokens_w8(const void* x, const int8_t* gu_codes, const 
     MoeBuffers b;
     const size_t need = carve_moe(T, K, E, H, F, static_cast<char*>(workspace), &b);
     LEMOQ_REQUIRE(workspace_bytes >= need, LEMOQ_ERR_INVALID, "moe_tokens_w8: workspace of %zu bytes, needs %zu", workspace_bytes, need);
+    if (!err_flag) err_flag = status_word();
     LaunchCfg lc;
     lc.stream = static_cast<cudaStream_t>(stream);
     LaunchCfg chained = lc;

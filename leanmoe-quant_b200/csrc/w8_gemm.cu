@@ -703,7 +703,7 @@ extern "C" int lemoq_w8_gemm(const void* x, int T, const int8_t* codes, const vo
     g.y = reinterpret_cast<__half*>(y);
     g.T = T; g.N = N; g.K = K; g.group_size = group_size; g.E = E; g.gate_up = gate_up != 0;
     g.exact = exact != 0;
-    g.err_flag = err_flag;
+    g.err_flag = err_flag ? err_flag : status_word();
     LaunchCfg lc;
     lc.stream = static_cast<cudaStream_t>(stream);
     return launch_w8_gemm(g, lc);

@@ -48,6 +48,7 @@ class StepDesc(Structure):
 _SIGNATURES = {
     "lemoq_version": (c_char_p, []),
     "lemoq_last_error": (c_char_p, []),
+    "lemoq_status_word": (c_void_p, []),
     "lemoq_set_tuning": (c_int, [c_int, c_int]),
     "lemoq_rtn_quantize_w8": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "lemoq_dequant_gemv_w8": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p]),
@@ -174,6 +175,23 @@ def check_flags(word: int, what: str) -> None:
     """Raise ``RuntimeError`` for an error word that a kernel has left (its results are void)."""
     if word:
         raise RuntimeError("%s: %s" % (what, ", ".join(text for bit, text in _FLAG_TEXT.items() if word & bit) or "flags %d" % word))
+
+
+def error_flags(device: Any = None, *, clear: bool = False) -> int:
+    """``FLAG_*`` that kernels of short operator calls (attention, W8 linears, experts) have left on ``device`` since the word was last
+    cleared: ids, lengths and positions that were clamped, waits that ran out.  Does not wait for calls that are still running.  (A wait that
+    ran out also raises at the next such call.)"""
+    import torch
+
+    with torch.cuda.device(device):
+        address = lib().lemoq_status_word()
+    if not address:
+        return 0
+    word = c_int.from_address(address)
+    flags = word.value
+    if clear:
+        word.value = 0
+    return flags
 
 
 def ptr(t: Any) -> int | None:

@@ -52,3 +52,40 @@ def test_quant_linear_native_and_fallback_agree(mode, shape):
     assert linear._counters["fused_calls"] == (2 if single and mode == "fused" else 0)
     assert linear._counters["separate_calls"] == (0 if single and mode == "fused" else 2)
     assert linear._counters["fallbacks"] == ({"multi_token": 2} if mode == "fused" and not single else {})
+
+
+def test_calls_leave_their_flags_where_the_host_sees_them():
+    """The short calls pass no error word: clamped ids and lengths are in the device's status word, and a wait that ran out raises at the next
+    call (the host sets the bit here: no kernel is made to wait)."""
+    from ctypes import c_int
+
+    from lemoq import _cabi
+    from lemoq.kernels.attn_decode import attn_decode_forward_int8
+    from lemoq.kernels.moe_grouped_quant import QuantFusedExperts, grouped_moe_forward_quant, grouped_moe_forward_quant_tokens
+    from lemoq.quant.linear import QuantLinear, SchemeSpec
+
+    g = torch.Generator().manual_seed(1)
+    own = QuantFusedExperts(*(t.to(DEV) for s in ((256, 128), (128, 128)) for t in ops.rtn_quantize_w8(torch.randn(4, *s, generator=g), 128)), 8, 128)
+    x, ids, weights = torch.randn(3, 128, generator=g).half().to(DEV), torch.tensor([[0], [3], [1]], device=DEV), torch.ones(3, 1, device=DEV).half()
+    q, codes, scale = torch.randn(1, 2, 1, 128, device=DEV).half(), torch.ones(1, 2, 40, 128, dtype=torch.int8, device=DEV), torch.ones(1, 2, 40, device=DEV).half()
+    linear = QuantLinear(nn.Linear(128, 64, device=DEV, dtype=torch.float16), SchemeSpec.from_flags("w8a16", 128, dequant="fused"))
+    calls = {"tokens": lambda n=0: grouped_moe_forward_quant_tokens(x, own, ids + n, weights), "token": lambda n=0: grouped_moe_forward_quant(x[0], own, ids[0] + n, weights[0]),
+             "attention": lambda n=0: attn_decode_forward_int8(q, codes, scale, codes, scale, torch.tensor([40 + n], dtype=torch.int32, device=DEV)),
+             "linear": lambda n=0: linear(x), "one": lambda n=0: linear(x[:1])}
+
+    def flags():
+        torch.cuda.synchronize()
+        return _cabi.error_flags(clear=True)
+
+    flags()
+    with torch.no_grad():
+        for name, call in calls.items():
+            call()
+            assert flags() == 0, name
+            call(9)  # clamped, as ever
+            assert flags() == {"tokens": _cabi.FLAG_BAD_EXPERT, "token": _cabi.FLAG_BAD_EXPERT, "attention": _cabi.FLAG_BAD_LENGTH}.get(name, 0), name
+            c_int.from_address(_cabi.lib().lemoq_status_word()).value = _cabi.FLAG_WAIT_TIMEOUT | _cabi.FLAG_BAD_EXPERT
+            with pytest.raises(RuntimeError, match="wait ran out"):
+                call()
+            call()
+            assert flags() == _cabi.FLAG_BAD_EXPERT, name
