@@ -289,10 +289,16 @@ class ExpertParallelDecoder:
     """Lockstep greedy decode of ``sequences`` sequences that share one prefilled prompt.
 
     ``model`` is the canonical quantised module tree (after ``install_replacements``); ``session`` a batch-1
-    ``StaticCacheDecodeSession`` on it whose prefill filled the fp16 cache for the common prompt."""
+    ``StaticCacheDecodeSession`` on it whose prefill filled the fp16 cache for the common prompt.
+
+    On one rank with the static exchange the step is one native call, which has no exchange and chooses the attention's
+    splits itself.  ``exchange_kernels=False`` or an ``attn_splits`` other than the default asks for the step by parts,
+    which has both."""
+
+    DEFAULT_SPLITS = 4
 
     def __init__(self, model: Any, session: Any, *, sequences: int, world: int, rank: int, group: Any = None,
-                 attn_splits: int = 4, static_exchange: bool = False, exchange_kernels: bool = True) -> None:
+                 attn_splits: int = DEFAULT_SPLITS, static_exchange: bool = False, exchange_kernels: bool = True) -> None:
         from lemoq import _cabi
         from lemoq.prompt import lockstep_plan
 
@@ -337,8 +343,9 @@ class ExpertParallelDecoder:
         self.pos_t = torch.zeros(1, dtype=torch.int64, device=self.device)
         self.filled_t = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.err = torch.zeros(1, dtype=torch.int32, device=self.device)
-        # on one rank nothing leaves the device: the whole step is one native call
-        self.native = lockstep_plan(model, self.kv, self.b, self.max_len) if world == 1 and static_exchange else None
+        # on one rank nothing leaves the device: the whole step is one native call, unless the caller chose parts of it
+        chosen = not exchange_kernels or attn_splits != self.DEFAULT_SPLITS
+        self.native = lockstep_plan(model, self.kv, self.b, self.max_len) if world == 1 and static_exchange and not chosen else None
         self.sections = None  # name -> list of (start, end) CUDA events while a timing split is being taken
 
     def _section(self, name: str) -> Any:

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("exchange", ["dynamic", "static-tensor-library", "static-kernels"])
+@pytest.mark.parametrize("exchange", ["dynamic", "static-tensor-library", "static-kernels", "static-native"])
 def test_batched_lockstep_decode_matches_oracle_per_sequence(exchange):
     from benchmarks.cudagraph import StaticCacheDecodeSession, compare_logits
     from benchmarks.expert_parallel import ExpertParallelDecoder
@@ -33,9 +33,10 @@ def test_batched_lockstep_decode_matches_oracle_per_sequence(exchange):
     for i, cl in enumerate(session.cache.layers):  # identical inputs on both sides: the oracle's prefilled cache
         cl.keys.copy_(st0.keys[i].to(DEV))
         cl.values.copy_(st0.values[i].to(DEV))
-    dec = ExpertParallelDecoder(model, session, sequences=seqs, world=1, rank=0, attn_splits=3,
-                                static_exchange=exchange != "dynamic", exchange_kernels=exchange == "static-kernels")
-    assert dec.exchange_kernels == (exchange == "static-kernels")
+    chosen = {} if exchange == "static-native" else {"attn_splits": 3, "exchange_kernels": exchange == "static-kernels"}
+    dec = ExpertParallelDecoder(model, session, sequences=seqs, world=1, rank=0, static_exchange=exchange != "dynamic", **chosen)
+    assert dec.exchange_kernels == (exchange in ("static-kernels", "static-native"))
+    assert (dec.native is not None) == (exchange == "static-native")  # what the caller chose is what runs
     first = [5, 77, 300]
     tokens = torch.tensor(first, dtype=torch.int64, device=DEV)
     got_logits, got_tokens = [], []
