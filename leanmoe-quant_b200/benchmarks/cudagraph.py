@@ -447,9 +447,8 @@ class StaticCacheDecodeSession:
 
         stream = None
         for i, layer in enumerate(self.model.model.layers):
-            attn = getattr(layer, "self_attn", None)
-            bufs = getattr(attn, "_lemoq_kv_int8_bufs", None)
-            ref = getattr(attn, "_lemoq_kv_int8_src_cache_ref", None)
+            here = getattr(getattr(layer, "self_attn", None), "__dict__", {})  # (a missing attribute of a module takes a microsecond)
+            bufs, ref = here.get("_lemoq_kv_int8_bufs"), here.get("_lemoq_kv_int8_src_cache_ref")
             cl = self.cache.layers[i]
             if bufs is None or ref is None or ref() is not self.cache or not cl.is_initialized:
                 continue

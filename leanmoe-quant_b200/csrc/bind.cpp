@@ -231,6 +231,35 @@ PyObject* pointers(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(words.data()), static_cast<Py_ssize_t>(8 * words.size()));
 }
 
+// plain(modules, forwards): True when no module of the list has a forward (pre-)hook, nor a forward of its own other than a bound method of one
+// of the functions `forwards`; else None.  (200 modules: 6 us here, 30 us as Python expressions.)
+PyObject* plain(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    static PyObject *const hooks = PyUnicode_InternFromString("_forward_hooks"), *const pre_hooks = PyUnicode_InternFromString("_forward_pre_hooks"),
+                            *const forward = PyUnicode_InternFromString("forward");
+    if (n != 2 || !PyList_Check(args[0]) || !PyTuple_Check(args[1]) || !hooks || !pre_hooks || !forward) return none();
+    auto is_plain = [&](PyObject* dict) {
+        for (PyObject* name : {hooks, pre_hooks}) {
+            PyObject* registered = PyDict_GetItemWithError(dict, name);
+            if (!registered || !PyDict_Check(registered) || PyDict_Size(registered) != 0) return false;
+        }
+        PyObject* own = PyDict_GetItemWithError(dict, forward);
+        if (!own) return !PyErr_Occurred();
+        for (Py_ssize_t j = 0; PyMethod_Check(own) && j < PyTuple_GET_SIZE(args[1]); ++j)
+            if (PyMethod_GET_FUNCTION(own) == PyTuple_GET_ITEM(args[1], j)) return true;
+        return false;
+    };
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[0]); ++i) {
+        PyObject* dict = PyObject_GenericGetDict(PyList_GET_ITEM(args[0], i), nullptr);
+        const bool yes = dict && PyDict_Check(dict) && is_plain(dict);
+        Py_XDECREF(dict);
+        if (!yes) {
+            PyErr_Clear();
+            return none();
+        }
+    }
+    Py_RETURN_TRUE;
+}
+
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     try {
@@ -246,6 +275,7 @@ PyMethodDef kMethods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<linear>)), METH_FASTCALL, "W8 linear, or None"},
     {"experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<experts>)), METH_FASTCALL, "routed W8 experts, or None"},
     {"pointers", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<pointers>)), METH_FASTCALL, "addresses of tensors of given forms, or None"},
+    {"plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<plain>)), METH_FASTCALL, "True for modules without hooks, or None"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_bind", "native call path of the lemoq operators", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

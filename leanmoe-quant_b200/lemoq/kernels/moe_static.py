@@ -177,6 +177,7 @@ def _block_forward(block: Any) -> Callable[[Any], tuple[Any, Any]]:
         return static_moe_forward(hidden_states, block._static_router, block._static_experts, top_k=block._static_top_k,
                                   norm_topk_prob=block._static_norm, act_fn=block._static_act, impl=block._static_impl)
 
+    forward.of_block = block  # tells this forward from one that somebody else has put in its place
     return forward
 
 

@@ -9,12 +9,19 @@ call is kept for the next by the address or identity of a tensor or module.
 from __future__ import annotations
 
 from array import array
+from itertools import chain
 from typing import Any, NamedTuple
 
 import torch
 import torch.nn.functional as F
+from torch import nn
 
 from lemoq import _cabi, _native
+from lemoq.kernels.attn_decode import _decode_forward_impl
+from lemoq.kernels.moe_grouped_quant import QuantFusedExperts
+from lemoq.kernels.rmsnorm import _fused_norm_forward
+from lemoq.model import OlmoeAttention, OlmoeDecoderLayer, OlmoeRMSNorm, OlmoeRotaryEmbedding, StaticCache
+from lemoq.quant.linear import QuantLinear
 
 _PLAN = "_lemoq_prompt_plan"  # on the cache object: what the last native call over that cache was given
 
@@ -29,6 +36,7 @@ class Weights(NamedTuple):
 
     own: dict      # field of ``StepDesc`` -> tensor
     layers: list   # per layer, in the order of ``_LAYER_WEIGHTS``
+    modules: tuple  # what a forward of the module tree calls: (W8 linears, norms, attention and expert blocks, embedding and decoder layers)
 
     def tensors(self) -> list:
         return [*self.own.values(), *(t for layer in self.layers for t in layer)]
@@ -38,10 +46,6 @@ def _read(model: Any) -> tuple[Weights | None, str | None]:
     """The tensors that the model's forwards would use now, or None and the reason why one ``StepDesc`` does not stand for the model: it has
     ONE group size, top_k, eps and so on, so what every block was really built with is compared here.  (Through the modules' own
     dictionaries: 300 attribute look-ups of ``nn.Module`` would take longer than the launches of a short prompt.)"""
-    from lemoq.kernels.attn_decode import _decode_forward_impl
-    from lemoq.kernels.moe_grouped_quant import QuantFusedExperts
-    from lemoq.model import OlmoeAttention, OlmoeDecoderLayer
-    from lemoq.quant.linear import QuantLinear
 
     cfg, m, lm = model.config, model.model, model.lm_head
     if type(lm) is not QuantLinear or lm.bias is not None:
@@ -51,7 +55,7 @@ def _read(model: Any) -> tuple[Weights | None, str | None]:
     group, eps, routing = lm.group_size, cfg.rms_norm_eps, (cfg.num_experts_per_tok, bool(cfg.norm_topk_prob))
     if getattr(m.norm, "variance_epsilon", None) != eps:
         return None, "the final norm has an eps of its own"
-    layers = []
+    layers, linears, norms, blocks = [], [lm], [m.norm], []
     for i, layer in enumerate(m.layers):
         if type(layer) is not OlmoeDecoderLayer:
             return None, "layer %d is a %s" % (i, type(layer).__name__)
@@ -71,18 +75,45 @@ def _read(model: Any) -> tuple[Weights | None, str | None]:
                           % (i, packed.group_size, o_proj.group_size, stacks.group_size, group))
         if (moe["_static_top_k"], moe["_static_norm"]) != routing:
             return None, "layer %d: top_k %d (normalised: %s) is not the configuration's" % (i, moe["_static_top_k"], moe["_static_norm"])
-        weights = []
-        for norm in (parts["input_layernorm"], parts["post_attention_layernorm"], inner["q_norm"], inner["k_norm"]):
-            if "weight" not in norm._parameters or getattr(norm, "variance_epsilon", None) != eps:
-                return None, "layer %d: a norm is not RMSNorm with the configuration's eps" % i
-            weights.append(norm._parameters["weight"])
-        layers.append((*weights, packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"], moe["_static_router"].contiguous(),
+        ln1, ln2, q_norm, k_norm = own = parts["input_layernorm"], parts["post_attention_layernorm"], inner["q_norm"], inner["k_norm"]
+        if any([type(norm) is not OlmoeRMSNorm or norm.variance_epsilon != eps or "weight" not in norm._parameters for norm in own]):
+            return None, "layer %d: a norm is not RMSNorm with the configuration's eps" % i
+        linears += inner["q_proj"], inner["k_proj"], inner["v_proj"], o_proj
+        norms += own
+        blocks += attn, mlp
+        layers.append((ln1._parameters["weight"], ln2._parameters["weight"], q_norm._parameters["weight"], k_norm._parameters["weight"], packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"], moe["_static_router"].contiguous(),
                        stacks.packed_gate_up, stacks.scale_gate_up, stacks.packed_down, stacks.scale_down))
-    return Weights({"embed": m.embed_tokens.weight, "final_norm": m.norm.weight, "lm_head_codes": lm.packed, "lm_head_scale": lm.scale}, layers), None
+    return Weights({"embed": m.embed_tokens.weight, "final_norm": m.norm.weight, "lm_head_codes": lm.packed, "lm_head_scale": lm.scale}, layers,
+                   (linears, norms, blocks, [m.embed_tokens, m.rotary_emb, *m.layers])), None
 
 
 def read_weights(model: Any) -> Weights | None:
     return _read(model)[0]
+
+
+def _skippable(weights: Weights) -> bool:
+    """May the module tree's forward be left out?  Not when that would be noticed: a hook on one of the modules it calls or on all modules, or a
+    module with another forward than the one the native path computes."""
+
+    linears, norms, blocks, plain = weights.modules
+    embed, rotary = plain[:2]
+    if set(map(type, linears)) != {QuantLinear} or type(embed) is not nn.Embedding or embed.max_norm is not None or type(rotary) is not OlmoeRotaryEmbedding:
+        return False
+    if any([getattr(mlp.__dict__.get("forward"), "of_block", None) is not mlp for mlp in blocks[1::2]]):
+        return False
+    every = torch.nn.modules.module
+    if every._global_forward_hooks or every._global_forward_pre_hooks:
+        return False
+    groups = ((linears + plain, ()), (norms, (_fused_norm_forward, OlmoeRMSNorm.forward)), (blocks[::2], (_decode_forward_impl,)))
+    if any(x._forward_hooks or x._forward_pre_hooks for x in blocks[1::2]):
+        return False
+    return all(_native.plain(modules, forwards) or all(_plain(x, forwards) for x in modules) for modules, forwards in groups)
+
+
+def _plain(module: Any, forwards: tuple) -> bool:
+    """No hook, and no forward of its own but a bound method of one of ``forwards``."""
+    own = module.__dict__.get("forward")
+    return not (module._forward_hooks or module._forward_pre_hooks) and (own is None or getattr(own, "__func__", None) in forwards)
 
 
 _HALF, _CODE = 0, 1  # element types of a form: (type, *shape)
@@ -129,14 +160,13 @@ def form_blocker(model: Any) -> str | None:
             or _misfit([t for tensors in weights.layers for t in tensors], layer, _LAYER_WEIGHTS, device))
 
 
-def describe(model: Any, weights: Weights, max_len: int, caches: list[dict], cache_forms: dict) -> tuple[Any, Any] | None:
-    """``(StepDesc, LayerDesc array)`` of the model over one set of cache tensors per layer (named as in ``LayerDesc``, each with its form):
+def describe(model: Any, weights: Weights, max_len: int, caches: list[tuple], cache_forms: tuple) -> tuple[Any, Any] | None:
+    """``(StepDesc, LayerDesc array)`` of the model over one set of cache tensors per layer (in the order of ``_CACHES``, each None or of its form):
     pointers only, the caller keeps the tensors for as long as the C side may read them.  None when a tensor misfits."""
     cfg, m = model.config, model.model
     device, (own_forms, layer_forms) = weights.own["embed"].device, _forms(model)
     own = _pointers(list(weights.own.values()), own_forms, tuple(weights.own), device)
-    words = _pointers([t for layer, slots in zip(weights.layers, caches) for t in (*layer, *map(slots.get, _CACHES))],
-                      layer_forms + tuple(cache_forms.get(name, (_HALF,)) for name in _CACHES), _LAYER_WEIGHTS + _CACHES, device)
+    words = _pointers(list(chain.from_iterable(chain.from_iterable(zip(weights.layers, caches)))), layer_forms + cache_forms, _LAYER_WEIGHTS + _CACHES, device)
     if own is None or words is None:
         return None
     cos, sin = m.rotary_emb.tables(max_len, torch.float16, device)
@@ -154,7 +184,6 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
     """Logits ``(1, T, V)`` of the prompt ``input_ids (1, T)``, with its K/V rows written into ``cache`` - or None when the
     model, the cache or the call is not of the kind the native path takes.  A token id outside the vocabulary, a position outside the cache
     and a wait that ran out raise ``RuntimeError`` (the kernels clamp and flag; the call waits for the flag unless the cache's owner does)."""
-    from lemoq.model import StaticCache
 
     weight = model.model.embed_tokens.weight
     if (torch.is_grad_enabled() or type(cache) is not StaticCache or input_ids.shape[0] != 1 or not weight.is_cuda or weight.dtype != torch.float16
@@ -163,14 +192,14 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
             or len(cache.layers) != len(model.model.layers) or not _cabi.available()):
         return None
     weights = read_weights(model)
-    if weights is None:
+    if weights is None or not _skippable(weights):
         return None
     cfg, device = model.config, weight.device
     for slot in cache.layers:
         if not slot.is_initialized:
             slot.lazy_initialization(torch.empty((1, cfg.num_attention_heads, 1, cfg.head_dim), dtype=torch.float16, device=device))
-    slots = (_HALF, 1, cfg.num_attention_heads, cache.max_cache_len, cfg.head_dim)
-    described = describe(model, weights, cache.max_cache_len, [{"keys": s.keys, "values": s.values} for s in cache.layers], {"keys": slots, "values": slots})
+    described = describe(model, weights, cache.max_cache_len, [(s.keys, s.values, None, None, None, None) for s in cache.layers],
+                         6 * ((_HALF, 1, cfg.num_attention_heads, cache.max_cache_len, cfg.head_dim),))
     if described is None:
         return None
     desc, layers = described
@@ -187,21 +216,24 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     _cabi.call("lemoq_prompt_run", desc, layers, _cabi.ptr(ids), _cabi.ptr(cache_position), tokens, _cabi.ptr(logits),
                _cabi.ptr(workspace), size, _cabi.ptr(flags), _cabi.current_stream(device))
+    for linear in weights.modules[0]:
+        linear.count_separate(several=True)
     if carried is None and not torch.cuda.is_current_stream_capturing():
         _cabi.check_flags(int(flags), "prompt")
     return logits
 
 
-def _lockstep_forms(model: Any, sequences: int, max_len: int) -> dict:
+def _describe_lockstep(model: Any, weights: Weights, kv: list[dict], sequences: int, max_len: int) -> tuple[Any, Any] | None:
     heads, dim = sequences * model.config.num_attention_heads, model.config.head_dim
-    return {"kc": (_CODE, heads, max_len, dim), "vc": (_CODE, heads, max_len, dim), "ks": (_HALF, heads, max_len), "vs": (_HALF, heads, max_len)}
+    codes, scales = (_CODE, heads, max_len, dim), (_HALF, heads, max_len)
+    return describe(model, weights, max_len, [tuple(map(slots.get, _CACHES)) for slots in kv], (codes, codes, codes, scales, codes, scales))
 
 
 def lockstep_plan(model: Any, kv: list[dict], sequences: int, max_len: int) -> dict | None:
     """What :func:`run_lockstep` keeps from step to step for ``sequences`` sequences with the int8 caches ``kv`` (per layer ``kc/vc
     (B*heads, S, D)``, ``ks/vs (B*heads, S)``), or None when the model is not in the canonical form."""
     weights = read_weights(model) if _cabi.available() else None
-    described = None if weights is None else describe(model, weights, max_len, kv, _lockstep_forms(model, sequences, max_len))
+    described = None if weights is None else _describe_lockstep(model, weights, kv, sequences, max_len)
     if described is None:
         return None
     size = int(_cabi.lib().lemoq_lockstep_workspace_bytes(described[0], sequences))
@@ -216,7 +248,7 @@ def run_lockstep(plan: dict, tokens: Any, position: Any, filled: Any, vocab: int
     canonical form.  ``plan["weights"]``: the tensors this call reads (a captured step's graph reads them at every replay)."""
     model, max_len = plan["model"], plan["max_len"]
     weights = read_weights(model)
-    described = None if weights is None else describe(model, weights, max_len, plan["kv"], _lockstep_forms(model, plan["sequences"], max_len))
+    described = None if weights is None else _describe_lockstep(model, weights, plan["kv"], plan["sequences"], max_len)
     if described is None:
         return None
     desc, layers = described

@@ -210,3 +210,30 @@ def test_a_flagged_prompt_raises():
         for ids, at, told in ((prompt + spec.vocab, slots, "token id"), (prompt, slots + 5, "position")):
             with pytest.raises(RuntimeError, match=told):
                 model(ids, past_key_values=cache, cache_position=at)
+
+
+def test_a_prompt_is_counted_and_hooks_fire():
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+    from lemoq.quant.linear import dequant_activity, reset_dequant_counters
+
+    spec = glue.OlmoeSpec(layers=2, hidden=256, heads=2, head_dim=128, experts=8, top_k=2, ffn=128, vocab=512)
+    model = lemoq_model_from_oracle(glue.random_float_weights(spec, seed=6, dtype=torch.float16, std=0.05))
+    install_canonical(model, 20, 4)
+    session = StaticCacheDecodeSession(model, torch.arange(20, device=DEV).unsqueeze(0), ctx=20, max_new_tokens=4, engine="ops")
+
+    def counted():
+        reset_dequant_counters(model)
+        del session.cache._lemoq_prompt_plan
+        logits = session.prefill().logits.clone()
+        return dequant_activity(model), logits
+
+    native, logits = counted()
+    assert "_lemoq_prompt_plan" in session.cache.__dict__ and native["separate_calls"] == 9 and native["fallbacks"] == {"multi_token": 9}
+    session.cache._lemoq_prompt_plan = seen = []
+    handle = model.model.layers[1].self_attn.o_proj.register_forward_hook(lambda module, args, out: seen.append(tuple(out.shape)))
+    by_modules, same = counted()
+    assert seen == [(1, 20, 256)] and "_lemoq_prompt_plan" not in session.cache.__dict__
+    assert by_modules == native and rel_err(logits, same) < 2e-2
+    handle.remove()
+    session.prefill()
+    assert len(seen) == 1 and "_lemoq_prompt_plan" in session.cache.__dict__

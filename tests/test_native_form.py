@@ -45,8 +45,8 @@ def test_a_description_follows_the_tensors_of_the_model(canonical):
     """Nothing is kept by a module's identity: whatever replaces a parameter or a buffer is what the next call is given."""
     from lemoq.prompt import _HALF, describe, read_weights
 
-    model, forms = canonical(), dict.fromkeys(("keys", "values"), (_HALF, 1, 2, 8, 128))
-    caches = [{"keys": torch.zeros(1, 2, 8, 128, dtype=torch.float16), "values": torch.zeros(1, 2, 8, 128, dtype=torch.float16)} for _ in range(2)]
+    model, forms = canonical(), 6 * ((_HALF, 1, 2, 8, 128),)
+    caches = [(torch.zeros(1, 2, 8, 128, dtype=torch.float16), torch.zeros(1, 2, 8, 128, dtype=torch.float16), *4 * (None,)) for _ in range(2)]
 
     def pointers():
         desc, layers = describe(model, read_weights(model), 8, caches, forms)
@@ -69,8 +69,8 @@ def test_a_description_follows_the_tensors_of_the_model(canonical):
                              (lambda: setattr(last.mlp._static_experts, "scale_down", last.mlp._static_experts.scale_down.clone()), ["dn_scale"]),
                              (lambda: model.lm_head.load_state_dict({k: v.clone() for k, v in model.lm_head.state_dict().items()}, assign=True),
                               ["lm_head_codes", "lm_head_scale"]),
-                             (lambda: caches[-1].update(keys=caches[-1]["keys"].clone()), ["keys"])):
-        keep.append([t.detach() for t in read_weights(model).tensors()] + [c["keys"] for c in caches])
+                             (lambda: caches.append((caches.pop()[0].clone(), *caches[0][1:])), ["keys", "values"])):
+        keep.append([t.detach() for t in read_weights(model).tensors()] + [t for c in caches for t in c[:2]])
         change()
         assert moved() == expected
     last.self_attn.o_proj.bias = torch.zeros(256)
@@ -111,8 +111,8 @@ def test_a_tensor_of_another_form_is_not_described(canonical, bound, monkeypatch
 
     if not bound:
         monkeypatch.setattr(_native, "pointers", lambda *a: None)
-    model, forms = canonical(), dict.fromkeys(("keys", "values"), (_HALF, 1, 2, 8, 128))
-    cache = lambda n: [{"keys": torch.zeros(1, 2, n, 128, dtype=torch.float16), "values": torch.zeros(1, 2, 8, 128, dtype=torch.float16)} for _ in range(2)]  # noqa: E731
+    model, forms = canonical(), 6 * ((_HALF, 1, 2, 8, 128),)
+    cache = lambda n: [(torch.zeros(1, 2, n, 128, dtype=torch.float16), torch.zeros(1, 2, 8, 128, dtype=torch.float16), *4 * (None,)) for _ in range(2)]  # noqa: E731
     assert describe(model, read_weights(model), 8, cache(8), forms) is not None and describe(model, read_weights(model), 8, cache(9), forms) is None
     mlp = model.model.layers[1].mlp
     whole = mlp._static_experts.packed_down
@@ -120,3 +120,33 @@ def test_a_tensor_of_another_form_is_not_described(canonical, bound, monkeypatch
                   torch.zeros(whole.numel() + 1, dtype=torch.int8)[1:].view_as(whole)):
         mlp._static_experts.packed_down = other
         assert describe(model, read_weights(model), 8, cache(8), forms) is None
+
+
+@pytest.mark.parametrize("bound", [True, False])
+def test_a_forward_that_is_seen_or_replaced_is_not_skipped(canonical, bound, monkeypatch):
+    from lemoq import _native
+    from lemoq.prompt import _skippable, read_weights
+
+    if not bound:
+        monkeypatch.setattr(_native, "plain", lambda *a: None)
+    model = canonical()
+    layer = model.model.layers[1]
+    skippable = lambda: (lambda weights: weights is not None and _skippable(weights))(read_weights(model))  # noqa: E731
+    assert skippable() and len(read_weights(model).modules[0]) == 9
+    called = [model.lm_head, model.model.norm, model.model.embed_tokens, model.model.rotary_emb, layer, layer.self_attn, layer.mlp, layer.input_layernorm,
+              *(getattr(layer.self_attn, n) for n in ("q_proj", "k_proj", "v_proj", "o_proj", "q_norm", "k_norm")), layer.post_attention_layernorm]
+    for module in called:
+        for register in (module.register_forward_hook, module.register_forward_pre_hook):
+            handle = register(lambda *a: None)
+            assert not skippable(), module
+            handle.remove()
+        own = module.__dict__.get("forward")
+        module.forward = lambda *a, **k: None
+        assert not skippable(), module
+        del module.forward
+        if own is not None:
+            module.forward = own
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    assert not skippable()
+    handle.remove()
+    assert skippable()
