@@ -353,7 +353,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_i8_kernel(const __grid_const
 
 }  // namespace
 
-bool attn_i8_eligible(const AttnParams& p) { return p.D == 128 && p.kv_head_stride == static_cast<int64_t>(p.S) * 128 && static_cast<int64_t>(p.heads) * p.S <= 0x7fffffff && p.heads <= 65535; }
+// (The query is read eight bytes at a time; one that starts elsewhere takes the split kernel, which reads it by element.)
+bool attn_i8_eligible(const AttnParams& p) {
+    return p.D == 128 && p.kv_head_stride == static_cast<int64_t>(p.S) * 128 && static_cast<int64_t>(p.heads) * p.S <= 0x7fffffff && p.heads <= 65535 &&
+           (reinterpret_cast<uintptr_t>(p.q) & 7u) == 0;
+}
 
 int launch_attn_i8(const AttnParams& a, const LaunchCfg& lc) {
     CUtensorMap map_k, map_v;

@@ -41,3 +41,17 @@ def test_attn_i8_edges(heads, capacity, filled, splits):
     k, v = (c[:, :filled].double() * s[:, :filled].double()[..., None] for c, s in ((kc, ks), (vc, vs)))
     weights = torch.softmax(torch.einsum("hd,hsd->hs", q.double(), k) * 128 ** -0.5, dim=-1)
     assert rel_err(out, torch.einsum("hs,hsd->hd", weights, v)) < PER_KERNEL_REL_TOL
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4])
+def test_query_at_any_element(offset):
+    """A contiguous query may start anywhere in its storage (a slice of a projection row): every start gives what an aligned copy gives."""
+    from lemoq.kernels.attn_decode import attn_decode_forward_int8
+
+    g = torch.Generator().manual_seed(offset)
+    codes, scales = torch.randint(-127, 128, (1, 3, 300, 128), generator=g, dtype=torch.int8).to(DEV), (torch.rand(1, 3, 300, generator=g) * 0.02).half().to(DEV)
+    row = torch.randn(offset + 3 * 128, generator=g).half().to(DEV)
+    q = row[offset:].view(1, 3, 1, 128)
+    length = torch.tensor([290], dtype=torch.int32, device=DEV)
+    got, ref = (attn_decode_forward_int8(x, codes, scales, codes, scales, length) for x in (q, q.clone()))
+    assert rel_err(got, ref) < PER_KERNEL_REL_TOL
