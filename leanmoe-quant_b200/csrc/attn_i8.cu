@@ -210,13 +210,14 @@ __global__ void __launch_bounds__(kThreads, 2) attn_i8_kernel(const __grid_const
         };
         auto query_digits = [&](const uint2& v, int round) {  // every warp finds the scale, warp 0 writes the digits
             const __half* h = reinterpret_cast<const __half*>(&v);
-            float f[4], amax = 0.f, sx, inv;
+            float f[4], sx, inv;
+            uint32_t top = 0;
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
                 f[x] = __half2float(h[x]);
-                amax = fmaxf(amax, fabsf(f[x]));
+                top = max(top, __float_as_uint(fabsf(f[x])));
             }
-            digit_scale(warp_max(amax), sx, inv);
+            digit_scale(__reduce_max_sync(0xffffffffu, top), sx, inv);
             if (warp == 0) {
 #pragma unroll
                 for (int x = 0; x < 4; ++x) sts_digits(q_at(round & 1), 0, 4 * lane + x, digit_round(f[x], inv));
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_i8_kernel(const __grid_const
                 l = fmaf(l, alpha, e);
                 m = m_new;
                 float sx, inv;
-                digit_scale(warp_max(fabsf(ev)), sx, inv);
+                digit_scale(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(ev))), sx, inv);
                 // the sums of the tile before the last leave TMEM; its digits' buffer is free then
                 if (t > 1 && !(ok = take(j - 2))) break;
                 if (lane == 0) s_step[j & 3][warp] = make_float2(alpha, sx);

@@ -24,11 +24,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 
 // Power-of-two scale of a group of fp32 values and its inverse: |x| / scale < 2^20, so x is three 7-bit digits
-// d2 * 2^14 + d1 * 2^7 + d0 (fp16 values within 2^9 of the maximum are exact, the rest good to 2^-20 of it).
-__device__ __forceinline__ void digit_scale(float amax, float& sx, float& inv) {
-    const int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xffu);  // biased exponent
-    const int k = amax > 0.f && e > 20 ? e - 19 : 2;  // zero or denormal range: a fixed tiny scale keeps the arithmetic exact
-    sx = __uint_as_float(static_cast<uint32_t>(k) << 23);
+// d2 * 2^14 + d1 * 2^7 + d0 (fp16 values within 2^9 of the maximum are exact, the rest good to 2^-20 of it).  `top`: the largest of the
+// absolute values' bit patterns, in whose order NaN and infinity come last; digits cannot express those, so the scale is NaN then.
+__device__ __forceinline__ void digit_scale(uint32_t top, float& sx, float& inv) {
+    const int e = static_cast<int>(top >> 23);  // biased exponent
+    const int k = e > 20 ? e - 19 : 2;  // zero or denormal range: a fixed tiny scale keeps the arithmetic exact
+    sx = e == 255 ? __uint_as_float(0x7fffffffu) : __uint_as_float(static_cast<uint32_t>(k) << 23);
     inv = __uint_as_float(static_cast<uint32_t>(254 - k) << 23);
 }
 __device__ __forceinline__ int digit_round(float x, float inv) {  // round to nearest even, |x| * inv < 2^20

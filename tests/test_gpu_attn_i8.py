@@ -55,3 +55,25 @@ def test_query_at_any_element(offset):
     length = torch.tensor([290], dtype=torch.int32, device=DEV)
     got, ref = (attn_decode_forward_int8(x, codes, scales, codes, scales, length) for x in (q, q.clone()))
     assert rel_err(got, ref) < PER_KERNEL_REL_TOL
+
+
+@pytest.mark.parametrize("what", ["q", "ks", "vs"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("filled", [40, 300])
+def test_values_that_are_not_numbers_are_not_hidden(what, value, filled):
+    """Digits cannot express them: the head they are in must come out as not finite, as the arithmetic has it, and no other head."""
+    from lemoq.kernels.attn_decode import attn_decode_forward_int8
+
+    g = torch.Generator().manual_seed(filled)
+    t = {"q": torch.randn(1, 3, 1, 128, generator=g).half(), "kc": torch.randint(1, 128, (1, 3, 320, 128), generator=g, dtype=torch.int8),
+         "ks": (torch.rand(1, 3, 320, generator=g) * 0.02).half()}
+    t["vc"], t["vs"] = t["kc"].flip(2), t["ks"].flip(2)
+    call = lambda: attn_decode_forward_int8(*(t[n].to(DEV) for n in ("q", "kc", "ks", "vc", "vs")), torch.tensor([filled], dtype=torch.int32, device=DEV)).cpu()  # noqa: E731
+    ref = call()
+    assert bool(ref.isfinite().all())
+    t[what].view(3, -1)[1, 7] = value
+    if what == "ks":
+        t["q"][0, 1] = t["q"][0, 1].abs()  # the score is then plus infinity, not minus: such a position is not simply left out
+    got = call()
+    assert not got[0, 1].isfinite().any()
+    assert torch.equal(got[0, 0], ref[0, 0]) and torch.equal(got[0, 2], ref[0, 2])
