@@ -90,6 +90,7 @@ struct GemmShape {
     float* y32;            // or: (T, N) in fp32
     int* err_flag;
     int parts;             // SPLIT: blocks of a cluster that share a tile's groups
+    int wide;              // rows of y (and resid) begin on 16 bytes: eight values a store
     int scale_vecs;        // 16-byte vectors of a row's scales when they fit the shared rows (1 or 2), else 0
 };
 
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 const int64_t ld = gu ? half_rows : p.N;
                 __half* y = p.y + static_cast<int64_t>(t.t0 + j0) * ld;
                 const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * ld : nullptr;
-                if (ld % 8 == 0 && mrow - lane + 32 <= lim) {
+                if (p.wide && mrow - lane + 32 <= lim) {
                     // A thread has one row of many tokens; turned over in shared memory 32 x 32 at a time, a lane stores eight rows of a token
                     // (two bytes a lane instead: a down tile of 128 tokens spent longer in its stores than in its MMAs).
                     const uint32_t turn = stage0 + kStages * S::kStage + warp * 2048u;
@@ -640,6 +641,7 @@ int launch_nt(GemmShape p, const __half* x, const int8_t* codes, const LaunchCfg
     if (int rc = encode_rows_map(&map_x, x, 2, p.T, p.K, Shape<NT>::kBox)) return rc;
     const size_t smem = Shape<NT>::kSmem + 8 * (static_cast<size_t>(p.E) + 1);
     const int gk = p.K / p.group;
+    p.wide = (p.gate_up ? p.N / 2 : p.N) % 8 == 0 && aligned16(p.y) && aligned16(p.resid);
     p.scale_vecs = aligned16(p.scale) && (gk == 8 || gk == 16) ? gk / 8 : 0;
     const int64_t mt = p.gate_up ? (p.N / 2 + 127) / 128 : (p.N + kTileRows - 1) / kTileRows;
     const int64_t most = mt * (p.seg ? p.T / NT + std::min<int64_t>(p.E, p.T) : (p.T + NT - 1) / NT);  // tiles, at most

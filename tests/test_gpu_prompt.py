@@ -49,6 +49,26 @@ def test_w8_gemm_edges(tokens, n, k, exact):
     assert rel_err(_gemm(*args, exact=exact, gate_up=True), gate * torch.sigmoid(gate) * up) < 2 * PER_KERNEL_REL_TOL
 
 
+@pytest.mark.parametrize("tokens", [3, 70, 130])  # exact form; scaled form, one token tile and two
+def test_w8_gemm_results_and_residuals_at_any_element(tokens):
+    """Only x and the codes have to begin on 16 bytes."""
+    from lemoq import _cabi
+
+    codes, scale = _w8(256, 256, tokens)
+    x = torch.randn(tokens, 256, generator=torch.Generator().manual_seed(5)).half()
+    resid = torch.randn(tokens, 256, generator=torch.Generator().manual_seed(6)).half()
+    ref = ops.dense_w8_gemv(x, codes, scale, 128).half() + resid
+    dev = [t.to(DEV) for t in (x, codes, scale)]
+    for y_at, resid_at in ((1, 0), (0, 1), (4, 4), (0, 0)):
+        y = torch.full((tokens * 256 + 8,), float("nan"), dtype=torch.float16, device=DEV)
+        held = torch.zeros(tokens * 256 + 8, dtype=torch.float16, device=DEV)
+        held[resid_at: resid_at + tokens * 256] = resid.flatten().to(DEV)
+        _cabi.call("lemoq_w8_gemm", _cabi.ptr(dev[0]), tokens, _cabi.ptr(dev[1]), _cabi.ptr(dev[2]), 256, 256, 128, None, 1, 0, 0,
+                   _cabi.ptr(held) + 2 * resid_at, _cabi.ptr(y) + 2 * y_at, None, _cabi.current_stream())
+        assert rel_err(y[y_at: y_at + tokens * 256].view(tokens, 256), ref) < PER_KERNEL_REL_TOL
+        assert bool(y[:y_at].isnan().all()) and bool(y[y_at + tokens * 256:].isnan().all())
+
+
 @pytest.mark.parametrize("counts,exact", [((0, 1, 16, 17, 0), True), ((70, 0, 3), True), ((128, 129, 0, 257, 1), False)])
 def test_w8_gemm_segments(counts, exact):
     n, k, rows = 258, 256, sum(counts)
