@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include "common.cuh"
 
 namespace lemoq {
@@ -18,6 +20,14 @@ struct LaunchCfg {
     int cluster = 1;         // blocks of a thread-block cluster along x
     int* launch_count = nullptr;
 };
+
+// The weights of a layer are there and begin on 16 bytes, as the vector loads and TMA copies of every form of the model need them.
+inline bool weights_placed(const lemoq_layer_desc& l) {
+    for (const void* p : {l.ln1, l.ln2, l.q_norm, l.k_norm, static_cast<const void*>(l.qkv_codes), l.qkv_scale, static_cast<const void*>(l.o_codes), l.o_scale, l.router,
+                          static_cast<const void*>(l.gu_codes), l.gu_scale, static_cast<const void*>(l.dn_codes), l.dn_scale})
+        if (!p || !aligned16(p)) return false;
+    return true;
+}
 
 // Launch through cudaLaunchKernelEx so that the PDL attribute can be attached.
 template <typename... KArgs, typename... Args>

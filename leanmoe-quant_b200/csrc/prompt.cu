@@ -81,9 +81,16 @@ int run_rows(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const 
     LEMOQ_REQUIRE(T > 0 && static_cast<int64_t>(T) * d.top_k <= (1 << 24), LEMOQ_ERR_INVALID, "prompt: T=%d out of range", T);
     LEMOQ_REQUIRE(d.embed && d.final_norm && d.lm_head_codes && d.lm_head_scale && d.rope_cos && d.rope_sin, LEMOQ_ERR_INVALID,
                   "prompt: null pointer in descriptor");
+    const bool lockstep = filled != nullptr;
+    for (const void* p : {d.embed, d.final_norm, static_cast<const void*>(d.lm_head_codes), d.lm_head_scale, d.rope_cos, d.rope_sin})
+        LEMOQ_REQUIRE(aligned16(p), LEMOQ_ERR_INVALID, "prompt: unaligned pointer in descriptor");
+    for (int i = 0; i < d.layers; ++i) {
+        const lemoq_layer_desc& L = layers[i];
+        const bool caches = lockstep ? L.kc && L.ks && L.vc && L.vs && aligned16(L.kc) && aligned16(L.vc) : L.keys && L.values && aligned16(L.keys) && aligned16(L.values);
+        LEMOQ_REQUIRE(weights_placed(L) && caches, LEMOQ_ERR_INVALID, "prompt: null or unaligned pointer in layer %d", i);
+    }
     LEMOQ_REQUIRE(aligned16(logits) && aligned16(workspace), LEMOQ_ERR_INVALID, "prompt: logits and workspace must be 16-byte aligned");
     PromptBuffers b;
-    const bool lockstep = filled != nullptr;
     const size_t rows_bytes = carve_prompt(d, T, static_cast<char*>(workspace), &b), need = rows_bytes + (lockstep ? attn_scratch_bytes(T * d.heads) : 0);
     LEMOQ_REQUIRE(workspace_bytes >= need, LEMOQ_ERR_INVALID, "prompt: workspace of %zu bytes, needs %zu", workspace_bytes, need);
     if (!err_flag) err_flag = status_word();

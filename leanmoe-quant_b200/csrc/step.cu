@@ -172,9 +172,8 @@ extern "C" int lemoq_step_create(const lemoq_step_desc* desc, const lemoq_layer_
                   "step_create: workspace must be 32-byte aligned");
     for (int l = 0; l < desc->layers; ++l) {
         const lemoq_layer_desc& L = layers[l];
-        LEMOQ_REQUIRE(L.ln1 && L.ln2 && L.q_norm && L.k_norm && L.qkv_codes && L.qkv_scale && L.o_codes && L.o_scale &&
-                          L.router && L.gu_codes && L.gu_scale && L.dn_codes && L.dn_scale && L.keys && L.values,
-                      LEMOQ_ERR_INVALID, "step_create: null pointer in layer %d", l);
+        LEMOQ_REQUIRE(weights_placed(L) && L.keys && L.values && aligned16(L.keys) && aligned16(L.values), LEMOQ_ERR_INVALID,
+                      "step_create: null or unaligned pointer in layer %d", l);
         LEMOQ_REQUIRE(!desc->kv_int8 || (L.kc && L.ks && L.vc && L.vs), LEMOQ_ERR_INVALID,
                       "step_create: layer %d has no int8 KV mirror", l);
     }

@@ -56,6 +56,45 @@ def test_cabi_argument_validation_needs_no_gpu():
         _cabi.check(_cabi.ERR_CUDA)
 
 
+def test_whole_model_calls_look_at_every_pointer():
+    """A null or misplaced pointer in a descriptor is an error of the call, before anything is launched (no GPU needed)."""
+    import ctypes
+
+    from lemoq import _cabi
+
+    lib = _cabi.lib()
+    desc, layers = _cabi.StepDesc(), (_cabi.LayerDesc * 2)()
+    for name, value in dict(layers=2, hidden=256, heads=2, head_dim=128, experts=8, top_k=2, ffn=128, vocab=64, group_size=128, max_len=16, eps=1e-5).items():
+        setattr(desc, name, value)
+    own = ("embed", "final_norm", "lm_head_codes", "lm_head_scale", "rope_cos", "rope_sin")
+    for name in own + ("token", "cache_position", "filled_len", "logits", "workspace"):
+        setattr(desc, name, 4096)
+    desc.workspace_bytes = 1 << 30
+    names = [name for name, _ in _cabi.LayerDesc._fields_]
+    for layer in layers:
+        for name in names:
+            setattr(layer, name, 4096)
+    # the workspace is a byte short, the last thing looked at: with sound pointers that is what is told
+    prompt = lambda: lib.lemoq_prompt_run(desc, layers, 4096, 4096, 4, 4096, 4096, lib.lemoq_prompt_workspace_bytes(desc, 4) - 1, None, None)  # noqa: E731
+    lockstep = lambda: lib.lemoq_lockstep_run(desc, layers, 4096, 4096, 4096, 4, 4096, 4096, lib.lemoq_lockstep_workspace_bytes(desc, 4) - 1, None, None)  # noqa: E731
+    calls = {"keys": [prompt], "values": [prompt], "kc": [lockstep], "vc": [lockstep], "ks": [lockstep], "vs": [lockstep]}
+    for call in (prompt, lockstep):
+        assert call() == _cabi.ERR_INVALID and "workspace of" in _cabi.last_error()
+    handle = ctypes.c_void_p()
+    for name in names:
+        for value in (None,) if name in ("ks", "vs") else (None, 4104):
+            setattr(layers[1], name, value)
+            for call in calls.get(name, [prompt, lockstep]):
+                assert call() == _cabi.ERR_INVALID and "pointer in layer 1" in _cabi.last_error(), name
+            if name not in ("kc", "ks", "vc", "vs"):
+                assert lib.lemoq_step_create(ctypes.byref(desc), layers, ctypes.byref(handle)) == _cabi.ERR_INVALID and "pointer in layer 1" in _cabi.last_error()
+            setattr(layers[1], name, 4096)
+    for name in own:
+        setattr(desc, name, 4104)
+        assert prompt() == _cabi.ERR_INVALID and "in descriptor" in _cabi.last_error()
+        setattr(desc, name, 4096)
+
+
 def test_ops_refuse_cpu_tensors_instead_of_falling_back():
     from lemoq.kernels.dequant_gemv import dequant_gemm_fused
     from lemoq.kernels.kv_int8 import kv_int8_rows_applicable, quantize_per_token_int8
