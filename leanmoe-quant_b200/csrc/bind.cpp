@@ -4,7 +4,11 @@
 // the kernel.  A function here takes the tensors of an ordinary call, and returns None for everything else (a wrong shape, another dtype,
 // a capture without a workspace, ...): the caller then goes its Python way, which raises the error or serves the call.
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/TracerMode.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContextLight.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -45,6 +49,17 @@ const at::Tensor* cuda_tensor(PyObject* o, int device) {
     const at::Tensor& t = THPVariable_Unpack(o);
     return t.is_cuda() && t.get_device() == device ? &t : nullptr;
 }
+
+// Nothing but the numbers of this call is wanted: no tensor class or mode that has to see the operation, no tangent, no trace, no autocast, no
+// gradient.  (The Python ways that remain are made of torch's operators where those matter.)
+bool ordinary(PyObject* o, const at::Tensor& x, const at::Tensor& scale) {
+    static const c10::DispatchKeySet wrapped({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                              c10::DispatchKey::Functionalize, c10::DispatchKey::ZeroTensor, c10::DispatchKey::Negative});
+    return THPVariable_CheckExact(o) && !x.unsafeGetTensorImpl()->key_set().has_any(wrapped) && !x._fw_grad(0).defined() && !scale._fw_grad(0).defined() &&
+           !(at::GradMode::is_enabled() && (x.requires_grad() || scale.requires_grad())) && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+           !at::impl::torch_function_mode_enabled() && !at::tracer::impl::is_dispatch_enabled() && !at::autocast::is_autocast_enabled(at::kCUDA);
+}
+bool aligned(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 
 bool is(const at::Tensor* t, at::ScalarType type, int dim) { return t && t->scalar_type() == type && t->dim() == dim; }
 bool rows(const at::Tensor* t, at::ScalarType type, int dim) { return is(t, type, dim) && t->is_contiguous(); }
@@ -125,6 +140,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int device = c10::cuda::current_device();
     const at::Tensor *x = cuda_tensor(args[0], device), *codes = cuda_tensor(args[1], device), *scale = cuda_tensor(args[2], device);
     if (!x || x->scalar_type() != at::kHalf || x->dim() < 1 || !x->is_contiguous() || !rows(codes, at::kChar, 2) || !rows(scale, at::kHalf, 2)) return none();
+    if (!ordinary(args[0], *x, *scale) || !aligned(*x) || !aligned(*codes)) return none();
     const int64_t N = codes->size(0), K = codes->size(1), group = PyLong_AsLongLong(args[3]);
     if (group <= 0 || K % group || scale->size(0) != N || scale->size(1) != K / group || x->size(-1) != K || K == 0 || N == 0) {
         PyErr_Clear();

@@ -89,3 +89,49 @@ def test_calls_leave_their_flags_where_the_host_sees_them():
                 call()
             call()
             assert flags() == _cabi.FLAG_BAD_EXPERT, name
+
+
+class _Marked(torch.Tensor):
+    """A tensor class whose operations have to be seen to keep it."""
+
+
+def _jvp(f, x):
+    import torch.autograd.forward_ad as fw
+
+    with fw.dual_level():
+        return fw.unpack_dual(f(fw.make_dual(x, x + 1))).tangent
+
+
+def _autocast(f, x):
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        return f(x)
+
+
+def _scale_gradient(f, x):
+    with torch.enable_grad():
+        scale = f.scale.detach().requires_grad_()
+        f.scale = scale
+        return torch.autograd.grad(f(x).float().square().mean(), scale)[0]
+
+
+@pytest.mark.parametrize("tokens", [4, 70])  # (vmap: two halves)
+@pytest.mark.parametrize("way", [_jvp, _autocast, _scale_gradient, lambda f, x: torch.func.vmap(f)(x.view(2, -1, 256)).flatten(0, 1),
+                                 lambda f, x: torch.func.jvp(f, (x,), (x + 1,))[1], lambda f, x: torch.jit.trace(f, (x + 1,), check_trace=False)(x),
+                                 lambda f, x: f(x.as_subclass(_Marked)), lambda f, x: f(torch.cat([x.flatten()[:1], x.flatten()])[1:].view_as(x)),
+                                 lambda f, x: torch.compile(f, backend="eager", fullgraph=True)(x)],
+                         ids=["tangent", "autocast", "scale gradient", "vmap", "jvp", "trace", "subclass", "misaligned", "compile"])
+def test_quant_linear_where_the_operation_itself_matters(way, tokens):
+    """What torch does with a linear it does with this one: the same result and kind of result as with the rebuilt weight."""
+    from lemoq.quant.linear import QuantLinear, SchemeSpec
+
+    class Rebuilt(QuantLinear):
+        def forward(self, x):
+            return torch.nn.functional.linear(x, self.dequantized_weight(dtype=x.dtype), self.bias)
+
+    torch.manual_seed(tokens)
+    dense = nn.Linear(256, 130, bias=True, device=DEV, dtype=torch.float16)
+    x = torch.randn(tokens, 256, device=DEV).half()
+    with torch.no_grad():
+        got, ref = (way(kind(dense, SchemeSpec.from_flags("w8a16", 128, dequant="fused")), x) for kind in (QuantLinear, Rebuilt))
+    assert type(got) is type(ref) and got.dtype == ref.dtype and got.shape == ref.shape
+    assert rel_err(got, ref) < (PER_KERNEL_REL_TOL if ref.dtype != torch.bfloat16 else 8 * PER_KERNEL_REL_TOL)
