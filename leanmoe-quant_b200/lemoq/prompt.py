@@ -180,11 +180,18 @@ def describe(model: Any, weights: Weights, max_len: int, caches: list[tuple], ca
     return desc, (_cabi.LayerDesc * len(m.layers)).from_buffer_copy(words)
 
 
+def _operations_matter() -> bool:
+    """Is somebody to see or change the single operations of this call (autocast, a dispatch mode, a trace, a compilation)?"""
+    return bool(torch.compiler.is_compiling() or torch.is_autocast_enabled("cuda") or torch._C._len_torch_dispatch_stack() or torch.jit.is_tracing())
+
+
 def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, position_ids: Any) -> Any:
     """Logits ``(1, T, V)`` of the prompt ``input_ids (1, T)``, with its K/V rows written into ``cache`` - or None when the
     model, the cache or the call is not of the kind the native path takes.  A token id outside the vocabulary, a position outside the cache
     and a wait that ran out raise ``RuntimeError`` (the kernels clamp and flag; the call waits for the flag unless the cache's owner does)."""
 
+    if _operations_matter():
+        return None
     weight = model.model.embed_tokens.weight
     if (torch.is_grad_enabled() or type(cache) is not StaticCache or input_ids.shape[0] != 1 or not weight.is_cuda or weight.dtype != torch.float16
             or input_ids.dtype != torch.int64 or cache_position.dtype != torch.int64 or not cache_position.is_cuda or cache_position.numel() != input_ids.shape[1]

@@ -257,3 +257,29 @@ def test_a_prompt_is_counted_and_hooks_fire():
     handle.remove()
     session.prefill()
     assert len(seen) == 1 and "_lemoq_prompt_plan" in session.cache.__dict__
+
+
+def test_a_prompt_whose_operations_matter_goes_through_the_modules():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+
+    class Seen(TorchDispatchMode):
+        count = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.count += func is torch.ops.aten.index_copy_.default
+            return func(*args, **(kwargs or {}))
+
+    spec = glue.OlmoeSpec(layers=2, hidden=256, heads=2, head_dim=128, experts=8, top_k=2, ffn=128, vocab=512)
+    model = lemoq_model_from_oracle(glue.random_float_weights(spec, seed=8, dtype=torch.float16, std=0.05))
+    install_canonical(model, 20, 4)
+    session = StaticCacheDecodeSession(model, torch.arange(20, device=DEV).unsqueeze(0), ctx=20, max_new_tokens=4, engine="ops")
+    native = session.prefill().logits.clone()
+    for mode in (Seen(), torch.autocast("cuda", dtype=torch.float16)):
+        del session.cache._lemoq_prompt_plan
+        with mode:
+            logits = session.prefill().logits.clone()
+        assert "_lemoq_prompt_plan" not in session.cache.__dict__ and rel_err(logits, native) < 2e-2
+        assert not isinstance(mode, Seen) or mode.count == 4  # k and v rows of both layers
+        assert torch.equal(session.prefill().logits, native) and "_lemoq_prompt_plan" in session.cache.__dict__
