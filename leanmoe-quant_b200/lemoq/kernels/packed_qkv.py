@@ -4,7 +4,8 @@ stacked ``[q; k; v]`` (the interface of the reference's src/lemoq/kernels/packed
 The GEMV kernel reduces every output row on its own, in an order that does not depend on how many rows
 the call has, so the stacked call returns the very bits three separate calls return
 (tests/test_gpu_ops.py checks that).  The stacked buffers are built once, after quantisation and before
-any graph capture; the decode step hands their pointers to the native step engine.
+any graph capture; the decode step, the lockstep step and native prompts hand their pointers to the C side.
+They are copies: whoever changes a projection's codes afterwards calls :func:`install_packed_qkv` again.
 """
 
 from __future__ import annotations

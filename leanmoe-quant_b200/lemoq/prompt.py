@@ -78,7 +78,8 @@ def _read(model: Any) -> tuple[Weights | None, str | None]:
         ln1, ln2, q_norm, k_norm = own = parts["input_layernorm"], parts["post_attention_layernorm"], inner["q_norm"], inner["k_norm"]
         if any([type(norm) is not OlmoeRMSNorm or norm.variance_epsilon != eps or "weight" not in norm._parameters for norm in own]):
             return None, "layer %d: a norm is not RMSNorm with the configuration's eps" % i
-        linears += inner["q_proj"], inner["k_proj"], inner["v_proj"], o_proj
+        linears.append(o_proj)
+        linears.extend(filter(None, map(inner.get, ("q_proj", "k_proj", "v_proj"))))  # (absent where only the stacked rows were kept)
         norms += own
         blocks += attn, mlp
         layers.append((ln1._parameters["weight"], ln2._parameters["weight"], q_norm._parameters["weight"], k_norm._parameters["weight"], packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"], moe["_static_router"].contiguous(),

@@ -150,3 +150,12 @@ def test_a_forward_that_is_seen_or_replaced_is_not_skipped(canonical, bound, mon
     assert not skippable()
     handle.remove()
     assert skippable()
+
+
+def test_projections_may_be_given_up_once_they_are_stacked(canonical):
+    from lemoq.prompt import _skippable, form_blocker, read_weights
+
+    model = canonical()
+    for layer in model.model.layers:
+        del layer.self_attn.q_proj, layer.self_attn.k_proj, layer.self_attn.v_proj
+    assert form_blocker(model) is None and _skippable(read_weights(model))
