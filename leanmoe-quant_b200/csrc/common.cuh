@@ -13,7 +13,6 @@ constexpr int kWarp = 32;
 
 // ---- error plumbing (host) -------------------------------------------------
 int set_error(int code, const char* fmt, ...);
-int check_launch(const char* what);
 int* status_word();  // where a call without an error word has its flags left: the current device's lemoq_status_word, or null before the first of it
 
 #define LEMOQ_REQUIRE(cond, code, ...)                 \

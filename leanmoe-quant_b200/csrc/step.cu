@@ -307,7 +307,6 @@ extern "C" int lemoq_step_run(lemoq_step* s, void* stream, int* launches) {
         p.fl_logits = s->flagged + kFlLogits; p.fl_act = s->flagged + kFlAct;
         p.fl_attn = s->flagged + kFlAttn; p.fl_part = s->flagged + kFlPart;
         p.router_logits = s->router_logits; p.top_w = s->top_w; p.top_i = s->top_i; p.attn_part = s->attn_part;
-        p.barriers_per_launch = 1;  // the end of the step
         p.stamps = s->stamps;
         if (int rc = launch_step_tile(p, s->whole_grid, static_cast<cudaStream_t>(stream))) return rc;
         if (launches) *launches = 1;

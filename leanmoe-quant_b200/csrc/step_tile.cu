@@ -1240,7 +1240,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
     unsigned char* const my_stage = S.ring + static_cast<size_t>(warp) * kStageBytes;
 
     const uint32_t epoch = ld_acquire_u32(p.bar_epoch);
-    unsigned int bar_target = epoch * static_cast<unsigned int>(p.barriers_per_launch) * gridDim.x;
+    unsigned int bar_target = epoch * gridDim.x;  // one barrier a launch: the end of the step
     const uint32_t tag0 = epoch * 64u;  // tag of layer l's exchanges: tag0 + l + 1 (at most 33 layers per launch)
     const __half* const embed_row = p.embed + tok * static_cast<int64_t>(p.H);
     float pw1v[4];

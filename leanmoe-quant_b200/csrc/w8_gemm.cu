@@ -33,7 +33,7 @@
 
 namespace lemoq {
 
-int encode_rows_map(CUtensorMap* map, const void* base, int elem_bytes, int64_t rows, int64_t cols, int box_rows, int64_t row_stride) {
+int encode_rows_map(CUtensorMap* map, const void* base, int elem_bytes, int64_t rows, int64_t cols, int box_rows) {
     using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static Encode encode = nullptr;
@@ -46,9 +46,8 @@ int encode_rows_map(CUtensorMap* map, const void* base, int elem_bytes, int64_t 
             encode = reinterpret_cast<Encode>(fn);
     });
     if (!encode) return set_error(LEMOQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available in this driver");
-    if (row_stride == 0) row_stride = cols;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_stride) * elem_bytes};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * elem_bytes};
     const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / elem_bytes), static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t elem[2] = {1, 1};
     const CUresult rc = encode(map, elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims,
