@@ -6,7 +6,9 @@
  *   - plain C: device pointers, sizes and a CUDA stream handle (`cudaStream_t`
  *     passed as `void*`; NULL = the legacy default stream);
  *   - no allocation, no synchronisation, no host<->device copies: work is only
- *     enqueued on `stream`, so every call is legal under stream capture;
+ *     enqueued on `stream`, so every call is legal under stream capture (but for
+ *     lemoq_step_create, lemoq_set_tuning, lemoq_status_word and lemoq_step_replay,
+ *     as said there);
  *   - tensors are contiguous unless a stride argument says otherwise; weight,
  *     cache and activation base pointers must be 16-byte aligned;
  *   - return value: LEMOQ_OK, or an error code with a message available from
@@ -67,7 +69,7 @@ LEMOQ_API int* lemoq_status_word(void);
  *   key 5  whole-step kernel, current device: polls of a flagged word before a wait gives up with
  *          LEMOQ_FLAG_WAIT_TIMEOUT (1 .. 2^24, default 2^21).  A step whose wait ran out has gone on with
  *          stale values: its results are void, the flag says so, the next step is unaffected.  Exists so
- *          that the time-out path can be exercised (value 1) without anything hanging.
+ *          that the time-out path can be exercised (value 1) without anything hanging.  Waits for the device.
  * Keys 0, 1 and 4 give the same results up to fp32 summation order.
  * No counterpart in the reference, whose tile configs are module dicts
  * (ref: src/lemoq/kernels/moe_grouped.py:78, src/lemoq/kernels/_dequant_triton.py:83).
@@ -383,6 +385,8 @@ typedef struct lemoq_step_desc {
 
 typedef struct lemoq_step lemoq_step; /* host-side plan, owns no device memory */
 
+/* lemoq_step_create reads desc and layers and, for the whole-step kernel, writes the zeroed workspace: it waits for the
+ * device before and after (set-up time, not under capture). */
 LEMOQ_API size_t lemoq_step_workspace_bytes(const lemoq_step_desc* desc);
 LEMOQ_API int lemoq_step_create(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, lemoq_step** out);
 LEMOQ_API void lemoq_step_destroy(lemoq_step* step);

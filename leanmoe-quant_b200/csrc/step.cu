@@ -229,8 +229,12 @@ extern "C" int lemoq_step_create(const lemoq_step_desc* desc, const lemoq_layer_
                     host[desc->layers].ln1 = reinterpret_cast<const __half*>(desc->final_norm);
                     host[desc->layers].qkv_codes = desc->lm_head_codes;
                     host[desc->layers].qkv_scale = reinterpret_cast<const __half*>(desc->lm_head_scale);
-                    // set-up time only: the descriptors move to the device once (synchronous copy)
-                    const cudaError_t err = cudaMemcpy(s->whole_layers, host, sizeof(StepLayer) * (desc->layers + 1), cudaMemcpyHostToDevice);
+                    // Set-up time only: the descriptors move to the device once.  The copy is ordered with nothing on a non-blocking
+                    // stream: neither with the zeroing of the workspace it goes into, which the caller may still have under way on one, nor
+                    // with the first step (for pageable memory the call returns before the bytes have arrived).  Hence a wait on either side.
+                    cudaError_t err = cudaDeviceSynchronize();
+                    if (err == cudaSuccess) err = cudaMemcpy(s->whole_layers, host, sizeof(StepLayer) * (desc->layers + 1), cudaMemcpyHostToDevice);
+                    if (err == cudaSuccess) err = cudaDeviceSynchronize();
                     delete[] host;
                     if (err == cudaSuccess) {
                         s->whole_grid = grid;

@@ -1590,7 +1590,8 @@ size_t tile_smem_bytes() { return sizeof(tile::Smem) + 128; }
 int set_flag_spin_limit(int polls) {
     if (polls < 1 || polls > (1 << 24)) return set_error(LEMOQ_ERR_INVALID, "set_tuning: flag poll limit %d outside [1, 2^24]", polls);
     const uint32_t v = static_cast<uint32_t>(polls);
-    const cudaError_t err = cudaMemcpyToSymbol(tile::c_flag_spin_limit, &v, sizeof(v));
+    cudaError_t err = cudaMemcpyToSymbol(tile::c_flag_spin_limit, &v, sizeof(v));
+    if (err == cudaSuccess) err = cudaDeviceSynchronize();  // the copy is ordered with no other stream's kernels
     if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "set_tuning: %s", cudaGetErrorString(err));
     return LEMOQ_OK;
 }

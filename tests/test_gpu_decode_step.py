@@ -588,3 +588,24 @@ def test_a_wait_that_runs_out_raises_the_flag_and_the_next_step_is_unaffected():
     assert decode() == good
     assert session.step_error_flags() == 0
     session.close()
+
+
+def test_a_step_is_built_while_its_stream_is_busy():
+    """The workspace's zeroing may still be queued on the caller's stream when the plan writes its layer table into the workspace, and the first
+    step follows at once: neither may overtake the other."""
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+
+    spec = glue.OlmoeSpec(layers=2, hidden=512, heads=4, head_dim=128, experts=8, top_k=2, ffn=512, vocab=1024)
+    model = lemoq_model_from_oracle(glue.random_float_weights(spec, seed=2, dtype=torch.float16, std=0.05))
+    install_canonical(model, 40, 4)
+    prompt = torch.arange(40, device="cuda").unsqueeze(0)
+    logits = []
+    for cycles in (0, 100_000_000):
+        session = StaticCacheDecodeSession(model, prompt, ctx=40, max_new_tokens=4, engine="step")
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(cycles)
+            logits.append(session.decode_eager().clone())
+        assert session.capture_info["step_kernel"] == "whole-step" and session.step_error_flags() == 0
+        session.close()
+    assert torch.equal(logits[0], logits[1])
