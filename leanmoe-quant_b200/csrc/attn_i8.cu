@@ -369,8 +369,12 @@ int launch_attn_i8(const AttnParams& a, const LaunchCfg& lc) {
     if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
     Shape p;
     p.q = a.q; p.ks = a.ks; p.vs = a.vs; p.filled = a.filled; p.out = a.out; p.part = a.part; p.counters = a.counters; p.err_flag = a.err_flag;
-    // num_splits is the most a caller wants.  With a head for every SM no split is worth its partial sums: 176 heads x 701 positions
-    // 17 us without and 23 us with two, 1024 x 2049 111 and 122 us.
+    // num_splits is the most a caller wants.  With a head for every SM a split is not worth its partial sums, also where half of the two
+    // places an SM has stay empty (us with 1 / 2 / 3 / 4 splits, cold caches):
+    //   160 heads    700 positions 16 / 25 / 23 / 23    2048: 29 / 37 / 33 / 37    4096: 47 / 59 / 49 / 55
+    //   240 heads    700 positions 20 / 25 / 29 / 29    2048: 35 / 41 / 45 / 45    4096: 59 / 64 / 68 / 70
+    //   512 heads    700 positions 31 / 41 / 47 / 49    2048: 62 / 72 / 76 / 76    4096: 102 / 115 / 119 / 117
+    // The exceptions are small: 148 heads x 4096 45 / 43 / 47 / 47, 320 (a third round of items) x 4096 92 / 88 / 86 / 84.
     p.heads = a.heads; p.S = a.S; p.splits = a.heads >= sm_count() ? 1 : a.num_splits; p.scale_log2 = a.qk_scale_log2;
     const int64_t items = static_cast<int64_t>(a.heads) * p.splits;
     return launch_kernel(attn_i8_kernel, dim3(static_cast<unsigned>(std::min<int64_t>(items, 2 * sm_count()))), dim3(kThreads), kSmem, lc, map_k, map_v, p);

@@ -7,7 +7,8 @@
 //   PV          A = the fp16 weights from TMEM, B = V (d is the contiguous side: MN-major), 128 x 128 fp32 in TMEM
 //   O           accumulates in TMEM.  The maximum a row's weights are taken against follows the true one only when that has grown by more
 //               than 2^8 (the weights stay below 256, the sum of them in fp32): then, which is rare after the first steps, O is rescaled.
-// Blocks are handed out longest first.  No S x S matrix exists anywhere.
+// Blocks are handed out longest first.  No S x S matrix exists anywhere.  (Two query tiles taking turns, sums in TMEM and rescaling only
+// beyond a slack are the published method of FlashAttention-4.)
 //
 // Bounded by exp2 (16 per SM and clock: 2048 cycles for the two tiles of a step) and the MMAs (2048 cycles as well), which the two tiles
 // overlap.  (With O in registers, 128 of them beside a row of S, the kernel spilled: 412 us at 4096 rows and 16 heads

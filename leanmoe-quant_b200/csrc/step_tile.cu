@@ -1608,9 +1608,16 @@ bool tile_eligible(const lemoq_step_desc& d) {
 }
 
 // Attention splits per head for the tile form: every (head, split) unit should have at most one KV tile per
-// streaming warp.  A tile is one warp's serial work and every further split makes the merge of the partials longer
-// (it takes the splits four at a time), so a short int8 cache is cut into tiles of 32 positions, about 8 per unit and
-// at most 6 splits, and a long one into tiles of 64, 10 per unit (measured at 1024 and 4096 cached positions).
+// streaming warp, since a tile is one warp's serial work.  A short int8 cache is cut into tiles of 32 positions, about 8 per
+// unit and at most 6 splits, a long one into tiles of 64, 10 per unit; fp16 tiles have 32 positions.  More splits cost little: the head's
+// first block collects all the others in one pass.  Whole step in us, the number this gives first, then 3 / 4 / 5 / 6 / 7 / 8 / 9 splits:
+//   int8     48 cached   1: 547   546 / 552 / 552 / 555 / 554 / 558 / 558      fp16     48 cached   1: 543   552 / 555 / 554 / 554 / 555 / 558 / 560
+//           256          2: 556   550 / 549 / 552 / 554 / 556 / 556 / 560              1537          6: 584   625 / 618 / 586 / 585 / 583 / 584 / 584
+//          1024          5: 564   573 / 568 / 564 / 564 / 566 / 567 / 566              4096          9: 652   768 / 724 / 688 / 681 / 664 / 661 / 653
+//          2048          4: 591   627 / 589 / 588 / 584 / 578 / 578 / 575
+//          3000          5: 599   644 / 639 / 602 / 599 / 595 / 599 / 599
+//          4096          7: 605   683 / 645 / 641 / 635 / 603 / 606 / 601
+// So the line is right within 1.3 %, but for 2.4 % around 2048 positions.
 int tile_attention_splits(const lemoq_step_desc& d, int grid) {
     const int tiles64 = (d.max_len + tile::kKvTile - 1) / tile::kKvTile, tiles32 = (d.max_len + 31) / 32;
     int s;
