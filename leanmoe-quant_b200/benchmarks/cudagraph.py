@@ -757,9 +757,12 @@ class StaticCacheDecodeSession:
         self.prefill()
 
     def close(self) -> None:
+        """Give the native step back: its workspace, and with it the graph that works in it."""
         if self._step is not None:
             from lemoq import _cabi
 
+            if self.stream is not None:
+                self.stream.synchronize()  # a step that was only queued still works in the workspace
+            self.graph = self._graph_exec = None
             _cabi.lib().lemoq_step_destroy(self._step["handle"])
             self._step = None
-            self._graph_exec = None

@@ -609,3 +609,22 @@ def test_a_step_is_built_while_its_stream_is_busy():
         assert session.capture_info["step_kernel"] == "whole-step" and session.step_error_flags() == 0
         session.close()
     assert torch.equal(logits[0], logits[1])
+
+
+def test_a_closed_session_replays_nothing():
+    """The graph works in the step's workspace: once that is given back, there is nothing to replay (or to time)."""
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+
+    spec = glue.OlmoeSpec(layers=1, hidden=512, heads=4, head_dim=128, experts=8, top_k=2, ffn=512, vocab=1024)
+    model = lemoq_model_from_oracle(glue.random_float_weights(spec, seed=2, dtype=torch.float16, std=0.05))
+    install_canonical(model, 20, 4)
+    session = StaticCacheDecodeSession(model, torch.arange(20, device="cuda").unsqueeze(0), ctx=20, max_new_tokens=4, engine="step")
+    session.capture(warmup=1)
+    session.replay()
+    session.replay(synchronize=False)
+    last = session.logits_cpu()
+    session.close()
+    assert torch.equal(session.logits_cpu(), last)  # what it answered last stays
+    for call in (session.replay, lambda: session.replay(synchronize=False), lambda: session.replay_chained(1), session.time_graph_only):
+        with pytest.raises(RuntimeError):
+            call()
