@@ -178,8 +178,8 @@ PyObject* experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
         ids.scalar_type() != at::kLong || w.scalar_type() != at::kHalf || (x.dim() != 1 && x.dim() != 2))
         return none();
     const int64_t E = gu.size(0), H = gu.size(2), F = dn.size(2), T = x.dim() == 2 ? x.size(0) : 1;
-    if (T < 1 || T > 65535 || x.size(-1) != H || gu.size(1) != 2 * F || dn.size(0) != E || dn.size(1) != H || H % group || F % group || ids.numel() % T ||
-        w.numel() != ids.numel() || gu.numel() >= (int64_t(1) << 31) || gs.numel() * group != gu.numel() || ds.numel() * group != dn.numel())
+    if (T < 1 || T > 65535 || x.size(-1) != H || gu.size(1) != 2 * F || dn.size(0) != E || dn.size(1) != H || H % group || F % group ||
+        (x.dim() == 2 && (ids.dim() != 2 || ids.size(0) != T || w.sizes() != ids.sizes())) || w.numel() != ids.numel() || gu.numel() >= (int64_t(1) << 31) || gs.numel() * group != gu.numel() || ds.numel() * group != dn.numel())
         return none();
     const int64_t K = ids.numel() / T;
     if (K < 1 || K > 64 || group % 16 || (T > 1 && (H % 128 || F % 128 || group % 128))) return none();

@@ -192,6 +192,8 @@ def grouped_moe_forward_quant_tokens(x: Any, q: QuantFusedExperts, ids: Any, top
     out = _native.experts(x, q.packed_gate_up, q.scale_gate_up, q.packed_down, q.scale_down, ids, top_w, q.group_size) if x.dim() == 2 else None
     if out is not None:
         return out
+    if x.dim() != 2 or ids.dim() != 2 or ids.shape[0] != x.shape[0] or top_w.shape != ids.shape or x.shape[1] != q.hidden:
+        raise ValueError("需要 x (T, %d)、ids 与 top_w (T, K)，得到 %r、%r、%r" % (q.hidden, tuple(x.shape), tuple(ids.shape), tuple(top_w.shape)))
     t, hidden = int(x.shape[0]), int(x.shape[1])
     k = int(ids.shape[1])
     dt = q.scale_gate_up.dtype

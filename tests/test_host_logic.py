@@ -173,6 +173,19 @@ def test_contract_errors_match_the_reference_types_and_keywords():
         qe.to(torch.float32)
 
 
+def test_batched_experts_refuse_shapes_that_do_not_belong_together():
+    """The kernel reads ``T * K`` ids and weights: fewer of them would be read past their end (no GPU needed)."""
+    from lemoq.kernels.moe_grouped_quant import QuantFusedExperts, grouped_moe_forward_quant_tokens
+
+    q = QuantFusedExperts(torch.zeros(4, 256, 128, dtype=torch.int8), torch.zeros(4, 256, 1).half(), torch.zeros(4, 128, 128, dtype=torch.int8), torch.zeros(4, 128, 1).half(), 8, 128)
+    x, ids, weights = torch.zeros(3, 128).half(), torch.zeros(3, 2, dtype=torch.int64), torch.zeros(3, 2).half()
+    for bad in ((x, ids[:2], weights), (x, ids, weights[:2]), (x, ids, weights[:, :1]), (x, ids.t(), weights.t()), (x, ids.flatten(), weights.flatten()), (x[:, :64], ids, weights), (x[0], ids, weights)):
+        with pytest.raises(ValueError):
+            grouped_moe_forward_quant_tokens(bad[0], q, bad[1], bad[2])
+    with pytest.raises(RuntimeError):  # and sound ones get as far as the device
+        grouped_moe_forward_quant_tokens(x, q, ids, weights)
+
+
 def test_fusion_switches():
     from lemoq.kernels.fusion_switches import ENV_VARS, FUSION_DEFAULTS, fusion_enabled, fusion_states
 
