@@ -34,13 +34,14 @@ def test_experts_for_several_tokens(tokens, top_k, experts):
     assert rel_err(got, ref) < PER_KERNEL_REL_TOL
 
 
+@pytest.mark.parametrize("bias", [True, False])
 @pytest.mark.parametrize("mode", ["fused", "separate"])
 @pytest.mark.parametrize("shape", [(256,), (1, 1, 256), (1, 3, 256), (70, 256)])
-def test_quant_linear_native_and_fallback_agree(mode, shape):
+def test_quant_linear_native_and_fallback_agree(mode, shape, bias):
     from lemoq.quant.linear import QuantLinear, SchemeSpec
 
     torch.manual_seed(len(shape))
-    dense = nn.Linear(256, 130, bias=True, device=DEV, dtype=torch.float16)
+    dense = nn.Linear(256, 130, bias=bias, device=DEV, dtype=torch.float16)
     linear = QuantLinear(dense, SchemeSpec.from_flags("w8a16", 128, dequant=mode))
     x = torch.randn(*shape, device=DEV).half()
     with torch.no_grad():
@@ -49,6 +50,7 @@ def test_quant_linear_native_and_fallback_agree(mode, shape):
         strided = linear(torch.cat([x, x], dim=-1)[..., :256])  # not contiguous: the Python way
     assert got.shape == ref.shape and rel_err(got, ref) < PER_KERNEL_REL_TOL and rel_err(strided, ref) < PER_KERNEL_REL_TOL
     single = x.numel() == 256
+    assert single or not bias or torch.equal(got, ref)  # the bias is added before the one rounding
     assert linear._counters["fused_calls"] == (2 if single and mode == "fused" else 0)
     assert linear._counters["separate_calls"] == (0 if single and mode == "fused" else 2)
     assert linear._counters["fallbacks"] == ({"multi_token": 2} if mode == "fused" and not single else {})
@@ -68,7 +70,7 @@ def test_calls_leave_their_flags_where_the_host_sees_them():
     own = QuantFusedExperts(*(t.to(DEV) for s in ((256, 128), (128, 128)) for t in ops.rtn_quantize_w8(torch.randn(4, *s, generator=g), 128)), 8, 128)
     x, ids, weights = torch.randn(3, 128, generator=g).half().to(DEV), torch.tensor([[0], [3], [1]], device=DEV), torch.ones(3, 1, device=DEV).half()
     q, codes, scale = torch.randn(1, 2, 1, 128, device=DEV).half(), torch.ones(1, 2, 40, 128, dtype=torch.int8, device=DEV), torch.ones(1, 2, 40, device=DEV).half()
-    linear = QuantLinear(nn.Linear(128, 64, device=DEV, dtype=torch.float16), SchemeSpec.from_flags("w8a16", 128, dequant="fused"))
+    linear = QuantLinear(nn.Linear(128, 64, bias=False, device=DEV, dtype=torch.float16), SchemeSpec.from_flags("w8a16", 128, dequant="fused"))
     calls = {"tokens": lambda n=0: grouped_moe_forward_quant_tokens(x, own, ids + n, weights), "token": lambda n=0: grouped_moe_forward_quant(x[0], own, ids[0] + n, weights[0]),
              "attention": lambda n=0: attn_decode_forward_int8(q, codes, scale, codes, scale, torch.tensor([40 + n], dtype=torch.int32, device=DEV)),
              "linear": lambda n=0: linear(x), "one": lambda n=0: linear(x[:1])}
@@ -114,13 +116,14 @@ def _scale_gradient(f, x):
         return torch.autograd.grad(f(x).float().square().mean(), scale)[0]
 
 
+@pytest.mark.parametrize("bias", [True, False])
 @pytest.mark.parametrize("tokens", [4, 70])  # (vmap: two halves)
 @pytest.mark.parametrize("way", [_jvp, _autocast, _scale_gradient, lambda f, x: torch.func.vmap(f)(x.view(2, -1, 256)).flatten(0, 1),
                                  lambda f, x: torch.func.jvp(f, (x,), (x + 1,))[1], lambda f, x: torch.jit.trace(f, (x + 1,), check_trace=False)(x),
                                  lambda f, x: f(x.as_subclass(_Marked)), lambda f, x: f(torch.cat([x.flatten()[:1], x.flatten()])[1:].view_as(x)),
                                  lambda f, x: torch.compile(f, backend="eager", fullgraph=True)(x)],
                          ids=["tangent", "autocast", "scale gradient", "vmap", "jvp", "trace", "subclass", "misaligned", "compile"])
-def test_quant_linear_where_the_operation_itself_matters(way, tokens):
+def test_quant_linear_where_the_operation_itself_matters(way, tokens, bias):
     """What torch does with a linear it does with this one: the same result and kind of result as with the rebuilt weight."""
     from lemoq.quant.linear import QuantLinear, SchemeSpec
 
@@ -129,7 +132,7 @@ def test_quant_linear_where_the_operation_itself_matters(way, tokens):
             return torch.nn.functional.linear(x, self.dequantized_weight(dtype=x.dtype), self.bias)
 
     torch.manual_seed(tokens)
-    dense = nn.Linear(256, 130, bias=True, device=DEV, dtype=torch.float16)
+    dense = nn.Linear(256, 130, bias=bias, device=DEV, dtype=torch.float16)
     x = torch.randn(tokens, 256, device=DEV).half()
     with torch.no_grad():
         got, ref = (way(kind(dense, SchemeSpec.from_flags("w8a16", 128, dequant="fused")), x) for kind in (QuantLinear, Rebuilt))
