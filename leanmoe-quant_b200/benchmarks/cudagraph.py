@@ -266,8 +266,6 @@ class StaticCacheDecodeSession:
     def prefill(self) -> Any:
         """Run the prompt through the model eagerly into the emptied static cache; the arg-max of the last position
         seeds the decode.  A prompt with a token id outside the vocabulary raises ``RuntimeError``."""
-        from lemoq import _cabi
-
         torch, ctx = self.torch, self.config.ctx
         self.current_token_id = None
         self._clear_cache()
@@ -277,6 +275,8 @@ class StaticCacheDecodeSession:
                                 use_cache=True, cache_position=slots, position_ids=slots.unsqueeze(0))
         picked, flags = torch.stack((output.logits[0, -1].argmax(), self._error_word)).tolist()  # one read-back
         if flags:
+            from lemoq import _cabi
+
             self._error_word.zero_()
             _cabi.check_flags(flags, "prefill")
         self.current_token_id, self.position = picked, ctx

@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
+#include <initializer_list>
 #include <map>
 #include <tuple>
 #include <vector>
@@ -200,80 +201,196 @@ PyObject* experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return rc ? raise(rc) : THPVariable_Wrap(out);
 }
 
-// ---- a model's tensors ----------------------------------------------------------------------------------------------------
-// pointers(tensors, forms, device): the addresses of the tensors as bytes, 64 bits each (None: 0).  Tensor i has the form forms[i % n], a tuple
-// (0 for fp16 or 1 for int8, *sizes).  None when one is not contiguous, 16-byte aligned, of its form and on the device (-1: the CPU).  A prompt
-// asks this of some 250 tensors: 2 us here, 200 us as Python expressions.
-PyObject* pointers(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 3 || !PyList_Check(args[0]) || !PyTuple_Check(args[1])) return none();
-    const Py_ssize_t count = PyList_GET_SIZE(args[0]), period = PyTuple_GET_SIZE(args[1]);
-    const long device = PyLong_AsLong(args[2]);
-    if (period == 0 || (device == -1 && PyErr_Occurred())) {
-        PyErr_Clear();
-        return none();
-    }
-    struct Form {
-        at::ScalarType type;
-        c10::DimVector sizes;
-    };
-    std::vector<Form> forms;
-    for (Py_ssize_t i = 0; i < period; ++i) {
-        PyObject* f = PyTuple_GET_ITEM(args[1], i);
-        if (!PyTuple_Check(f) || PyTuple_GET_SIZE(f) < 1) return none();
-        Form form;
+// ---- a whole model ---------------------------------------------------------------------------------------------------------
+// A prompt asks about some 250 tensors and 200 modules before it launches anything: 20 us here, 110 us as Python expressions.  Each function
+// answers the ordinary case and returns None for anything else; the Python expressions it stands for then decide, and name the reason.
+struct Form {
+    at::ScalarType type;
+    c10::DimVector sizes;
+};
+// forms: a tuple of tuples (0 for fp16 or 1 for int8, *sizes)
+bool read_forms(PyObject* o, std::vector<Form>& forms) {
+    if (!PyTuple_Check(o) || PyTuple_GET_SIZE(o) == 0) return false;
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(o); ++i) {
+        PyObject* f = PyTuple_GET_ITEM(o, i);
+        if (!PyTuple_Check(f) || PyTuple_GET_SIZE(f) < 1) return false;
+        Form form{};
         for (Py_ssize_t d = 0; d < PyTuple_GET_SIZE(f); ++d) {
             const int64_t v = PyLong_AsLongLong(PyTuple_GET_ITEM(f, d));
-            if (v == -1 && PyErr_Occurred()) {
-                PyErr_Clear();
-                return none();
-            }
+            if (v == -1 && PyErr_Occurred()) return false;
             if (d == 0) form.type = v ? at::kChar : at::kHalf;
             else form.sizes.push_back(v);
         }
         forms.push_back(std::move(form));
     }
-    std::vector<uint64_t> words(static_cast<size_t>(count), 0);
-    for (Py_ssize_t i = 0; i < count; ++i) {
-        PyObject* o = PyList_GET_ITEM(args[0], i);
-        if (o == Py_None) continue;
-        if (!THPVariable_Check(o)) return none();
-        const at::Tensor& t = THPVariable_Unpack(o);
-        const Form& form = forms[static_cast<size_t>(i % period)];
-        if (t.scalar_type() != form.type || t.sizes() != at::IntArrayRef(form.sizes) || !t.is_contiguous()) return none();
-        if (device < 0 ? !t.device().is_cpu() : !t.is_cuda() || t.get_device() != device) return none();
-        words[static_cast<size_t>(i)] = reinterpret_cast<uint64_t>(t.data_ptr());
-        if (words[static_cast<size_t>(i)] & 15) return none();
+    return true;
+}
+// The address of a tensor that is contiguous, 16-byte aligned, of the form and on the device (-1: the CPU); 0 for any other.
+uint64_t address(PyObject* o, const Form& form, long device) {
+    if (!THPVariable_Check(o)) return 0;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (t.scalar_type() != form.type || t.sizes() != at::IntArrayRef(form.sizes) || !t.is_contiguous()) return 0;
+    if (device < 0 ? !t.device().is_cpu() : !t.is_cuda() || t.get_device() != device) return 0;
+    const auto at = reinterpret_cast<uint64_t>(t.data_ptr());
+    return at & 15 ? 0 : at;
+}
+
+// pointers(weights, forms, device[, caches, cache_forms]): the addresses as bytes, 64 bits each.  Weight i has the form forms[i % n]; behind every n
+// weights come the next m caches (None: 0).  None when a tensor misfits.
+PyObject* pointers(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if ((n != 3 && n != 5) || !PyList_Check(args[0]) || (n == 5 && !PyList_Check(args[3]))) return none();
+    std::vector<Form> forms, more;
+    const long device = PyLong_AsLong(args[2]);
+    if ((device == -1 && PyErr_Occurred()) || !read_forms(args[1], forms) || (n == 5 && !read_forms(args[4], more))) {
+        PyErr_Clear();
+        return none();
+    }
+    const size_t w = forms.size(), c = more.size(), rounds = static_cast<size_t>(PyList_GET_SIZE(args[0])) / w;
+    if (rounds * w != static_cast<size_t>(PyList_GET_SIZE(args[0])) || (c && rounds * c != static_cast<size_t>(PyList_GET_SIZE(args[3])))) return none();
+    std::vector<uint64_t> words;
+    words.reserve(rounds * (w + c));
+    for (size_t r = 0; r < rounds; ++r) {
+        for (size_t i = 0; i < w; ++i) {
+            words.push_back(address(PyList_GET_ITEM(args[0], static_cast<Py_ssize_t>(r * w + i)), forms[i], device));
+            if (!words.back()) return none();
+        }
+        for (size_t i = 0; i < c; ++i) {
+            PyObject* o = PyList_GET_ITEM(args[3], static_cast<Py_ssize_t>(r * c + i));
+            words.push_back(o == Py_None ? 0 : address(o, more[i], device));
+            if (o != Py_None && !words.back()) return none();
+        }
     }
     return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(words.data()), static_cast<Py_ssize_t>(8 * words.size()));
 }
 
-// plain(modules, forwards): True when no module of the list has a forward (pre-)hook, nor a forward of its own other than a bound method of one
-// of the functions `forwards`; else None.  (200 modules: 6 us here, 30 us as Python expressions.)
-PyObject* plain(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    static PyObject *const hooks = PyUnicode_InternFromString("_forward_hooks"), *const pre_hooks = PyUnicode_InternFromString("_forward_pre_hooks"),
-                            *const forward = PyUnicode_InternFromString("forward");
-    if (n != 2 || !PyList_Check(args[0]) || !PyTuple_Check(args[1]) || !hooks || !pre_hooks || !forward) return none();
-    auto is_plain = [&](PyObject* dict) {
-        for (PyObject* name : {hooks, pre_hooks}) {
-            PyObject* registered = PyDict_GetItemWithError(dict, name);
-            if (!registered || !PyDict_Check(registered) || PyDict_Size(registered) != 0) return false;
+struct Name {
+    PyObject* o;
+    explicit Name(const char* text) : o(PyUnicode_InternFromString(text)) {}
+};
+PyObject* item(PyObject* dict, const Name& name) {  // borrowed; null when absent
+    PyObject* v = dict && PyDict_Check(dict) ? PyDict_GetItemWithError(dict, name.o) : nullptr;
+    if (!v) PyErr_Clear();
+    return v;
+}
+// The attribute dictionaries of objects, held until the end of a call.
+struct Dicts {
+    std::vector<PyObject*> held;
+    PyObject* of(PyObject* o) {
+        PyObject* d = o ? PyObject_GenericGetDict(o, nullptr) : nullptr;
+        if (d) held.push_back(d);
+        else PyErr_Clear();
+        return d;
+    }
+    ~Dicts() {
+        for (PyObject* d : held) Py_DECREF(d);
+    }
+};
+bool equal(PyObject* a, PyObject* b) {
+    if (!a || !b) return false;
+    const int eq = PyObject_RichCompareBool(a, b, Py_EQ);
+    if (eq < 0) PyErr_Clear();
+    return eq == 1;
+}
+PyObject* function_of(PyObject* method) { return method && PyMethod_Check(method) ? PyMethod_GET_FUNCTION(method) : nullptr; }
+
+// No forward (pre-)hook on a module, and no forward of its own other than a bound method of one of the functions given.
+bool unwatched(PyObject* dict, std::initializer_list<PyObject*> forwards) {
+    static const Name hooks("_forward_hooks"), pre_hooks("_forward_pre_hooks"), forward("forward");
+    for (const Name* name : {&hooks, &pre_hooks}) {
+        PyObject* registered = item(dict, *name);
+        if (!registered || !PyDict_Check(registered) || PyDict_Size(registered) != 0) return false;
+    }
+    PyObject* own = item(dict, forward);
+    if (!own) return true;
+    for (PyObject* f : forwards)
+        if (function_of(own) == f) return true;
+    return false;
+}
+
+// layers(decoder layers, known, wanted) -> (tensors, linears, unwatched): of every layer the thirteen weights in the order of LayerDesc, the W8 linears
+// that a forward of the module tree calls, and whether no module would notice that the tree's forward is left out.  known: (OlmoeDecoderLayer,
+// QuantLinear, QuantFusedExperts, OlmoeRMSNorm, decode forward, plain attention forward, silu, fused norm forward, plain norm forward); wanted:
+// (group size, eps, top_k, renormalised).  None for a layer that is not of that kind.
+PyObject* layers(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    static const Name modules("_modules"), buffers("_buffers"), parameters("_parameters"), self_attn("self_attn"), mlp_name("mlp"), o_proj_name("o_proj"),
+        packed_qkv("_lemoq_packed_qkv"), original("_lemoq_original_forward"), forward("forward"), groups("num_key_value_groups"), bias("bias"), packed_name("packed"),
+        scale("scale"), group_size("group_size"), bits("bits"), experts_name("_static_experts"), act("_static_act"), top_k("_static_top_k"), norm_name("_static_norm"),
+        router_name("_static_router"), eps_name("variance_epsilon"), weight("weight"), of_block("of_block");
+    static const Name norm_names[4] = {Name("input_layernorm"), Name("post_attention_layernorm"), Name("q_norm"), Name("k_norm")};
+    static const Name expert_tensors[4] = {Name("packed_gate_up"), Name("scale_gate_up"), Name("packed_down"), Name("scale_down")};
+    static const Name projections[3] = {Name("q_proj"), Name("k_proj"), Name("v_proj")};
+    static PyObject *const one = PyLong_FromLong(1), *const eight = PyLong_FromLong(8);
+    if (n != 3 || !PyList_Check(args[0]) || !PyTuple_Check(args[1]) || PyTuple_GET_SIZE(args[1]) != 9 || !PyTuple_Check(args[2]) || PyTuple_GET_SIZE(args[2]) != 4) return none();
+    auto known = [&](int i) { return PyTuple_GET_ITEM(args[1], i); };
+    auto wanted = [&](int i) { return PyTuple_GET_ITEM(args[2], i); };
+    auto is_a = [&](PyObject* o, int i) { return o && reinterpret_cast<PyObject*>(Py_TYPE(o)) == known(i); };
+    Dicts dicts;
+    std::vector<PyObject*> tensors, linears;  // borrowed from the dictionaries
+    bool quiet = true;
+    for (Py_ssize_t l = 0; l < PyList_GET_SIZE(args[0]); ++l) {
+        PyObject* layer = PyList_GET_ITEM(args[0], l);
+        if (!is_a(layer, 0)) return none();
+        PyObject *own = dicts.of(layer), *parts = item(own, modules), *attn = item(parts, self_attn), *mlp = item(parts, mlp_name);
+        PyObject *attn_own = dicts.of(attn), *inner = item(attn_own, modules), *mlp_own = dicts.of(mlp);
+        PyObject *packed = dicts.of(item(attn_own, packed_qkv)), *o_proj = item(inner, o_proj_name), *o_own = dicts.of(o_proj), *o_buffers = item(o_own, buffers);
+        PyObject *stacks = item(mlp_own, experts_name), *stacks_own = dicts.of(stacks);
+        if (!is_a(o_proj, 1) || item(o_buffers, bias) != Py_None || !is_a(stacks, 2) || !equal(item(stacks_own, bits), eight)) return none();
+        PyObject* activation = item(mlp_own, act);
+        if (activation != Py_None && activation != known(6)) return none();
+        PyObject* attn_forward = function_of(item(attn_own, forward));
+        if (attn_forward != known(4) || function_of(item(attn_own, original)) != known(5) || !equal(item(attn_own, groups), one)) return none();
+        for (PyObject* of : {packed, o_own, stacks_own})
+            if (!equal(item(of, group_size), wanted(0))) return none();
+        if (!equal(item(mlp_own, top_k), wanted(2)) || !equal(item(mlp_own, norm_name), wanted(3))) return none();
+        PyObject* mlp_forward = item(mlp_own, forward);
+        PyObject* block = mlp_forward ? PyObject_GetAttr(mlp_forward, of_block.o) : nullptr;
+        if (!block) PyErr_Clear();
+        quiet = quiet && block == mlp && unwatched(own, {}) && unwatched(attn_own, {known(4)}) && unwatched(o_own, {});
+        Py_XDECREF(block);
+        if (quiet) {  // (its forward is the block's: looked at above)
+            static const Name hooks("_forward_hooks"), pre_hooks("_forward_pre_hooks");
+            for (const Name* name : {&hooks, &pre_hooks}) {
+                PyObject* registered = item(mlp_own, *name);
+                quiet = quiet && registered && PyDict_Check(registered) && PyDict_Size(registered) == 0;
+            }
         }
-        PyObject* own = PyDict_GetItemWithError(dict, forward);
-        if (!own) return !PyErr_Occurred();
-        for (Py_ssize_t j = 0; PyMethod_Check(own) && j < PyTuple_GET_SIZE(args[1]); ++j)
-            if (PyMethod_GET_FUNCTION(own) == PyTuple_GET_ITEM(args[1], j)) return true;
-        return false;
-    };
-    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[0]); ++i) {
-        PyObject* dict = PyObject_GenericGetDict(PyList_GET_ITEM(args[0], i), nullptr);
-        const bool yes = dict && PyDict_Check(dict) && is_plain(dict);
-        Py_XDECREF(dict);
-        if (!yes) {
-            PyErr_Clear();
-            return none();
+        for (int i = 0; i < 4; ++i) {
+            PyObject *norm = item(i < 2 ? parts : inner, norm_names[i]), *norm_own = dicts.of(norm);
+            if (!is_a(norm, 3) || !equal(item(norm_own, eps_name), wanted(1))) return none();
+            tensors.push_back(item(item(norm_own, parameters), weight));
+            quiet = quiet && unwatched(norm_own, {known(7), known(8)});
+        }
+        tensors.push_back(item(packed, packed_name));
+        tensors.push_back(item(packed, scale));
+        tensors.push_back(item(o_buffers, packed_name));
+        tensors.push_back(item(o_buffers, scale));
+        PyObject* router = item(mlp_own, router_name);
+        if (!router || !THPVariable_Check(router) || !THPVariable_Unpack(router).is_contiguous()) return none();  // Python lays it out
+        tensors.push_back(router);
+        for (const Name& name : expert_tensors) tensors.push_back(item(stacks_own, name));
+        linears.push_back(o_proj);
+        for (const Name& name : projections) {
+            PyObject* linear = item(inner, name);
+            if (!linear) continue;  // absent where only the stacked rows were kept
+            quiet = quiet && is_a(linear, 1) && unwatched(dicts.of(linear), {});
+            linears.push_back(linear);
         }
     }
-    Py_RETURN_TRUE;
+    for (PyObject* t : tensors)
+        if (!t || !THPVariable_Check(t)) return none();
+    auto list = [](const std::vector<PyObject*>& from) {
+        PyObject* to = PyList_New(static_cast<Py_ssize_t>(from.size()));
+        for (size_t i = 0; to && i < from.size(); ++i) {
+            Py_INCREF(from[i]);
+            PyList_SET_ITEM(to, static_cast<Py_ssize_t>(i), from[i]);
+        }
+        return to;
+    };
+    PyObject *a = list(tensors), *b = list(linears);
+    PyObject* answer = a && b ? PyTuple_Pack(3, a, b, quiet ? Py_True : Py_False) : nullptr;
+    Py_XDECREF(a);
+    Py_XDECREF(b);
+    return answer;
 }
 
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
@@ -291,7 +408,7 @@ PyMethodDef kMethods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<linear>)), METH_FASTCALL, "W8 linear, or None"},
     {"experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<experts>)), METH_FASTCALL, "routed W8 experts, or None"},
     {"pointers", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<pointers>)), METH_FASTCALL, "addresses of tensors of given forms, or None"},
-    {"plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<plain>)), METH_FASTCALL, "True for modules without hooks, or None"},
+    {"layers", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<layers>)), METH_FASTCALL, "weights and linears of decoder layers, or None"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_bind", "native call path of the lemoq operators", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -1,5 +1,5 @@
-"""The native call path of the short operators (``csrc/bind.cpp``): ``attention``, ``linear``, ``experts``, and ``pointers`` and ``plain``,
-which look over the tensors and the modules of a whole model.  Each returns None for a call it does not take; the callers then go their Python way, which raises the
+"""The native call path of the short operators (``csrc/bind.cpp``): ``attention``, ``linear``, ``experts``, and ``layers`` and ``pointers``,
+which look over the modules and the tensors of a whole model.  Each returns None for a call it does not take; the callers then go their Python way, which raises the
 error or serves the call.  Without the built module they always do."""
 
 from __future__ import annotations
@@ -7,11 +7,11 @@ from __future__ import annotations
 try:
     import torch  # noqa: F401  (the module links against torch's libraries)
 
-    from lemoq._bind import attention, experts, linear, plain, pointers
+    from lemoq._bind import attention, experts, layers, linear, pointers
 except ImportError:  # not built: same results through ctypes
     def _absent(*args: object) -> None:
         return None
 
-    attention = experts = linear = plain = pointers = _absent
+    attention = experts = layers = linear = pointers = _absent
 
-__all__ = ["attention", "experts", "linear", "plain", "pointers"]
+__all__ = ["attention", "experts", "layers", "linear", "pointers"]

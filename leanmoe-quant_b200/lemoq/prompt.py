@@ -9,7 +9,7 @@ call is kept for the next by the address or identity of a tensor or module.
 from __future__ import annotations
 
 from array import array
-from itertools import chain
+from itertools import chain, cycle
 from typing import Any, NamedTuple
 
 import torch
@@ -34,58 +34,81 @@ assert _LAYER_WEIGHTS + _CACHES == tuple(name for name, _ in _cabi.LayerDesc._fi
 class Weights(NamedTuple):
     """The tensors of a model in the canonical form."""
 
-    own: dict      # field of ``StepDesc`` -> tensor
-    layers: list   # per layer, in the order of ``_LAYER_WEIGHTS``
-    modules: tuple  # what a forward of the module tree calls: (W8 linears, norms, attention and expert blocks, embedding and decoder layers)
+    own: dict       # field of ``StepDesc`` -> tensor
+    layers: list    # in the order of ``_LAYER_WEIGHTS``, layer after layer
+    linears: list   # the W8 linears that a forward of the module tree calls
+    unwatched: bool  # no hook on a module that such a forward calls, and none has another forward than the one computed natively
 
     def tensors(self) -> list:
-        return [*self.own.values(), *(t for layer in self.layers for t in layer)]
+        return [*self.own.values(), *self.layers]
 
 
-def _read(model: Any) -> tuple[Weights | None, str | None]:
-    """The tensors that the model's forwards would use now, or None and the reason why one ``StepDesc`` does not stand for the model: it has
-    ONE group size, top_k, eps and so on, so what every block was really built with is compared here.  (Through the modules' own
-    dictionaries: 300 attribute look-ups of ``nn.Module`` would take longer than the launches of a short prompt.)"""
+_KNOWN = (OlmoeDecoderLayer, QuantLinear, QuantFusedExperts, OlmoeRMSNorm, _decode_forward_impl, OlmoeAttention.forward, F.silu, _fused_norm_forward, OlmoeRMSNorm.forward)
+_NORM_FORWARDS = (_fused_norm_forward, OlmoeRMSNorm.forward)
 
-    cfg, m, lm = model.config, model.model, model.lm_head
-    if type(lm) is not QuantLinear or lm.bias is not None:
-        return None, "lm_head is not a W8 linear without bias"
-    if cfg.clip_qkv is not None or not len(m.layers):
-        return None, "clip_qkv is set, or there are no layers"
-    group, eps, routing = lm.group_size, cfg.rms_norm_eps, (cfg.num_experts_per_tok, bool(cfg.norm_topk_prob))
-    if getattr(m.norm, "variance_epsilon", None) != eps:
-        return None, "the final norm has an eps of its own"
-    layers, linears, norms, blocks = [], [lm], [m.norm], []
-    for i, layer in enumerate(m.layers):
+
+def _plain(module: Any, forwards: tuple = ()) -> bool:
+    """No hook, and no forward of its own but a bound method of one of ``forwards``."""
+    own = module.__dict__.get("forward")
+    return not (module._forward_hooks or module._forward_pre_hooks) and (own is None or getattr(own, "__func__", None) in forwards)
+
+
+def _read_layers(layers: list, group: int, eps: float, top_k: int, renormalised: bool) -> tuple[list, list, bool] | str:
+    """(weights, linears, unwatched) of the decoder layers as ``Weights`` has them, or the reason why one description does not stand for them."""
+    tensors, linears, unwatched = [], [], True
+    for i, layer in enumerate(layers):
         if type(layer) is not OlmoeDecoderLayer:
-            return None, "layer %d is a %s" % (i, type(layer).__name__)
+            return "layer %d is a %s" % (i, type(layer).__name__)
         parts = layer._modules
         attn, mlp = parts["self_attn"], parts["mlp"]
         inner, here, moe = attn._modules, attn.__dict__, mlp.__dict__
         packed, o_proj, stacks = here.get("_lemoq_packed_qkv"), inner.get("o_proj"), moe.get("_static_experts")
         if packed is None or type(o_proj) is not QuantLinear or o_proj._buffers["bias"] is not None:
-            return None, "layer %d: packed q/k/v not installed, or o_proj is not a W8 linear without bias" % i
+            return "layer %d: packed q/k/v not installed, or o_proj is not a W8 linear without bias" % i
         if not isinstance(stacks, QuantFusedExperts) or stacks.bits != 8 or moe["_static_act"] not in (None, F.silu):
-            return None, "layer %d: experts are not W8 with SiLU" % i
+            return "layer %d: experts are not W8 with SiLU" % i
         if (getattr(here.get("forward"), "__func__", None) is not _decode_forward_impl or here["num_key_value_groups"] != 1
                 or getattr(here.get("_lemoq_original_forward"), "__func__", None) is not OlmoeAttention.forward):
-            return None, "layer %d: attention core not replaced, or GQA" % i
+            return "layer %d: attention core not replaced, or GQA" % i
         if not packed.group_size == o_proj.group_size == stacks.group_size == group:
-            return None, ("layer %d: group sizes %d (q.k.v), %d (o_proj), %d (experts) beside %d (lm_head)"
-                          % (i, packed.group_size, o_proj.group_size, stacks.group_size, group))
-        if (moe["_static_top_k"], moe["_static_norm"]) != routing:
-            return None, "layer %d: top_k %d (normalised: %s) is not the configuration's" % (i, moe["_static_top_k"], moe["_static_norm"])
-        ln1, ln2, q_norm, k_norm = own = parts["input_layernorm"], parts["post_attention_layernorm"], inner["q_norm"], inner["k_norm"]
-        if any([type(norm) is not OlmoeRMSNorm or norm.variance_epsilon != eps or "weight" not in norm._parameters for norm in own]):
-            return None, "layer %d: a norm is not RMSNorm with the configuration's eps" % i
-        linears.append(o_proj)
-        linears.extend(filter(None, map(inner.get, ("q_proj", "k_proj", "v_proj"))))  # (absent where only the stacked rows were kept)
-        norms += own
-        blocks += attn, mlp
-        layers.append((ln1._parameters["weight"], ln2._parameters["weight"], q_norm._parameters["weight"], k_norm._parameters["weight"], packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"], moe["_static_router"].contiguous(),
-                       stacks.packed_gate_up, stacks.scale_gate_up, stacks.packed_down, stacks.scale_down))
-    return Weights({"embed": m.embed_tokens.weight, "final_norm": m.norm.weight, "lm_head_codes": lm.packed, "lm_head_scale": lm.scale}, layers,
-                   (linears, norms, blocks, [m.embed_tokens, m.rotary_emb, *m.layers])), None
+            return ("layer %d: group sizes %d (q.k.v), %d (o_proj), %d (experts) beside %d (lm_head)"
+                    % (i, packed.group_size, o_proj.group_size, stacks.group_size, group))
+        if (moe["_static_top_k"], moe["_static_norm"]) != (top_k, renormalised):
+            return "layer %d: top_k %d (normalised: %s) is not the configuration's" % (i, moe["_static_top_k"], moe["_static_norm"])
+        norms = (parts["input_layernorm"], parts["post_attention_layernorm"], inner.get("q_norm"), inner.get("k_norm"))
+        if any(type(norm) is not OlmoeRMSNorm or norm.variance_epsilon != eps or norm._parameters.get("weight") is None for norm in norms):
+            return "layer %d: a norm is not RMSNorm with the configuration's eps" % i
+        mine = [o_proj, *filter(None, map(inner.get, ("q_proj", "k_proj", "v_proj")))]  # (absent where only the stacked rows were kept)
+        block_forward = getattr(moe.get("forward"), "of_block", None) is mlp and not (mlp._forward_hooks or mlp._forward_pre_hooks)
+        unwatched = (unwatched and block_forward and _plain(layer) and _plain(attn, (_decode_forward_impl,)) and all(_plain(n, _NORM_FORWARDS) for n in norms)
+                     and all(type(x) is QuantLinear and _plain(x) for x in mine))
+        linears += mine
+        tensors += [*(norm._parameters["weight"] for norm in norms), packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"],
+                    moe["_static_router"].contiguous(), stacks.packed_gate_up, stacks.scale_gate_up, stacks.packed_down, stacks.scale_down]
+    return tensors, linears, unwatched
+
+
+def _read(model: Any) -> tuple[Weights | None, str | None]:
+    """The tensors that the model's forwards would use now, or None and the reason why one ``StepDesc`` does not stand for the model: it has
+    ONE group size, top_k, eps and so on, so what every block was really built with is compared here."""
+    cfg, m, lm = model.config, model._modules["model"], model._modules["lm_head"]
+    parts = m._modules
+    embed, norm, rotary, layers = parts["embed_tokens"], parts["norm"], parts["rotary_emb"], list(parts["layers"]._modules.values())
+    if type(lm) is not QuantLinear or lm._buffers["bias"] is not None:
+        return None, "lm_head is not a W8 linear without bias"
+    if cfg.clip_qkv is not None or not layers:
+        return None, "clip_qkv is set, or there are no layers"
+    if type(norm) is not OlmoeRMSNorm or norm.variance_epsilon != cfg.rms_norm_eps or embed._parameters.get("weight") is None or norm._parameters.get("weight") is None:
+        return None, "the embedding or the final norm is not the configuration's"
+    wanted = (lm.group_size, cfg.rms_norm_eps, cfg.num_experts_per_tok, bool(cfg.norm_topk_prob))
+    found = _native.layers(layers, _KNOWN, wanted) or _read_layers(layers, *wanted)
+    if isinstance(found, str):
+        return None, found
+    tensors, linears, unwatched = found
+    unwatched = (unwatched and type(embed) is nn.Embedding and embed.max_norm is None and type(rotary) is OlmoeRotaryEmbedding
+                 and _plain(lm) and _plain(embed) and _plain(rotary) and _plain(norm, _NORM_FORWARDS))
+    own = {"embed": embed._parameters["weight"], "final_norm": norm._parameters["weight"], "lm_head_codes": lm._buffers["packed"], "lm_head_scale": lm._buffers["scale"]}
+    return Weights(own, tensors, [lm, *linears], unwatched), None
 
 
 def read_weights(model: Any) -> Weights | None:
@@ -93,28 +116,9 @@ def read_weights(model: Any) -> Weights | None:
 
 
 def _skippable(weights: Weights) -> bool:
-    """May the module tree's forward be left out?  Not when that would be noticed: a hook on one of the modules it calls or on all modules, or a
-    module with another forward than the one the native path computes."""
-
-    linears, norms, blocks, plain = weights.modules
-    embed, rotary = plain[:2]
-    if set(map(type, linears)) != {QuantLinear} or type(embed) is not nn.Embedding or embed.max_norm is not None or type(rotary) is not OlmoeRotaryEmbedding:
-        return False
-    if any([getattr(mlp.__dict__.get("forward"), "of_block", None) is not mlp for mlp in blocks[1::2]]):
-        return False
+    """May the module tree's forward be left out?  Not when that would be noticed."""
     every = torch.nn.modules.module
-    if every._global_forward_hooks or every._global_forward_pre_hooks:
-        return False
-    groups = ((linears + plain, ()), (norms, (_fused_norm_forward, OlmoeRMSNorm.forward)), (blocks[::2], (_decode_forward_impl,)))
-    if any(x._forward_hooks or x._forward_pre_hooks for x in blocks[1::2]):
-        return False
-    return all(_native.plain(modules, forwards) or all(_plain(x, forwards) for x in modules) for modules, forwards in groups)
-
-
-def _plain(module: Any, forwards: tuple) -> bool:
-    """No hook, and no forward of its own but a bound method of one of ``forwards``."""
-    own = module.__dict__.get("forward")
-    return not (module._forward_hooks or module._forward_pre_hooks) and (own is None or getattr(own, "__func__", None) in forwards)
+    return weights.unwatched and not (every._global_forward_hooks or every._global_forward_pre_hooks)
 
 
 _HALF, _CODE = 0, 1  # element types of a form: (type, *shape)
@@ -130,22 +134,29 @@ def _forms(model: Any) -> tuple[tuple, tuple]:
 
 
 def _misfit(tensors: list, forms: tuple, names: tuple, device: Any) -> str | None:
-    """The first tensor (None: absent) that is not contiguous, 16-byte aligned, on ``device`` and of its form."""
+    """The first tensor that is not contiguous, 16-byte aligned, on ``device`` and of its form."""
     for i, t in enumerate(tensors):
         form, name = forms[i % len(forms)], names[i % len(names)]
-        if t is not None and (t.dtype is not (torch.float16, torch.int8)[form[0]] or tuple(t.shape) != form[1:] or t.device != device):
+        if t.dtype is not (torch.float16, torch.int8)[form[0]] or tuple(t.shape) != form[1:] or t.device != device:
             return "%s is %s %s on %s" % (name, tuple(t.shape), t.dtype, t.device)
-        if t is not None and (not t.is_contiguous() or t.data_ptr() & 15):
+        if not t.is_contiguous() or t.data_ptr() & 15:
             return "%s is not contiguous and 16-byte aligned" % name
     return None
 
 
-def _pointers(tensors: list, forms: tuple, names: tuple, device: Any) -> bytes | bytearray | None:
-    """The tensors' addresses, 64 bits each; None when one of them misfits."""
-    words = _native.pointers(tensors, forms, -1 if device.index is None else device.index)
-    if words is None and _misfit(tensors, forms, names, device) is None:
-        words = array("Q", [0 if t is None else t.data_ptr() for t in tensors]).tobytes()
-    return words
+def _pointers(tensors: list, forms: tuple, names: tuple, device: Any, caches: list = [], cache_forms: tuple = ()) -> bytes | None:  # noqa: B006
+    """The tensors' addresses, 64 bits each, behind the weights of every layer those of its caches (None: 0); None when one of them misfits."""
+    index = -1 if device.index is None else device.index
+    words = _native.pointers(tensors, forms, index, caches, cache_forms) if caches else _native.pointers(tensors, forms, index)
+    if words is not None:
+        return words
+    there = [(t, form, name) for t, form, name in zip(caches, cycle(cache_forms), cycle(_CACHES)) if t is not None]
+    if _misfit(tensors, forms, names, device) or any(_misfit([t], (form,), (name,), device) for t, form, name in there):
+        return None
+    address = lambda t: 0 if t is None else t.data_ptr()  # noqa: E731
+    w, c = len(forms), len(cache_forms)
+    rounds = [[*map(address, tensors[r * w: (r + 1) * w]), *map(address, caches[r * c: (r + 1) * c])] for r in range(len(tensors) // w)]
+    return array("Q", chain.from_iterable(rounds)).tobytes()
 
 
 def form_blocker(model: Any) -> str | None:
@@ -158,27 +169,22 @@ def form_blocker(model: Any) -> str | None:
     own, layer = _forms(model)
     device = weights.own["embed"].device
     return (_misfit(list(weights.own.values()), own, tuple(weights.own), device)
-            or _misfit([t for tensors in weights.layers for t in tensors], layer, _LAYER_WEIGHTS, device))
+            or _misfit(weights.layers, layer, _LAYER_WEIGHTS, device))
 
 
 def describe(model: Any, weights: Weights, max_len: int, caches: list[tuple], cache_forms: tuple) -> tuple[Any, Any] | None:
     """``(StepDesc, LayerDesc array)`` of the model over one set of cache tensors per layer (in the order of ``_CACHES``, each None or of its form):
     pointers only, the caller keeps the tensors for as long as the C side may read them.  None when a tensor misfits."""
-    cfg, m = model.config, model.model
-    device, (own_forms, layer_forms) = weights.own["embed"].device, _forms(model)
+    cfg, device, (own_forms, layer_forms) = model.config, weights.own["embed"].device, _forms(model)
     own = _pointers(list(weights.own.values()), own_forms, tuple(weights.own), device)
-    words = _pointers(list(chain.from_iterable(chain.from_iterable(zip(weights.layers, caches)))), layer_forms + cache_forms, _LAYER_WEIGHTS + _CACHES, device)
+    words = _pointers(weights.layers, layer_forms, _LAYER_WEIGHTS, device, list(chain.from_iterable(caches)), cache_forms)
     if own is None or words is None:
         return None
-    cos, sin = m.rotary_emb.tables(max_len, torch.float16, device)
-    desc = _cabi.StepDesc()
-    desc.layers, desc.hidden, desc.heads, desc.head_dim = len(m.layers), cfg.hidden_size, cfg.num_attention_heads, cfg.head_dim
-    desc.experts, desc.top_k, desc.ffn, desc.vocab = cfg.num_experts, cfg.num_experts_per_tok, cfg.intermediate_size, cfg.vocab_size
-    desc.group_size, desc.max_len, desc.eps = int(model.lm_head.group_size), max_len, float(cfg.rms_norm_eps)
-    desc.norm_topk_prob = int(bool(cfg.norm_topk_prob))
-    desc.embed, desc.final_norm, desc.lm_head_codes, desc.lm_head_scale = array("Q", own)
-    desc.rope_cos, desc.rope_sin = cos.data_ptr(), sin.data_ptr()
-    return desc, (_cabi.LayerDesc * len(m.layers)).from_buffer_copy(words)
+    cos, sin = model.model.rotary_emb.tables(max_len, torch.float16, device)
+    desc = _cabi.StepDesc(len(caches), cfg.hidden_size, cfg.num_attention_heads, cfg.head_dim, cfg.num_experts, cfg.num_experts_per_tok, cfg.intermediate_size,
+                          cfg.vocab_size, int(model.lm_head.group_size), max_len, float(cfg.rms_norm_eps), int(bool(cfg.norm_topk_prob)), 0, 0, 0,
+                          *array("Q", own), cos.data_ptr(), sin.data_ptr())
+    return desc, (_cabi.LayerDesc * len(caches)).from_buffer_copy(words)
 
 
 def _operations_matter() -> bool:
@@ -224,7 +230,7 @@ def run_prompt(model: Any, input_ids: Any, cache: Any, cache_position: Any, posi
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     _cabi.call("lemoq_prompt_run", desc, layers, _cabi.ptr(ids), _cabi.ptr(cache_position), tokens, _cabi.ptr(logits),
                _cabi.ptr(workspace), size, _cabi.ptr(flags), _cabi.current_stream(device))
-    for linear in weights.modules[0]:
+    for linear in weights.linears:
         linear.count_separate(several=True)
     if carried is None and not torch.cuda.is_current_stream_capturing():
         _cabi.check_flags(int(flags), "prompt")

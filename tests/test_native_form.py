@@ -8,9 +8,11 @@ import torch
 from oracle import lemoq_oracle as ops
 
 
-@pytest.fixture
-def canonical(monkeypatch):
-    """Builder of a small canonical model on the CPU; ``experts``: group size of the experts' scales."""
+@pytest.fixture(params=["binding", "python"])
+def canonical(request, monkeypatch):
+    """Builder of a small canonical model on the CPU; ``experts``: group size of the experts' scales.  Everything is asked of the binding's
+    functions and of the Python expressions they stand for."""
+    from lemoq import _native
     import lemoq.quant.rtn as rtn
     from lemoq.kernels.attn_decode import replace_attention_cores
     from lemoq.kernels.moe_grouped_quant import QuantFusedExperts
@@ -38,6 +40,18 @@ def canonical(monkeypatch):
         install_packed_qkv(model)
         return model
 
+    if request.param == "python":
+        for name in ("layers", "pointers"):
+            monkeypatch.setattr(_native, name, lambda *a: None)
+    else:  # an ordinary model is the binding's business: nothing of it is asked of the Python expressions
+        from lemoq import prompt
+
+        model = build()
+        with monkeypatch.context() as patch:
+            patch.setattr(prompt, "_read_layers", None)
+            patch.setattr(prompt, "_misfit", None)
+            assert prompt._skippable(prompt.read_weights(model))
+            assert prompt.describe(model, prompt.read_weights(model), 8, 2 * [6 * (None,)], 6 * ((prompt._HALF,),)) is not None
     return build
 
 
@@ -103,14 +117,9 @@ def test_every_block_is_compared_with_the_configuration(canonical):
     assert form_blocker(model) is None
 
 
-@pytest.mark.parametrize("bound", [True, False])
-def test_a_tensor_of_another_form_is_not_described(canonical, bound, monkeypatch):
-    """The binding and the Python expressions it stands for refuse the same."""
-    from lemoq import _native
+def test_a_tensor_of_another_form_is_not_described(canonical):
     from lemoq.prompt import _HALF, describe, read_weights
 
-    if not bound:
-        monkeypatch.setattr(_native, "pointers", lambda *a: None)
     model, forms = canonical(), 6 * ((_HALF, 1, 2, 8, 128),)
     cache = lambda n: [(torch.zeros(1, 2, n, 128, dtype=torch.float16), torch.zeros(1, 2, 8, 128, dtype=torch.float16), *4 * (None,)) for _ in range(2)]  # noqa: E731
     assert describe(model, read_weights(model), 8, cache(8), forms) is not None and describe(model, read_weights(model), 8, cache(9), forms) is None
@@ -122,17 +131,13 @@ def test_a_tensor_of_another_form_is_not_described(canonical, bound, monkeypatch
         assert describe(model, read_weights(model), 8, cache(8), forms) is None
 
 
-@pytest.mark.parametrize("bound", [True, False])
-def test_a_forward_that_is_seen_or_replaced_is_not_skipped(canonical, bound, monkeypatch):
-    from lemoq import _native
+def test_a_forward_that_is_seen_or_replaced_is_not_skipped(canonical):
     from lemoq.prompt import _skippable, read_weights
 
-    if not bound:
-        monkeypatch.setattr(_native, "plain", lambda *a: None)
     model = canonical()
     layer = model.model.layers[1]
     skippable = lambda: (lambda weights: weights is not None and _skippable(weights))(read_weights(model))  # noqa: E731
-    assert skippable() and len(read_weights(model).modules[0]) == 9
+    assert skippable() and len(read_weights(model).linears) == 9
     called = [model.lm_head, model.model.norm, model.model.embed_tokens, model.model.rotary_emb, layer, layer.self_attn, layer.mlp, layer.input_layernorm,
               *(getattr(layer.self_attn, n) for n in ("q_proj", "k_proj", "v_proj", "o_proj", "q_norm", "k_norm")), layer.post_attention_layernorm]
     for module in called:
@@ -159,3 +164,12 @@ def test_projections_may_be_given_up_once_they_are_stacked(canonical):
     for layer in model.model.layers:
         del layer.self_attn.q_proj, layer.self_attn.k_proj, layer.self_attn.v_proj
     assert form_blocker(model) is None and _skippable(read_weights(model))
+
+
+def test_a_router_of_other_strides_is_laid_out(canonical):
+    from lemoq.prompt import form_blocker, read_weights
+
+    model = canonical()
+    mlp = model.model.layers[1].mlp
+    mlp._static_router = mlp._static_router.t().contiguous().t()
+    assert form_blocker(model) is None and torch.equal(read_weights(model).layers[13 + 8], mlp._static_router)
