@@ -151,14 +151,15 @@ __device__ __forceinline__ bool thread_wait(uint32_t bar, uint32_t parity, volat
 // Bounded wait of a whole warp: the same outcome in every lane.  `abort` is a flag in shared memory: a warp that gave up
 // sets it, and every later wait in the block ends at once.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
-    bool ok = mbar_test(bar, parity);
-    for (uint32_t i = 0; !__all_sync(0xffffffffu, ok) && i < kWaitLimit; ++i) {
+    bool ok = mbar_try_wait(bar, parity);
+    if (__all_sync(0xffffffffu, ok)) return true;
+    for (uint32_t i = 0; i < kWaitLimit; ++i) {
         if ((i & 1023u) == 1023u && __any_sync(0xffffffffu, *abort)) break;
         ok = ok || mbar_try_wait(bar, parity);
+        if (__all_sync(0xffffffffu, ok)) return true;
     }
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) *abort = 1;
-    return ok;
+    *abort = 1;
+    return false;
 }
 
 }  // namespace lemoq

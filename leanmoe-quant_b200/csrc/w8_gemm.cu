@@ -5,11 +5,10 @@
 //
 // The weight rows are the M side of tcgen05.mma (128 rows a tile, lane = row), the tokens the N side: an expert with nine
 // tokens costs an N of 16 and not a tile of 128.  Two forms:
-//   exact   up to 64 tokens a tile.  int8 codes are exact in fp16, so the products are those of the integer kernels: the codes
+//   exact   here, up to 64 tokens a tile.  int8 codes are exact in fp16, so the products are those of the integer kernels: the codes
 //           are widened, not scaled.  The fp32 sum of one group of 128 codes leaves TMEM, is scaled in fp32 and added to
 //           the row's accumulators in registers.
-//   scaled  up to 128 tokens a tile, for prompts: the widened code is multiplied by its group scale and rounded to fp16 (what
-//           dequantising the weights to fp16 in memory does), the sum over all of K stays in TMEM.
+//   scaled  more tokens, for prompts: w8_pair.cu.
 //
 // One persistent block per SM, a tile = two M tiles (256 weight rows; for gate/up 128 gate rows and their 128 up rows)
 // x up to NT tokens of one expert:
@@ -17,16 +16,15 @@
 //   warps 8-15   a warpgroup per M tile, thread = weight row: widen the codes of a group into TMEM (two buffers)
 //   warps 17, 18 issue the MMAs, one warp per M tile: A = widened codes from TMEM, B = tokens from shared memory, D in TMEM
 //   warps 0-7    a warpgroup per M tile, thread = weight row: collect the sums (per group / at the end), finish the rows
-// TMEM: D of tile w at column 128 w (exact: two buffers of 64), A of tile w, buffer b at 256 + 128 w + 64 b.
+// TMEM: D of tile w, buffer b at column 128 w + 64 b, A of tile w, buffer b at 256 + 128 w + 64 b.
 //
-// What bounds it: with few tokens per expert the bytes of the codes (HBM); with 128 per tile shared memory (160 KB of TMA
-// writes, code reads and B reads per group against 1024 cycles of MMAs).  A in TMEM instead of shared memory, because widened
+// What bounds it: with few tokens per expert the bytes of the codes (HBM).  A in TMEM instead of shared memory, because widened
 // codes in shared memory would add a write and a read of twice the codes' size.  Widening and collecting are different warps
 // because either is a chain of waits, and the TMA and MMA loops are one thread each because a vote after every wait cost
-// that warp 160 cycles (exact, NT = 16: 3200 cycles per group with both by the same warps and `lane == 0` issue, 1700 with
+// that warp 160 cycles (NT = 16: 3200 cycles per group with both by the same warps and `lane == 0` issue, 1700 with
 // separate warps and elect.sync).  One MMA thread for both tiles left the tensor pipe idle for a quarter of the time (a wait
 // that is over costs it 200 cycles): with two, one waits while the other's MMAs run.
-#include "tc.cuh"
+#include "w8_tile.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -50,8 +48,10 @@ int encode_rows_map(CUtensorMap* map, const void* base, int elem_bytes, int64_t 
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * elem_bytes};
     const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / elem_bytes), static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t elem[2] = {1, 1};
+    // 256-byte promotion: a box is 128 bytes of each row, and the next one along the rows comes soon.  With 128 the experts of 64 tokens took 73.8 and
+    // 43.0 us (gate/up, down), with 256 69.7 and 39.9.
     const CUresult rc = encode(map, elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims,
-                               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) return set_error(LEMOQ_ERR_CUDA, "cuTensorMapEncodeTiled: error %d", static_cast<int>(rc));
     return LEMOQ_OK;
@@ -61,7 +61,7 @@ namespace {
 
 constexpr int kThreads = 640;       // five warpgroups: two collect, two widen, the fifth has the TMA warp and the MMA warp
 // Registers: 640 threads are launched with 96 each (61,440); 256 x 144 + 256 x 56 + 128 x 72 = 60,416 afterwards.
-constexpr int kExactTokens = 64, kScaledTokens = 128;  // most tokens of a tile
+constexpr int kExactTokens = 64;    // most tokens of a tile
 constexpr int kRegsCollect = 144, kRegsWiden = 56, kRegsIssue = 72;
 constexpr int kTileRows = 256;      // weight rows of a tile (two M tiles of 128)
 constexpr int kCodeBytes = 2 * 128 * 128;
@@ -70,79 +70,12 @@ constexpr uint32_t kColA = 256;     // first TMEM column of the widened codes
 
 template <int NT>
 struct Shape {
-    static constexpr int kBox = NT >= 128 ? 32 : 16;                    // token rows of one TMA box
+    static constexpr int kBox = 16;                                     // token rows of one TMA box
     static constexpr int kHalf = NT * 128;                              // bytes of one 64-wide half of the tokens
     static constexpr int kStage = kCodeBytes + 2 * kHalf;
-    static constexpr bool kScaled = NT > kExactTokens;
-    static constexpr int kDBufs = kScaled ? 1 : 2;                      // accumulator buffers per M tile
-    static constexpr int kStages = NT >= 128 ? 3 : (NT == 64 ? 4 : 5);
-    static constexpr int kTurn = kScaled ? 8 * 32 * 32 * 2 : 0;         // a collecting warp's 32 rows x 32 tokens, turned for wide stores
-    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + kTurn + 1024;  // + 8 (E + 1) bytes of tile table
+    static constexpr int kStages = NT == 64 ? 4 : 5;
+    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStage + 1024;  // + 8 (E + 1) bytes of tile table
 };
-
-struct GemmShape {
-    int T, N, K, group, E, gate_up;
-    const int32_t* seg;    // (E + 1) or null: one segment [0, T)
-    const __half* scale;   // (E, N, K / group)
-    const __half* resid;   // (T, N) or null
-    __half* y;             // (T, N), or (T, N / 2) in gate/up mode
-    float* y32;            // or: (T, N) in fp32
-    int* err_flag;
-    int parts;             // SPLIT: blocks of a cluster that share a tile's groups
-    int wide;              // rows of y (and resid) begin on 16 bytes: eight values a store
-    int scale_vecs;        // 16-byte vectors of a row's scales when they fit the shared rows (1 or 2), else 0
-};
-
-struct Tile {
-    int row0, row1;    // first weight row of the two M tiles inside the expert
-    int e, t0, n;      // expert, first token, tokens
-};
-
-// Tiles before expert e: first[e].  A tile number -> expert by binary search, then (M tile pair, token tile): neighbours in
-// the order share their weight rows and meet in L2.  The tokens of an expert are split evenly.
-template <int NT>
-__device__ __forceinline__ Tile tile_at(int i, const int* first, const int* tok, const GemmShape& p) {
-    if (i >= first[p.E]) return Tile{0, 0, 0, 0, 0};
-    int lo = 0, hi = p.E;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (first[mid] <= i) lo = mid; else hi = mid;
-    }
-    Tile t;
-    t.e = lo;
-    const int cnt = tok[lo + 1] - tok[lo], nt = (cnt + NT - 1) / NT, r = i - first[lo], m = r / nt, b = r - m * nt;
-    const int per = ((cnt + nt - 1) / nt + 15) & ~15;
-    t.t0 = tok[lo] + b * per;
-    t.n = max(0, min(per, tok[lo + 1] - t.t0));
-    t.row0 = p.gate_up ? m * 128 : m * kTileRows;
-    t.row1 = p.gate_up ? p.N / 2 + m * 128 : m * kTileRows + 128;
-    return t;
-}
-
-// silu(gate) * up of two pairs, for fp16 results: exp and the quotients to about 2^-21, one reciprocal for both.  Below -43 the exponential is
-// held at e^43 (its square is finite): such a gate gives less than 1e-12 whatever `up` is.  (With expf and rounded divisions the epilogue of a
-// gate/up tile of 128 tokens took 9900 cycles, half as long as its MMAs.)
-__device__ __forceinline__ void swiglu2(float g0, float u0, float g1, float u1, float& y0, float& y1) {
-    const float a = 1.0f + __expf(-fmaxf(g0, -43.f)), b = 1.0f + __expf(-fmaxf(g1, -43.f)), r = __fdividef(1.0f, a * b);
-    y0 = g0 * (r * b) * u0;
-    y1 = g1 * (r * a) * u1;
-}
-
-// 16 codes -> 8 words of two exact fp16 each: bytes with the sign flipped dropped into 0x64__ are 1024 + 128 + c.
-template <bool SCALED>
-__device__ __forceinline__ void widen16(const uint4& w, __half scale, uint32_t* out) {
-    const uint32_t u[4] = {w.x ^ 0x80808080u, w.y ^ 0x80808080u, w.z ^ 0x80808080u, w.w ^ 0x80808080u};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        __half2 a = codes_half2(u[i], 0x4140), b = codes_half2(u[i], 0x4342);
-        if (SCALED) {
-            a = __hmul2(a, __half2half2(scale));
-            b = __hmul2(b, __half2half2(scale));
-        }
-        out[2 * i] = *reinterpret_cast<const uint32_t*>(&a);
-        out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&b);
-    }
-}
 
 // The group scales of one weight row: the thread of the row asks for those of its next tile a tile ahead (a load takes up to three
 // groups under load), keeps them in registers until the tile is done and then leaves them in its own row of shared memory.
@@ -150,12 +83,12 @@ struct RowScales {
     uint4 ahead[2];
     const __half* row;
     uint32_t at;
-    __device__ __forceinline__ void ask(const GemmShape& p, const Tile& t, int wrow) {
-        row = p.scale + (static_cast<int64_t>(t.e) * p.N + min(wrow, p.N - 1)) * (p.K / p.group);
+    __device__ __forceinline__ void ask(const W8Shape& p, int e, int wrow) {
+        row = p.scale + (static_cast<int64_t>(e) * p.N + min(wrow, p.N - 1)) * (p.K / p.group);
         if (p.scale_vecs > 0) ahead[0] = __ldg(reinterpret_cast<const uint4*>(row));
         if (p.scale_vecs > 1) ahead[1] = __ldg(reinterpret_cast<const uint4*>(row) + 1);
     }
-    __device__ __forceinline__ void keep(const GemmShape& p) {
+    __device__ __forceinline__ void keep(const W8Shape& p) {
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
             if (v < p.scale_vecs) {
@@ -166,7 +99,7 @@ struct RowScales {
         }
     }
     // `mine`: the row this tile works on (the one asked for last belongs to the next tile)
-    __device__ __forceinline__ __half get(const GemmShape& p, const __half* mine, int g) const {
+    __device__ __forceinline__ __half get(const W8Shape& p, const __half* mine, int g) const {
         const int k = p.group == 128 ? g : (g << 7) / p.group;
         if (p.scale_vecs == 0) return __ldg(mine + k);
         unsigned short h;
@@ -175,9 +108,15 @@ struct RowScales {
     }
 };
 
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+template <int NT>
+__device__ __forceinline__ Tile tile_at(int i, const int* first, const int* tok, const W8Shape& p) {
+    Tile t = find_tile(i, first, tok, p.E, NT, 16);
+    const int m = t.row0;
+    t.row0 = p.gate_up ? m * 128 : m * kTileRows;
+    t.row1 = p.gate_up ? p.N / 2 + m * 128 : m * kTileRows + 128;
+    return t;
 }
+
 __device__ __forceinline__ float ld_peer(uint32_t addr, int rank) {
     uint32_t there;
     float v;
@@ -190,28 +129,26 @@ __device__ __forceinline__ float ld_peer(uint32_t addr, int rank) {
 // block leaves its sums in its own shared memory and finishes a part of the tokens from those of all, in rank order.
 template <int NT, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                                                              const GemmShape p) {
+                                                              const W8Shape p) {
     using S = Shape<NT>;
     constexpr int kStages = S::kStages;
     extern __shared__ uint8_t raw[];
-    __shared__ __align__(8) uint64_t s_bar[2 * kStages + 10];
+    __shared__ __align__(8) uint64_t s_bar[2 * kStages + 9];
     __shared__ __align__(16) uint8_t s_scale[kTileRows * kScaleStride];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage0 = (smem_u32(raw) + 1023u) & ~1023u;
-    int* s_first = reinterpret_cast<int*>(raw + (stage0 - smem_u32(raw)) + static_cast<size_t>(kStages) * S::kStage + S::kTurn);
+    int* s_first = reinterpret_cast<int*>(raw + (stage0 - smem_u32(raw)) + static_cast<size_t>(kStages) * S::kStage);
     int* s_tok = s_first + p.E + 1;
     const uint32_t bars = smem_u32(s_bar);
     auto full = [&](int s) { return bars + 8u * s; };
     auto done = [&](int s) { return bars + 8u * (kStages + s); };
     auto a_full = [&](int w, int b) { return bars + 8u * (2 * kStages + 2 * w + b); };
     auto d_free = [&](int b) { return bars + 8u * (2 * kStages + 4 + b); };
-    const uint32_t ex = bars + 8u * (2 * kStages + 6), d_full = ex + 8u;
-    auto drained = [&](int w) { return ex + 16u + 8u * w; };
-    constexpr int kD = S::kDBufs;
-    constexpr bool kScaled = S::kScaled;
+    const uint32_t ex = bars + 8u * (2 * kStages + 6);
+    auto drained = [&](int w) { return ex + 8u + 8u * w; };
 
     if (tid == 0) {
         s_abort = 0;
@@ -226,7 +163,6 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
             mbar_init(drained(b), 1);
         }
         mbar_init(ex, 8);
-        mbar_init(d_full, 2);
         mbar_fence_init();
     }
     if (warp == 17) tmem_alloc(smem_u32(&s_tmem), 512);
@@ -237,29 +173,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
     if (p.seg) pdl_wait();  // segments and tokens come from earlier kernels; without segments only the token loads wait
     pdl_trigger();
     const int mt = p.gate_up ? (p.N / 2 + 127) / 128 : (p.N + kTileRows - 1) / kTileRows;
-    if (warp == 0) {  // tokens and tiles before each expert
-        int carry = 0;
-        for (int e0 = 0; e0 < p.E; e0 += 32) {
-            const int e = e0 + lane;
-            int a = 0, b = 0;
-            if (e < p.E) {
-                a = p.seg ? min(max(p.seg[e], 0), p.T) : 0;
-                b = p.seg ? min(max(p.seg[e + 1], a), p.T) : p.T;
-                s_tok[e] = a;
-                if (e == p.E - 1) s_tok[p.E] = b;
-            }
-            const int mine = (b - a + NT - 1) / NT * mt;
-            int v = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += up;
-            }
-            if (e < p.E) s_first[e] = carry + v - mine;
-            carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) s_first[p.E] = carry;
-    }
+    if (warp == 0) fill_tiles(p, NT, mt, s_first, s_tok, lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -317,26 +231,23 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
         // ---- MMA: one thread per M tile ------------------------------------------------------------------------------
         if (elect_one()) {
             const int w = warp - 17;
-            int s = 0, it = 0, dn = 0;  // dn counts the accumulations: one per group (exact) or per tile (scaled)
+            int s = 0, it = 0;
             bool ok = true;
             Tile t = tile(tile0);
             for (int i = tile0; i < tiles && ok; i += stride) {
                 const uint32_t idesc = idesc_f16(128, max(16, (t.n + 15) & ~15), false);
                 for (int g = g0; g < g1; ++g, ++it) {
-                    const int b = it & 1, db = kD == 2 ? dn & 1 : 0;
-                    const bool begins = !kScaled || g == g0, ends = !kScaled || g + 1 == g1;
+                    const int b = it & 1;
                     // a widening warp has seen the stage's copies land before it arrives: no wait on full(s) here
                     if (!(ok = thread_wait(a_full(w, b), (it >> 1) & 1, abort))) break;
-                    if (begins && !(ok = thread_wait(d_free(db), ((kD == 2 ? dn >> 1 : dn) & 1) ^ 1, abort))) break;
+                    if (!(ok = thread_wait(d_free(b), ((it >> 1) & 1) ^ 1, abort))) break;
                     tc_fence_after();
                     const uint64_t x0 = smem_desc_sw128(stage0 + static_cast<uint32_t>(s) * S::kStage + kCodeBytes, 1024);
-                    const uint32_t a = tmem + kColA + 128u * w + 64u * b, d = tmem + 128u * w + 64u * db;
+                    const uint32_t a = tmem + kColA + 128u * w + 64u * b, d = tmem + 128u * w + 64u * b;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) mma_f16_ts(d, a + 8u * k, x0 + (k >> 2) * (S::kHalf >> 4) + (k & 3) * 2u, idesc, !(begins && k == 0));
+                    for (int k = 0; k < 8; ++k) mma_f16_ts(d, a + 8u * k, x0 + (k >> 2) * (S::kHalf >> 4) + (k & 3) * 2u, idesc, k != 0);
                     // one event ends the group for everybody: the stage may be refilled, the A buffer rewritten, D read
                     tc_commit(done(s));
-                    if (kScaled && ends) tc_commit(d_full);  // (a parity wait cannot look past the next phase of done(s))
-                    if (ends) ++dn;
                     if (++s == kStages) s = 0;
                     if (g + 1 == g1) t = tile(i + stride);
                 }
@@ -355,18 +266,9 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
         int s = 0, it = 0, s2 = kStages - 2;       // s2, ph2: stage and phase of group it - 2, the last user of this A buffer
         uint32_t ph = 0, ph2 = 1;
         bool ok = true;
-        RowScales sc;
-        sc.at = smem_u32(s_scale) + (w * 128 + row) * kScaleStride;
-        if (kScaled && tile0 < tiles) {
-            const Tile t = tile(tile0);
-            sc.ask(p, t, (w ? t.row1 : t.row0) + row);
-        }
         for (int i = tile0; i < tiles && ok; i += stride) {
-            const __half* mine = sc.row;
-            if (kScaled) sc.keep(p);
             for (int g = g0; g < g1; ++g, ++it) {
                 const int b = it & 1;
-                const __half scale = kScaled ? sc.get(p, mine, g) : __half();
                 if (!(ok = warp_wait(full(s), ph, abort) && warp_wait(done(s2), ph2, abort))) break;
                 tc_fence_after();
                 const uint32_t from = from0 + static_cast<uint32_t>(s) * S::kStage, to = to0 + 64u * b;
@@ -374,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 for (int h = 0; h < 4; ++h) {
                     uint32_t a[16];
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) widen16<kScaled>(lds128(from + ((static_cast<uint32_t>(2 * h + c) ^ swz) << 4)), scale, a + 8 * c);
+                    for (int c = 0; c < 2; ++c) widen16<false>(lds128(from + ((static_cast<uint32_t>(2 * h + c) ^ swz) << 4)), __half(), a + 8 * c);
                     tmem_st16(to + 16u * h, a);
                 }
                 tmem_wait_st();
@@ -382,10 +284,6 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
                 warp_arrive(a_full(w, b));
                 if (++s == kStages) { s = 0; ph ^= 1; }
                 if (++s2 == kStages) { s2 = 0; ph2 ^= 1; }
-                if (kScaled && g == g0 && i + stride < tiles) {
-                    const Tile t = tile(i + stride);
-                    sc.ask(p, t, (w ? t.row1 : t.row0) + row);
-                }
             }
         }
     } else if (warp < 8) {
@@ -401,196 +299,103 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
         Tile t = tile(tile0);
         RowScales sc;
         sc.at = smem_u32(s_scale) + (w * 128 + row) * kScaleStride;
-        if (!kScaled && tile0 < tiles) sc.ask(p, t, (w ? t.row1 : t.row0) + row);
+        if (tile0 < tiles) sc.ask(p, t.e, (w ? t.row1 : t.row0) + row);
         for (int i = tile0; i < tiles && ok; i += stride, ++round) {
             const int lim = p.gate_up ? half_rows : p.N;                 // rows of this tile's kind
             const int mrow = (p.gate_up ? t.row0 : (w ? t.row1 : t.row0)) + row;  // gate/up: both tiles count gate rows
             const bool live = mrow < lim;
             Tile next = t;
-            if constexpr (kScaled) {
-                // the sums are complete: take them out of TMEM as fp16, hand the columns back, then store
-                constexpr int H = NT / 2;
-                const bool gu = p.gate_up;
-                const int j0 = gu ? w * H : 0, nj = max(0, min(t.n - j0, gu ? H : NT));  // this warpgroup's tokens
-                next = tile(i + stride);
-                if (!(ok = warp_wait(d_full, round & 1, abort))) break;
+            float acc[NT];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) acc[j] = 0.f;
+            const __half* mine = sc.row;
+            sc.keep(p);
+            for (int g = g0; g < g1; ++g, ++it) {
+                const int db = it & 1;
+                const float scale = __half2float(sc.get(p, mine, g));
+                if (!(ok = warp_wait(done(s), ph, abort))) break;
                 tc_fence_after();
-                __half2 out[H];
-                if (gu) {
+                const uint32_t d = tmem + lanes + 128u * w + 64u * db;
 #pragma unroll
-                    for (int c = 0; c < H; c += 32) {
-                        if (c < nj) {
-                            uint32_t r[32], u[32];
-                            tmem_ld32(r, tmem + lanes + j0 + c);
-                            tmem_ld32(u, tmem + lanes + 128u + j0 + c);
-                            tmem_wait_ld();
-                            if (c + 32 >= nj) {  // everything has left TMEM: the next tile may begin
-                                tc_fence_before();
-                                warp_arrive(d_free(0));
-                            }
+                for (int c = 0; c < NT; c += 16) {
+                    if (c < t.n) {
+                        uint32_t r[16];
+                        tmem_ld16(r, d + c);
+                        tmem_wait_ld();
 #pragma unroll
-                            for (int j = 0; j < 32; j += 2) {
-                                float y0, y1;
-                                swiglu2(__uint_as_float(r[j]), __uint_as_float(u[j]), __uint_as_float(r[j + 1]), __uint_as_float(u[j + 1]), y0, y1);
-                                out[(c + j) / 2] = __floats2half2_rn(y0, y1);
-                            }
-                        }
-                    }
-                    if (nj == 0) {
-                        tc_fence_before();
-                        warp_arrive(d_free(0));
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < NT; c += 32) {
-                        if (c < nj) {
-                            uint32_t r[32];
-                            tmem_ld32(r, tmem + lanes + 128u * w + c);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 32; j += 2) out[(c + j) / 2] = __floats2half2_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-                        }
-                    }
-                    tc_fence_before();
-                    warp_arrive(d_free(0));
-                }
-                const int64_t ld = gu ? half_rows : p.N;
-                __half* y = p.y + static_cast<int64_t>(t.t0 + j0) * ld;
-                const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * ld : nullptr;
-                if (p.wide && mrow - lane + 32 <= lim) {
-                    // A thread has one row of many tokens; turned over in shared memory 32 x 32 at a time, a lane stores eight rows of a token
-                    // (two bytes a lane instead: a down tile of 128 tokens spent longer in its stores than in its MMAs).
-                    const uint32_t turn = stage0 + kStages * S::kStage + warp * 2048u;
-#pragma unroll
-                    for (int c = 0; c < NT; c += 32) {
-                        if (c < nj) {
-                            __syncwarp();
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                const __half v = j & 1 ? __high2half(out[(c + j) / 2]) : __low2half(out[(c + j) / 2]);
-                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(turn + 64u * j + 2u * lane), "h"(__half_as_ushort(v)) : "memory");
-                            }
-                            __syncwarp();
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                const int j = 8 * k + (lane >> 2), at = mrow - lane + 8 * (lane & 3);
-                                if (c + j < nj) {
-                                    uint4 v = lds128(turn + 64u * j + 16u * (lane & 3));
-                                    if (res) {
-                                        const uint4 r4 = __ldcg(reinterpret_cast<const uint4*>(res + (c + j) * ld + at));
-                                        __half2* vh = reinterpret_cast<__half2*>(&v);
-                                        const __half2* rh = reinterpret_cast<const __half2*>(&r4);
-#pragma unroll
-                                        for (int e = 0; e < 4; ++e) vh[e] = __hadd2(vh[e], rh[e]);
-                                    }
-                                    *reinterpret_cast<uint4*>(y + (c + j) * ld + at) = v;
-                                }
-                            }
-                        }
-                    }
-                } else if (live) {
-#pragma unroll
-                    for (int j = 0; j < NT; ++j) {
-                        if (j < nj) {
-                            __half v = j & 1 ? __high2half(out[j / 2]) : __low2half(out[j / 2]);
-                            if (res) v = __hadd(v, res[j * ld + mrow]);
-                            y[j * ld + mrow] = v;
-                        }
+                        for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(scale, __uint_as_float(r[j]), acc[c + j]);
                     }
                 }
-            } else {
-                float acc[NT];
-#pragma unroll
-                for (int j = 0; j < NT; ++j) acc[j] = 0.f;
-                const __half* mine = sc.row;
-                sc.keep(p);
-                for (int g = g0; g < g1; ++g, ++it) {
-                    const int db = it & 1;
-                    const float scale = __half2float(sc.get(p, mine, g));
-                    if (!(ok = warp_wait(done(s), ph, abort))) break;
-                    tc_fence_after();
-                    const uint32_t d = tmem + lanes + 128u * w + 64u * db;
-#pragma unroll
-                    for (int c = 0; c < NT; c += 16) {
-                        if (c < t.n) {
-                            uint32_t r[16];
-                            tmem_ld16(r, d + c);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(scale, __uint_as_float(r[j]), acc[c + j]);
-                        }
-                    }
-                    tc_fence_before();
-                    // gate/up: the last sums' columns carry the exchange below and are freed after it
-                    if (!p.gate_up || g + 1 < g1) warp_arrive(d_free(db));
-                    if (++s == kStages) { s = 0; ph ^= 1; }
-                    if (g == g0) {
-                        next = tile(i + stride);
-                        if (i + stride < tiles) sc.ask(p, next, (w ? next.row1 : next.row0) + row);
-                    }
+                tc_fence_before();
+                // gate/up: the last sums' columns carry the exchange below and are freed after it
+                if (!p.gate_up || g + 1 < g1) warp_arrive(d_free(db));
+                if (++s == kStages) { s = 0; ph ^= 1; }
+                if (g == g0) {
+                    next = tile(i + stride);
+                    if (i + stride < tiles) sc.ask(p, next.e, (w ? next.row1 : next.row0) + row);
                 }
-                if (!ok) break;
-                const int dl = (it - 1) & 1;  // buffer of the last group
+            }
+            if (!ok) break;
+            const int dl = (it - 1) & 1;  // buffer of the last group
 
-                if (SPLIT) {
-                    // every group of this block has been read: the stages are free for its sums, [token][row]
-                    const uint32_t at = stage0 + 4u * (w * 128 + row);
+            if (SPLIT) {
+                // every group of this block has been read: the stages are free for its sums, [token][row]
+                const uint32_t at = stage0 + 4u * (w * 128 + row);
 #pragma unroll
-                    for (int j = 0; j < NT; ++j)
-                        if (j < t.n) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 4u * kTileRows * j), "f"(acc[j]) : "memory");
-                } else if (p.gate_up) {
-                    // SwiGLU: the gate tile's threads finish the first half of the tokens, the up tile's the second; what the other
-                    // needs goes through the accumulators' own columns of TMEM (same lanes, so no shared memory)
-                    constexpr int H = NT / 2;
-                    uint32_t r[16];
+                for (int j = 0; j < NT; ++j)
+                    if (j < t.n) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 4u * kTileRows * j), "f"(acc[j]) : "memory");
+            } else if (p.gate_up) {
+                // SwiGLU: the gate tile's threads finish the first half of the tokens, the up tile's the second; what the other
+                // needs goes through the accumulators' own columns of TMEM (same lanes, so no shared memory)
+                constexpr int H = NT / 2;
+                uint32_t r[16];
 #pragma unroll
-                    for (int c = 0; c < H; c += 16) {
+                for (int c = 0; c < H; c += 16) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) r[j] = c + j < H ? __float_as_uint(w ? acc[c + j < H ? c + j : 0] : acc[H + (c + j < H ? c + j : 0)]) : 0u;
-                        tmem_st16(tmem + lanes + 128u * w + 64u * dl + c, r);
-                    }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    warp_arrive(ex);
-                    if (!(ok = warp_wait(ex, round & 1, abort))) break;
-                    tc_fence_after();
-                    const uint32_t d_other = tmem + lanes + 128u * (w ^ 1) + 64u * dl;
-                    const int first = w ? H : 0;
+                    for (int j = 0; j < 16; ++j) r[j] = c + j < H ? __float_as_uint(w ? acc[c + j < H ? c + j : 0] : acc[H + (c + j < H ? c + j : 0)]) : 0u;
+                    tmem_st16(tmem + lanes + 128u * w + 64u * dl + c, r);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                warp_arrive(ex);
+                if (!(ok = warp_wait(ex, round & 1, abort))) break;
+                tc_fence_after();
+                const uint32_t d_other = tmem + lanes + 128u * (w ^ 1) + 64u * dl;
+                const int first = w ? H : 0;
 #pragma unroll
-                    for (int c = 0; c < H; c += 16) {
-                        if (first + c < t.n) {
-                            tmem_ld16(r, d_other + c);
-                            tmem_wait_ld();
+                for (int c = 0; c < H; c += 16) {
+                    if (first + c < t.n) {
+                        tmem_ld16(r, d_other + c);
+                        tmem_wait_ld();
 #pragma unroll
-                            for (int j = 0; j < 16 && c + j < H; j += 2) {
-                                float y[2];
-                                const float o0 = __uint_as_float(r[j]), o1 = __uint_as_float(r[j + 1]);
-                                if (w) swiglu2(o0, acc[H + c + j], o1, acc[H + c + j + 1], y[0], y[1]);
-                                else swiglu2(acc[c + j], o0, acc[c + j + 1], o1, y[0], y[1]);
+                        for (int j = 0; j < 16 && c + j < H; j += 2) {
+                            float y[2];
+                            const float o0 = __uint_as_float(r[j]), o1 = __uint_as_float(r[j + 1]);
+                            if (w) swiglu2(o0, acc[H + c + j], o1, acc[H + c + j + 1], y[0], y[1]);
+                            else swiglu2(acc[c + j], o0, acc[c + j + 1], o1, y[0], y[1]);
 #pragma unroll
-                                for (int v = 0; v < 2; ++v)
-                                    if (live && first + c + j + v < t.n)
-                                        p.y[static_cast<int64_t>(t.t0 + first + c + j + v) * half_rows + mrow] = __float2half_rn(y[v]);
-                            }
+                            for (int v = 0; v < 2; ++v)
+                                if (live && first + c + j + v < t.n)
+                                    p.y[static_cast<int64_t>(t.t0 + first + c + j + v) * half_rows + mrow] = __float2half_rn(y[v]);
                         }
                     }
-                    tc_fence_before();
-                    warp_arrive(d_free(dl));
-                } else if (live) {
-                    __half* y = p.y + static_cast<int64_t>(t.t0) * p.N + mrow;
-                    float* y32 = p.y32 + static_cast<int64_t>(t.t0) * p.N + mrow;
-                    const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * p.N + mrow : nullptr;
+                }
+                tc_fence_before();
+                warp_arrive(d_free(dl));
+            } else if (live) {
+                __half* y = p.y + static_cast<int64_t>(t.t0) * p.N + mrow;
+                float* y32 = p.y32 + static_cast<int64_t>(t.t0) * p.N + mrow;
+                const __half* res = p.resid ? p.resid + static_cast<int64_t>(t.t0) * p.N + mrow : nullptr;
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) {
-                        if (j < t.n) {
-                            if (p.y32) {
-                                y32[static_cast<int64_t>(j) * p.N] = acc[j];
-                                continue;
-                            }
-                            __half v = __float2half_rn(acc[j]);
-                            if (res) v = __hadd(v, res[static_cast<int64_t>(j) * p.N]);
-                            y[static_cast<int64_t>(j) * p.N] = v;
+                for (int j = 0; j < NT; ++j) {
+                    if (j < t.n) {
+                        if (p.y32) {
+                            y32[static_cast<int64_t>(j) * p.N] = acc[j];
+                            continue;
                         }
+                        __half v = __float2half_rn(acc[j]);
+                        if (res) v = __hadd(v, res[static_cast<int64_t>(j) * p.N]);
+                        y[static_cast<int64_t>(j) * p.N] = v;
                     }
                 }
             }
@@ -626,37 +431,27 @@ __global__ void __launch_bounds__(kThreads, 1) w8_gemm_kernel(const __grid_const
     }
 }
 
-// Per device and idempotent; not a stream operation, so legal under capture.
-template <typename K>
-int allow_smem(K kernel, size_t bytes) {
-    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-    return err == cudaSuccess ? LEMOQ_OK : set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
-}
-
 template <int NT>
-int launch_nt(GemmShape p, const __half* x, const int8_t* codes, const LaunchCfg& lc) {
+int launch_nt(W8Shape p, const __half* x, const int8_t* codes, const LaunchCfg& lc) {
     CUtensorMap map_w, map_x;
     if (int rc = encode_rows_map(&map_w, codes, 1, static_cast<int64_t>(p.E) * p.N, p.K, 128)) return rc;
     if (int rc = encode_rows_map(&map_x, x, 2, p.T, p.K, Shape<NT>::kBox)) return rc;
     const size_t smem = Shape<NT>::kSmem + 8 * (static_cast<size_t>(p.E) + 1);
     const int gk = p.K / p.group;
-    p.wide = (p.gate_up ? p.N / 2 : p.N) % 8 == 0 && aligned16(p.y) && aligned16(p.resid);
     p.scale_vecs = aligned16(p.scale) && (gk == 8 || gk == 16) ? gk / 8 : 0;
     const int64_t mt = p.gate_up ? (p.N / 2 + 127) / 128 : (p.N + kTileRows - 1) / kTileRows;
     const int64_t most = mt * (p.seg ? p.T / NT + std::min<int64_t>(p.E, p.T) : (p.T + NT - 1) / NT);  // tiles, at most
     const int sms = sm_count();
-    if constexpr (NT <= kExactTokens) {
-        // A linear of few rows is a tile on every sixth SM or fewer (2048 rows: 8 tiles), each a chain of K / 128 groups of half a
-        // microsecond: its groups are shared out over a cluster while that leaves every block two of them and an SM of its own.
-        int parts = 1;
-        while (parts < 8 && most * 2 * parts <= sms && 4 * parts <= p.K >> 7) parts *= 2;
-        if (parts > 1 && !p.seg && !p.gate_up && !p.y32 && p.T <= NT) {
-            if (int rc = allow_smem(w8_gemm_kernel<NT, true>, smem)) return rc;
-            p.parts = parts;
-            LaunchCfg clustered = lc;
-            clustered.cluster = parts;
-            return launch_kernel(w8_gemm_kernel<NT, true>, dim3(static_cast<unsigned>(most) * parts), dim3(kThreads), smem, clustered, map_w, map_x, p);
-        }
+    // A linear of few rows is a tile on every sixth SM or fewer (2048 rows: 8 tiles), each a chain of K / 128 groups of half a
+    // microsecond: its groups are shared out over a cluster while that leaves every block two of them and an SM of its own.
+    int parts = 1;
+    while (parts < 8 && most * 2 * parts <= sms && 4 * parts <= p.K >> 7) parts *= 2;
+    if (parts > 1 && !p.seg && !p.gate_up && !p.y32 && p.T <= NT) {
+        if (int rc = allow_smem(w8_gemm_kernel<NT, true>, smem)) return rc;
+        p.parts = parts;
+        LaunchCfg clustered = lc;
+        clustered.cluster = parts;
+        return launch_kernel(w8_gemm_kernel<NT, true>, dim3(static_cast<unsigned>(most) * parts), dim3(kThreads), smem, clustered, map_w, map_x, p);
     }
     if (int rc = allow_smem(w8_gemm_kernel<NT, false>, smem)) return rc;
     const int grid = static_cast<int>(std::min<int64_t>(sms, std::max<int64_t>(most, 1)));
@@ -666,7 +461,7 @@ int launch_nt(GemmShape p, const __half* x, const int8_t* codes, const LaunchCfg
 }  // namespace
 
 int launch_w8_gemm(const W8GemmParams& g, const LaunchCfg& lc) {
-    GemmShape p = {};
+    W8Shape p = {};
     p.T = g.T; p.N = g.N; p.K = g.K; p.group = g.group_size; p.E = g.E; p.gate_up = g.gate_up ? 1 : 0;
     p.seg = g.seg; p.scale = g.scale; p.resid = g.resid; p.y = g.y; p.y32 = g.y32; p.err_flag = g.err_flag;
     // NT bounds the tokens of a tile, the MMA's N follows the real count: a small NT only saves registers and stage bytes, a
@@ -675,7 +470,7 @@ int launch_w8_gemm(const W8GemmParams& g, const LaunchCfg& lc) {
     if (want <= 16) return launch_nt<16>(p, g.x, g.codes, lc);
     if (want <= 32) return launch_nt<32>(p, g.x, g.codes, lc);
     if (want <= kExactTokens || g.exact) return launch_nt<kExactTokens>(p, g.x, g.codes, lc);
-    return launch_nt<kScaledTokens>(p, g.x, g.codes, lc);
+    return launch_w8_pair(p, g.x, g.codes, lc);
 }
 
 }  // namespace lemoq
