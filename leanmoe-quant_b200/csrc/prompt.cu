@@ -3,7 +3,7 @@
 //   lemoq_lockstep_run  one token of each of T sequences, all at the same slot: K/V rows quantised into each sequence's int8 caches,
 //                       decode attention over those
 //
-// Nine kernels per layer (ten with more than a thousand routed pairs), launched from here with programmatic dependent launch: the prompt of a short question is
+// Nine kernels per layer, launched from here with programmatic dependent launch: the prompt of a short question is
 // bound by the 6.9 GB of weights all experts together have (1.1 ms), so a launch gap or a host call per expert is what it
 // must not pay; a long prompt is bound by the tensor cores (w8_gemm.cu, prompt_attn.cu); a lockstep step by the weights and its
 // sequences' caches (attn_i8.cu).
@@ -19,7 +19,7 @@ size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 struct PromptBuffers {
     __half *x, *x1, *h, *qkv, *q, *ctx, *pairs, *act;
     float* top_w;
-    int32_t *top_i, *place, *pair_of, *seg;
+    int32_t *top_i, *place, *pair_of, *seg, *counts;
 };
 
 size_t carve_prompt(const lemoq_step_desc& d, int T, char* base, PromptBuffers* b) {
@@ -42,8 +42,9 @@ size_t carve_prompt(const lemoq_step_desc& d, int T, char* base, PromptBuffers* 
     o.top_w = reinterpret_cast<float*>(take(4 * P));
     o.top_i = reinterpret_cast<int32_t*>(take(4 * P));
     o.place = reinterpret_cast<int32_t*>(take(4 * P));
-    o.pair_of = reinterpret_cast<int32_t*>(take(4 * P));
+    o.pair_of = reinterpret_cast<int32_t*>(take(4 * P));  // norm_route's ranks, then (very many tokens) the pair of a row
     o.seg = reinterpret_cast<int32_t*>(take(4 * (static_cast<size_t>(d.experts) + 1)));
+    o.counts = reinterpret_cast<int32_t*>(take(4 * ((t + 15) / 16) * d.experts));
     if (b) *b = o;
     return off;
 }
@@ -144,8 +145,11 @@ int run_rows(const lemoq_step_desc* desc, const lemoq_layer_desc* layers, const 
             LEMOQ_TRY(launch_prompt_attn(a, chained));
         }
         LEMOQ_TRY(gemm(b.ctx, T, L.o_codes, L.o_scale, d.hidden, A, b.x, b.x1));
-        LEMOQ_TRY(launch_norm_route(b.x1, half(L.ln2), d.eps, half(L.router), T, d.hidden, d.experts, d.top_k, d.norm_topk_prob, b.h, b.top_w, b.top_i, chained));
-        LEMOQ_TRY(launch_pairs(b.top_i, P, d.experts, b.h, d.top_k, d.hidden, b.place, b.pair_of, b.seg, b.pairs, nullptr, chained));
+        LEMOQ_TRY(launch_norm_route(b.x1, half(L.ln2), d.eps, half(L.router), T, d.hidden, d.experts, d.top_k, d.norm_topk_prob, b.h, b.top_w, b.top_i, b.pair_of, b.counts, chained));
+        if (T <= kPlaceTokens)
+            LEMOQ_TRY(launch_place_rows(b.top_i, b.pair_of, b.counts, T, d.top_k, d.experts, b.h, d.hidden, b.place, b.seg, b.pairs, chained));
+        else
+            LEMOQ_TRY(launch_pairs(b.top_i, P, d.experts, b.h, d.top_k, d.hidden, b.place, b.pair_of, b.seg, b.pairs, nullptr, chained));
         W8GemmParams g;
         g.x = b.pairs; g.T = P; g.codes = L.gu_codes; g.scale = half(L.gu_scale); g.N = 2 * d.ffn; g.K = d.hidden; g.group_size = d.group_size;
         g.seg = b.seg; g.E = d.experts; g.gate_up = true; g.y = b.act; g.exact = lockstep; g.err_flag = err_flag;

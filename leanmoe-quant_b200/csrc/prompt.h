@@ -25,9 +25,14 @@ struct QkvRows {
 };
 int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc);
 
-// h = RMSNorm(x); logits fp16(h . router^T), softmax + top-k of every row.  E a multiple of 8, <= 128; H a multiple of 64, <= 4096.
+// h = RMSNorm(x); logits fp16(h . router^T), softmax + top-k of every row.  E a multiple of 8, <= 128; H a multiple of 64, <= 4096.  Of the pairs of
+// every 16 tokens also: counts (ceil(T / 16), E) by expert, and rank (T, top_k), the place of a pair among those of its expert.
 int launch_norm_route(const __half* x, const __half* norm_w, float eps, const __half* router, int T, int H, int E, int top_k, int norm, __half* h, float* top_w,
-                      int32_t* top_i, const LaunchCfg& lc);
+                      int32_t* top_i, int32_t* rank, int32_t* counts, const LaunchCfg& lc);
+// Stable sort of the pairs by expert from those: place[p] = row of pair p in expert order, seg[e] = first row of e, x_sorted[place[p]] = h[p / K].
+constexpr int kPlaceTokens = 16384;  // at most
+int launch_place_rows(const int32_t* top_i, const int32_t* rank, const int32_t* counts, int T, int K, int E, const __half* h, int H, int32_t* place, int32_t* seg,
+                      __half* x_sorted, const LaunchCfg& lc);
 // Stable sort of the P = T * K pairs by expert: place[p] = row of pair p in expert order, pair_of[row] = p, seg[e] = first row of e,
 // x_sorted[row] = h[pair_of[row] / K].  Ids outside [0, E) are clamped and flagged.
 int launch_pairs(const int32_t* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,

@@ -5,13 +5,15 @@
 //   embed_norm     embedding row, input RMSNorm                                   one block per token
 //   qkv_rows       q/k RMSNorm over the projection width, RoPE, rows into the caches one block per token
 //   norm_route     post-attention RMSNorm, router logits (fp16 mma), softmax, top-k  one block per 16 tokens
-//   pair_plan      stable counting sort of the (token, slot) pairs by expert         one block per expert
-//   gather_rows    activations into expert order (few pairs: done by pair_plan)     one block per pair
+//   place_rows     activations into expert order, from norm_route's counts           one block per 1 to 16 tokens
+//   pair_plan      the same where only expert ids are given, or of very many tokens: stable counting sort, one block per expert
+//   gather_rows    and the copy (few pairs: done by pair_plan)                       one block per pair
 //   combine_norm   routing-weighted sum in slot order (fp32) + residual, next norm   one block per token
 #include "prompt.h"
 #include "stream.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace lemoq {
 namespace {
@@ -214,8 +216,10 @@ constexpr int kRouteTokens = 16;
 template <int TILES>  // expert tiles of 8
 __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __half* __restrict__ x, const __half* __restrict__ norm_w, float eps,
                                                                       const __half* __restrict__ router, int T, int H, int E, int top_k, int norm,
-                                                                      __half* __restrict__ h, float* __restrict__ top_w, int32_t* __restrict__ top_i) {
+                                                                      __half* __restrict__ h, float* __restrict__ top_w, int32_t* __restrict__ top_i, int32_t* __restrict__ rank,
+                                                                      int32_t* __restrict__ counts) {
     extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ int s_ids[kRouteTokens * 32];  // expert of the block's pairs, -1 behind the end
     float* part = reinterpret_cast<float*>(smem);    // [warp][16 tokens][E], after the rows
     __half* rows = reinterpret_cast<__half*>(smem);  // [16][H + 8]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
@@ -288,6 +292,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
     constexpr int PER = TILES / 4 < 1 ? 1 : TILES / 4;  // experts of a lane: lane + 32 i
     for (int j = warp; j < kRouteTokens; j += kRouteWarps) {
         const int t = t0 + j;
+        if (lane < top_k) s_ids[j * top_k + lane] = -1;
         if (t >= T) break;
         float p[PER];
         float mx = -INFINITY;
@@ -348,7 +353,21 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
         if (lane < top_k) {
             top_w[static_cast<int64_t>(t) * top_k + lane] = norm ? kept / wsum : kept;
             top_i[static_cast<int64_t>(t) * top_k + lane] = kept_i;
+            s_ids[j * top_k + lane] = kept_i;
         }
+    }
+    // A warp's experts: how many of the block's pairs go to each, and which of them a pair is (in pair order).
+    __syncthreads();
+    for (int e = warp; e < E; e += kRouteWarps) {
+        int n = 0;
+        for (int i0 = 0; i0 < kRouteTokens * top_k; i0 += 32) {
+            const int i = i0 + lane;
+            const bool hit = i < kRouteTokens * top_k && s_ids[i] == e;
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            if (hit) rank[static_cast<int64_t>(t0) * top_k + i] = n + __popc(m & ((1u << lane) - 1u));
+            n += __popc(m);
+        }
+        if (lane == 0) counts[blockIdx.x * E + e] = n;
     }
 }
 
@@ -431,6 +450,95 @@ __global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const ID* __res
     }
 }
 
+// Rows into expert order after norm_route, whose blocks left the pairs of every expert among their 16 tokens (`counts`) and the place of a
+// pair among those (`rank`): a block sums the counts of all blocks and of those before its tokens', which gives the first row of every
+// expert and of its own tokens in it, and writes each of its rows `K` times.  Bounded by those writes.  Us of this kernel / of a counting sort by a
+// block per expert and a gather by a block per pair: see launch_place_rows.
+constexpr int kPlaceThreads = 256;
+__global__ void __launch_bounds__(kPlaceThreads) place_rows_kernel(const int32_t* __restrict__ top_i, const int32_t* __restrict__ rank, const int32_t* __restrict__ counts,
+                                                                   int T, int K, int E, const __half* __restrict__ h, int H, int per_block, int32_t* __restrict__ place,
+                                                                   int32_t* __restrict__ seg, __half* __restrict__ x_sorted) {
+    __shared__ int s_all[kPlaceThreads], s_below[kPlaceThreads], s_base[128], s_row[kRouteTokens * 32];
+    const int tid = threadIdx.x, t0 = blockIdx.x * per_block, chunks = (T + kRouteTokens - 1) / kRouteTokens, chunk = t0 / kRouteTokens;
+    const int n = min(per_block, T - t0), pairs = n * K;
+    pdl_wait();
+    pdl_trigger();
+    uint4 v[kRowVecs];
+    auto load = [&](int j) {
+#pragma unroll
+        for (int u = 0; u < kRowVecs; ++u) {
+            const int i = 8 * (tid + kPlaceThreads * u);
+            if (i < H) v[u] = ld_cg16(h + static_cast<int64_t>(t0 + j) * H + i);
+        }
+    };
+    load(0);
+    const int lanes = E <= 64 ? 64 : 128, e = tid & (lanes - 1);
+    int all = 0, below = 0;
+    if (e < E) {
+#pragma unroll 8
+        for (int c = tid / lanes; c < chunks; c += kPlaceThreads / lanes) {
+            const int k = __ldcg(counts + c * E + e);
+            all += k;
+            below += c < chunk ? k : 0;
+        }
+    }
+    s_all[tid] = all;
+    s_below[tid] = below;
+    __syncthreads();
+    if (tid < 32) {  // four neighbouring experts a lane, then over the lanes
+        int sum[4], mine = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int x = 4 * tid + i;
+            sum[i] = 0;
+            if (x < E)
+                for (int u = x; u < kPlaceThreads; u += lanes) sum[i] += s_all[u];
+            mine += sum[i];
+        }
+        int first = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, first, o);
+            if (tid >= o) first += up;
+        }
+        first -= mine;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int x = 4 * tid + i;
+            if (x < E) {
+                int before = first;
+                for (int u = x; u < kPlaceThreads; u += lanes) before += s_below[u];
+                s_base[x] = before;
+                if (blockIdx.x == 0) seg[x] = first;
+            }
+            first += sum[i];
+        }
+        if (blockIdx.x == 0 && tid == 31) seg[E] = first;
+    }
+    __syncthreads();
+    for (int i = tid; i < pairs; i += kPlaceThreads) {
+        const int64_t p = static_cast<int64_t>(t0) * K + i;
+        const int row = s_base[__ldcg(top_i + p)] + __ldcg(rank + p);
+        s_row[i] = row;
+        place[p] = row;
+    }
+    __syncthreads();
+    for (int j = 0; j < n; ++j) {
+        uint4 w[kRowVecs];
+#pragma unroll
+        for (int u = 0; u < kRowVecs; ++u) w[u] = v[u];
+        if (j + 1 < n) load(j + 1);
+        for (int k = 0; k < K; ++k) {
+            __half* dst = x_sorted + static_cast<int64_t>(s_row[j * K + k]) * H;
+#pragma unroll
+            for (int u = 0; u < kRowVecs; ++u) {
+                const int i = 8 * (tid + kPlaceThreads * u);
+                if (i < H) *reinterpret_cast<uint4*>(dst + i) = w[u];
+            }
+        }
+    }
+}
+
 // out[t] = fp16(sum_k w[t, k] * y[place[t, k]]), products and sums in slot order in fp32, y not rounded before.
 __global__ void __launch_bounds__(kRowThreads) weighted_sum_kernel(const float* __restrict__ y, const int32_t* __restrict__ place, const __half* __restrict__ top_w, int K,
                                                                    int H, __half* __restrict__ out) {
@@ -481,22 +589,31 @@ int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc) {
 }
 
 int launch_norm_route(const __half* x, const __half* norm_w, float eps, const __half* router, int T, int H, int E, int top_k, int norm, __half* h, float* top_w,
-                      int32_t* top_i, const LaunchCfg& lc) {
+                      int32_t* top_i, int32_t* rank, int32_t* counts, const LaunchCfg& lc) {
     const dim3 grid((T + kRouteTokens - 1) / kRouteTokens), block(kRouteWarps * 32);
     const size_t smem = std::max(static_cast<size_t>(kRouteWarps) * kRouteTokens * E * sizeof(float), static_cast<size_t>(kRouteTokens) * (H + 8) * sizeof(__half));
     auto run = [&](auto* kernel) {
         const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
-        return launch_kernel(kernel, grid, block, smem, lc, x, norm_w, eps, router, T, H, E, top_k, norm, h, top_w, top_i);
+        return launch_kernel(kernel, grid, block, smem, lc, x, norm_w, eps, router, T, H, E, top_k, norm, h, top_w, top_i, rank, counts);
     };
     return E <= 64 ? run(norm_route_kernel<8>) : run(norm_route_kernel<16>);
+}
+
+// Tokens of a block: enough blocks for the chip, and no more than that, because each of them reads all counts.  With more tokens than kPlaceTokens
+// those reads (a block 256 bytes for 16 tokens, and one block for 16) outgrow the copies.
+int launch_place_rows(const int32_t* top_i, const int32_t* rank, const int32_t* counts, int T, int K, int E, const __half* h, int H, int32_t* place, int32_t* seg,
+                      __half* x_sorted, const LaunchCfg& lc) {
+    int per = 1;
+    while (per < kRouteTokens && T / per > 8 * sm_count() / 2) per *= 2;
+    return launch_kernel(place_rows_kernel, dim3((T + per - 1) / per), dim3(kPlaceThreads), 0, lc, top_i, rank, counts, T, K, E, h, H, per, place, seg, x_sorted);
 }
 
 template <typename ID>
 static int plan_and_gather(const ID* ids, int P, int E, const __half* h, int K, int H, int32_t* place, int32_t* pair_of, int32_t* seg, __half* x_sorted, int* err,
                            const LaunchCfg& lc) {
-    if (P <= kGatherPairs)
-        return launch_kernel(pair_plan_kernel<ID, true>, dim3(E), dim3(kPlanThreads), 0, lc, ids, P, E, place, pair_of, seg, h, K, H, x_sorted, err);
+    if (std::is_same<ID, int64_t>::value && P <= kGatherPairs)
+        return launch_kernel(pair_plan_kernel<int64_t, true>, dim3(E), dim3(kPlanThreads), 0, lc, reinterpret_cast<const int64_t*>(ids), P, E, place, pair_of, seg, h, K, H, x_sorted, err);
     if (int rc = launch_kernel(pair_plan_kernel<ID, false>, dim3(E), dim3(kPlanThreads), 0, lc, ids, P, E, place, pair_of, seg, h, K, H, x_sorted, err)) return rc;
     return launch_kernel(gather_rows_kernel, dim3(P), dim3(kRowThreads), 0, lc, h, pair_of, K, H, x_sorted);
 }

@@ -283,3 +283,27 @@ def test_a_prompt_whose_operations_matter_goes_through_the_modules():
         assert "_lemoq_prompt_plan" not in session.cache.__dict__ and rel_err(logits, native) < 2e-2
         assert not isinstance(mode, Seen) or mode.count == 4  # k and v rows of both layers
         assert torch.equal(session.prefill().logits, native) and "_lemoq_prompt_plan" in session.cache.__dict__
+
+
+# either side of 16 tokens (the blocks that route), one, two, four and eight tokens a block that copies, and more tokens than those blocks take
+@pytest.mark.parametrize("tokens", [15, 16, 17, 610, 1201, 2405, 4800, 16390])
+def test_rows_of_a_prompt_reach_their_experts(tokens):
+    """The native prompt against the same prompt through the modules (which a hook asks for)."""
+    from benchmarks.cudagraph import StaticCacheDecodeSession
+
+    spec = glue.OlmoeSpec(layers=1, hidden=256, heads=2, head_dim=128, experts=72, top_k=5, ffn=128, vocab=512)
+    wf = glue.random_float_weights(spec, seed=tokens, dtype=torch.float16, std=0.05, norm_weight_jitter=0.1)
+    wf.embed.mul_(20.0)
+    wf.layers[0].router.mul_(5.0)
+    model = lemoq_model_from_oracle(wf)
+    install_canonical(model, tokens, 4)
+    prompt = torch.randint(0, spec.vocab, (1, tokens), generator=torch.Generator().manual_seed(tokens)).to(DEV)
+    session = StaticCacheDecodeSession(model, prompt, ctx=tokens, max_new_tokens=4, engine="ops")
+    native = session.prefill().logits
+    assert "_lemoq_prompt_plan" in session.cache.__dict__
+    del session.cache._lemoq_prompt_plan
+    model.model.layers[0].mlp.register_forward_hook(lambda module, args, out: None)
+    by_modules = session.prefill().logits
+    assert "_lemoq_prompt_plan" not in session.cache.__dict__
+    # over all rows: now and then a token has another, nearly equal expert in its last slot
+    assert float((native.float() - by_modules.float()).norm() / by_modules.float().norm()) < 1e-2
