@@ -210,10 +210,12 @@ constexpr int kRouteTokens = 16;
 
 // A warp normalises one of the block's 16 rows; then the warps split H for the logits of all 16 rows and all experts.  Their partial
 // sums meet in shared memory (over the rows) and are added in warp order.  With 0.27 GFLOP per thousand tokens the work is too small for
-// a tcgen05 pipeline to fill: what counts is one round of loads.  The router does not depend on earlier kernels: it is asked into L2
-// while those finish.  A and B use the same permutation of k inside 32 values, so that 128-bit loads feed the fragments.
-// (As a norm kernel and a router kernel of eight warps with all loads in turn: 3.5 + 19 us at 64 tokens.)
-template <int TILES>  // expert tiles of 8
+// a tcgen05 pipeline to fill: what counts is one round of loads, so a row and its norm weights are asked for together, and a warp's first router
+// values before the previous kernel ends (the rest of the router is asked into L2).  A and B use the same permutation of k inside 32
+// values, so that 128-bit loads feed the fragments.  The top-k takes the bits of a probability as a whole number: two warp-wide reductions a choice.
+// (As a norm kernel and a router kernel of eight warps with all loads in turn: 3.5 + 19 us at 64 tokens; with loads inside loops and a choice by
+// ten shuffles a layer of a prompt of 61 tokens took 2.8 us more than with this, of a step of 11 sequences 5.6, of one of 64 at 2048 3.)
+template <int TILES, int VECS>  // expert tiles of 8; vectors of eight values a lane has of a row
 __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __half* __restrict__ x, const __half* __restrict__ norm_w, float eps,
                                                                       const __half* __restrict__ router, int T, int H, int E, int top_k, int norm,
                                                                       __half* __restrict__ h, float* __restrict__ top_w, int32_t* __restrict__ top_i, int32_t* __restrict__ rank,
@@ -226,6 +228,19 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
     const int t0 = blockIdx.x * kRouteTokens, tiles = E >> 3, pitch = H + 8;
     for (int i = (blockIdx.x % 4) * kRouteWarps * 32 + threadIdx.x; i < E * H / 64; i += 4 * kRouteWarps * 32)  // four blocks share it
         asm volatile("prefetch.global.L2 [%0];" ::"l"(router + 64 * static_cast<int64_t>(i)));
+    const __half* wr = router + static_cast<int64_t>(g) * H + 8 * q;
+    constexpr bool kAhead = TILES <= 8, kNormAhead = VECS <= 8;  // (where the registers are there for it)
+    uint4 w[8];
+    auto load_router = [&](int k, int n0) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+            if (n0 + n < tiles) w[n] = __ldg(reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(8 * (n0 + n)) * H + k));
+    };
+    if (kAhead && 32 * warp < H) load_router(32 * warp, 0);
+    uint4 wv[VECS];
+#pragma unroll
+    for (int v = 0; v < VECS; ++v)
+        if (kNormAhead && 8 * lane + 256 * v < H) wv[v] = __ldg(reinterpret_cast<const uint4*>(norm_w + 8 * lane + 256 * v));
     pdl_wait();
     pdl_trigger();
     {
@@ -233,24 +248,30 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
         __half* mine = rows + warp * pitch;
         if (t < T) {
             const __half* src = x + static_cast<int64_t>(t) * H;
-            float ss = 0.f;
-            for (int i = 8 * lane; i < H; i += 256) {
-                const uint4 v = ld_cg16(src + i);
-                *reinterpret_cast<uint4*>(mine + i) = v;
-                float f[8];
-                unpack8_h(v, f);
+            uint4 r[VECS];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+            for (int v = 0; v < VECS; ++v) r[v] = 8 * lane + 256 * v < H ? ld_cg16(src + 8 * lane + 256 * v) : make_uint4(0, 0, 0, 0);
+            float ss = 0.f;
+#pragma unroll
+            for (int v = 0; v < VECS; ++v) {
+                float f[8];
+                unpack8_h(r[v], f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);  // vectors behind the row are zero
             }
             const float rstd = 1.0f / sqrtf(warp_sum(ss) / static_cast<float>(H) + eps);
-            for (int i = 8 * lane; i < H; i += 256) {
-                const uint4 v = *reinterpret_cast<const uint4*>(mine + i), wv = __ldg(reinterpret_cast<const uint4*>(norm_w + i));
-                const __half *vh = reinterpret_cast<const __half*>(&v), *wh = reinterpret_cast<const __half*>(&wv);
-                __align__(16) __half o[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(__half2float(vh[j]) * rstd), wh[j]);
-                *reinterpret_cast<uint4*>(mine + i) = *reinterpret_cast<const uint4*>(o);
-                *reinterpret_cast<uint4*>(h + static_cast<int64_t>(t) * H + i) = *reinterpret_cast<const uint4*>(o);
+            for (int v = 0; v < VECS; ++v) {
+                const int i = 8 * lane + 256 * v;
+                if (i < H) {
+                    if (!kNormAhead) wv[v] = __ldg(reinterpret_cast<const uint4*>(norm_w + i));
+                    const __half *vh = reinterpret_cast<const __half*>(&r[v]), *wh = reinterpret_cast<const __half*>(&wv[v]);
+                    __align__(16) __half o[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(__half2float(vh[j]) * rstd), wh[j]);
+                    *reinterpret_cast<uint4*>(mine + i) = *reinterpret_cast<const uint4*>(o);
+                    *reinterpret_cast<uint4*>(h + static_cast<int64_t>(t) * H + i) = *reinterpret_cast<const uint4*>(o);
+                }
             }
         } else {
             for (int i = 8 * lane; i < H; i += 256) *reinterpret_cast<uint4*>(mine + i) = make_uint4(0, 0, 0, 0);
@@ -260,21 +281,20 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
     float c[TILES][4];
 #pragma unroll
     for (int n = 0; n < TILES; ++n) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
-    const __half* wr = router + static_cast<int64_t>(g) * H + 8 * q;
-#pragma unroll(TILES <= 8 ? 2 : 1)
     for (int k = 32 * warp; k < H; k += 32 * kRouteWarps) {
         const uint4 a = *reinterpret_cast<const uint4*>(rows + g * pitch + 8 * q + k), b = *reinterpret_cast<const uint4*>(rows + (g + 8) * pitch + 8 * q + k);
 #pragma unroll
         for (int n0 = 0; n0 < TILES; n0 += 8) {
-            uint4 w[8];
+            if (!kAhead) load_router(k, n0);
+            uint4 u[8];
 #pragma unroll
-            for (int n = 0; n < 8; ++n)
-                if (n0 + n < tiles) w[n] = __ldg(reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(8 * (n0 + n)) * H + k));
+            for (int n = 0; n < 8; ++n) u[n] = w[n];
+            if (kAhead && k + 32 * kRouteWarps < H) load_router(k + 32 * kRouteWarps, 0);  // on its way under the work on this
 #pragma unroll
             for (int n = 0; n < 8; ++n) {
                 if (n0 + n < tiles) {
-                    mma_f16(c[n0 + n], a.x, b.x, a.y, b.y, w[n].x, w[n].y);
-                    mma_f16(c[n0 + n], a.z, b.z, a.w, b.w, w[n].z, w[n].w);
+                    mma_f16(c[n0 + n], a.x, b.x, a.y, b.y, u[n].x, u[n].y);
+                    mma_f16(c[n0 + n], a.z, b.z, a.w, b.w, u[n].z, u[n].w);
                 }
             }
         }
@@ -290,10 +310,10 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
     }
     __syncthreads();
     constexpr int PER = TILES / 4 < 1 ? 1 : TILES / 4;  // experts of a lane: lane + 32 i
-    for (int j = warp; j < kRouteTokens; j += kRouteWarps) {
-        const int t = t0 + j;
-        if (lane < top_k) s_ids[j * top_k + lane] = -1;
-        if (t >= T) break;
+    const int t = t0 + warp;
+    static_assert(kRouteTokens == kRouteWarps, "a warp chooses for one token");
+    if (lane < top_k) s_ids[warp * top_k + lane] = -1;
+    if (t < T) {
         float p[PER];
         float mx = -INFINITY;
 #pragma unroll
@@ -303,7 +323,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
             if (e < E) {
                 float v = 0.f;
 #pragma unroll
-                for (int w = 0; w < kRouteWarps; ++w) v += part[(w * kRouteTokens + j) * E + e];
+                for (int u = 0; u < kRouteWarps; ++u) v += part[(u * kRouteTokens + warp) * E + e];
                 p[i] = __half2float(__float2half_rn(v));  // the logits are fp16 values
             }
             mx = fmaxf(mx, p[i]);
@@ -318,29 +338,26 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
             }
         }
         sum = warp_sum(sum);
+        int key[PER];  // order of the probabilities; -1 taken, no expert, or not a number
 #pragma unroll
-        for (int i = 0; i < PER; ++i) p[i] = lane + 32 * i < E ? p[i] / sum : -1.f;
+        for (int i = 0; i < PER; ++i) {
+            const float v = p[i] / sum;
+            key[i] = lane + 32 * i < E && v >= 0.f ? __float_as_int(v) : -1;
+        }
         float kept = 0.f, wsum = 0.f;
         int kept_i = 0;
         for (int k = 0; k < top_k; ++k) {
-            float best = -1.f;
-            int bi = 0x7fffffff;
+            int top = key[0];
 #pragma unroll
-            for (int i = 0; i < PER; ++i)
-                if (p[i] > best) {  // ascending e inside a lane: the first maximum wins
-                    best = p[i];
-                    bi = lane + 32 * i;
-                }
+            for (int i = 1; i < PER; ++i) top = max(top, key[i]);
+            top = __reduce_max_sync(0xffffffffu, top);
+            unsigned first = 0x7fffffffu;  // the lowest expert that has it
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) {
-                    best = ob;
-                    bi = oi;
-                }
-            }
-            if (bi >= E) bi = 0;  // only with NaN logits: any valid expert
+            for (int i = PER - 1; i >= 0; --i)
+                if (key[i] == top) first = lane + 32 * i;
+            int bi = static_cast<int>(__reduce_min_sync(0xffffffffu, first));
+            if (top < 0) bi = 0;  // only with NaN logits: any valid expert
+            const float best = top < 0 ? -1.f : __int_as_float(top);
             wsum += best;
             if (lane == k) {
                 kept = best;
@@ -348,12 +365,12 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
             }
 #pragma unroll
             for (int i = 0; i < PER; ++i)
-                if (bi == lane + 32 * i) p[i] = -1.f;
+                if (bi == lane + 32 * i) key[i] = -1;
         }
         if (lane < top_k) {
             top_w[static_cast<int64_t>(t) * top_k + lane] = norm ? kept / wsum : kept;
             top_i[static_cast<int64_t>(t) * top_k + lane] = kept_i;
-            s_ids[j * top_k + lane] = kept_i;
+            s_ids[warp * top_k + lane] = kept_i;
         }
     }
     // A warp's experts: how many of the block's pairs go to each, and which of them a pair is (in pair order).
@@ -597,7 +614,8 @@ int launch_norm_route(const __half* x, const __half* norm_w, float eps, const __
         if (err != cudaSuccess) return set_error(LEMOQ_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(err));
         return launch_kernel(kernel, grid, block, smem, lc, x, norm_w, eps, router, T, H, E, top_k, norm, h, top_w, top_i, rank, counts);
     };
-    return E <= 64 ? run(norm_route_kernel<8>) : run(norm_route_kernel<16>);
+    if (H <= 2048) return E <= 64 ? run(norm_route_kernel<8, 8>) : run(norm_route_kernel<16, 8>);
+    return E <= 64 ? run(norm_route_kernel<8, 16>) : run(norm_route_kernel<16, 16>);
 }
 
 // Tokens of a block: enough blocks for the chip, and no more than that, because each of them reads all counts.  With more tokens than kPlaceTokens

@@ -286,12 +286,16 @@ def test_a_prompt_whose_operations_matter_goes_through_the_modules():
 
 
 # either side of 16 tokens (the blocks that route), one, two, four and eight tokens a block that copies, and more tokens than those blocks take
-@pytest.mark.parametrize("tokens", [15, 16, 17, 610, 1201, 2405, 4800, 16390])
-def test_rows_of_a_prompt_reach_their_experts(tokens):
+@pytest.mark.parametrize("tokens,shape", [(t, {}) for t in (15, 16, 17, 610, 1201, 2405, 4800, 16390)] +
+                         # rows shorter than a warp's stride and of more than 2048 values, one and 32 experts a token, 128 of them
+                         [(17, dict(hidden=2048, experts=8, top_k=1)), (33, dict(hidden=1024, experts=128, top_k=32)),
+                          (20, dict(hidden=4096, experts=64, top_k=8)), (18, dict(hidden=4096, experts=128, top_k=8)), (5, dict(hidden=128, experts=40, top_k=3))])
+def test_rows_of_a_prompt_reach_their_experts(tokens, shape):
     """The native prompt against the same prompt through the modules (which a hook asks for)."""
     from benchmarks.cudagraph import StaticCacheDecodeSession
 
-    spec = glue.OlmoeSpec(layers=1, hidden=256, heads=2, head_dim=128, experts=72, top_k=5, ffn=128, vocab=512)
+    shape = {"hidden": 256, "experts": 72, "top_k": 5, **shape}
+    spec = glue.OlmoeSpec(layers=1, heads=shape["hidden"] // 128, head_dim=128, ffn=128, vocab=512, **shape)
     wf = glue.random_float_weights(spec, seed=tokens, dtype=torch.float16, std=0.05, norm_weight_jitter=0.1)
     wf.embed.mul_(20.0)
     wf.layers[0].router.mul_(5.0)
