@@ -23,6 +23,10 @@ constexpr int kRowVecs = 2;  // 8-value vectors a thread keeps: rows up to 4096
 
 // RMSNorm of a row held as fp32 in registers (vector v at 8 * (tid + 256 v)); HF rounding chain, fp16 out.
 __device__ __forceinline__ void norm_row_store(const float (&f)[kRowVecs][8], int H, const __half* __restrict__ w, float eps, __half* __restrict__ y, float* red) {
+    uint4 wv[kRowVecs];  // on their way under the reduction
+#pragma unroll
+    for (int v = 0; v < kRowVecs; ++v)
+        if (8 * (threadIdx.x + kRowThreads * v) < H) wv[v] = __ldg(reinterpret_cast<const uint4*>(w + 8 * (threadIdx.x + kRowThreads * v)));
     float ss = 0.f;
 #pragma unroll
     for (int v = 0; v < kRowVecs; ++v)
@@ -34,8 +38,7 @@ __device__ __forceinline__ void norm_row_store(const float (&f)[kRowVecs][8], in
     for (int v = 0; v < kRowVecs; ++v) {
         const int i = 8 * (threadIdx.x + kRowThreads * v);
         if (i < H) {
-            const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + i));
-            const __half* wh = reinterpret_cast<const __half*>(&wv);
+            const __half* wh = reinterpret_cast<const __half*>(&wv[v]);
             __align__(16) __half o[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(f[v][j] * rstd), wh[j]);
@@ -64,7 +67,10 @@ __global__ void __launch_bounds__(kRowThreads) embed_norm_kernel(const int64_t* 
     norm_row_store(f, H, w, eps, h + t * H, red);
 }
 
-// out[t] = fp16(sum_k w[t, k] * y[place[t, k]]) + x1[t]; then the next RMSNorm of it.
+// out[t] = fp16(sum_k w[t, k] * y[place[t, k]]) + x1[t]; then the next RMSNorm of it.  Bounded by the K rows a token reads: eight of them are in
+// flight at a time, the residual and the norm weights beside them.  (Four at a time, the residual first and the norm weights
+// last: 5.9 us alone at 61 tokens, now 4.6; the same 40 us at 4096, 4.6 TB/s.)
+template <int VECS>  // vectors of eight values a thread has of a row
 __global__ void __launch_bounds__(kRowThreads) combine_norm_kernel(const __half* __restrict__ y, const int32_t* __restrict__ place, const float* __restrict__ top_w,
                                                                    int K, const __half* __restrict__ x1, int H, const __half* __restrict__ w, float eps,
                                                                    __half* __restrict__ x2, __half* __restrict__ h) {
@@ -73,26 +79,55 @@ __global__ void __launch_bounds__(kRowThreads) combine_norm_kernel(const __half*
     pdl_trigger();
     const int64_t t = blockIdx.x;
     float f[kRowVecs][8];
+    uint4 r[VECS];
 #pragma unroll
-    for (int v = 0; v < kRowVecs; ++v) {
-        const int i = 8 * (threadIdx.x + kRowThreads * v);
+    for (int v = 0; v < kRowVecs; ++v)
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[v][j] = 0.f;
-        if (i < H) {
-            uint4 r = ld_cg16(x1 + t * H + i);
-#pragma unroll 4
-            for (int k = 0; k < K; ++k) {
-                const float wk = __half2float(__float2half_rn(__ldg(top_w + t * K + k)));
-                float g[8];
-                unpack8_h(ld_cg16(y + static_cast<int64_t>(__ldg(place + t * K + k)) * H + i), g);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) f[v][j] = __fadd_rn(f[v][j], __fmul_rn(g[j], wk));
+    for (int v = 0; v < VECS; ++v) {
+        const int i = 8 * (threadIdx.x + kRowThreads * v);
+        if (i < H) r[v] = ld_cg16(x1 + t * H + i);
+    }
+    for (int k0 = 0; k0 < K; k0 += 8) {
+        uint4 e[VECS][8];
+        float wk[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k0 + k < K) {
+                wk[k] = __half2float(__float2half_rn(__ldg(top_w + t * K + k0 + k)));
+                const __half* src = y + static_cast<int64_t>(__ldg(place + t * K + k0 + k)) * H;
+#pragma unroll
+                for (int v = 0; v < VECS; ++v) {
+                    const int i = 8 * (threadIdx.x + kRowThreads * v);
+                    if (i < H) e[v][k] = ld_cg16(src + i);
+                }
             }
-            __half* rh = reinterpret_cast<__half*>(&r);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k0 + k < K) {
+#pragma unroll
+                for (int v = 0; v < VECS; ++v) {
+                    if (8 * (threadIdx.x + kRowThreads * v) < H) {
+                        float g[8];
+                        unpack8_h(e[v][k], g);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) f[v][j] = __fadd_rn(f[v][j], __fmul_rn(g[j], wk[k]));
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < VECS; ++v) {
+        const int i = 8 * (threadIdx.x + kRowThreads * v);
+        if (i < H) {
+            __half* rh = reinterpret_cast<__half*>(&r[v]);
 #pragma unroll
             for (int j = 0; j < 8; ++j) rh[j] = __hadd(__float2half_rn(f[v][j]), rh[j]);
-            *reinterpret_cast<uint4*>(x2 + t * H + i) = r;
-            unpack8_h(r, f[v]);
+            *reinterpret_cast<uint4*>(x2 + t * H + i) = r[v];
+            unpack8_h(r[v], f[v]);
         }
     }
     norm_row_store(f, H, w, eps, h + t * H, red);
@@ -117,68 +152,101 @@ __device__ __forceinline__ void quantise_head_store(const __half* x, int8_t* cod
     if (first_lane) *scale = __float2half_rn(s);
 }
 
+// Sums over the block of two values per thread at once.
+__device__ __forceinline__ float2 block_sum2(float2 v, float2* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v.x = warp_sum(v.x);
+    v.y = warp_sum(v.y);
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    float2 t = lane < kRowThreads / 32 ? red[lane] : make_float2(0.f, 0.f);
+    t.x = warp_sum(t.x);
+    t.y = warp_sum(t.y);
+    return t;
+}
+
 // One block per token, A = heads * 128 <= 4096.  qkv (T, 3A) -> q (T, A) normalised and rotated.  The k and v rows go into slot pos[t] of
 // the fp16 caches (heads, S, 128), or (INT8, lockstep decoding) quantised into slot *pos of the row's own caches (T * heads, S, 128).
-template <bool INT8>
+// Bounded by the rows read and written; everything a thread needs is asked for at once.  (v rows, norm weights and angles where they were used,
+// a reduction for q and one for k: 5.5, 10.5 and 33.5 us alone at 61, 1024 and 4096 tokens; now 3.6, 7.5 and 22.)
+template <bool INT8, int VECS>  // vectors of eight values a thread has of a row
 __global__ void __launch_bounds__(kRowThreads) qkv_rows_kernel(const QkvRows p) {
-    __shared__ float red[40];
-    __shared__ __align__(16) __half row[2][kRowThreads * 8 * kRowVecs];
-    pdl_wait();
-    pdl_trigger();
+    __shared__ float2 red[kRowThreads / 32];
+    __shared__ __align__(16) __half row[2][kRowThreads * 8 * VECS];
     const int64_t t = blockIdx.x;
     const int A = p.heads * 128, tid = threadIdx.x;
+    uint4 w[2][VECS];  // norm weights: not an earlier kernel's
+#pragma unroll
+    for (int v = 0; v < VECS; ++v) {
+        const int i = 8 * (tid + kRowThreads * v);
+        if (i < A) {
+            w[0][v] = __ldg(reinterpret_cast<const uint4*>(p.q_norm + i));
+            w[1][v] = __ldg(reinterpret_cast<const uint4*>(p.k_norm + i));
+        }
+    }
+    pdl_wait();
+    pdl_trigger();
+    const __half* src = p.qkv + t * 3 * A;
+    uint4 x[3][VECS];
+#pragma unroll
+    for (int v = 0; v < VECS; ++v) {
+        const int i = 8 * (tid + kRowThreads * v);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) x[m][v] = i < A ? ld_cg16(src + m * A + i) : make_uint4(0, 0, 0, 0);
+    }
     int64_t pos = p.pos[INT8 ? 0 : t];
     if (pos < 0 || pos >= p.S) {
         if (p.err_flag && tid == 0) atomicOr(p.err_flag, LEMOQ_FLAG_BAD_POSITION);
         pos = pos < 0 ? 0 : p.S - 1;
     }
-    const __half* src = p.qkv + t * 3 * A;
-    float f[2][kRowVecs][8];
-    float ss[2] = {0.f, 0.f};
+    const int d = 8 * tid & 127;  // the same in every vector of a thread
+    const uint4 cos = __ldg(reinterpret_cast<const uint4*>(p.rope_cos + pos * 128 + d)), sin = __ldg(reinterpret_cast<const uint4*>(p.rope_sin + pos * 128 + d));
+    float2 ss = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int v = 0; v < VECS; ++v) {
+        float f[8];
+        unpack8_h(x[0][v], f);
 #pragma unroll
-        for (int v = 0; v < kRowVecs; ++v) {
-            const int i = 8 * (tid + kRowThreads * v);
-            unpack8_h(i < A ? ld_cg16(src + m * A + i) : make_uint4(0, 0, 0, 0), f[m][v]);
+        for (int j = 0; j < 8; ++j) ss.x = fmaf(f[j], f[j], ss.x);
+        unpack8_h(x[1][v], f);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) ss[m] = fmaf(f[m][v][j], f[m][v][j], ss[m]);
-        }
+        for (int j = 0; j < 8; ++j) ss.y = fmaf(f[j], f[j], ss.y);
+    }
+    ss = block_sum2(ss, red);
+    const float rstd[2] = {1.0f / sqrtf(ss.x / static_cast<float>(A) + p.eps), 1.0f / sqrtf(ss.y / static_cast<float>(A) + p.eps)};
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
-        const float rstd = 1.0f / sqrtf(block_sum(ss[m], red) / static_cast<float>(A) + p.eps);
-        const __half* w = m ? p.k_norm : p.q_norm;
 #pragma unroll
-        for (int v = 0; v < kRowVecs; ++v) {
+        for (int v = 0; v < VECS; ++v) {
             const int i = 8 * (tid + kRowThreads * v);
             if (i < A) {
-                const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + i));
-                const __half* wh = reinterpret_cast<const __half*>(&wv);
+                const __half* wh = reinterpret_cast<const __half*>(&w[m][v]);
+                float f[8];
+                unpack8_h(x[m][v], f);
                 __align__(16) __half o[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(f[m][v][j] * rstd), wh[j]);
-                *reinterpret_cast<uint4*>(&row[m][i]) = *reinterpret_cast<const uint4*>(o);
+                for (int j = 0; j < 8; ++j) o[j] = __hmul(__float2half_rn(f[j] * rstd[m]), wh[j]);
+                x[m][v] = *reinterpret_cast<const uint4*>(o);
+                *reinterpret_cast<uint4*>(&row[m][i]) = x[m][v];
             }
         }
     }
-    __syncthreads();
-    const __half* cos = p.rope_cos + pos * 128;
-    const __half* sin = p.rope_sin + pos * 128;
+    __syncwarp();  // the other half of a head is eight lanes away
+    float c[8], s[8];
+    unpack8_h(cos, c);
+    unpack8_h(sin, s);
+    const int away = d < 64 ? 64 : -64;
+    const float sign = d < 64 ? -1.f : 1.f;
 #pragma unroll
-    for (int v = 0; v < kRowVecs; ++v) {
+    for (int v = 0; v < VECS; ++v) {
         const int i = 8 * (tid + kRowThreads * v);
         if (i < A) {
-            const int d = i & 127, other = d < 64 ? i + 64 : i - 64;
-            const float sign = d < 64 ? -1.f : 1.f;
-            float c[8], s[8];
-            unpack8_h(__ldg(reinterpret_cast<const uint4*>(cos + d)), c);
-            unpack8_h(__ldg(reinterpret_cast<const uint4*>(sin + d)), s);
             const int64_t row_at = (INT8 ? t * p.heads + (i >> 7) : static_cast<int64_t>(i >> 7)) * p.S + pos, slot = row_at * 128 + d;
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 float a[8], b[8];
-                unpack8_h(*reinterpret_cast<const uint4*>(&row[m][i]), a);
-                unpack8_h(*reinterpret_cast<const uint4*>(&row[m][other]), b);
+                unpack8_h(x[m][v], a);
+                unpack8_h(*reinterpret_cast<const uint4*>(&row[m][i + away]), b);
                 __align__(16) __half o[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) o[j] = __float2half_rn(__fadd_rn(__fmul_rn(a[j], c[j]), __fmul_rn(sign * b[j], s[j])));
@@ -189,11 +257,10 @@ __global__ void __launch_bounds__(kRowThreads) qkv_rows_kernel(const QkvRows p) 
                     *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
                 }
             }
-            const uint4 v4 = ld_cg16(src + 2 * A + i);
             if (INT8)
-                quantise_head_store(reinterpret_cast<const __half*>(&v4), p.vc + slot, p.vs + row_at, d == 0);
+                quantise_head_store(reinterpret_cast<const __half*>(&x[2][v]), p.vc + slot, p.vs + row_at, d == 0);
             else
-                *reinterpret_cast<uint4*>(p.values + slot) = v4;
+                *reinterpret_cast<uint4*>(p.values + slot) = x[2][v];
         }
     }
 }
@@ -470,7 +537,8 @@ __global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const ID* __res
 // Rows into expert order after norm_route, whose blocks left the pairs of every expert among their 16 tokens (`counts`) and the place of a
 // pair among those (`rank`): a block sums the counts of all blocks and of those before its tokens', which gives the first row of every
 // expert and of its own tokens in it, and writes each of its rows `K` times.  Bounded by those writes.  Us of this kernel / of a counting sort by a
-// block per expert and a gather by a block per pair: see launch_place_rows.
+// block per expert and a gather by a block per pair,
+// alone: 5.3 / 5.5 at 61 tokens, 12 / 23 at 1024, 39 / 77 at 4096.
 constexpr int kPlaceThreads = 256;
 __global__ void __launch_bounds__(kPlaceThreads) place_rows_kernel(const int32_t* __restrict__ top_i, const int32_t* __restrict__ rank, const int32_t* __restrict__ counts,
                                                                    int T, int K, int E, const __half* __restrict__ h, int H, int per_block, int32_t* __restrict__ place,
@@ -597,12 +665,13 @@ int launch_embed_norm(const int64_t* tokens, const __half* embed, int64_t vocab,
 
 int launch_combine_norm(const __half* y, const int32_t* place, const float* top_w, int T, int K, const __half* x1, int H, const __half* w, float eps, __half* x2,
                         __half* h, const LaunchCfg& lc) {
-    return launch_kernel(combine_norm_kernel, dim3(T), dim3(kRowThreads), 0, lc, y, place, top_w, K, x1, H, w, eps, x2, h);
+    return launch_kernel(H <= 8 * kRowThreads ? combine_norm_kernel<1> : combine_norm_kernel<2>, dim3(T), dim3(kRowThreads), 0, lc, y, place, top_w, K, x1, H, w, eps, x2, h);
 }
 
 int launch_qkv_rows(const QkvRows& p, const LaunchCfg& lc) {
-    return p.kc ? launch_kernel(qkv_rows_kernel<true>, dim3(p.T), dim3(kRowThreads), 0, lc, p)
-                : launch_kernel(qkv_rows_kernel<false>, dim3(p.T), dim3(kRowThreads), 0, lc, p);
+    const bool one = p.heads * 128 <= 8 * kRowThreads;
+    auto* kernel = p.kc ? (one ? qkv_rows_kernel<true, 1> : qkv_rows_kernel<true, 2>) : (one ? qkv_rows_kernel<false, 1> : qkv_rows_kernel<false, 2>);
+    return launch_kernel(kernel, dim3(p.T), dim3(kRowThreads), 0, lc, p);
 }
 
 int launch_norm_route(const __half* x, const __half* norm_w, float eps, const __half* router, int T, int H, int E, int top_k, int norm, __half* h, float* top_w,
@@ -618,12 +687,12 @@ int launch_norm_route(const __half* x, const __half* norm_w, float eps, const __
     return E <= 64 ? run(norm_route_kernel<8, 16>) : run(norm_route_kernel<16, 16>);
 }
 
-// Tokens of a block: enough blocks for the chip, and no more than that, because each of them reads all counts.  With more tokens than kPlaceTokens
+// Tokens of a block: up to eight blocks an SM, and no more than that, because each of them reads all counts.  With more tokens than kPlaceTokens
 // those reads (a block 256 bytes for 16 tokens, and one block for 16) outgrow the copies.
 int launch_place_rows(const int32_t* top_i, const int32_t* rank, const int32_t* counts, int T, int K, int E, const __half* h, int H, int32_t* place, int32_t* seg,
                       __half* x_sorted, const LaunchCfg& lc) {
     int per = 1;
-    while (per < kRouteTokens && T / per > 8 * sm_count() / 2) per *= 2;
+    while (per < kRouteTokens && T / per > 8 * sm_count()) per *= 2;
     return launch_kernel(place_rows_kernel, dim3((T + per - 1) / per), dim3(kPlaceThreads), 0, lc, top_i, rank, counts, T, K, E, h, H, per, place, seg, x_sorted);
 }
 
