@@ -404,7 +404,7 @@ struct Smem {
     __align__(128) unsigned char ring[kStreamWarps * kStageBytes];
     __align__(8) unsigned long long full_bars[kStreamWarps];   // a tile has landed in the stage
     __align__(8) unsigned long long empty_bars[kStreamWarps];  // the consumer is done with the stage
-    volatile int ready_layer;                                  // the routing of layers <= this is in route_id
+    volatile uint32_t route[32];                               // a layer's routed experts: {layer + 1, id} in 16 bits each
     __align__(128) unsigned char xplanes[kXPlaneBytes];
     __align__(16) float xsx[16];
     __align__(128) unsigned char xh[4 * (1024 + kPad)];  // fp16 copy of the normalised vector, in quarters (router rows)
@@ -413,7 +413,6 @@ struct Smem {
     __half xres[kPartFloats];  // residual stream, the rows of this block's o_proj and down tiles (the same rows): row j * 8 + r
     float red[64];
     float cs[2 * kHeadDim];
-    int route_id[32];
     float route_w[32];
     Geo geo;
     StepLayer layers[kMaxLayers];
@@ -443,11 +442,11 @@ __device__ __forceinline__ TileSource weight_tile(const Smem& S, const Geo& geo,
         const int j = udiv_small(lt, geo.f_magic), pp = lt - j * geo.ftiles;
         const uint32_t first = (geo.b + j * geo.G) * 8;
         const int slot = geo.fpair ? 2 * pp : pp;
-        const size_t r0 = static_cast<size_t>(S.route_id[slot]) * geo.H + first;
+        const size_t r0 = static_cast<size_t>(S.route[slot] & 0xffffu) * geo.H + first;
         w.codes[0] = reinterpret_cast<const char*>(L.dn_codes) + r0 * K;
         w.scales[0] = reinterpret_cast<const char*>(L.dn_scale) + r0 * sb;
         if (geo.fpair && slot + 1 < geo.K) {
-            const size_t r1 = static_cast<size_t>(S.route_id[slot + 1]) * geo.H + first;
+            const size_t r1 = static_cast<size_t>(S.route[slot + 1] & 0xffffu) * geo.H + first;
             w.codes[1] = reinterpret_cast<const char*>(L.dn_codes) + r1 * K;
             w.scales[1] = reinterpret_cast<const char*>(L.dn_scale) + r1 * sb;
             w.pairs = w.scale_runs = 2;
@@ -461,7 +460,7 @@ __device__ __forceinline__ TileSource weight_tile(const Smem& S, const Geo& geo,
     if (kind == KE) {  // 4 gate rows + 4 up rows of one routed expert
         const uint32_t K = geo.H, sb = (K >> 7) * 2;
         const int slot = tg >> geo.shF4, n0 = (tg - (slot << geo.shF4)) * 4;
-        const size_t row = static_cast<size_t>(S.route_id[slot]) * 2 * geo.F + n0;
+        const size_t row = static_cast<size_t>(S.route[slot] & 0xffffu) * 2 * geo.F + n0;
         w.codes[0] = reinterpret_cast<const char*>(L.gu_codes) + row * K;
         w.scales[0] = reinterpret_cast<const char*>(L.gu_scale) + row * sb;
         w.scales[1] = w.scales[0] + static_cast<size_t>(geo.F) * sb;
@@ -569,18 +568,19 @@ __device__ __forceinline__ void producer_loop(Smem& S, int* err_flag, int first_
     while (ok && (c.kind != KEND || other.kind != KEND)) {
         if (c.kind != KEND) {
             if (c.kind >= KE) {
-                // expert tiles: the routing of the layer must be known.  (A word and not a barrier: a producer need not have
-                // tiles in every layer, so it may come two phases late.  Asleep between looks: looking all the time costs the
-                // consumer warps of the block 2 % of the step.)
+                // expert tiles: the routed expert must be known (down tiles: all of them; they come in order).  (Words and not a barrier: a
+                // producer need not have tiles in every layer, so it may come two phases late.  Asleep between looks: looking all
+                // the time costs the consumer warps of the block 2 % of the step.  With one
+                // word for the whole choice, announced after it, the phase took 1.5 us longer.)
+                const int slot = c.kind == KE ? (geo.b + c.lt * geo.G) >> geo.shF4 : geo.K - 1;
                 uint32_t n = 0;
-                while (S.ready_layer < c.layer) {
+                while (S.route[slot] >> 16 != static_cast<uint32_t>(c.layer + 1)) {
                     __nanosleep(64);
                     if (++n > (1u << 22)) {
                         ok = false;
                         break;
                     }
                 }
-                __threadfence_block();
             }
             if (ok && used > 0) ok = mbar_wait(smem_u32(&S.empty_bars[stage]), (used - 1) & 1u);
             if (!ok) break;
@@ -618,7 +618,7 @@ __device__ __forceinline__ void stage_release(uint32_t empty_bar) {
 // ---------------------------------------------------------------------------------------------
 template <int PER>  // experts per lane: 2 for E <= 64, 4 for E <= 128
 __device__ __forceinline__ void warp_topk_per(const unsigned long long* logits, uint32_t tag, int* err_flag, int E, int K, bool norm,
-                                              int lane, int& id_reg, float& w_reg) {
+                                              int lane, int& id_reg, float& w_reg, volatile uint32_t* route, uint32_t mark) {
     float v[PER];
     float mx = -INFINITY;
     {
@@ -675,6 +675,7 @@ __device__ __forceinline__ void warp_topk_per(const unsigned long long* logits, 
             const unsigned int b = __ballot_sync(0xffffffffu, key[j] == top);
             if (b) bi = 32 * j + __ffs(b) - 1;
         }
+        if (lane == 0) route[k] = mark | static_cast<uint32_t>(bi);  // the producers may start this expert's tiles
         const float best = __uint_as_float(top - 1u);
         wsum += best;
         if (lane == k) {
@@ -691,9 +692,9 @@ __device__ __forceinline__ void warp_topk_per(const unsigned long long* logits, 
     w_reg = __half2float(__float2half_rn(w_reg));  // the routing weights are used in fp16
 }
 __device__ __noinline__ void warp_topk(const unsigned long long* logits, uint32_t tag, int* err_flag, int E, int K, bool norm, int lane,
-                                       int& id_reg, float& w_reg) {
-    if (E <= 64) warp_topk_per<2>(logits, tag, err_flag, E, K, norm, lane, id_reg, w_reg);
-    else warp_topk_per<4>(logits, tag, err_flag, E, K, norm, lane, id_reg, w_reg);
+                                       int& id_reg, float& w_reg, volatile uint32_t* route, uint32_t mark) {
+    if (E <= 64) warp_topk_per<2>(logits, tag, err_flag, E, K, norm, lane, id_reg, w_reg, route, mark);
+    else warp_topk_per<4>(logits, tag, err_flag, E, K, norm, lane, id_reg, w_reg, route, mark);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1226,7 +1227,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
             mbar_init(smem_u32(&S.empty_bars[st]), 1u);
         }
         mbar_fence_init();
-        S.ready_layer = -1;
+        for (int i = 0; i < 32; ++i) S.route[i] = 0u;
     }
     __syncthreads();  // the one barrier of all warps: from here on producers and consumers only meet at the stages
     if (warp >= kStreamWarps) {
@@ -1345,16 +1346,12 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                 if (warp == 0) {  // one warp routes, the others pick the result up from shared memory
                     int id;
                     float w;
-                    warp_topk(f_logits, tag, p.err_flag, p.E, p.K, p.norm_topk != 0, lane, id, w);
-                    S.route_id[lane] = id;
+                    warp_topk(f_logits, tag, p.err_flag, p.E, p.K, p.norm_topk != 0, lane, id, w, S.route, static_cast<uint32_t>(l + 1) << 16);
                     S.route_w[lane] = lane < p.K ? w : 0.f;
                     if (b == 0 && lane < p.K) {
                         p.top_i[static_cast<int64_t>(l) * p.K + lane] = id;
                         p.top_w[lane] = __float2half_rn(w);
                     }
-                    __threadfence_block();
-                    __syncwarp();  // the lanes may leave the top-k apart: lane 0 must not announce ids that others still hold
-                    if (lane == 0) S.ready_layer = l;  // the producers may start the expert tiles of this layer
                 }
                 consumer_sync();
             } else if (ph == 2) {
