@@ -423,6 +423,9 @@ __device__ __forceinline__ int udiv_small(int q, int magic) { return (q * magic)
 // ---------------------------------------------------------------------------------------------
 // per-warp tile stream
 // ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // Where tile (layer, kind, lt) of this block lies in memory.  Global tile index of local tile lt: b + lt * G (down
 // phase: row block b + j * G with the top_k routed experts as consecutive tiles).  An int8 weight tile is one or two
 // pairs of code runs (a run: four rows, adjacent in memory; the second run of a pair `run_step` bytes after the first)
@@ -519,6 +522,15 @@ __device__ __forceinline__ void issue_tile(const Smem& S, const Geo& geo, int la
     if (w.scale_runs == 2) bulk_g2s(stage + kScaleOff + w.scale_bytes, w.scales[1], w.scale_bytes, bar);
 }
 
+// The rows of an expert gate/up tile that goes through a stage in a later round, asked into L2 while the stage is in use.
+__device__ __forceinline__ void ask_tile(const Smem& S, const Geo& geo, int layer, int lt) {
+    const TileSource w = weight_tile(S, geo, S.layers[layer], KE, lt);
+    bulk_prefetch(w.codes[0], 4 * w.K);
+    bulk_prefetch(w.codes[0] + w.run_step, 4 * w.K);
+    bulk_prefetch(w.scales[0], w.scale_bytes);
+    bulk_prefetch(w.scales[1], w.scale_bytes);
+}
+
 // Place in the block's tile sequence of the tiles that go through one stage.  The tiles of a block form one
 // sequence over all phases of the step; tile q of the sequence goes through stage q mod 10 and is consumed by warp
 // q mod 10, so the stages that free up first in a phase take the tiles that are needed first in the next one.
@@ -552,6 +564,19 @@ struct Cursor {
     }
 };
 
+// Expert tiles: the routed expert must be known (down tiles: all of them; they come in order).  (Words and not a barrier: a
+// producer need not have tiles in every layer, so it may come two phases late.  Asleep between looks: looking all
+// the time costs the consumer warps of the block 2 % of the step.  With one word for the whole choice, announced after it, the phase took
+// 1.5 us longer.)
+__device__ __forceinline__ bool route_wait(const Smem& S, const Geo& geo, const Cursor& c) {
+    const int slot = c.kind == KE ? (geo.b + c.lt * geo.G) >> geo.shF4 : geo.K - 1;
+    for (uint32_t n = 0; S.route[slot] >> 16 != static_cast<uint32_t>(c.layer + 1); ++n) {
+        if (n > (1u << 22)) return false;
+        __nanosleep(32);
+    }
+    return true;
+}
+
 // One thread of a producer warp: fills the warp's two stages in sequence order for the whole step.  A stage is
 // refilled as soon as its consumer gives it back, whatever phase the consumers are in; only the expert tiles wait for
 // the routing of their layer.  Every wait is bounded: a producer that gives up raises the flag word and stops, and the
@@ -563,26 +588,24 @@ __device__ __forceinline__ void producer_loop(Smem& S, int* err_flag, int first_
     other.start(geo, first_stage + 1);
     int stage = first_stage;
     uint32_t used = 0, other_used = 0;  // fills of each stage so far
-    bool ok = true;
+    bool ok = true, asked = false, other_asked = false;  // the next tile of a stage has been asked into L2
 #pragma unroll 1
     while (ok && (c.kind != KEND || other.kind != KEND)) {
         if (c.kind != KEND) {
-            if (c.kind >= KE) {
-                // expert tiles: the routed expert must be known (down tiles: all of them; they come in order).  (Words and not a barrier: a
-                // producer need not have tiles in every layer, so it may come two phases late.  Asleep between looks: looking all
-                // the time costs the consumer warps of the block 2 % of the step.  With one
-                // word for the whole choice, announced after it, the phase took 1.5 us longer.)
-                const int slot = c.kind == KE ? (geo.b + c.lt * geo.G) >> geo.shF4 : geo.K - 1;
-                uint32_t n = 0;
-                while (S.route[slot] >> 16 != static_cast<uint32_t>(c.layer + 1)) {
-                    __nanosleep(64);
-                    if (++n > (1u << 22)) {
-                        ok = false;
-                        break;
-                    }
+            // A later round of a layer's expert tiles: asked into L2 as soon as the stage's tile of the round before has landed (earlier it
+            // would compete with the first round: 5.6 % of a step), for both stages before either is waited for.  (545 -> 538 us a step at 1024
+            // cached positions, with the stage waited for before the routing.)
+            if (c.kind == KE && c.lt >= kStreamWarps && !asked) {
+                ok = route_wait(S, geo, c);
+                if (ok && mbar_wait(smem_u32(&S.full_bars[stage]), (used - 1) & 1u)) ask_tile(S, geo, c.layer, c.lt);
+                if (other.kind == KE && other.lt >= kStreamWarps && other.layer == c.layer && !other_asked) {
+                    other_asked = true;
+                    if (ok && route_wait(S, geo, other) && mbar_wait(smem_u32(&S.full_bars[stage ^ 1]), (other_used - 1) & 1u)) ask_tile(S, geo, other.layer, other.lt);
                 }
             }
+            asked = false;
             if (ok && used > 0) ok = mbar_wait(smem_u32(&S.empty_bars[stage]), (used - 1) & 1u);
+            if (ok && c.kind >= KE) ok = route_wait(S, geo, c);
             if (!ok) break;
             issue_tile(S, geo, c.layer, c.kind, c.lt, smem_u32(S.ring) + static_cast<uint32_t>(stage) * kStageBytes, smem_u32(&S.full_bars[stage]));
             ++used;
@@ -595,6 +618,9 @@ __device__ __forceinline__ void producer_loop(Smem& S, int* err_flag, int first_
         const uint32_t n = used;
         used = other_used;
         other_used = n;
+        const bool a = asked;
+        asked = other_asked;
+        other_asked = a;
         stage ^= 1;
     }
     if (!ok && err_flag) atomicOr(err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
@@ -620,7 +646,7 @@ template <int PER>  // experts per lane: 2 for E <= 64, 4 for E <= 128
 __device__ __forceinline__ void warp_topk_per(const unsigned long long* logits, uint32_t tag, int* err_flag, int E, int K, bool norm,
                                               int lane, int& id_reg, float& w_reg, volatile uint32_t* route, uint32_t mark) {
     float v[PER];
-    float mx = -INFINITY;
+    int order = -0x8000;
     {
         uint32_t d[PER];
         bool on[PER];
@@ -645,10 +671,12 @@ __device__ __forceinline__ void warp_topk_per(const unsigned long long* logits, 
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             v[j] = on[j] ? __half2float(__ushort_as_half(static_cast<unsigned short>(d[j] & 0xffffu))) : -INFINITY;
-            mx = fmaxf(mx, v[j]);
+            const int h = static_cast<short>(d[j] & 0xffffu);  // fp16 bits, ordered as whole numbers
+            if (on[j]) order = max(order, h ^ ((h >> 31) & 0x7fff));
         }
     }
-    mx = warp_max(mx);
+    order = __reduce_max_sync(0xffffffffu, order);
+    const float mx = __half2float(__ushort_as_half(static_cast<unsigned short>(order ^ ((order >> 31) & 0x7fff))));
     float sum = 0.f;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
