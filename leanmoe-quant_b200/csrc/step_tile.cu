@@ -835,28 +835,31 @@ __device__ __forceinline__ void attention_prologue(const StepParams& p, const St
     if (warp == 0 || (geo.owner && warp < 3)) {
         const int A = geo.A, h = geo.h;
         // this lane's four values of the head's q (k, v) row: flagged words written by the q.k.v phase
+        uint2 wv = make_uint2(0u, 0u);  // asked for before the wait: they come from memory
+        if (warp < 2) wv = *reinterpret_cast<const uint2*>((warp == 0 ? L.q_norm : L.k_norm) + h * D + lane * 4);
         uint32_t d4[4];
         bool good = flag_wait4(fqkv + warp * A + h * D + lane * 4, tag, d4, p.err_flag);
         const uint2 raw = make_uint2((d4[0] & 0xffffu) | (d4[1] << 16), (d4[2] & 0xffffu) | (d4[3] << 16));
         const __half* rh = reinterpret_cast<const __half*>(&raw);
         float f[4];
         if (warp < 2) {
-            const uint2 wv = *reinterpret_cast<const uint2*>((warp == 0 ? L.q_norm : L.k_norm) + h * D + lane * 4);
             const __half* wh = reinterpret_cast<const __half*>(&wv);
-            // sum of squares of the whole q (k) row: one partial per block of the grid, added in a fixed order
+            // sum of squares of the whole q (k) row: one partial per block of the grid, added in a fixed order.  All in one look (four words
+            // a lane and a second look for the last twenty of 148 blocks took another trip to L2 a layer).
+            constexpr int kLook = 5;
             float s = 0.f;
 #pragma unroll 1
-            for (int b0 = 0; b0 < geo.G; b0 += 128) {
-                uint32_t d[4];
-                bool on[4];
+            for (int b0 = 0; b0 < geo.G; b0 += 32 * kLook) {
+                uint32_t d[kLook];
+                bool on[kLook];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) on[i] = b0 + lane + 32 * i < geo.G;
+                for (int i = 0; i < kLook; ++i) on[i] = b0 + lane + 32 * i < geo.G;
                 const uint32_t limit = c_flag_spin_limit;
 #pragma unroll 1
                 for (uint32_t it = 0; it < limit; ++it) {
                     bool ok = true;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < kLook; ++i) {
                         const unsigned long long w = on[i] ? flag_load(fstats + warp * 1024 + b0 + lane + 32 * i) : (static_cast<unsigned long long>(tag) << 32);
                         ok = ok && tag_reached(w, tag);
                         d[i] = static_cast<uint32_t>(w);
@@ -868,7 +871,7 @@ __device__ __forceinline__ void attention_prologue(const StepParams& p, const St
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s += on[i] ? __uint_as_float(d[i]) : 0.f;
+                for (int i = 0; i < kLook; ++i) s += on[i] ? __uint_as_float(d[i]) : 0.f;
             }
             __syncwarp();
             s = warp_sum(s);
@@ -1140,12 +1143,12 @@ __device__ __forceinline__ void attention_finish(const StepParams& p, Smem& S, u
     }
     if (tid < D) {
         float m = big;
-#pragma unroll 1
+#pragma unroll 4
         for (int j = 0; j < others; ++j) m = fmaxf(m, sm.other[j][D]);
         const float ref = m > -INFINITY ? m : 0.f;
         const float own = exp2f(big - ref);
         float num = a * own, den = l * own;
-#pragma unroll 1
+#pragma unroll 4
         for (int j = 0; j < others; ++j) {
             const float w = exp2f(sm.other[j][D] - ref);
             den = fmaf(sm.other[j][D + 1], w, den);
