@@ -13,7 +13,9 @@ DEV = "cuda"
 
 # nothing filled; one position; either side of a tile; a last tile of one position in a split of its own; more heads than two blocks per SM
 @pytest.mark.parametrize("heads,capacity,filled,splits", [(3, 40, 0, 1), (3, 40, 0, 4), (2, 40, 1, 3), (2, 200, 127, 2), (2, 200, 128, 2), (2, 200, 129, 2),
-                                                          (5, 700, 641, 19), (5, 700, 700, 6), (300, 300, 259, 4), (700, 131, 131, 1)])
+                                                          (5, 700, 641, 19), (5, 700, 700, 6), (300, 300, 259, 4), (700, 131, 131, 1),
+                                                          # as many splits as are merged in one trip, one more, more than a warp has lanes
+                                                          (2, 2600, 2560, 20), (2, 2700, 2561, 21), (3, 4300, 4225, 40)])
 def test_attn_i8_edges(heads, capacity, filled, splits):
     from lemoq import _cabi
 
