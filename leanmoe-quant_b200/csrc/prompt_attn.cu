@@ -1,6 +1,6 @@
 // Attention of a prompt over the fp16 cache: row t sees slots [0, pos[t]] (head_dim 128), tcgen05 for both products.
 //
-// One block = one head x 256 query rows, as two tiles of 128 that take turns: while the warpgroup of one tile is in its softmax,
+// One block = one head x 256 query rows (few blocks: 128), as two tiles of 128 that take turns: while the warpgroup of one tile is in its softmax,
 // the tensor pipe works for the other.  Per 128 cache slots and tile:
 //   S = Q K^T   A, B from shared memory, 128 x 128 fp32 in TMEM
 //   softmax     one thread per row, in base 2: its row in registers, maximum, exp2, fp16, back into TMEM over S
@@ -31,7 +31,7 @@ constexpr size_t kSmem = static_cast<size_t>(2 * kTile + 2 * kKvStages * kTile) 
 struct AttnShape {
     const int64_t* pos;
     __half* out;
-    int T, heads, S;
+    int T, heads, S, tiles;  // tiles: of a block, 1 or 2
     float scale_log2;
     int* err_flag;
 };
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_c
     auto p_full = [&](int i) { return bars + 8u * (11 + i); };
     auto o_full = [&](int i) { return bars + 8u * (13 + i); };
     const uint32_t drained = bars + 8u * 15;
-    const int head = blockIdx.y, t0 = (gridDim.x - 1 - blockIdx.x) * 2 * kRows;  // the last rows see most: they start first
+    const int head = blockIdx.y, t0 = (gridDim.x - 1 - blockIdx.x) * p.tiles * kRows;  // the last rows see most: they start first
     volatile int* abort = &s_abort;
 
     if (tid == 0) {
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_c
     pdl_wait();
     pdl_trigger();
     int my_pos = -1;  // rows behind the end see nothing
-    if (warp < 8 && t0 + tid < p.T) {
+    if (warp < 4 * p.tiles && t0 + tid < p.T) {
         const int64_t q = p.pos[t0 + tid];
         my_pos = static_cast<int>(q < 0 ? 0 : (q >= p.S ? p.S - 1 : q));
         atomicMax(&s_most[warp >> 2], my_pos);
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_attn_kernel(const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const int live = t0 + kRows < p.T ? 2 : 1;
+    const int live = p.tiles == 2 && t0 + kRows < p.T ? 2 : 1;
     const int steps = max(s_most[0], s_most[1]) / kSlots + 1;  // both tiles run over the same slots
 
     if (warp == 8) {
@@ -281,7 +281,10 @@ int launch_prompt_attn(const PromptAttn& a, const LaunchCfg& lc) {
     p.pos = a.pos; p.out = a.out; p.T = a.T; p.heads = a.heads; p.S = a.S;
     p.scale_log2 = a.scale * 1.4426950408889634f;
     p.err_flag = a.err_flag;
-    return launch_kernel(prompt_attn_kernel, dim3((a.T + 2 * kRows - 1) / (2 * kRows), a.heads), dim3(kThreads), kSmem, lc, map_q, map_k, map_v, p);
+    // One tile a block while every such block has an SM of its own: the pair shares the SM's exp2 unit, which is idle elsewhere (us of four layers of
+    // a prompt with two tiles a block / one: 512 tokens 965 / 945, 1024 1251 / 1237; 1500 tokens, 192 tiles, 1510 / 1530, 4096 3820 / 4100).
+    p.tiles = static_cast<int64_t>((a.T + kRows - 1) / kRows) * a.heads <= sm_count() ? 1 : 2;
+    return launch_kernel(prompt_attn_kernel, dim3((a.T + p.tiles * kRows - 1) / (p.tiles * kRows), a.heads), dim3(kThreads), kSmem, lc, map_q, map_k, map_v, p);
 }
 
 }  // namespace lemoq

@@ -289,7 +289,9 @@ def test_a_prompt_whose_operations_matter_goes_through_the_modules():
 @pytest.mark.parametrize("tokens,shape", [(t, {}) for t in (15, 16, 17, 610, 1201, 2405, 4800, 16390)] +
                          # rows shorter than a warp's stride and of more than 2048 values, one and 32 experts a token, 128 of them
                          [(17, dict(hidden=2048, experts=8, top_k=1)), (33, dict(hidden=1024, experts=128, top_k=32)),
-                          (20, dict(hidden=4096, experts=64, top_k=8)), (18, dict(hidden=4096, experts=128, top_k=8)), (5, dict(hidden=128, experts=40, top_k=3))])
+                          (20, dict(hidden=4096, experts=64, top_k=8)), (18, dict(hidden=4096, experts=128, top_k=8)), (5, dict(hidden=128, experts=40, top_k=3)),
+                          # more heads and tiles of 128 queries than SMs: two tiles a block of the attention, the last one ragged
+                          (650, dict(hidden=4096, experts=8, top_k=1))])
 def test_rows_of_a_prompt_reach_their_experts(tokens, shape):
     """The native prompt against the same prompt through the modules (which a hook asks for)."""
     from benchmarks.cudagraph import StaticCacheDecodeSession
