@@ -536,9 +536,8 @@ __global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const ID* __res
 
 // Rows into expert order after norm_route, whose blocks left the pairs of every expert among their 16 tokens (`counts`) and the place of a
 // pair among those (`rank`): a block sums the counts of all blocks and of those before its tokens', which gives the first row of every
-// expert and of its own tokens in it, and writes each of its rows `K` times.  Bounded by those writes.  Us of this kernel / of a counting sort by a
-// block per expert and a gather by a block per pair,
-// alone: 5.3 / 5.5 at 61 tokens, 12 / 23 at 1024, 39 / 77 at 4096.
+// expert and of its own tokens in it, and writes each of its rows `K` times.  Bounded by those writes.  Us of this kernel / of a counting sort
+// by a block per expert and a gather by a block per pair, alone: 5.3 / 5.5 at 61 tokens, 12 / 23 at 1024, 39 / 77 at 4096.
 constexpr int kPlaceThreads = 256;
 __global__ void __launch_bounds__(kPlaceThreads) place_rows_kernel(const int32_t* __restrict__ top_i, const int32_t* __restrict__ rank, const int32_t* __restrict__ counts,
                                                                    int T, int K, int E, const __half* __restrict__ h, int H, int per_block, int32_t* __restrict__ place,

@@ -22,7 +22,7 @@
 // 1024 cached positions), and code beyond the first-level instruction cache runs at a third of the speed.  With the
 // barrier in every layer, fp32 partials read by all blocks and three copies of the tile product the step took 646 us.
 // Keeping the block's own residual rows in shared memory and inlining the attention code (its calls saved registers on the
-// stack) made 553 of the 568.
+// stack) made 553 of the 568; the expert tiles' earlier start (route_wait, ask_tile) and the attention's loads about 520 of the 553.
 //
 // Arithmetic: the activation vector of a phase is turned once per block into three planes of signed
 // 7-bit digits with one power-of-two scale per group of 128 (x = sx * (d2*2^14 + d1*2^7 + d0)).  The
