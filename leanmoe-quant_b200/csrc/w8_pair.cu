@@ -9,7 +9,8 @@
 //   warps 8-15   widen: thread = weight row and half of the group's codes; times the group's scale, rounded to fp16, into TMEM
 //   warp 17      of the even block: issues the MMAs (A from TMEM, B from shared memory, D in TMEM over all of k)
 //   warps 0-7    collect: the sums out of TMEM, finished, turned over in shared memory for 16-byte stores
-// TMEM: D in columns [0, 256) (tiles of at most 128 tokens take its halves in turn), A of stage s at 256 + 64 s.
+// TMEM: D in the first columns (256, or twice the most tokens of a tile if those are fewer than 128; tiles of up to 128 take its halves in
+// turn), behind it A of stage s at 64 s: with few tokens a tile there is room for up to six stages.
 //
 // What bounds it: large tiles the tensor pipe at the clock that the power cap leaves; tiles of 128 tokens and less the widening warps, 900 to 1000
 // cycles a group (neither more of them, nor two groups at once, nor fewer operations a code changed that).  One block per tile of 256
