@@ -173,3 +173,34 @@ def test_a_router_of_other_strides_is_laid_out(canonical):
     mlp = model.model.layers[1].mlp
     mlp._static_router = mlp._static_router.t().contiguous().t()
     assert form_blocker(model) is None and torch.equal(read_weights(model).layers[13 + 8], mlp._static_router)
+
+
+@pytest.mark.parametrize("tokens", [1, 3])
+@pytest.mark.parametrize("mode", ["fused", "separate"])
+@pytest.mark.parametrize("name", ["bias", "scale"])
+@pytest.mark.parametrize("kind", ["assigned", "parametrised"])
+def test_a_tensor_of_a_quant_linear_need_not_be_a_buffer(monkeypatch, kind, name, mode, tokens):
+    """A bias or scale assigned as a parameter (for tuning), or parametrised, is what the linear computes with, and its gradient is there."""
+    import lemoq.quant.rtn as rtn
+    from lemoq.quant.linear import QuantLinear, SchemeSpec
+
+    monkeypatch.setattr(rtn, "quantize_w8", lambda w, g=128: ops.rtn_quantize_w8(w.detach().float(), g))
+    torch.manual_seed(tokens)
+    linear = QuantLinear(torch.nn.Linear(128, 64), SchemeSpec.from_flags("w8a16", 128, dequant=mode))
+    codes, tensors = linear.packed.float(), {"scale": linear.scale.float(), "bias": linear.bias.float()}
+    if kind == "assigned":
+        setattr(linear, name, torch.nn.Parameter(2 * tensors[name]))
+    else:
+        class Twice(torch.nn.Module):
+            def forward(self, t):
+                return 2 * t.float()
+
+        torch.nn.utils.parametrize.register_parametrization(linear, name, Twice(), unsafe=True)
+    tensors[name] = 2 * tensors[name]
+    x = torch.randn(tokens, 128)
+    got = linear(x)
+    # fp32 throughout, the same weight: sums of 128 products in another order, 128 x 2^-24
+    assert torch.allclose(got, x @ (codes * tensors["scale"]).t() + tensors["bias"], rtol=1e-5, atol=1e-5)
+    if kind == "assigned":
+        got.sum().backward()
+        assert getattr(linear, name).grad.abs().sum() > 0
