@@ -53,6 +53,13 @@ def _plain(module: Any, forwards: tuple = ()) -> bool:
     return not (module._forward_hooks or module._forward_pre_hooks) and (own is None or getattr(own, "__func__", None) in forwards)
 
 
+def _w8(linear: Any) -> tuple[Any, Any] | None:
+    """Codes and scales of a W8 linear without bias that has them in the buffers it was built with, else None."""
+    own = linear._buffers if type(linear) is QuantLinear else {}
+    codes, scale = own.get("packed"), own.get("scale")
+    return (codes, scale) if own.get("bias", linear) is None and codes is not None and scale is not None else None
+
+
 def _read_layers(layers: list, group: int, eps: float, top_k: int, renormalised: bool) -> tuple[list, list, bool] | str:
     """(weights, linears, unwatched) of the decoder layers as ``Weights`` has them, or the reason why one description does not stand for them."""
     tensors, linears, unwatched = [], [], True
@@ -63,7 +70,8 @@ def _read_layers(layers: list, group: int, eps: float, top_k: int, renormalised:
         attn, mlp = parts["self_attn"], parts["mlp"]
         inner, here, moe = attn._modules, attn.__dict__, mlp.__dict__
         packed, o_proj, stacks = here.get("_lemoq_packed_qkv"), inner.get("o_proj"), moe.get("_static_experts")
-        if packed is None or type(o_proj) is not QuantLinear or o_proj._buffers["bias"] is not None:
+        o_own = _w8(o_proj)
+        if packed is None or o_own is None:
             return "layer %d: packed q/k/v not installed, or o_proj is not a W8 linear without bias" % i
         if not isinstance(stacks, QuantFusedExperts) or stacks.bits != 8 or moe["_static_act"] not in (None, F.silu):
             return "layer %d: experts are not W8 with SiLU" % i
@@ -83,7 +91,7 @@ def _read_layers(layers: list, group: int, eps: float, top_k: int, renormalised:
         unwatched = (unwatched and block_forward and _plain(layer) and _plain(attn, (_decode_forward_impl,)) and all(_plain(n, _NORM_FORWARDS) for n in norms)
                      and all(type(x) is QuantLinear and _plain(x) for x in mine))
         linears += mine
-        tensors += [*(norm._parameters["weight"] for norm in norms), packed.packed, packed.scale, o_proj._buffers["packed"], o_proj._buffers["scale"],
+        tensors += [*(norm._parameters["weight"] for norm in norms), packed.packed, packed.scale, *o_own,
                     moe["_static_router"].contiguous(), stacks.packed_gate_up, stacks.scale_gate_up, stacks.packed_down, stacks.scale_down]
     return tensors, linears, unwatched
 
@@ -94,7 +102,8 @@ def _read(model: Any) -> tuple[Weights | None, str | None]:
     cfg, m, lm = model.config, model._modules["model"], model._modules["lm_head"]
     parts = m._modules
     embed, norm, rotary, layers = parts["embed_tokens"], parts["norm"], parts["rotary_emb"], list(parts["layers"]._modules.values())
-    if type(lm) is not QuantLinear or lm._buffers["bias"] is not None:
+    lm_own = _w8(lm)
+    if lm_own is None:
         return None, "lm_head is not a W8 linear without bias"
     if cfg.clip_qkv is not None or not layers:
         return None, "clip_qkv is set, or there are no layers"
@@ -107,7 +116,7 @@ def _read(model: Any) -> tuple[Weights | None, str | None]:
     tensors, linears, unwatched = found
     unwatched = (unwatched and type(embed) is nn.Embedding and embed.max_norm is None and type(rotary) is OlmoeRotaryEmbedding
                  and _plain(lm) and _plain(embed) and _plain(rotary) and _plain(norm, _NORM_FORWARDS))
-    own = {"embed": embed._parameters["weight"], "final_norm": norm._parameters["weight"], "lm_head_codes": lm._buffers["packed"], "lm_head_scale": lm._buffers["scale"]}
+    own = {"embed": embed._parameters["weight"], "final_norm": norm._parameters["weight"], "lm_head_codes": lm_own[0], "lm_head_scale": lm_own[1]}
     return Weights(own, tensors, [lm, *linears], unwatched), None
 
 

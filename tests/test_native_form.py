@@ -175,6 +175,20 @@ def test_a_router_of_other_strides_is_laid_out(canonical):
     assert form_blocker(model) is None and torch.equal(read_weights(model).layers[13 + 8], mlp._static_router)
 
 
+@pytest.mark.parametrize("name", ["bias", "scale", "packed"])
+def test_a_linear_whose_tensors_are_no_buffers_goes_through_the_modules(canonical, name):
+    from lemoq.prompt import form_blocker, read_weights
+
+    model = canonical()
+    for linear in (model.lm_head, model.model.layers[1].self_attn.o_proj):
+        kept = getattr(linear, name)
+        setattr(linear, name, torch.nn.Parameter(torch.ones(64) if kept is None else kept.clone(), requires_grad=False))
+        assert read_weights(model) is None and "not a W8 linear without bias" in form_blocker(model)
+        delattr(linear, name)
+        linear.register_buffer(name, kept)
+    assert form_blocker(model) is None
+
+
 @pytest.mark.parametrize("tokens", [1, 3])
 @pytest.mark.parametrize("mode", ["fused", "separate"])
 @pytest.mark.parametrize("name", ["bias", "scale"])
