@@ -57,6 +57,7 @@
 #include <cstdlib>
 
 #include "step_kernel.h"
+#include "step_route.h"
 #include "stream.cuh"
 
 namespace lemoq {
@@ -404,7 +405,7 @@ struct Smem {
     __align__(128) unsigned char ring[kStreamWarps * kStageBytes];
     __align__(8) unsigned long long full_bars[kStreamWarps];   // a tile has landed in the stage
     __align__(8) unsigned long long empty_bars[kStreamWarps];  // the consumer is done with the stage
-    volatile uint32_t route[32];                               // a layer's routed experts: {layer + 1, id} in 16 bits each
+    volatile uint32_t route[32];                               // a layer's routed experts (step_route.h)
     __align__(128) unsigned char xplanes[kXPlaneBytes];
     __align__(16) float xsx[16];
     __align__(128) unsigned char xh[4 * (1024 + kPad)];  // fp16 copy of the normalised vector, in quarters (router rows)
@@ -444,12 +445,12 @@ __device__ __forceinline__ TileSource weight_tile(const Smem& S, const Geo& geo,
         const uint32_t K = geo.F, sb = (K >> 7) * 2;
         const int j = udiv_small(lt, geo.f_magic), pp = lt - j * geo.ftiles;
         const uint32_t first = (geo.b + j * geo.G) * 8;
-        const int slot = geo.fpair ? 2 * pp : pp;
-        const size_t r0 = static_cast<size_t>(S.route[slot] & 0xffffu) * geo.H + first;
+        const RouteSlots slots = slots_of_down(pp, geo.fpair != 0, geo.K);
+        const size_t r0 = static_cast<size_t>(route_expert(S.route[slots.first])) * geo.H + first;
         w.codes[0] = reinterpret_cast<const char*>(L.dn_codes) + r0 * K;
         w.scales[0] = reinterpret_cast<const char*>(L.dn_scale) + r0 * sb;
-        if (geo.fpair && slot + 1 < geo.K) {
-            const size_t r1 = static_cast<size_t>(S.route[slot + 1] & 0xffffu) * geo.H + first;
+        if (slots.count == 2) {
+            const size_t r1 = static_cast<size_t>(route_expert(S.route[slots.first + 1])) * geo.H + first;
             w.codes[1] = reinterpret_cast<const char*>(L.dn_codes) + r1 * K;
             w.scales[1] = reinterpret_cast<const char*>(L.dn_scale) + r1 * sb;
             w.pairs = w.scale_runs = 2;
@@ -462,8 +463,8 @@ __device__ __forceinline__ TileSource weight_tile(const Smem& S, const Geo& geo,
     const int tg = geo.b + lt * geo.G;
     if (kind == KE) {  // 4 gate rows + 4 up rows of one routed expert
         const uint32_t K = geo.H, sb = (K >> 7) * 2;
-        const int slot = tg >> geo.shF4, n0 = (tg - (slot << geo.shF4)) * 4;
-        const size_t row = static_cast<size_t>(S.route[slot] & 0xffffu) * 2 * geo.F + n0;
+        const int slot = slots_of_gate_up(tg, geo.shF4).first, n0 = (tg - (slot << geo.shF4)) * 4;
+        const size_t row = static_cast<size_t>(route_expert(S.route[slot])) * 2 * geo.F + n0;
         w.codes[0] = reinterpret_cast<const char*>(L.gu_codes) + row * K;
         w.scales[0] = reinterpret_cast<const char*>(L.gu_scale) + row * sb;
         w.scales[1] = w.scales[0] + static_cast<size_t>(geo.F) * sb;
@@ -564,13 +565,13 @@ struct Cursor {
     }
 };
 
-// Expert tiles: the routed expert must be known (down tiles: all of them; they come in order).  (Words and not a barrier: a
-// producer need not have tiles in every layer, so it may come two phases late.  Asleep between looks: looking all
-// the time costs the consumer warps of the block 2 % of the step.  With one word for the whole choice, announced after it, the phase took
-// 1.5 us longer.)
+// Expert tiles: every routed expert whose rows the tile holds must be known.  (Words and not a barrier: a producer need not have tiles in every
+// layer, so it may come two phases late.  Asleep between looks: looking all the time costs the consumer warps of the block 2 % of the step.  With
+// one word for the whole choice, announced after it, the phase took 1.5 us longer.)
 __device__ __forceinline__ bool route_wait(const Smem& S, const Geo& geo, const Cursor& c) {
-    const int slot = c.kind == KE ? (geo.b + c.lt * geo.G) >> geo.shF4 : geo.K - 1;
-    for (uint32_t n = 0; S.route[slot] >> 16 != static_cast<uint32_t>(c.layer + 1); ++n) {
+    const RouteSlots slots = c.kind == KE ? slots_of_gate_up(geo.b + c.lt * geo.G, geo.shF4)
+                                          : slots_of_down(c.lt - udiv_small(c.lt, geo.f_magic) * geo.ftiles, geo.fpair != 0, geo.K);
+    for (uint32_t n = 0; !route_known(S.route, c.layer, slots); ++n) {
         if (n > (1u << 22)) return false;
         __nanosleep(32);
     }
@@ -1377,7 +1378,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_tile_kernel(const __grid_con
                 if (warp == 0) {  // one warp routes, the others pick the result up from shared memory
                     int id;
                     float w;
-                    warp_topk(f_logits, tag, p.err_flag, p.E, p.K, p.norm_topk != 0, lane, id, w, S.route, static_cast<uint32_t>(l + 1) << 16);
+                    warp_topk(f_logits, tag, p.err_flag, p.E, p.K, p.norm_topk != 0, lane, id, w, S.route, route_mark(l));
                     S.route_w[lane] = lane < p.K ? w : 0.f;
                     if (b == 0 && lane < p.K) {
                         p.top_i[static_cast<int64_t>(l) * p.K + lane] = id;

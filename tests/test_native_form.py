@@ -2,6 +2,8 @@
 
 from __future__ import annotations
 
+import os
+
 import pytest
 import torch
 
@@ -218,3 +220,41 @@ def test_a_tensor_of_a_quant_linear_need_not_be_a_buffer(monkeypatch, kind, name
     if kind == "assigned":
         got.sum().backward()
         assert getattr(linear, name).grad.abs().sum() > 0
+
+
+def test_an_expert_tile_waits_for_every_word_it_reads(tmp_path):
+    """The routing words of the whole-step kernel may become visible in any order: whatever words have come, a tile is taken up only when each of
+    its own carries the layer's mark, and the tiles of a layer hold every slot once."""
+    import ctypes
+    import subprocess
+
+    from conftest import PKG
+
+    source, lib = tmp_path / "route.cpp", tmp_path / "route.so"
+    source.write_text("""#include "step_route.h"
+    using namespace lemoq::tile;
+    extern "C" int slots(int down, int tile, int shift, int paired, int top_k, int* count) {
+        const RouteSlots s = down ? slots_of_down(tile, paired, top_k) : slots_of_gate_up(tile, shift);
+        *count = s.count;
+        return s.first;
+    }
+    extern "C" int known(const uint32_t* route, int layer, int first, int count) { return route_known(route, layer, RouteSlots{first, count}); }
+    extern "C" uint32_t word(int layer, int expert) { return route_mark(layer) | static_cast<uint32_t>(expert); }
+    extern "C" uint32_t expert(uint32_t word) { return route_expert(word); }
+    """)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(PKG, "csrc"), str(source), "-o", str(lib)], check=True)
+    native, layer = ctypes.CDLL(str(lib)), 31
+    assert native.expert(native.word(layer, 127)) == 127
+    for down, paired, top_k in [(0, 0, 4), *((1, p, k) for p in (0, 1) for k in (1, 2, 5, 8))]:
+        tiles = 4 * top_k if not down else -(-top_k // 2) if paired else top_k
+        held = []
+        for tile in range(tiles):
+            count = ctypes.c_int()
+            first = native.slots(down, tile, 2, paired, top_k, ctypes.byref(count))
+            own = set(range(first, first + count.value))
+            held += own
+            for come in range(1 << top_k):  # the words of this layer that can be seen; the others still hold the layer before's
+                words = [native.word(layer if come >> k & 1 else layer - 1, k) for k in range(top_k)]
+                ready = native.known((ctypes.c_uint32 * 32)(*words), layer, first, count.value)
+                assert bool(ready) == all(come >> k & 1 for k in own), (down, paired, top_k, tile, come)
+        assert sorted(held) == sorted(list(range(top_k)) * (1 if down else 4))
