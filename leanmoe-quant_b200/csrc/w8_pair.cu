@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                 const __half scale = sc.next(p, g);
                 // the stage was refilled when its last MMAs were over: its A buffer is free
                 if (!(ok = warp_wait(full(s), ph, abort))) break;
+                tc_fence_after();
                 const uint32_t from = from0 + static_cast<uint32_t>(s) * stage_bytes, to = to0 + 64u * s;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {

@@ -62,6 +62,26 @@ def test_segments(counts):
     assert rel_err(_run(x, codes, scale, 128, seg=seg, gate_up=True), _swiglu(ref)) < 2 * PER_KERNEL_REL_TOL
 
 
+# counts repeated: tiles of up to 160 tokens, some of more than 128 (all of the accumulator's columns) between some of fewer (a half in turn), and tiles
+# of up to 96, all in halves; several tiles and more groups than stages a pair; rows: off 32, and gate/up rows off eight and off 32
+@pytest.mark.parametrize("counts,k", [((20, 160, 130, 40, 97, 170), 640), ((20, 97, 60, 40), 896)])
+@pytest.mark.parametrize("n", [264, 1008])
+def test_accumulators_are_handed_over(counts, k, n):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    counts = counts * (1 + 2 * sms // (len(counts) * (n // 250)))  # four tiles a pair and more
+    codes, scale, w = _weights(n, k, 128, n, (len(counts),))
+    seg = torch.tensor(counts).cumsum(0).roll(1).tolist()
+    seg = torch.tensor([0, *seg[1:], seg[0]], dtype=torch.int32, device=DEV)
+    x = torch.randn(sum(counts), k, generator=torch.Generator().manual_seed(k)).half().to(DEV)
+    resid = torch.randn(sum(counts), n, generator=torch.Generator().manual_seed(n)).half().to(DEV)
+    refs = [part.double() @ w[e].double().T for e, part in enumerate(x.split(counts))]
+    for kind, tol in (({}, 1), ({"resid": resid}, 1), ({"gate_up": True}, 2)):
+        got = _run(x, codes, scale, 128, seg=seg, **kind).split(counts)
+        for e, ref in enumerate(refs):  # each expert by itself: a wrong tile is not lost among right ones
+            ref = _swiglu(ref) if "gate_up" in kind else ref.half() + resid[seg[e]: seg[e + 1]] if kind else ref
+            assert rel_err(got[e], ref) < tol * PER_KERNEL_REL_TOL, (kind, e, counts[e])
+
+
 def test_more_tiles_a_pair_than_are_looked_up_ahead():
     tokens = 256 * 66 * (torch.cuda.get_device_properties(0).multi_processor_count // 2) + 33
     codes, scale, w = _weights(2, 128, 128, 3)
