@@ -20,8 +20,11 @@
 // 300, 1024 and 4096 tokens 85 / 76, 112 / 89 and 267 / 228, down 50 / 47, 64 / 57 and 152 / 118; 2048 x 2048 by 300 and 1024 tokens 35 / 20 and
 // 37 / 25.
 //
-// Arrivals at the other block's barriers and waits for them carry no scope: what they order are TMEM and TMA, which have their own fences.  With
-// `.release.cluster` and `.acquire.cluster` every group waited for the memory system (4096 x 6144 x 2048: 168 us instead of 94).
+// Arrivals at the other block's barriers and waits for them are the instructions' default, release and acquire at the scope of a block: they order no
+// shared memory between the blocks.  What crosses over is of two other kinds.  TMEM (codes widened, sums taken out) is ordered by tcgen05's fences
+// before an arrival and after a wait.  The odd block's tokens are reported to the even block's barrier by the TMA itself, which counts their
+// bytes there (`x_full`).  (With `.release.cluster` and `.acquire.cluster` on the arrivals instead, every group waited for the memory system:
+// 4096 x 6144 x 2048 168 us, not 94.)
 #include "w8_tile.cuh"
 
 #include <algorithm>
@@ -66,6 +69,19 @@ __device__ __forceinline__ uint32_t at_even_block(uint32_t addr) {
     uint32_t there;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(there) : "r"(addr));
     return there;
+}
+// One arrival on a barrier of either block, which then waits for `bytes` of copies too.
+__device__ __forceinline__ void expect_tx_at(uint32_t cluster_bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_bar), "r"(bytes) : "memory");
+}
+// tma_load_2d into this block's shared memory, completing on a barrier of either block of the pair.
+__device__ __forceinline__ void tma_load_2d_at(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t cluster_bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+                 "l"(map), "r"(c0), "r"(c1), "r"(cluster_bar)
+                 : "memory");
+}
+__device__ __forceinline__ void store_at(uint32_t cluster_addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 // Of a converged warp, on a barrier of either block.
 __device__ __forceinline__ void warp_arrive_at(uint32_t cluster_bar) {
@@ -141,22 +157,25 @@ struct RowScales {
 __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                               const __grid_constant__ CUtensorMap map_x16, const W8Shape p) {
     extern __shared__ uint8_t raw[];
-    __shared__ __align__(8) uint64_t s_bar[3 * kStages + 5];
+    __shared__ __align__(8) uint64_t s_bar[4 * kStages + 5];
     __shared__ int4 s_list[kListed];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
+    __shared__ int s_issued;           // odd block: stages its TMA thread has filled, when that gave up ...
+    __shared__ volatile int s_copies;  // ... and even block: that number + 1
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage0 = (smem_u32(raw) + 1023u) & ~1023u;
     int* s_first = reinterpret_cast<int*>(raw + (stage0 - smem_u32(raw)) + kRing + kTurn);
     int* s_tok = s_first + p.E + 1;
     const uint32_t bars = smem_u32(s_bar);
-    auto full = [&](int s) { return bars + 8u * s; };                    // the stage's copies have landed
+    auto full = [&](int s) { return bars + 8u * s; };                    // the stage's copies have landed (odd block: its codes)
     auto done = [&](int s) { return bars + 8u * (kStages + s); };        // its MMAs are over: stage and A buffer are free
     auto a_full = [&](int s) { return bars + 8u * (2 * kStages + s); };  // even block: both blocks' codes are widened
     auto d_full = [&](int b) { return bars + 8u * (3 * kStages + b); };
     auto d_free = [&](int b) { return bars + 8u * (3 * kStages + 2 + b); };  // even block: both blocks have taken the sums out
     const uint32_t drained = bars + 8u * (3 * kStages + 4);
+    auto x_full = [&](int s) { return bars + 8u * (3 * kStages + 5 + s); };  // even block: the odd block's tokens have landed there
     const int rank = blockIdx.x & 1;
     // A stage: the block's codes, then its half of up to `cap` tokens as two halves of 64 k.  As many of them as there are A buffers
     // beside two accumulators of `twice` tokens.
@@ -164,8 +183,9 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
     const uint32_t half_bytes = 64u * p.cap, stage_bytes = kCodeBytes + 2u * half_bytes, col_a = p.cap > 128 ? 256u : 2u * p.cap;
 
     if (tid == 0) {
-        s_abort = 0;
+        s_abort = s_copies = 0;
         for (int s = 0; s < kStages; ++s) {
+            mbar_init(x_full(s), 1);
             mbar_init(full(s), 1);
             mbar_init(done(s), 1);
             mbar_init(a_full(s), 16);
@@ -228,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
             auto stage_at = [&](int k) { return stage0 + static_cast<uint32_t>(k) * stage_bytes; };
             auto half_of = [&](const Tile& x) { return (x.n + kUnit - 1) / kUnit * (kUnit / 2); };  // tokens of one block
             auto load_codes = [&](const Tile& x, int g, int k) {
-                mbar_expect_tx(full(k), kCodeBytes + 2u * half_of(x) * 128u);
+                mbar_expect_tx(full(k), kCodeBytes + (rank ? 0u : 2u * half_of(x) * 128u));
                 tma_load_2d(stage_at(k), &map_w, g * 128, x.e * p.N + x.row0, full(k));
                 tma_load_2d(stage_at(k) + kCodeBytes / 2, &map_w, g * 128, x.e * p.N + x.row1, full(k));
             };
@@ -245,11 +265,12 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                         if (!(ok = thread_wait(done(s), ph, abort))) break;
                         load_codes(t, g, s);
                     }
-                    const uint32_t at = stage_at(s) + kCodeBytes;
+                    const uint32_t at = stage_at(s) + kCodeBytes, landed = at_even_block(rank ? x_full(s) : full(s));
+                    if (rank) expect_tx_at(landed, 2u * half * 128u);
                     for (int b = 0; b < half; b += kBox) {
                         const CUtensorMap* map = half - b >= kBox ? &map_x : &map_x16;
-                        tma_load_2d(at + b * 128, map, g * 128, row + b, full(s));
-                        tma_load_2d(at + half_bytes + b * 128, map, g * 128 + 64, row + b, full(s));
+                        tma_load_2d_at(at + b * 128, map, g * 128, row + b, landed);
+                        tma_load_2d_at(at + half_bytes + b * 128, map, g * 128 + 64, row + b, landed);
                     }
                     ++issued;
                     if (++s == stages) { s = 0; ph ^= 1; }
@@ -262,6 +283,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
             if (!ok) {  // gave up: the copies in flight still land in this block's shared memory
                 for (int j = max(0, issued - stages); j < issued; ++j) mbar_wait(full(j % stages), (j / stages) & 1);
             }
+            s_issued = issued;
         }
     } else if (warp == 17 && rank == 0) {
         // ---- MMA: one thread of the pair -----------------------------------------------------------------------------
@@ -278,8 +300,8 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                 if (round > 0 && max(n, before) > twice && !(ok = thread_wait_pair(d_free(b ^ 1), ((round - 1) >> 1) & 1, abort))) break;
                 before = n;
                 for (int g = 0; g < groups; ++g) {
-                    // a widening warp has seen the stage's copies land before it arrives: no wait on full(s) here
-                    if (!(ok = thread_wait_pair(a_full(s), ph, abort))) break;
+                    // a widening warp has seen its block's copies land before it arrives: no wait on full(s) here
+                    if (!(ok = thread_wait_pair(x_full(s), ph, abort) && thread_wait_pair(a_full(s), ph, abort))) break;
                     tc_fence_after();
                     const uint64_t x0 = smem_desc_sw128(stage0 + static_cast<uint32_t>(s) * stage_bytes + kCodeBytes, 1024);
                     const uint32_t a = tmem + col_a + 64u * s;
@@ -442,8 +464,16 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
         }
     }
     __syncthreads();
-    if (tid == 0 && s_abort && p.err_flag) atomicOr(p.err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+    if (tid == 0 && s_abort) {
+        if (p.err_flag) atomicOr(p.err_flag, LEMOQ_FLAG_WAIT_TIMEOUT);
+        if (rank) store_at(at_even_block(smem_u32(const_cast<int*>(&s_copies))), s_issued + 1);
+    }
     cluster_sync();  // the other block's arrivals and MMAs are over
+    if (rank ? s_abort : s_copies) {  // the odd block gave up: it stays until the even block has seen its last tokens land
+        if (rank == 0 && tid == 0)
+            for (int j = max(0, s_copies - 1 - stages); j < s_copies - 1; ++j) mbar_wait(x_full(j % stages), (j / stages) & 1);
+        cluster_sync();
+    }
     if (warp == 17) {
         tc_fence_after();
         tmem_free_pair(tmem);
