@@ -16,6 +16,7 @@
 #include <cmath>
 #include <initializer_list>
 #include <map>
+#include <set>
 #include <tuple>
 #include <vector>
 
@@ -91,6 +92,12 @@ void* attn_scratch(int device, const c10::cuda::CUDAStream& stream, int64_t head
     return at->second.data_ptr();
 }
 
+// The first call of a shape goes the Python way, which makes the workspace that captures of the shape take (they take none from here).
+bool first_of_shape(int device, int64_t heads, int64_t dim, int splits) {
+    static auto* seen = new std::set<std::tuple<int, int64_t, int64_t, int>>;
+    return seen->emplace(device, heads, dim, splits).second;
+}
+
 // attention(q, k, ks | None, v, vs | None, filled, scale | None): the default split count, as resolve_num_splits gives it
 PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 7 || !on_cuda(args[0])) return none();
@@ -122,6 +129,7 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return none();
     const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     const int splits = static_cast<int>(std::min<int64_t>(64, std::max<int64_t>(1, (2 * sms + heads - 1) / heads)));
+    if (first_of_shape(device, heads, dim, splits)) return none();
     at::Tensor out = fp16({1, heads, 1, dim}, device);
     void* ws = attn_scratch(device, stream, heads, dim, splits);
     const int S = static_cast<int>(capacity), H = static_cast<int>(heads), D = static_cast<int>(dim);

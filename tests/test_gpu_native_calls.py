@@ -138,3 +138,34 @@ def test_quant_linear_where_the_operation_itself_matters(way, tokens, bias):
         got, ref = (way(kind(dense, SchemeSpec.from_flags("w8a16", 128, dequant="fused")), x) for kind in (QuantLinear, Rebuilt))
     assert type(got) is type(ref) and got.dtype == ref.dtype and got.shape == ref.shape
     assert rel_err(got, ref) < (PER_KERNEL_REL_TOL if ref.dtype != torch.bfloat16 else 8 * PER_KERNEL_REL_TOL)
+
+
+@pytest.mark.parametrize("int8", [True, False])
+@pytest.mark.parametrize("before,heads", [("warm", 5), ("call", 6), ("nothing", 7)])
+def test_attention_is_captured_after_a_call_of_its_shape(before, heads, int8):
+    """``warm()`` or an ordinary call leaves the workspace that a capture needs; without either a capture is refused."""
+    from lemoq.kernels.attn_decode import attn_decode_forward, attn_decode_forward_int8, warm
+    from lemoq.kernels.kv_int8 import kv_int8_bulk_quantize
+
+    heads += 20 * int8  # a shape of its own for every case
+    g = torch.Generator(DEV).manual_seed(heads)
+    q, k, v = (torch.randn(1, heads, n, 128, device=DEV, generator=g).half() for n in (1, 96, 96))
+    filled = torch.tensor([70], dtype=torch.int32, device=DEV)
+    cache = kv_int8_bulk_quantize(k, v)
+    call = (lambda: attn_decode_forward_int8(q, cache["kc"], cache["ks"], cache["vc"], cache["vs"], filled)) if int8 else lambda: attn_decode_forward(q, k, v, filled)
+    if before == "warm":
+        warm(heads=heads, head_dim=128, kv_len=96)
+    elif before == "call":
+        call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    if before == "nothing":
+        with pytest.raises(RuntimeError, match="before capture"), torch.cuda.graph(graph):
+            call()
+        return
+    with torch.cuda.graph(graph):
+        out = call()
+    for _ in range(2):
+        graph.replay()
+        assert torch.equal(out, call())
+        q.neg_()
