@@ -123,7 +123,8 @@ __device__ void softmax_topk_warp(const float* __restrict__ logit_s, int E, int 
     }
     sum = warp_sum(sum);
     __syncwarp();
-    for (int e = lane; e < E; e += 32) scratch[e] = scratch[e] / sum;
+    const bool number = sum == sum;  // else (a logit that is not a number, or an infinite one) no probability is: the first experts, and weights that are none either
+    for (int e = lane; e < E; e += 32) scratch[e] = number ? scratch[e] / sum : 0.f;
     __syncwarp();
     float wsum = 0.f;
     for (int k = 0; k < top_k; ++k) {
@@ -147,7 +148,7 @@ __device__ void softmax_topk_warp(const float* __restrict__ logit_s, int E, int 
         }
         wsum += best;
         if (lane == 0) {
-            w_out[k] = best;
+            w_out[k] = number ? best : sum;
             i_out[k] = bi;
             scratch[bi] = -1.0e30f;
         }

@@ -294,6 +294,28 @@ def test_routing_golden_and_boundaries(ops_golden):
     assert e0.shape == (0, 8) and i0.shape == (0, 8)
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_logits_that_order_nothing_are_sent_to_valid_experts(value, norm, dtype):
+    """The softmax of a row with a NaN, with an infinity or of nothing but -infinity has no numbers: its weights are NaN, its experts are distinct and
+    inside the range; the rows beside it are what they are without it."""
+    from lemoq.kernels.routing import routing_softmax_topk
+
+    for e, k in ((64, 8), (12, 3), (8, 8), (200, 6)):
+        logits = torch.randn(5, e, generator=torch.Generator().manual_seed(e)).to(dtype).to(DEV)
+        clean_w, clean_i = routing_softmax_topk(logits, top_k=k, norm_topk_prob=norm)
+        logits[1, e // 2] = logits[3, :] = value
+        some = not torch.softmax(logits[1].float(), dim=-1).isnan().any()  # one -infinity is an expert that is never taken while there are others
+        w, i = routing_softmax_topk(logits, top_k=k, norm_topk_prob=norm)
+        for row in (3,) if some else (1, 3):
+            assert bool(w[row].isnan().all()) and i[row].tolist() == list(range(k))
+        assert torch.equal(w[0::2], clean_w[0::2]) and torch.equal(i[0::2], clean_i[0::2])
+        if some:
+            ref_w, ref_i = ops.routing_softmax_topk(logits[1:2].cpu(), k, norm)
+            assert torch.equal(i[1:2].cpu(), ref_i) and torch.allclose(w[1:2].cpu(), ref_w, atol=1e-6)
+
+
 def test_route_linear_plus_topk_matches_oracle():
     """The fused router kernel of the step engine (linear + softmax + top-k) through the C-ABI."""
     from lemoq import _cabi
