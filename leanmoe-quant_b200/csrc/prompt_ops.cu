@@ -405,11 +405,11 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
             }
         }
         sum = warp_sum(sum);
-        int key[PER];  // order of the probabilities; -1 taken, no expert, or not a number
+        int key[PER];  // order of the probabilities; -1 taken or no expert.  If one is not a number, none is: the first experts, and weights that are none either
 #pragma unroll
         for (int i = 0; i < PER; ++i) {
             const float v = p[i] / sum;
-            key[i] = lane + 32 * i < E && v >= 0.f ? __float_as_int(v) : -1;
+            key[i] = lane + 32 * i < E ? (v >= 0.f ? __float_as_int(v) : 0x7fffffff) : -1;
         }
         float kept = 0.f, wsum = 0.f;
         int kept_i = 0;
@@ -422,9 +422,8 @@ __global__ void __launch_bounds__(kRouteWarps * 32) norm_route_kernel(const __ha
 #pragma unroll
             for (int i = PER - 1; i >= 0; --i)
                 if (key[i] == top) first = lane + 32 * i;
-            int bi = static_cast<int>(__reduce_min_sync(0xffffffffu, first));
-            if (top < 0) bi = 0;  // only with NaN logits: any valid expert
-            const float best = top < 0 ? -1.f : __int_as_float(top);
+            const int bi = static_cast<int>(__reduce_min_sync(0xffffffffu, first));  // (there is one: top_k <= E)
+            const float best = __int_as_float(top);
             wsum += best;
             if (lane == k) {
                 kept = best;

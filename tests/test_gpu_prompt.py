@@ -357,3 +357,15 @@ def test_of_equal_logits_the_lowest_expert_is_taken(tokens, alike):
     clear = kept[:, -2] - kept[:, -1] > 2 ** -8 * logits.abs().amax(dim=-1) if alike > 1 else torch.ones(tokens, dtype=torch.bool, device=DEV)
     assert clear.float().mean() > 0.5 and float(_row_tol(logits).max()) < 0.05
     assert bool((_row_errors(native, by_modules) < _row_tol(logits))[clear].all())
+
+
+def test_a_token_whose_router_logits_overflow_keeps_to_its_row():
+    """Their softmax has no numbers: the token's own row has none either, and the tokens before it get what they get without it."""
+    rows = []
+    for last in (0, 511):
+        def change(wf, prompt):  # only token 511 has a first value, and hardly another one; it goes to expert 3 with more than fp16 holds
+            wf.embed[:, 0] = wf.embed[511] = wf.layers[0].o_w[0] = wf.layers[0].router[:, 0] = 0
+            wf.embed[511, 0], wf.layers[0].router[3, 0], prompt[0, -1] = 20, 60000, last
+
+        rows.append(_routed_session(77, {}, change)[0].prefill().logits[0])
+    assert bool(rows[0].isfinite().all()) and torch.equal(rows[0][:-1], rows[1][:-1]) and bool(rows[1][-1].isnan().all())
