@@ -75,7 +75,9 @@ struct Cursor {
 };
 
 // Dimension tid of a head from its splits (maximum, sum, values), in split order.  Everything of the first kMerge comes in one trip to L2, a
-// maximum and a sum in a lane each: 12.2 -> 10.3 us at 16 heads x 4097 positions, 10.3 -> 9 at 2049.  (A function of its own: inlined, its
+// maximum and a sum in a lane each.  Us a call without / with it, mean of 20 calls in a graph on the same cache (on caches from memory): 16 heads x 1025
+// positions 7.7 / 6.9 (8.4 / 7.5), 2049 8.4 / 7.4 (9.9 / 8.9), 4097 in 19 splits 9.5 / 8.5 (11.2 / 10.2); 8 heads x 4097 in 37 splits, seventeen of
+// them one after the other, 10.1 / 9.4 (11.6 / 10.8); 256 to 1024 heads, which have no splits, the same.  (A function of its own: inlined, its
 // registers made the tiles' loop slower, 1.5 us a layer of a lockstep step of five sequences.)
 __device__ __noinline__ float merged(const float* parts, int splits, int tid) {
     const int lane = tid & 31;

@@ -467,8 +467,9 @@ __device__ __forceinline__ int expert_of(const ID* __restrict__ ids, int p, int 
 
 // One block per expert: counts the pairs of lower experts, then gives its own pairs their rows in pair order.  GATHER: it also copies
 // the activations of its pairs, up to kGatherPairs of them in all: a launch less, but an expert with many pairs is one block's work.
-// Us of a layer of a prompt with the gather in a kernel of its own / in here: 128 pairs 123.7 / 124.0, 256 139.5 / 142, 512 155.6 / 157.8,
-// 768 186.7 / 192.1, 1024 191.6 / 199.4, 2048 226 / 241, 4096 235 / 261: even at 128 pairs and behind from 256 on.
+// Us of a call of the experts' block (64 experts, 8 a token) with the gather in here / in a kernel of its own: 16 pairs 32.4 / 33.0, 32 49.4 / 50.5,
+// 64 66.5 / 67.7, 128 77.3 / 78.0, 256 to 1024 the same within what two runs of one side differ by.  The pairs of very many tokens of a prompt,
+// which are plain int32 ids, are always above the line.
 constexpr int kGatherPairs = 1024;
 template <typename ID, bool GATHER>
 __global__ void __launch_bounds__(kPlanThreads) pair_plan_kernel(const ID* __restrict__ top_i, int P, int E, int32_t* __restrict__ place,

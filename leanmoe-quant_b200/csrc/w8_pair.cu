@@ -13,7 +13,7 @@
 // turn), behind it A of stage s at 64 s: with few tokens a tile there is room for up to six stages.
 //
 // What bounds it: large tiles the tensor pipe at the clock that the power cap leaves; tiles of 128 tokens and less the widening warps, 900 to 1000
-// cycles a group (neither more of them, nor two groups at once, nor fewer operations a code changed that).  One block per tile of 256
+// cycles a group (neither more of them, nor each half of them on groups of its own in turn, nor fewer operations a code changed that).  One block per tile of 256
 // rows x 128 tokens (the form before) moved 160 KB through shared memory per 1024 cycles of MMAs (TMA writes, code reads, token reads by the
 // MMAs), more than its 128 bytes a clock; a pair moves 96 KB a block, because a block holds half of the tokens only, and widens half as many
 // codes per product.  Us of that form / of this one: 50304 x 2048 by 1024 tokens 180 / 144, by 4096 720 / 575 (1.47 PFLOP/s); experts' gate/up at
@@ -87,23 +87,6 @@ __device__ __forceinline__ void store_at(uint32_t cluster_addr, uint32_t v) {
 __device__ __forceinline__ void warp_arrive_at(uint32_t cluster_bar) {
     __syncwarp();
     if (elect_one()) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-// Bounded wait of one thread for arrivals from both blocks.
-__device__ __forceinline__ bool thread_wait_pair(uint32_t bar, uint32_t parity, volatile int* abort) {
-    for (uint32_t i = 0; i < kWaitLimit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if ((i & 1023u) == 1023u && *abort) return false;
-    }
-    *abort = 1;
-    return false;
 }
 // 16 lanes x 32 columns: lane l has rows l / 4 (r[4 j], r[4 j + 1]) and 8 + l / 4 (r[4 j + 2], r[4 j + 3]) at columns 8 j + 2 (l mod 4), + 1.
 __device__ __forceinline__ void tmem_ld_16x32(uint32_t (&r)[16], uint32_t addr) {
@@ -296,12 +279,12 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                 const int n = (t.n + kUnit - 1) / kUnit * kUnit, b = round & 1;
                 const uint32_t idesc = idesc_f16(256, n, false), d = tmem + (n <= twice ? static_cast<uint32_t>(twice * b) : 0u);
                 // the tile before the last one is out of TMEM, and where one of two neighbours takes both halves so is the last
-                if (!(ok = thread_wait_pair(d_free(b), ((round >> 1) & 1) ^ 1, abort))) break;
-                if (round > 0 && max(n, before) > twice && !(ok = thread_wait_pair(d_free(b ^ 1), ((round - 1) >> 1) & 1, abort))) break;
+                if (!(ok = thread_wait(d_free(b), ((round >> 1) & 1) ^ 1, abort))) break;
+                if (round > 0 && max(n, before) > twice && !(ok = thread_wait(d_free(b ^ 1), ((round - 1) >> 1) & 1, abort))) break;
                 before = n;
                 for (int g = 0; g < groups; ++g) {
                     // a widening warp has seen its block's copies land before it arrives: no wait on full(s) here
-                    if (!(ok = thread_wait_pair(x_full(s), ph, abort) && thread_wait_pair(a_full(s), ph, abort))) break;
+                    if (!(ok = thread_wait(x_full(s), ph, abort) && thread_wait(a_full(s), ph, abort))) break;
                     tc_fence_after();
                     const uint64_t x0 = smem_desc_sw128(stage0 + static_cast<uint32_t>(s) * stage_bytes + kCodeBytes, 1024);
                     const uint32_t a = tmem + col_a + 64u * s;
