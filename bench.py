@@ -230,7 +230,7 @@ def run_reference(args) -> int:
 # dram__bytes_read.sum + dram__bytes_write.sum of one step_tile_kernel launch, from one ncu capture of
 # `python bench.py --steps 4 --warmup 3 --no-cpu-baseline --no-sub-records` (summary under profiles/):
 # (ctx, layers) -> bytes.
-WHOLE_STEP_DRAM_TRAFFIC = {(1024, 16): 1269527296 + 4218624}
+WHOLE_STEP_DRAM_TRAFFIC = {(1024, 16): 1270131968 + 8408320}
 
 
 def time_dominant_kernel(model, peaks, iters: int = 20) -> dict:
