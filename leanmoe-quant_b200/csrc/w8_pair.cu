@@ -22,8 +22,10 @@
 //
 // Arrivals at the other block's barriers and waits for them are the instructions' default, release and acquire at the scope of a block: they order no
 // shared memory between the blocks.  What crosses over is of two other kinds.  TMEM (codes widened, sums taken out) is ordered by tcgen05's fences
-// before an arrival and after a wait.  The odd block's tokens are reported to the even block's barrier by the TMA itself, which counts their
-// bytes there (`x_full`).  (With `.release.cluster` and `.acquire.cluster` on the arrivals instead, every group waited for the memory system:
+// before an arrival and after a wait.  The odd block's tokens are reported to the even block by the TMA itself, which counts their bytes on that block's
+// `full`: its widening warps wait for them too, and tell the MMA thread.  Us of gate/up by 300 and 600 tokens and of a prompt of 300 (two layers): the odd
+// block's tokens on no barrier of the even block 62.5, 72.8 and 543; on `full` 63.0, 73.2 and 545; on one that the MMA thread waits for besides 64.8, 74.6 and 557,
+// on `a_full` the same.  (With `.release.cluster` and `.acquire.cluster` on the arrivals instead, every group waited for the memory system:
 // 4096 x 6144 x 2048 168 us, not 94.)
 #include "w8_tile.cuh"
 
@@ -69,10 +71,6 @@ __device__ __forceinline__ uint32_t at_even_block(uint32_t addr) {
     uint32_t there;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(there) : "r"(addr));
     return there;
-}
-// One arrival on a barrier of either block, which then waits for `bytes` of copies too.
-__device__ __forceinline__ void expect_tx_at(uint32_t cluster_bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_bar), "r"(bytes) : "memory");
 }
 // tma_load_2d into this block's shared memory, completing on a barrier of either block of the pair.
 __device__ __forceinline__ void tma_load_2d_at(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t cluster_bar) {
@@ -140,25 +138,24 @@ struct RowScales {
 __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                               const __grid_constant__ CUtensorMap map_x16, const W8Shape p) {
     extern __shared__ uint8_t raw[];
-    __shared__ __align__(8) uint64_t s_bar[4 * kStages + 5];
+    __shared__ __align__(8) uint64_t s_bar[3 * kStages + 5];
     __shared__ int4 s_list[kListed];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
-    __shared__ int s_issued;           // odd block: stages its TMA thread has filled, when that gave up ...
-    __shared__ volatile int s_copies;  // ... and even block: that number + 1
+    __shared__ int s_issued;           // stages the block's TMA thread has filled
+    __shared__ volatile int s_copies;  // even block: those of the odd block + 1, when that gave up
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage0 = (smem_u32(raw) + 1023u) & ~1023u;
     int* s_first = reinterpret_cast<int*>(raw + (stage0 - smem_u32(raw)) + kRing + kTurn);
     int* s_tok = s_first + p.E + 1;
     const uint32_t bars = smem_u32(s_bar);
-    auto full = [&](int s) { return bars + 8u * s; };                    // the stage's copies have landed (odd block: its codes)
+    auto full = [&](int s) { return bars + 8u * s; };                    // the stage's copies have landed; even block: both blocks' tokens, odd block: codes only
     auto done = [&](int s) { return bars + 8u * (kStages + s); };        // its MMAs are over: stage and A buffer are free
     auto a_full = [&](int s) { return bars + 8u * (2 * kStages + s); };  // even block: both blocks' codes are widened
     auto d_full = [&](int b) { return bars + 8u * (3 * kStages + b); };
     auto d_free = [&](int b) { return bars + 8u * (3 * kStages + 2 + b); };  // even block: both blocks have taken the sums out
     const uint32_t drained = bars + 8u * (3 * kStages + 4);
-    auto x_full = [&](int s) { return bars + 8u * (3 * kStages + 5 + s); };  // even block: the odd block's tokens have landed there
     const int rank = blockIdx.x & 1;
     // A stage: the block's codes, then its half of up to `cap` tokens as two halves of 64 k.  As many of them as there are A buffers
     // beside two accumulators of `twice` tokens.
@@ -168,7 +165,6 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
     if (tid == 0) {
         s_abort = s_copies = 0;
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(x_full(s), 1);
             mbar_init(full(s), 1);
             mbar_init(done(s), 1);
             mbar_init(a_full(s), 16);
@@ -220,6 +216,8 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
         return t;
     };
 
+    auto half_of = [&](const Tile& x) { return (x.n + kUnit - 1) / kUnit * (kUnit / 2); };  // tokens of one block
+
     if (warp >= 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
     if (warp == 16) {
         // ---- TMA: one thread ---------------------------------------------------------------------------------------
@@ -229,9 +227,8 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
             bool ok = true;
             Tile t = tile(0);
             auto stage_at = [&](int k) { return stage0 + static_cast<uint32_t>(k) * stage_bytes; };
-            auto half_of = [&](const Tile& x) { return (x.n + kUnit - 1) / kUnit * (kUnit / 2); };  // tokens of one block
-            auto load_codes = [&](const Tile& x, int g, int k) {
-                mbar_expect_tx(full(k), kCodeBytes + (rank ? 0u : 2u * half_of(x) * 128u));
+            auto load_codes = [&](const Tile& x, int g, int k) {  // (the odd block's tokens may land before the even block expects them: its arrival is still missing)
+                mbar_expect_tx(full(k), kCodeBytes + (rank ? 0u : 4u * half_of(x) * 128u));
                 tma_load_2d(stage_at(k), &map_w, g * 128, x.e * p.N + x.row0, full(k));
                 tma_load_2d(stage_at(k) + kCodeBytes / 2, &map_w, g * 128, x.e * p.N + x.row1, full(k));
             };
@@ -248,8 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                         if (!(ok = thread_wait(done(s), ph, abort))) break;
                         load_codes(t, g, s);
                     }
-                    const uint32_t at = stage_at(s) + kCodeBytes, landed = at_even_block(rank ? x_full(s) : full(s));
-                    if (rank) expect_tx_at(landed, 2u * half * 128u);
+                    const uint32_t at = stage_at(s) + kCodeBytes, landed = at_even_block(full(s));
                     for (int b = 0; b < half; b += kBox) {
                         const CUtensorMap* map = half - b >= kBox ? &map_x : &map_x16;
                         tma_load_2d_at(at + b * 128, map, g * 128, row + b, landed);
@@ -264,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
             // the last MMAs' events arrive here before this block may leave
             for (int j = max(0, issued - stages); ok && j < issued; ++j) ok = thread_wait(done(j % stages), (j / stages) & 1, abort);
             if (!ok) {  // gave up: the copies in flight still land in this block's shared memory
-                for (int j = max(0, issued - stages); j < issued; ++j) mbar_wait(full(j % stages), (j / stages) & 1);
+                for (int j = max(0, issued - stages); j < issued && mbar_wait(full(j % stages), (j / stages) & 1);) ++j;
             }
             s_issued = issued;
         }
@@ -283,8 +279,8 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                 if (round > 0 && max(n, before) > twice && !(ok = thread_wait(d_free(b ^ 1), ((round - 1) >> 1) & 1, abort))) break;
                 before = n;
                 for (int g = 0; g < groups; ++g) {
-                    // a widening warp has seen its block's copies land before it arrives: no wait on full(s) here
-                    if (!(ok = thread_wait(x_full(s), ph, abort) && thread_wait(a_full(s), ph, abort))) break;
+                    // the widening warps have seen the copies land before they arrive: no wait on full(s) here
+                    if (!(ok = thread_wait(a_full(s), ph, abort))) break;
                     tc_fence_after();
                     const uint64_t x0 = smem_desc_sw128(stage0 + static_cast<uint32_t>(s) * stage_bytes + kCodeBytes, 1024);
                     const uint32_t a = tmem + col_a + 64u * s;
@@ -453,8 +449,13 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
     }
     cluster_sync();  // the other block's arrivals and MMAs are over
     if (rank ? s_abort : s_copies) {  // the odd block gave up: it stays until the even block has seen its last tokens land
-        if (rank == 0 && tid == 0)
-            for (int j = max(0, s_copies - 1 - stages); j < s_copies - 1; ++j) mbar_wait(x_full(j % stages), (j / stages) & 1);
+        if (rank == 0 && tid == 0) {
+            const int there = s_copies - 1;
+            for (int j = max(0, there - stages); j < there; ++j) {
+                if (j >= s_issued) mbar_expect_tx(full(j % stages), 2u * half_of(tile(j / groups)) * 128u);  // (this block gave up earlier)
+                if (!mbar_wait(full(j % stages), (j / stages) & 1)) break;
+            }
+        }
         cluster_sync();
     }
     if (warp == 17) {
