@@ -24,8 +24,8 @@
 // shared memory between the blocks.  What crosses over is of two other kinds.  TMEM (codes widened, sums taken out) is ordered by tcgen05's fences
 // before an arrival and after a wait.  The odd block's tokens are reported to the even block by the TMA itself, which counts their bytes on that block's
 // `full`: its widening warps wait for them too, and tell the MMA thread.  Us of gate/up by 300 and 600 tokens and of a prompt of 300 (two layers): the odd
-// block's tokens on no barrier of the even block 62.5, 72.8 and 543; on `full` 63.0, 73.2 and 545; on one that the MMA thread waits for besides 64.8, 74.6 and 557,
-// on `a_full` the same.  (With `.release.cluster` and `.acquire.cluster` on the arrivals instead, every group waited for the memory system:
+// block's tokens on no barrier of the even block 62.3, 72.3 and 543; on one that the MMA thread waits for besides 64.8, 74.6 and 557, on `a_full` the same; on
+// `full` 63.0, 73.1 and 545, and with the addresses of the even block's barriers looked up once, as now, 61.5, 71.4 and 536.  (With `.release.cluster` and `.acquire.cluster` on the arrivals instead, every group waited for the memory system:
 // 4096 x 6144 x 2048 168 us, not 94.)
 #include "w8_tile.cuh"
 
@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
             bool ok = true;
             Tile t = tile(0);
             auto stage_at = [&](int k) { return stage0 + static_cast<uint32_t>(k) * stage_bytes; };
+            const uint32_t even_full = at_even_block(full(0));  // (full(s) is 8 s behind)
             auto load_codes = [&](const Tile& x, int g, int k) {  // (the odd block's tokens may land before the even block expects them: its arrival is still missing)
                 mbar_expect_tx(full(k), kCodeBytes + (rank ? 0u : 4u * half_of(x) * 128u));
                 tma_load_2d(stage_at(k), &map_w, g * 128, x.e * p.N + x.row0, full(k));
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                         if (!(ok = thread_wait(done(s), ph, abort))) break;
                         load_codes(t, g, s);
                     }
-                    const uint32_t at = stage_at(s) + kCodeBytes, landed = at_even_block(full(s));
+                    const uint32_t at = stage_at(s) + kCodeBytes, landed = even_full + 8u * s;
                     for (int b = 0; b < half; b += kBox) {
                         const CUtensorMap* map = half - b >= kBox ? &map_x : &map_x16;
                         tma_load_2d_at(at + b * 128, map, g * 128, row + b, landed);
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
         const int slot = p.gate_up ? ((lane >> 3) & 1) * 64 + 16 * quarter + 8 * (lane >> 4) + (lane & 7) : 32 * quarter + lane;
         const uint32_t to0 = tmem + (static_cast<uint32_t>(quarter) << 21) + col_a + 32u * kh;
         const uint32_t from0 = stage0 + slot * 128u, swz = slot & 7;
+        const uint32_t even_a_full = at_even_block(a_full(0));
         auto weight_row = [&](const Tile& t) { return slot < 64 ? t.row0 + slot : t.row1 + slot - 64; };
         int s = 0;
         uint32_t ph = 0;
@@ -332,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1) w8_pair_kernel(const __grid_const
                 }
                 tmem_wait_st();
                 tc_fence_before();
-                warp_arrive_at(at_even_block(a_full(s)));
+                warp_arrive_at(even_a_full + 8u * s);
                 if (++s == stages) { s = 0; ph ^= 1; }
                 if (g == 0 && i + 1 < mine) {
                     const Tile t = tile(i + 1);
