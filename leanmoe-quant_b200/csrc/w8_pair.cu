@@ -25,8 +25,8 @@
 // before an arrival and after a wait.  The odd block's tokens are reported to the even block by the TMA itself, which counts their bytes on that block's
 // `full`: its widening warps wait for them too, and tell the MMA thread.  Us of gate/up by 300 and 600 tokens and of a prompt of 300 (two layers): the odd
 // block's tokens on no barrier of the even block 62.3, 72.3 and 543; on one that the MMA thread waits for besides 64.8, 74.6 and 557, on `a_full` the same; on
-// `full` 63.0, 73.1 and 545, and with the addresses of the even block's barriers looked up once, as now, 61.5, 71.4 and 536.  (With `.release.cluster` and `.acquire.cluster` on the arrivals instead, every group waited for the memory system:
-// 4096 x 6144 x 2048 168 us, not 94.)
+// `full` 63.0, 73.1 and 545, and with the addresses of the even block's barriers looked up once, as now, 61.5, 71.4 and 536.  (With
+// `.release.cluster` and `.acquire.cluster` on the arrivals instead, every group waited for the memory system: 4096 x 6144 x 2048 168 us, not 94.)
 #include "w8_tile.cuh"
 
 #include <algorithm>
